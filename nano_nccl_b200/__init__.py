@@ -6,8 +6,8 @@ Layout: ``communicator`` (ctypes binding of the C++ communicator), ``ops`` (torc
 ``parallel`` (bucketed gradient all-reduce, data-parallel wrapper), ``models`` (synthetic tensor
 stacks shaped like real models, for benchmarks), ``utils`` (timing, clocks, simulator binding).
 """
-from ._lib import B200CclError, lib_path, load  # noqa: F401
+from ._lib import B200CclError, lib_path, load, load_native_calls  # noqa: F401
 from .communicator import Communicator  # noqa: F401
 
-__all__ = ["Communicator", "B200CclError", "load", "lib_path"]
+__all__ = ["Communicator", "B200CclError", "load", "load_native_calls", "lib_path"]
 __version__ = "0.1.0"

@@ -4,9 +4,11 @@ The shared library is built in-tree (nano_nccl_b200/lib/) by ``__graft_entry__.b
 ``cmake``; nothing here falls back to another implementation when it is missing.
 """
 import ctypes
+import importlib.util
 import os
 
 _LIB = None
+_NATIVE = None
 
 
 class B2Config(ctypes.Structure):
@@ -93,3 +95,23 @@ def check(code):
         if code == 2:
             raise ValueError(msg)
         raise B200CclError(msg)
+
+
+def load_native_calls():
+    """The module with the collective calls (src/python/torch_binding.cc), bound to the library that
+    load() returns. Like the library it is built in-tree, and nothing stands in for it."""
+    global _NATIVE
+    if _NATIVE is None:
+        import torch  # noqa: F401  (the module needs torch's libraries in the process)
+
+        path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "_b200ccl_torch.so")
+        if not os.path.exists(path):
+            raise ImportError(f"{path} is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'`")
+        spec = importlib.util.spec_from_file_location("_b200ccl_torch", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        lib = load()
+        address = [ctypes.cast(f, ctypes.c_void_p).value for f in (lib.b2_collective, lib.b2_last_error)]
+        module.bind(address[0], address[1], B200CclError)
+        _NATIVE = module
+    return _NATIVE

@@ -11,14 +11,13 @@ import torch
 
 from . import _lib
 
-_DTYPES = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
-_OPS = {"sum": 0, "avg": 1, "max": 2, "min": 3}
-_COLL = {"all_reduce": 0, "reduce_scatter": 1, "all_gather": 2}
 _ALGO_NAMES = ["auto", "oneshot", "twoshot", "nvls", "ring", "ll", "copy", "pipeline"]
 
 
 class _SymmetricBlock:
-    """Owner of one symmetric allocation; exposes it to torch through the CUDA array interface."""
+    """Owner of one symmetric allocation; exposes it to torch through the CUDA array interface. The tensor
+    keeps this object, and this object the communicator; nothing points back, so that the last of them to
+    go takes the memory with it at once."""
 
     def __init__(self, comm, ptr, nbytes):
         self.comm, self.ptr, self.nbytes = comm, ptr, nbytes
@@ -43,7 +42,6 @@ class Communicator:
         self._lib = lib
         self._handle = ctypes.c_void_p()
         self._bootstrap = ctypes.c_void_p()
-        self._blocks = []
         cfg = _lib.B2Config()
         lib.b2_config_default(ctypes.byref(cfg))
         t, a = ctypes.c_int(), ctypes.c_int()
@@ -76,7 +74,8 @@ class Communicator:
         self.local_ranks = lib.b2_comm_local_ranks(self._handle)
         self.world_size = lib.b2_comm_global_ranks(self._handle)
         self.rank = lib.b2_comm_first_rank(self._handle)
-        self._one = ((ctypes.c_void_p * 1)(), (ctypes.c_void_p * 1)(), (ctypes.c_void_p * 1)())
+        places = self.devices if len(self.devices) > 1 else self.devices * self.local_ranks
+        self._call = _lib.load_native_calls().Caller(self._handle.value, tuple(places), self.world_size)
 
     @classmethod
     def from_env(cls, port=None, **kw):
@@ -141,7 +140,6 @@ class Communicator:
         for i in range(self.local_ranks):
             dev = self.devices[0] if len(self.devices) == 1 else self.devices[i]
             block = _SymmetricBlock(self, ptrs[i], nbytes)
-            self._blocks.append(block)
             with torch.cuda.device(dev):
                 raw = torch.as_tensor(block, device=f"cuda:{dev}")
             outs.append(raw[: numel * esize].view(dtype).view(*shape))
@@ -167,98 +165,19 @@ class Communicator:
         _lib.check(self._lib.b2_comm_unregister(self._handle, ptrs))
 
     # -- collectives -----------------------------------------------------------------------------
-    def _device_index(self, i):
-        return self.devices[0] if len(self.devices) == 1 else self.devices[i]
-
-    def _check_tensor(self, what, i, t, dtype, numel):
-        """Everything the C layer cannot see behind a raw pointer: a tensor that is too small, of
-        another dtype or on another GPU would make the kernel write outside the allocation."""
-        if not isinstance(t, torch.Tensor) or not t.is_cuda or not t.is_contiguous():
-            raise ValueError(f"{what}[{i}] must be a contiguous CUDA tensor")
-        if t.dtype != dtype:
-            raise ValueError(f"{what}[{i}] has dtype {t.dtype}, expected {dtype}")
-        if t.numel() != numel:
-            raise ValueError(f"{what}[{i}] has {t.numel()} elements, expected {numel}")
-        want = self._device_index(i)
-        if t.device.index != want:
-            raise ValueError(f"{what}[{i}] lives on cuda:{t.device.index}, local rank {i} of this communicator drives cuda:{want}")
-
-    def _run(self, coll, outs, inps, op, streams, count, in_numel, out_numel, in_place=False):
-        if op not in _OPS:
-            raise ValueError(f"unknown reduction '{op}'")
-        if isinstance(inps, torch.Tensor):
-            # Fast path: one local rank, one tensor each way.
-            if self.local_ranks != 1 or not isinstance(outs, torch.Tensor):
-                raise ValueError(f"need one tensor per local rank ({self.local_ranks})")
-            dtype = inps.dtype
-            code = _DTYPES.get(dtype)
-            if code is None:
-                raise ValueError(f"unsupported dtype {dtype}")
-            self._check_tensor("input", 0, inps, dtype, in_numel)
-            self._check_tensor("output", 0, outs, dtype, out_numel)
-            if streams is None:
-                sp = torch.cuda.current_stream(inps.device).cuda_stream
-            else:
-                s0 = streams[0] if isinstance(streams, (list, tuple)) else streams
-                sp = s0.cuda_stream if hasattr(s0, "cuda_stream") else int(s0)
-            a = self._one
-            a[0][0], a[1][0], a[2][0] = inps.data_ptr(), outs.data_ptr(), sp
-            rc = self._lib.b2_collective(self._handle, _COLL[coll], a[0], a[1], a[2], count, code, _OPS[op], 1 if in_place else 0)
-            if rc != 0:
-                _lib.check(rc)
-            return
-        if isinstance(outs, torch.Tensor) or len(inps) != self.local_ranks or len(outs) != self.local_ranks:
-            raise ValueError(f"need one tensor per local rank ({self.local_ranks})")
-        dtype = inps[0].dtype
-        if dtype not in _DTYPES:
-            raise ValueError(f"unsupported dtype {dtype}")
-        for i, (x, y) in enumerate(zip(inps, outs)):
-            self._check_tensor("input", i, x, dtype, in_numel)
-            self._check_tensor("output", i, y, dtype, out_numel)
-        if streams is None:
-            streams = [torch.cuda.current_stream(t.device).cuda_stream for t in inps]
-        elif not isinstance(streams, (list, tuple)):
-            streams = [streams] * len(inps)
-        if len(streams) != self.local_ranks:
-            raise ValueError(f"need one stream per local rank ({self.local_ranks})")
-        streams = [s.cuda_stream if hasattr(s, "cuda_stream") else int(s) for s in streams]
-        n = self.local_ranks
-        send = (ctypes.c_void_p * n)(*[t.data_ptr() for t in inps])
-        recv = (ctypes.c_void_p * n)(*[t.data_ptr() for t in outs])
-        st = (ctypes.c_void_p * n)(*streams)
-        _lib.check(self._lib.b2_collective(self._handle, _COLL[coll], send, recv, st, count, _DTYPES[dtype], _OPS[op],
-                                           1 if in_place else 0))
-
+    # Checks (one contiguous tensor per local rank, on its GPU, of one supported dtype and the right
+    # length), streams (``None``: the current stream of each GPU) and the call itself are native.
     def all_reduce(self, out, inp=None, op="sum", stream=None):
         """out = reduce(inp over all ranks). ``inp=None`` (or the same tensor) reduces in place."""
-        if inp is None:
-            inp = out
-        first_in = inp if isinstance(inp, torch.Tensor) else inp[0]
-        first_out = out if isinstance(out, torch.Tensor) else out[0]
-        in_place = first_in.data_ptr() == first_out.data_ptr()
-        n = first_in.numel()
-        self._run("all_reduce", out, inp, op, stream, n, n, n, in_place)
-        return out
+        return self._call.all_reduce(out, out if inp is None else inp, op, stream)
 
     def reduce_scatter(self, out, inp, op="sum", stream=None):
         """Rank r's ``out`` (numel = inp.numel() / world_size) receives block r of the reduction."""
-        first_out = out if isinstance(out, torch.Tensor) else out[0]
-        first_in = inp if isinstance(inp, torch.Tensor) else inp[0]
-        if first_in.numel() != first_out.numel() * self.world_size:
-            raise ValueError("reduce_scatter: input must hold world_size blocks of the output's size")
-        n = first_out.numel()
-        self._run("reduce_scatter", out, inp, op, stream, n, n * self.world_size, n)
-        return out
+        return self._call.reduce_scatter(out, inp, op, stream)
 
     def all_gather(self, out, inp, stream=None):
         """``out`` (numel = inp.numel() * world_size) receives every rank's ``inp``, in rank order."""
-        first_out = out if isinstance(out, torch.Tensor) else out[0]
-        first_in = inp if isinstance(inp, torch.Tensor) else inp[0]
-        if first_out.numel() != first_in.numel() * self.world_size:
-            raise ValueError("all_gather: output must hold world_size blocks of the input's size")
-        n = first_in.numel()
-        self._run("all_gather", out, inp, "sum", stream, n, n, n * self.world_size)
-        return out
+        return self._call.all_gather(out, inp, "sum", stream)
 
     def free(self, tensors):
         """Releases the symmetric allocation behind tensor(s) returned by ``empty()``. COLLECTIVE: every
@@ -270,11 +189,11 @@ class Communicator:
             raise ValueError(f"need one tensor per local rank ({self.local_ranks})")
         ptrs = (ctypes.c_void_p * self.local_ranks)(*[t.data_ptr() for t in tensors])
         _lib.check(self._lib.b2_comm_free_symmetric(self._handle, ptrs))
-        gone = {int(p) for p in ptrs}
-        self._blocks = [b for b in self._blocks if int(b.ptr) not in gone]
 
     def close(self):
         if self._handle:
+            if hasattr(self, "_call"):
+                self._call.close()
             self._lib.b2_comm_destroy(self._handle)
             self._handle = ctypes.c_void_p()
         if self._bootstrap:

@@ -132,10 +132,11 @@ int b2_collective(b2_comm* c, int collective, const void* const* send, void* con
                   size_t count, int dtype, int redop, int allow_in_place) {
     return guarded([&] {
         const int n = c->comm->local_rank_count();
-        CollectiveArgs a;
+        static thread_local CollectiveArgs a;  // keeps its vectors' memory from call to call
         a.send_buffers.assign(send, send + n);
         a.recv_buffers.assign(recv, recv + n);
-        for (int i = 0; i < n; ++i) a.streams.push_back(static_cast<cudaStream_t>(streams[i]));
+        a.streams.resize(n);
+        for (int i = 0; i < n; ++i) a.streams[i] = static_cast<cudaStream_t>(streams[i]);
         a.count = count;
         a.dtype = static_cast<DType>(dtype);
         a.redop = static_cast<RedOp>(redop);

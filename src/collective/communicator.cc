@@ -29,6 +29,7 @@
 #include "topo/topology.h"
 
 #include <algorithm>
+#include <array>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -47,14 +48,14 @@ struct Located {
     std::size_t offset = 0;
 };
 
-// FNV-1a over the facts of a launch that every rank must share; never 0 (0 means "no check").
+// Mixes the facts of a launch that every rank must share, one multiply-and-fold per fact (eight dependent
+// multiplies per fact, as in a byte-wise FNV-1a, are a microsecond a call at eight ranks); never 0
+// (0 means "no check").
 unsigned long long plan_fingerprint(std::initializer_list<unsigned long long> facts) {
     unsigned long long h = 1469598103934665603ull;
     for (unsigned long long f : facts) {
-        for (int b = 0; b < 8; ++b) {
-            h ^= (f >> (8 * b)) & 0xffull;
-            h *= 1099511628211ull;
-        }
+        h = (h ^ f) * 0x9e3779b97f4a7c15ull;
+        h ^= h >> 29;
     }
     return h == 0 ? 1 : h;
 }
@@ -96,6 +97,7 @@ private:
         bool launched = false;
         cudaStream_t last_stream = nullptr;
         bool last_in_capture = false;  // the completion event was last recorded inside a stream capture
+        bool record_later = false;     // `done` does not cover the last launch yet (see record_done)
     };
 
     void resolve_transport();
@@ -109,17 +111,22 @@ private:
     char* stage_mc_out() const { return stage_mc_in() + staging_half_; }
     void check_canaries() const;
     Located locate(const void* p, std::size_t bytes, int grank) const;
+    // Launches that one call makes: one per local rank, or one that plays every emulated rank and is
+    // tracked by the first rank's event.
+    std::size_t launches_per_call() const { return loopback_ ? 1 : local_.size(); }
     void wait_previous(Local& l, cudaStream_t stream);
     void record_done(Local& l, cudaStream_t stream);
+    void record_pending(Local& l);
+    void synchronize(Local& l);
     // in_loc / out_loc: where each local rank's buffer lies; null when the buffers of this call do
     // not sit at one common offset of one window (then the window's peer addresses say nothing
     // about the other ranks' buffers and must not be used).
     void launch_all_reduce(const CollectiveArgs& args, const sched::Plan& plan, bool wide,
-                           const std::vector<Located>* in_loc, const std::vector<Located>* out_loc);
+                           const Located* in_loc, const Located* out_loc);
     void launch_reduce_scatter(const CollectiveArgs& args, const sched::Plan& plan, bool wide,
-                               const std::vector<Located>* in_loc);
+                               const Located* in_loc);
     void launch_all_gather(const CollectiveArgs& args, const sched::Plan& plan, bool wide,
-                           const std::vector<Located>* in_loc, const std::vector<Located>* out_loc);
+                           const Located* in_loc, const Located* out_loc);
     void fill_common(dev::CollArgs& a, const Local& l) const;
     void launch_reduce_ranks(const CollectiveArgs& args, std::vector<dev::CollArgs>& per_rank, int pack_bytes,
                              bool nvls, int grid);
@@ -437,12 +444,11 @@ Communicator::Impl::~Impl() {
     // Work in flight is waited for (destroying a communicator with unsynchronised streams is
     // allowed, as in tests/public_api.cu:904-916 of the reference).
     for (auto& l : local_) {
-        if (l.launched && l.done && !l.last_in_capture) {
-            const cudaError_t st = cudaEventSynchronize(l.done);
-            if (st != cudaSuccess) {
-                (void)cudaGetLastError();
-                log_warn("waiting for rank %d's last collective failed: %s", l.grank, cudaGetErrorString(st));
-            }
+        try {
+            synchronize(l);
+        } catch (const std::exception& e) {
+            (void)cudaGetLastError();
+            log_warn("waiting for rank %d's last collective failed: %s", l.grank, e.what());
         }
     }
     for (std::size_t i = 0; i < pipe_stats_.size(); ++i) {
@@ -609,8 +615,7 @@ void Communicator::Impl::release_window(const std::vector<void*>& ptrs, const ch
     if (ptrs.empty()) return;
     for (auto& w : windows_) {
         if (w.bytes != 0 && w.ptr[local_[0].grank] == ptrs[0]) {
-            for (auto& l : local_)
-                if (l.launched && !l.last_in_capture) B2_CUDA(cudaEventSynchronize(l.done));
+            for (auto& l : local_) synchronize(l);
             if (bootstrap_) bootstrap_->barrier();  // no peer may still be using it
             w.bytes = 0;
             w.region.reset();
@@ -641,24 +646,50 @@ void Communicator::Impl::unregister_buffers(const std::vector<void*>& ptrs) {
     release_window(ptrs, "unregister_buffers");
 }
 
+namespace {
+// The legacy default stream of a device.
+bool is_default_stream(cudaStream_t s) { return s == nullptr || s == cudaStreamLegacy; }
+
+bool is_capturing(cudaStream_t s) {
+    if (is_default_stream(s)) return false;  // cannot be captured
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    B2_CUDA(cudaStreamIsCapturing(s, &st));
+    return st == cudaStreamCaptureStatusActive;
+}
+}  // namespace
+
 void Communicator::Impl::wait_previous(Local& l, cudaStream_t stream) {
     if (!l.launched || l.last_stream == stream) return;
     // An event recorded outside a capture cannot be waited for inside one, and the other way
     // round; across that boundary the caller's own ordering (capture begin/end, graph launch) holds.
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    B2_CUDA(cudaStreamIsCapturing(stream, &st));
-    const bool capturing = st == cudaStreamCaptureStatusActive;
-    if (capturing != l.last_in_capture) return;
+    if (is_capturing(stream) != l.last_in_capture) return;
+    record_pending(l);
     B2_CUDA(cudaStreamWaitEvent(stream, l.done, 0));
 }
 
+// The event of a launch on the default stream is recorded only once somebody needs it: that stream
+// lives as long as its device, so it can still be recorded then, and it covers at least that launch.
+// Any other stream may be destroyed before the next call, so there the event is recorded at once.
 void Communicator::Impl::record_done(Local& l, cudaStream_t stream) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    B2_CUDA(cudaStreamIsCapturing(stream, &st));
-    B2_CUDA(cudaEventRecord(l.done, stream));
+    l.record_later = is_default_stream(stream);
+    l.last_in_capture = is_capturing(stream);
+    if (!l.record_later) B2_CUDA(cudaEventRecord(l.done, stream));
     l.launched = true;
     l.last_stream = stream;
-    l.last_in_capture = st == cudaStreamCaptureStatusActive;
+}
+
+void Communicator::Impl::record_pending(Local& l) {
+    if (!l.record_later) return;
+    DeviceGuard guard(l.device);
+    B2_CUDA(cudaEventRecord(l.done, l.last_stream));
+    l.record_later = false;
+}
+
+// Waits on the host for the last collective that `l` tracks.
+void Communicator::Impl::synchronize(Local& l) {
+    if (!l.launched || l.last_in_capture) return;
+    record_pending(l);
+    B2_CUDA(cudaEventSynchronize(l.done));
 }
 
 void Communicator::Impl::fill_common(dev::CollArgs& a, const Local& l) const {
@@ -692,9 +723,9 @@ void Communicator::Impl::launch_reduce_ranks(const CollectiveArgs& args, std::ve
             DeviceGuard guard(local_[0].device);
             cfg.stream = args.streams[0];
             cfg.loop_ranks = nranks_;
-            for (auto& l : local_) wait_previous(l, cfg.stream);
+            wait_previous(local_[0], cfg.stream);
             B2_CUDA(kernels::launch_reduce(args.dtype, args.redop, pack_bytes, nvls, per_rank.data(), cfg));
-            for (auto& l : local_) record_done(l, cfg.stream);
+            record_done(local_[0], cfg.stream);
         } else {
             for (std::size_t i = 0; i < local_.size(); ++i) {
                 DeviceGuard guard(local_[i].device);
@@ -727,9 +758,9 @@ void Communicator::Impl::launch_gather_ranks(const CollectiveArgs& args, std::ve
             DeviceGuard guard(local_[0].device);
             cfg.stream = args.streams[0];
             cfg.loop_ranks = nranks_;
-            for (auto& l : local_) wait_previous(l, cfg.stream);
+            wait_previous(local_[0], cfg.stream);
             B2_CUDA(kernels::launch_gather(per_rank.data(), cfg));
-            for (auto& l : local_) record_done(l, cfg.stream);
+            record_done(local_[0], cfg.stream);
         } else {
             for (std::size_t i = 0; i < local_.size(); ++i) {
                 DeviceGuard guard(local_[i].device);
@@ -758,7 +789,7 @@ void Communicator::Impl::run(Collective collective, const CollectiveArgs& args) 
     const std::size_t out_bytes = args.count * esz * (collective == Collective::AllGather ? n : 1);
 
     // Where do the buffers live?
-    std::vector<Located> in_loc(local_.size()), out_loc(local_.size());
+    std::array<Located, kMaxRanks> in_loc, out_loc;
     bool in_sym = true, out_sym = true, in_place = false;
     for (std::size_t i = 0; i < local_.size(); ++i) {
         in_loc[i] = locate(args.send_buffers[i], in_bytes, local_[i].grank);
@@ -843,14 +874,14 @@ void Communicator::Impl::run(Collective collective, const CollectiveArgs& args) 
             ring_.reset(new RingEngine(rc, alloc_.get(), ctrl_.get(), bootstrap_));
         }
         try {
-            for (std::size_t i = 0; i < local_.size(); ++i) {
+            for (std::size_t i = 0; i < launches_per_call(); ++i) {
                 DeviceGuard guard(local_[i].device);
-                wait_previous(local_[i], args.streams[loopback_ ? 0 : i]);
+                wait_previous(local_[i], args.streams[i]);
             }
             ring_->launch(collective, args);
-            for (std::size_t i = 0; i < local_.size(); ++i) {
+            for (std::size_t i = 0; i < launches_per_call(); ++i) {
                 DeviceGuard guard(local_[i].device);
-                record_done(local_[i], args.streams[loopback_ ? 0 : i]);
+                record_done(local_[i], args.streams[i]);
             }
         } catch (const std::invalid_argument&) {
             throw;
@@ -892,9 +923,9 @@ void Communicator::Impl::run(Collective collective, const CollectiveArgs& args) 
         return;
     }
     switch (collective) {
-        case Collective::AllReduce: launch_all_reduce(args, plan, wide, in_sym ? &in_loc : nullptr, out_sym ? &out_loc : nullptr); break;
-        case Collective::ReduceScatter: launch_reduce_scatter(args, plan, wide, in_sym ? &in_loc : nullptr); break;
-        case Collective::AllGather: launch_all_gather(args, plan, wide, in_sym ? &in_loc : nullptr, out_sym ? &out_loc : nullptr); break;
+        case Collective::AllReduce: launch_all_reduce(args, plan, wide, in_sym ? in_loc.data() : nullptr, out_sym ? out_loc.data() : nullptr); break;
+        case Collective::ReduceScatter: launch_reduce_scatter(args, plan, wide, in_sym ? in_loc.data() : nullptr); break;
+        case Collective::AllGather: launch_all_gather(args, plan, wide, in_sym ? in_loc.data() : nullptr, out_sym ? out_loc.data() : nullptr); break;
     }
 }
 
@@ -924,9 +955,9 @@ void Communicator::Impl::launch_low_latency(const CollectiveArgs& args) {
         if (loopback_) {
             DeviceGuard guard(local_[0].device);
             cudaStream_t stream = args.streams[0];
-            for (auto& l : local_) wait_previous(l, stream);
+            wait_previous(local_[0], stream);
             B2_CUDA(kernels::launch_ll_all_reduce(args.dtype, args.redop, per.data(), nranks_, stream));
-            for (auto& l : local_) record_done(l, stream);
+            record_done(local_[0], stream);
         } else {
             for (std::size_t i = 0; i < local_.size(); ++i) {
                 DeviceGuard guard(local_[i].device);
@@ -997,9 +1028,9 @@ void Communicator::Impl::launch_pipeline(const CollectiveArgs& args, const sched
             DeviceGuard guard(local_[0].device);
             cfg.stream = args.streams[0];
             cfg.loop_ranks = nranks_;
-            for (auto& l : local_) wait_previous(l, cfg.stream);
+            wait_previous(local_[0], cfg.stream);
             B2_CUDA(kernels::launch_staged_pipeline(args.dtype, args.redop, per.data(), cfg));
-            for (auto& l : local_) record_done(l, cfg.stream);
+            record_done(local_[0], cfg.stream);
         } else {
             for (std::size_t i = 0; i < local_.size(); ++i) {
                 DeviceGuard guard(local_[i].device);
@@ -1019,7 +1050,7 @@ void Communicator::Impl::launch_pipeline(const CollectiveArgs& args, const sched
 }
 
 void Communicator::Impl::launch_all_reduce(const CollectiveArgs& args, const sched::Plan& plan, bool wide,
-                                           const std::vector<Located>* in_win, const std::vector<Located>* out_win) {
+                                           const Located* in_win, const Located* out_win) {
     const std::size_t esz = dtype_size(args.dtype);
     const bool direct = direct_peer_pointers();
     const bool nvls = plan.algo == Algo::Nvls;
@@ -1031,11 +1062,11 @@ void Communicator::Impl::launch_all_reduce(const CollectiveArgs& args, const sch
     bool wide32 = wide && tuning_.wide32 && plan.algo == Algo::TwoShot && (args.count * esz) % 32 == 0;
     auto aligned32 = [](const void* p) { return (reinterpret_cast<std::uintptr_t>(p) & 31u) == 0; };
     if (wide32 && !plan.stage_in) {
-        if (in_win != nullptr) wide32 = aligned32(static_cast<const char*>(windows_[(*in_win)[0].region].ptr[0]) + (*in_win)[0].offset);
+        if (in_win != nullptr) wide32 = aligned32(static_cast<const char*>(windows_[in_win[0].region].ptr[0]) + in_win[0].offset);
         else for (const void* p : args.send_buffers) wide32 = wide32 && aligned32(p);
     }
     if (wide32 && !plan.stage_out) {
-        if (out_win != nullptr) wide32 = aligned32(static_cast<const char*>(windows_[(*out_win)[0].region].ptr[0]) + (*out_win)[0].offset);
+        if (out_win != nullptr) wide32 = aligned32(static_cast<const char*>(windows_[out_win[0].region].ptr[0]) + out_win[0].offset);
         else for (const void* p : args.recv_buffers) wide32 = wide32 && aligned32(p);
     }
     const std::size_t pack = wide32 ? 32 : (wide ? 16 : esz);
@@ -1058,13 +1089,13 @@ void Communicator::Impl::launch_all_reduce(const CollectiveArgs& args, const sch
                 // input table
                 if (plan.stage_in) a.in[p] = stage_in_ptr(p);
                 else if (in_win != nullptr)
-                    a.in[p] = static_cast<const char*>(windows_[(*in_win)[i].region].ptr[p]) + (*in_win)[i].offset + off;
+                    a.in[p] = static_cast<const char*>(windows_[in_win[i].region].ptr[p]) + in_win[i].offset + off;
                 else if (direct) a.in[p] = static_cast<const char*>(args.send_buffers[p]) + off;
                 // output table
                 if (plan.stage_out) a.out[p] = stage_out_ptr(p);
                 else if (oneshot) a.out[p] = nullptr;
                 else if (out_win != nullptr)
-                    a.out[p] = static_cast<char*>(windows_[(*out_win)[i].region].ptr[p]) + (*out_win)[i].offset + off;
+                    a.out[p] = static_cast<char*>(windows_[out_win[i].region].ptr[p]) + out_win[i].offset + off;
                 else if (direct) a.out[p] = static_cast<char*>(args.recv_buffers[p]) + off;
             }
             if (oneshot) a.out[local_[i].grank] = static_cast<char*>(args.recv_buffers[i]) + off;
@@ -1078,9 +1109,9 @@ void Communicator::Impl::launch_all_reduce(const CollectiveArgs& args, const sch
 #endif
             if (nvls) {
                 a.mc_in = plan.stage_in ? static_cast<const char*>(stage_mc_in())
-                                        : static_cast<const char*>(windows_[(*in_win)[i].region].mc) + (*in_win)[i].offset + off;
+                                        : static_cast<const char*>(windows_[in_win[i].region].mc) + in_win[i].offset + off;
                 a.mc_out = plan.stage_out ? stage_mc_out()
-                                          : static_cast<char*>(windows_[(*out_win)[i].region].mc) + (*out_win)[i].offset + off;
+                                          : static_cast<char*>(windows_[out_win[i].region].mc) + out_win[i].offset + off;
             }
         }
         last_.pack_bytes = static_cast<int>(pack);
@@ -1089,7 +1120,7 @@ void Communicator::Impl::launch_all_reduce(const CollectiveArgs& args, const sch
 }
 
 void Communicator::Impl::launch_reduce_scatter(const CollectiveArgs& args, const sched::Plan& plan, bool wide,
-                                               const std::vector<Located>* in_win) {
+                                               const Located* in_win) {
     const std::size_t esz = dtype_size(args.dtype);
     const std::size_t pack = wide ? 16 : esz;
     const std::size_t block_packs = args.count * esz / pack;  // one rank's block
@@ -1113,21 +1144,21 @@ void Communicator::Impl::launch_reduce_scatter(const CollectiveArgs& args, const
             for (int p = 0; p < nranks_; ++p) {
                 if (plan.stage_in) a.in[p] = stage_in_ptr(p);
                 else if (in_win != nullptr)
-                    a.in[p] = static_cast<const char*>(windows_[(*in_win)[i].region].ptr[p]) + (*in_win)[i].offset + off;
+                    a.in[p] = static_cast<const char*>(windows_[in_win[i].region].ptr[p]) + in_win[i].offset + off;
                 else if (direct) a.in[p] = static_cast<const char*>(args.send_buffers[p]) + off;
             }
             a.out[local_[i].grank] = static_cast<char*>(args.recv_buffers[i]) + off;
             a.in_extent = a.in_stride * static_cast<std::size_t>(nranks_ - 1) + len;
             a.out_extent = len;
             if (plan.stage_in) a.user_in = static_cast<const char*>(args.send_buffers[i]) + off;
-            if (nvls) a.mc_in = static_cast<const char*>(windows_[(*in_win)[i].region].mc) + (*in_win)[i].offset + off;
+            if (nvls) a.mc_in = static_cast<const char*>(windows_[in_win[i].region].mc) + in_win[i].offset + off;
         }
         launch_reduce_ranks(args, per, static_cast<int>(pack), nvls, plan.grid);
     }
 }
 
 void Communicator::Impl::launch_all_gather(const CollectiveArgs& args, const sched::Plan& plan, bool wide,
-                                           const std::vector<Located>* in_win, const std::vector<Located>* out_win) {
+                                           const Located* in_win, const Located* out_win) {
     const std::size_t esz = dtype_size(args.dtype);
     const std::size_t bytes = args.count * esz;
     std::size_t pack = wide ? 16 : (bytes % 4 == 0 ? 4 : 2);
@@ -1161,11 +1192,11 @@ void Communicator::Impl::launch_all_gather(const CollectiveArgs& args, const sch
                 if (plan.gather_mode == 1) {  // pull: need everyone's input
                     if (plan.stage_in) a.in[p] = stage_in_ptr(p);
                     else if (in_win != nullptr)
-                        a.in[p] = static_cast<const char*>(windows_[(*in_win)[i].region].ptr[p]) + (*in_win)[i].offset + off;
+                        a.in[p] = static_cast<const char*>(windows_[in_win[i].region].ptr[p]) + in_win[i].offset + off;
                     else if (direct) a.in[p] = static_cast<const char*>(args.send_buffers[p]) + off;
                 } else if (plan.gather_mode == 0) {  // push: need everyone's output
                     if (out_win != nullptr)
-                        a.out[p] = static_cast<char*>(windows_[(*out_win)[i].region].ptr[p]) + (*out_win)[i].offset + off;
+                        a.out[p] = static_cast<char*>(windows_[out_win[i].region].ptr[p]) + out_win[i].offset + off;
                     else if (direct) a.out[p] = static_cast<char*>(args.recv_buffers[p]) + off;
                 }
             }
@@ -1173,7 +1204,7 @@ void Communicator::Impl::launch_all_gather(const CollectiveArgs& args, const sch
             if (plan.gather_mode != 0) a.out[local_[i].grank] = static_cast<char*>(args.recv_buffers[i]) + off;
             if (plan.stage_in) a.user_in = static_cast<const char*>(args.send_buffers[i]) + off;
             if (plan.gather_mode == 2)
-                a.mc_out = static_cast<char*>(windows_[(*out_win)[i].region].mc) + (*out_win)[i].offset + off;
+                a.mc_out = static_cast<char*>(windows_[out_win[i].region].mc) + out_win[i].offset + off;
         }
         launch_gather_ranks(args, per, plan.grid);
     }

@@ -14,6 +14,8 @@
 #include "kernels/sm100/sync.cuh"
 #include "kernels/sm100/tma.cuh"
 
+#include <atomic>
+
 namespace b200ccl::kernels {
 
 using namespace b200ccl::dev;
@@ -96,22 +98,33 @@ __global__ void __launch_bounds__(32) bulk_copy_kernel(const unsigned char* src,
     tma_wait_group_all();  // stores read shared memory until they complete
 }
 
+// SM count of the current device. The first call on a device also raises the kernel's shared-memory
+// limit there (the attribute belongs to that device's copy of the function).
+cudaError_t prepare_device(int* sms) {
+    static std::atomic<int> known[64] = {};
+    int device = 0;
+    cudaError_t st = cudaGetDevice(&device);
+    if (st != cudaSuccess) return st;
+    const bool cached = device >= 0 && device < 64;
+    if (cached && (*sms = known[device].load(std::memory_order_acquire)) > 0) return cudaSuccess;
+    st = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, device);
+    if (st == cudaSuccess) st = cudaFuncSetAttribute(bulk_copy_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CopyShared));
+    if (st == cudaSuccess && cached) known[device].store(*sms, std::memory_order_release);
+    return st;
+}
+
 }  // namespace
 
 cudaError_t launch_local_copy(const void* src, void* dst, unsigned long long bytes, int max_ctas, Status* status,
                               cudaStream_t stream) {
     if (bytes == 0 || bytes % 16 != 0 || (reinterpret_cast<std::uintptr_t>(src) | reinterpret_cast<std::uintptr_t>(dst)) % 16 != 0)
         return cudaErrorInvalidValue;
-    int device = 0, sms = 0;
-    cudaError_t st = cudaGetDevice(&device);
-    if (st == cudaSuccess) st = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    int sms = 0;
+    cudaError_t st = prepare_device(&sms);
     if (st != cudaSuccess) return st;
     const u64 ntiles = (bytes + kTile - 1) / kTile;
     int grid = max_ctas > 0 ? (max_ctas < sms ? max_ctas : sms) : sms;
     if ((u64)grid > ntiles) grid = (int)ntiles;
-    // The attribute belongs to the current device's copy of the function.
-    st = cudaFuncSetAttribute(bulk_copy_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CopyShared));
-    if (st != cudaSuccess) return st;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(grid, 1, 1);
     config.blockDim = dim3(32, 1, 1);

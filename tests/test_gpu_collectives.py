@@ -301,3 +301,28 @@ def test_device_send_without_a_proxy():
     _lib.check(lib.b2_selftest_direct_send(0, 40, ctypes.byref(ok)))
     assert ok.value == 1
     assert torch.ones(4, device="cuda").sum().item() == 4
+
+
+@pytest.mark.parametrize("ranks", [1, 2])
+def test_native_call_checks_its_arguments(ranks):
+    comm = nn.Communicator(devices=[0], loopback_ranks=ranks if ranks > 1 else 0, wait_timeout_ms=2000)
+    x = [torch.full((64,), float(r + 1), device="cuda") for r in range(ranks)]
+    y = [torch.zeros(64, device="cuda") for _ in range(ranks)]
+    for out, inp, op, what in ((y, [t[:32] for t in x], "sum", "elements"), ([t.half() for t in y], x, "sum", "dtype"),
+                               ([t.cpu() for t in y], x, "sum", "CUDA tensor"), ([t[::2] for t in y], [t[:32] for t in x], "sum", "contiguous"),
+                               (y, x, "prod", "unknown reduction"), (y + y, x, "sum", "one tensor per local rank")):
+        with pytest.raises(ValueError, match=what):
+            comm.all_reduce(out, inp, op=op)
+    with pytest.raises(ValueError, match="one stream per local rank"):
+        comm.all_reduce(y, x, stream=[])
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    for stream in (None, side, [side] * ranks, side.cuda_stream):
+        assert comm.all_reduce(y, x, stream=stream) is y
+    if ranks == 1:
+        assert comm.all_reduce(y[0], x[0]) is y[0]
+    torch.cuda.synchronize()
+    assert all((t == ranks * (ranks + 1) / 2).all() for t in y)
+    comm.close()
+    with pytest.raises(RuntimeError, match="closed"):
+        comm.all_reduce(y, x)
