@@ -11,7 +11,7 @@ import torch
 
 from . import _lib
 
-_ALGO_NAMES = ["auto", "oneshot", "twoshot", "nvls", "ring", "ll", "copy", "pipeline"]
+_ALGO_NAMES = ["auto", "oneshot", "twoshot", "nvls", "ring", "ll", "copy", "pipeline", "local"]
 
 
 class _SymmetricBlock:

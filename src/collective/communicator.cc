@@ -20,7 +20,7 @@
 #include "kernels/sm100/dev_types.h"
 #include "kernels/sm100/direct_collectives.h"
 #include "kernels/sm100/ll_allreduce.h"
-#include "kernels/sm100/local_copy.h"
+#include "kernels/sm100/local_collectives.h"
 #include "kernels/sm100/staged_pipeline.h"
 #include "mem/ipc_window.h"
 #include "mem/symmetric.h"
@@ -132,6 +132,7 @@ private:
                              bool nvls, int grid);
     void launch_gather_ranks(const CollectiveArgs& args, std::vector<dev::GatherArgs>& per_rank, int grid);
     void launch_low_latency(const CollectiveArgs& args);
+    void launch_on_one_device(Collective collective, const CollectiveArgs& args, int max_ctas);
     void launch_pipeline(const CollectiveArgs& args, const sched::Plan& plan);
     bool direct_peer_pointers() const { return loopback_ || (!multiprocess_ && resolved_ == TransportKind::P2p); }
     void poison(const std::string& why) const {
@@ -835,6 +836,7 @@ void Communicator::Impl::run(Collective collective, const CollectiveArgs& args) 
     shape.peers_write_output = direct_peer_pointers() || out_sym;
     shape.input_multicast = in_sym && windows_[in_loc[0].region].mc != nullptr;
     shape.output_multicast = out_sym && windows_[out_loc[0].region].mc != nullptr;
+    shape.one_device = loopback_;
     shape.ring_only = resolved_ != TransportKind::P2p;  // shm, mixed, socket, rdma: only the ring crosses those edges
     shape.max_ctas = tuning_.max_ctas;
     shape.staging_multicast = alloc_ && alloc_->multicast_supported() && (!stage_ || stage_->multicast_ptr() != nullptr);
@@ -894,27 +896,12 @@ void Communicator::Impl::run(Collective collective, const CollectiveArgs& args) 
         return;
     }
 
-    if (plan.algo == Algo::LowLatency) {
-        launch_low_latency(args);
+    if (plan.algo == Algo::Local || nranks_ == 1) {
+        launch_on_one_device(collective, args, plan.grid);
         return;
     }
-    if (plan.algo == Algo::Copy) {
-        // One rank: input and output hold `count` elements for every collective.
-        Local& l = local_[0];
-        DeviceGuard guard(l.device);
-        cudaStream_t stream = args.streams[0];
-        try {
-            wait_previous(l, stream);
-            if (args.send_buffers[0] != args.recv_buffers[0])
-                B2_CUDA(kernels::launch_local_copy(args.send_buffers[0], args.recv_buffers[0], args.count * esz, plan.grid,
-                                                   l.status, stream));
-            record_done(l, stream);
-        } catch (const std::exception& e) {
-            poison(std::string("launch failed: ") + e.what());
-            throw;
-        }
-        last_.grid = plan.grid;
-        last_.block = 32;
+    if (plan.algo == Algo::LowLatency) {
+        launch_low_latency(args);
         return;
     }
     if (plan.stage_in || plan.stage_out) ensure_staging(args);
@@ -927,6 +914,33 @@ void Communicator::Impl::run(Collective collective, const CollectiveArgs& args) 
         case Collective::ReduceScatter: launch_reduce_scatter(args, plan, wide, in_sym ? in_loc.data() : nullptr); break;
         case Collective::AllGather: launch_all_gather(args, plan, wide, in_sym ? in_loc.data() : nullptr, out_sym ? out_loc.data() : nullptr); break;
     }
+}
+
+// All ranks on one device: emulated ranks, or a single one.
+void Communicator::Impl::launch_on_one_device(Collective collective, const CollectiveArgs& args, int max_ctas) {
+    kernels::LocalCall call;
+    call.collective = collective;
+    call.dtype = args.dtype;
+    call.redop = args.redop;
+    call.nranks = nranks_;
+    call.in = args.send_buffers.data();
+    call.out = args.recv_buffers.data();
+    call.count = args.count;
+    call.max_ctas = max_ctas;
+    call.stream = args.streams[0];
+    kernels::LocalLaunch made;
+    try {
+        DeviceGuard guard(local_[0].device);
+        wait_previous(local_[0], call.stream);
+        if (nranks_ > 1 || args.send_buffers[0] != args.recv_buffers[0]) B2_CUDA(kernels::launch_local(call, &made));
+        record_done(local_[0], call.stream);
+    } catch (const std::exception& e) {
+        poison(std::string("launch failed: ") + e.what());
+        throw;
+    }
+    last_.grid = made.grid;
+    last_.block = made.block;
+    last_.pack_bytes = made.pack_bytes;
 }
 
 // Low-latency AllReduce: the ranks exchange {data, call number} words through receive areas in

@@ -46,6 +46,7 @@ const char* algo_name(Algo a) {
         case Algo::LowLatency: return "ll";
         case Algo::Copy: return "copy";
         case Algo::Pipeline: return "pipeline";
+        case Algo::Local: return "local";
     }
     return "unknown";
 }
@@ -98,8 +99,8 @@ bool parse_algo(const char* text, Algo* out) {
     static const std::pair<const char*, Algo> t[] = {
         {"auto", Algo::Auto},       {"oneshot", Algo::OneShot}, {"twoshot", Algo::TwoShot},
         {"nvls", Algo::Nvls},       {"ring", Algo::Ring},       {"ring_simple", Algo::Ring},
-        {"ll", Algo::LowLatency},   {"pipeline", Algo::Pipeline}};
-    return parse_from(text, out, t, 8);
+        {"ll", Algo::LowLatency},   {"pipeline", Algo::Pipeline}, {"local", Algo::Local}};
+    return parse_from(text, out, t, 9);
 }
 
 bool parse_collective(const char* text, Collective* out) {

@@ -1,0 +1,379 @@
+// AllReduce, ReduceScatter and AllGather of ranks that share one device, in one plain launch.
+//
+// Bound by HBM: every input byte is read once and every output byte is written once. A thread loads the same
+// pack of every rank's input, combines them in rank order in fp32, rounds once and stores the result to every
+// output that holds it. Nothing waits for anything inside the kernel, so the launch needs no barrier, no flag
+// memory and no cooperative launch, any number of CTAs may run, and it is a programmatic dependent of the
+// kernel before it.
+//
+// Layout of the work: a call is cut into segments that share one set of addresses (all_reduce: one;
+// reduce_scatter: one per output block; all_gather: one per input), a segment into tiles of kThreads packs, and
+// there is one CTA per tile. CTAs start in order and live for one load and one store phase, which keeps the
+// window of addresses in flight narrow and the DRAM on reads, then on writes. Measured against CTAs that stay
+// and loop (one or two per SM, interleaved or contiguous, 16- to 256-byte windows per thread, and TMA bulk
+// copies through shared memory), float sum: 8 ranks x 64 MiB 157.8 us (6.81 TB/s) against 172.7-181.5 us;
+// 2 ranks x 512 MiB 308.8 us (6.96 TB/s) against 322-375 us; one rank, 64 MiB 21.2 us against 22.9 us for a
+// TMA bulk-copy kernel with one CTA per SM. More packs per thread, or 128 or 512 threads, change less than 1 %.
+// CTAs loop only where the caller caps their number.
+//
+// Lengths and addresses need no alignment beyond the element's. Packs are cut where the INPUTS are aligned; the
+// elements before the first and after the last pack of a segment are handled one by one by the CTA of its first
+// tile. Where the outputs are aligned differently (blocks of a ragged reduce_scatter or all_gather), results
+// move between neighbouring lanes by shuffle so that the stores are aligned 16-byte vectors all the same.
+#include "kernels/sm100/local_collectives.h"
+
+#include "kernels/sm100/vec.cuh"
+
+#include <algorithm>
+#include <cstdint>
+#include <type_traits>
+
+namespace b200ccl::kernels {
+
+using namespace b200ccl::dev;
+
+namespace {
+
+using u64 = unsigned long long;
+
+constexpr int kThreads = 256;
+
+struct LocalArgs {
+    const char* in[kMaxRanks];
+    char* out[kMaxRanks];
+    u64 count;           // elements of one segment
+    u64 in_step;         // bytes from one segment to the next in every input (reduce_scatter)
+    u64 out_step;        // bytes from one segment to the next in every output (all_gather)
+    unsigned tiles;      // of one segment
+    unsigned segments;
+    float scale;
+    int nranks;
+    int in_by_segment;   // all_gather: segment s reads in[s] only
+    int outs;            // outputs that a segment writes: all of them, or (1) out[s] only
+};
+
+// Bytes in flight per thread and input. A copy from one buffer to one buffer wants more (one rank, 64 MiB: 21.6 us
+// against 23.4 us with 32 bytes); one to eight buffers does not (8 ranks, 4 MiB blocks: 49.8 us against 46.7 us).
+constexpr int kBytes = 32, kCopyBytes = 128;
+
+// Word j.. of eight words shifted right by `bytes` (0 < bytes < 16, even).
+__device__ __forceinline__ uint4 shift_pair(const uint4& a, const uint4& b, unsigned bytes) {
+    unsigned w0, w1, w2, w3, w4;
+    switch (bytes >> 2) {
+        case 0: w0 = a.x; w1 = a.y; w2 = a.z; w3 = a.w; w4 = b.x; break;
+        case 1: w0 = a.y; w1 = a.z; w2 = a.w; w3 = b.x; w4 = b.y; break;
+        case 2: w0 = a.z; w1 = a.w; w2 = b.x; w3 = b.y; w4 = b.z; break;
+        default: w0 = a.w; w1 = b.x; w2 = b.y; w3 = b.z; w4 = b.w; break;
+    }
+    const unsigned bits = (bytes & 3u) * 8u;
+    return make_uint4(__funnelshift_r(w0, w1, bits), __funnelshift_r(w1, w2, bits), __funnelshift_r(w2, w3, bits),
+                      __funnelshift_r(w3, w4, bits));
+}
+
+template <typename T, typename Op, int N>
+__device__ __forceinline__ void reduce_one(const LocalArgs& a, unsigned seg, u64 in_off, u64 out_off, u64 e) {
+    T v;
+    if constexpr (N == 1) {
+        v = Narrow<T>::load(a.in[a.in_by_segment ? seg : 0] + in_off, e);
+    } else {
+        float acc = 0.0f;
+#pragma unroll
+        for (int p = 0; p < (N > 0 ? N : kMaxRanks); ++p) {
+            if (N > 0 || p < a.nranks) {
+                const float f = Elem<T>::to_f(Narrow<T>::load(a.in[p] + in_off, e));
+                acc = p == 0 ? f : Op::apply(acc, f);
+            }
+        }
+        v = Elem<T>::from_f(a.scale != 1.0f ? acc * a.scale : acc);
+    }
+    for (int q = 0; q < a.outs; ++q) reinterpret_cast<T*>(a.out[a.outs == 1 ? seg : q] + out_off)[e] = v;
+}
+
+// kPack 32: inputs and outputs are aligned alike. kPack 16: outputs may be aligned differently from inputs.
+template <typename T, typename Op, int N, int kPack, int kPerThread>
+__global__ void __launch_bounds__(kThreads, N <= 2 ? 4 : (N <= 4 ? 3 : 2)) local_kernel(const __grid_constant__ LocalArgs a) {
+    using P = std::conditional_t<kPack == 32, Wide32<T>, Wide<T>>;
+    using Raw = typename P::Raw;
+    constexpr int kElems = P::kElems;
+    constexpr int U = kPerThread / kPack;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const bool scaled = a.scale != 1.0f;
+    for (unsigned t = blockIdx.x; t < a.tiles * a.segments; t += gridDim.x) {
+        const unsigned seg = t / a.tiles, tile = t - seg * a.tiles;
+        const u64 in_off = seg * a.in_step, out_off = seg * a.out_step;
+        const char* src0 = a.in[a.in_by_segment ? seg : 0] + in_off;
+        const unsigned skew = (unsigned)(reinterpret_cast<std::uintptr_t>(src0) & (kPack - 1));
+        const unsigned before = ((unsigned)kPack - skew) & (kPack - 1);  // bytes until the inputs are aligned
+        const u64 head = before / sizeof(T) < a.count ? before / sizeof(T) : a.count;
+        const u64 packs = (a.count - head) / kElems;
+        if (tile == 0) {
+            const u64 tail0 = head + packs * kElems;
+            for (u64 e = threadIdx.x; e < head + (a.count - tail0); e += kThreads)
+                reduce_one<T, Op, N>(a, seg, in_off, out_off, e < head ? e : tail0 + (e - head));
+        }
+        const u64 in_body = in_off + before, out_body = out_off + before;
+        const u64 i0 = (u64)tile * (kThreads * U) + threadIdx.x;
+        Raw r[U][N];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (i0 + u * kThreads < packs) {
+#pragma unroll
+                for (int p = 0; p < N; ++p) r[u][p] = P::load((N == 1 ? src0 - in_off : a.in[p]) + in_body, i0 + u * kThreads);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const u64 i = i0 + u * kThreads;
+            Raw v = r[u][0];
+            if constexpr (N > 1) {
+                float acc[kElems];
+                P::unpack(r[u][0], acc);
+#pragma unroll
+                for (int p = 1; p < N; ++p) {
+                    float f[kElems];
+                    P::unpack(r[u][p], f);
+#pragma unroll
+                    for (int e = 0; e < kElems; ++e) acc[e] = Op::apply(acc[e], f[e]);
+                }
+                if (scaled) {
+#pragma unroll
+                    for (int e = 0; e < kElems; ++e) acc[e] *= a.scale;
+                }
+                v = P::pack(acc);
+            }
+            if constexpr (kPack == 32) {
+                if (i < packs)
+                    for (int q = 0; q < a.outs; ++q) P::store(a.out[a.outs == 1 ? seg : q] + out_body, i, v);
+            } else {
+                const unsigned m = (unsigned)(reinterpret_cast<std::uintptr_t>(a.out[a.outs == 1 ? seg : 0] + out_body) & 15u);
+                if (m == 0) {
+                    if (i < packs)
+                        for (int q = 0; q < a.outs; ++q) P::store(a.out[a.outs == 1 ? seg : q] + out_body, i, v);
+                } else {
+                    // The aligned vector that starts s bytes into this lane's pack ends m bytes into the next lane's.
+                    const unsigned s = 16u - m, lane = threadIdx.x & 31u;
+                    uint4 next;
+                    next.x = __shfl_down_sync(0xffffffffu, v.x, 1);
+                    next.y = __shfl_down_sync(0xffffffffu, v.y, 1);
+                    next.z = __shfl_down_sync(0xffffffffu, v.z, 1);
+                    next.w = __shfl_down_sync(0xffffffffu, v.w, 1);
+                    if (i < packs) {
+                        const bool last = lane == 31u || i + 1 >= packs;
+                        const uint4 w = shift_pair(v, next, s);
+                        T elems[kElems];
+                        *reinterpret_cast<uint4*>(elems) = v;
+                        for (int q = 0; q < a.outs; ++q) {
+                            char* dst = a.out[a.outs == 1 ? seg : q] + out_body + i * 16ull;
+                            if (!last) st16(reinterpret_cast<uint4*>(dst + s), w);
+                            if (lane == 0u || last) {
+#pragma unroll
+                                for (int e = 0; e < kElems; ++e)
+                                    if (e * sizeof(T) < s ? lane == 0u : last) reinterpret_cast<T*>(dst)[e] = elems[e];
+                            }
+                        }
+                    }
+                }
+            }
+        }
+    }
+}
+
+// Inputs (or outputs) that are not aligned alike among themselves: one element per access.
+template <typename T, typename Op>
+__global__ void __launch_bounds__(kThreads) local_scalar_kernel(const __grid_constant__ LocalArgs a) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (unsigned seg = 0; seg < a.segments; ++seg) {
+        const u64 in_off = seg * a.in_step, out_off = seg * a.out_step;
+        for (u64 e = (u64)blockIdx.x * kThreads + threadIdx.x; e < a.count; e += (u64)gridDim.x * kThreads) {
+            if (a.in_by_segment) reduce_one<T, Op, 1>(a, seg, in_off, out_off, e);
+            else reduce_one<T, Op, 0>(a, seg, in_off, out_off, e);
+        }
+    }
+}
+
+struct Plan {
+    LocalArgs args;
+    int pack = 0;  // 32, 16 or 0 (element by element)
+    int max_ctas = 0;  // 0: one CTA per tile
+    cudaStream_t stream = nullptr;
+};
+
+cudaError_t start(void (*kernel)(LocalArgs), const Plan& p, u64 work, LocalLaunch* made) {
+    const u64 grid = p.max_ctas > 0 ? std::min<u64>(work, (u64)p.max_ctas) : work;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3((unsigned)grid, 1, 1);
+    config.blockDim = dim3(kThreads, 1, 1);
+    config.stream = p.stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attr;
+    config.numAttrs = 1;
+    made->grid = (int)grid;
+    made->block = kThreads;
+    made->pack_bytes = p.pack;
+    return cudaLaunchKernelEx(&config, kernel, p.args);
+}
+
+template <typename T, typename Op, int N, int kPack, int kPerThread = kBytes>
+cudaError_t start_packed(Plan& p, LocalLaunch* made) {
+    constexpr u64 tile = (u64)kThreads * (kPerThread / sizeof(T));
+    const u64 tiles = (p.args.count + tile - 1) / tile;
+    if (tiles * p.args.segments > 0x7fffffffull) return cudaErrorInvalidValue;
+    p.args.tiles = (unsigned)tiles;
+    return start(local_kernel<T, Op, N, kPack, kPerThread>, p, tiles * p.args.segments, made);
+}
+
+template <typename T, typename Op>
+cudaError_t start_op(Plan& p, LocalLaunch* made) {
+    if (p.pack == 0) {
+        made->pack_bytes = (int)sizeof(T);
+        p.pack = (int)sizeof(T);
+        return start(local_scalar_kernel<T, Op>, p, std::min<u64>((p.args.count + kThreads - 1) / kThreads, 0x7fffffffull), made);
+    }
+    switch (p.args.nranks) {
+#define B2_LOCAL_N(n) \
+    case n: return p.pack == 32 ? start_packed<T, Op, n, 32>(p, made) : start_packed<T, Op, n, 16>(p, made);
+        B2_LOCAL_N(2)
+        B2_LOCAL_N(3)
+        B2_LOCAL_N(4)
+        B2_LOCAL_N(5)
+        B2_LOCAL_N(6)
+        B2_LOCAL_N(7)
+        B2_LOCAL_N(8)
+#undef B2_LOCAL_N
+    }
+    return cudaErrorInvalidValue;
+}
+
+// Copies: two-byte elements serve every type.
+cudaError_t start_copy(Plan& p, LocalLaunch* made) {
+    if (p.pack == 32 && p.args.nranks == 1) return start_packed<__half, OpAdd, 1, 32, kCopyBytes>(p, made);
+    if (p.pack == 32) return start_packed<__half, OpAdd, 1, 32>(p, made);
+    if (p.pack == 16) return start_packed<__half, OpAdd, 1, 16>(p, made);
+    return start_op<__half, OpAdd>(p, made);
+}
+
+template <typename T>
+cudaError_t start_type(RedOp op, Plan& p, LocalLaunch* made) {
+    switch (op) {
+        case RedOp::Sum:
+        case RedOp::Avg: return start_op<T, OpAdd>(p, made);
+        case RedOp::Max: return start_op<T, OpMax>(p, made);
+        case RedOp::Min: return start_op<T, OpMin>(p, made);
+    }
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace
+
+cudaError_t launch_local(const LocalCall& call, LocalLaunch* made) {
+    const int n = call.nranks;
+    if (n < 1 || n > kMaxRanks || call.count == 0) return cudaErrorInvalidValue;
+    const std::size_t bytes = call.count * dtype_size(call.dtype);
+    const bool copies = n == 1 || call.collective == Collective::AllGather;
+    Plan p;
+    LocalArgs& a = p.args;
+    a = LocalArgs{};
+    a.count = copies ? bytes / 2 : call.count;
+    a.nranks = n;
+    a.scale = !copies && call.redop == RedOp::Avg ? 1.0f / static_cast<float>(n) : 1.0f;
+    a.segments = call.collective == Collective::AllReduce ? 1u : (unsigned)n;
+    a.in_step = call.collective == Collective::ReduceScatter ? bytes : 0;
+    a.out_step = call.collective == Collective::AllGather ? bytes : 0;
+    a.in_by_segment = call.collective == Collective::AllGather ? 1 : 0;
+    a.outs = call.collective == Collective::ReduceScatter ? 1 : n;
+    // Bits in which the addresses of one side differ, and in which any two addresses of a segment differ.
+    std::uintptr_t in_bits = 0, out_bits = 0;
+    const auto in0 = reinterpret_cast<std::uintptr_t>(call.in[0]), out0 = reinterpret_cast<std::uintptr_t>(call.out[0]);
+    for (int r = 0; r < n; ++r) {
+        a.in[r] = static_cast<const char*>(call.in[r]);
+        a.out[r] = static_cast<char*>(call.out[r]);
+        in_bits |= reinterpret_cast<std::uintptr_t>(call.in[r]) ^ in0;
+        out_bits |= reinterpret_cast<std::uintptr_t>(call.out[r]) ^ out0;
+    }
+    const std::uintptr_t steps = a.segments > 1 ? bytes : 0;
+    if (((in_bits | out_bits | (in0 ^ out0) | steps) & 31u) == 0) p.pack = 32;
+    else if (((in_bits | out_bits) & 15u) == 0) p.pack = 16;
+    p.max_ctas = call.max_ctas;
+    p.stream = call.stream;
+    if (copies) return start_copy(p, made);
+    switch (call.dtype) {
+        case DType::Float: return start_type<float>(call.redop, p, made);
+        case DType::Float16: return start_type<__half>(call.redop, p, made);
+        case DType::BFloat16: return start_type<__nv_bfloat16>(call.redop, p, made);
+    }
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace b200ccl::kernels
+
+// ---------------------------------------------------------------------------------------------
+// Allocation-free single-GPU all-reduce (declaration and contract: kernels/sm100/no_alloc.h).
+// The launch above needs no memory of its own, so there is nothing to add but the checks.
+
+#include "kernels/sm100/no_alloc.h"
+
+#include <string>
+
+namespace b200ccl::kernels {
+// Message of the calling thread's last failure, shared with the C interface (b2_last_error).
+void set_last_error_message(const std::string& message);
+}  // namespace b200ccl::kernels
+
+extern "C" int b2_local_all_reduce_no_alloc(const void* const* inputs, void* const* outputs, int nranks, size_t count,
+                                            int dtype, int redop, void* stream, void* /*status_record*/) {
+    using namespace b200ccl;
+    auto reject = [](const std::string& why) {
+        kernels::set_last_error_message("b2_local_all_reduce_no_alloc: " + why);
+        return 2;
+    };
+    if (nranks < 1 || nranks > B2_NO_ALLOC_MAX_RANKS)
+        return reject("nranks = " + std::to_string(nranks) + " is outside 1.." + std::to_string(B2_NO_ALLOC_MAX_RANKS));
+    if (count == 0) return reject("count must be positive");
+    if (dtype < 0 || dtype > 2) return reject("unsupported dtype");
+    if (redop < 0 || redop > 3) return reject("unknown reduction operator");
+    if (inputs == nullptr || outputs == nullptr) return reject("inputs and outputs must be non-null");
+    const std::size_t elem_bytes = dtype_size(static_cast<DType>(dtype));
+    if (count > SIZE_MAX / elem_bytes) return reject("count * element size does not fit in size_t");
+    const std::size_t span = count * elem_bytes;
+    // Byte ranges [ptr, ptr + span) of two buffers share at least one byte.
+    auto overlap = [span](const void* a, const void* b) {
+        const std::uintptr_t x = reinterpret_cast<std::uintptr_t>(a), y = reinterpret_cast<std::uintptr_t>(b);
+        return x < y ? y - x < span : x - y < span;
+    };
+    for (int r = 0; r < nranks; ++r) {
+        if (inputs[r] == nullptr || outputs[r] == nullptr) return reject("every buffer must be non-null");
+        if (reinterpret_cast<std::uintptr_t>(inputs[r]) > UINTPTR_MAX - span ||
+            reinterpret_cast<std::uintptr_t>(outputs[r]) > UINTPTR_MAX - span)
+            return reject("a buffer's byte range wraps around the address space");
+    }
+    for (int r = 0; r < nranks; ++r) {
+        for (int q = 0; q < nranks; ++q) {
+            if (inputs[r] == outputs[q]) return reject("in-place operation is not supported");
+            if (overlap(inputs[r], outputs[q]))
+                return reject("input " + std::to_string(r) + " and output " + std::to_string(q) + " overlap");
+            if (q > r && overlap(outputs[r], outputs[q]))
+                return reject("outputs " + std::to_string(r) + " and " + std::to_string(q) + " overlap");
+        }
+    }
+    kernels::LocalCall call;
+    call.collective = Collective::AllReduce;
+    call.dtype = static_cast<DType>(dtype);
+    call.redop = static_cast<RedOp>(redop);
+    call.nranks = nranks;
+    call.in = inputs;
+    call.out = outputs;
+    call.count = count;
+    call.stream = static_cast<cudaStream_t>(stream);
+    kernels::LocalLaunch made;
+    const cudaError_t st = kernels::launch_local(call, &made);
+    if (st != cudaSuccess) {
+        kernels::set_last_error_message(std::string("b2_local_all_reduce_no_alloc: launch failed: ") + cudaGetErrorString(st));
+        (void)cudaGetLastError();
+        return 1;
+    }
+    return 0;
+}

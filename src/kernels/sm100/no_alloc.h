@@ -13,9 +13,9 @@
  *   - code that runs under a "no allocation after initialisation" rule (real-time or safety
  *     reviews often impose one).
  * The communicator's own entry points are of no use to them: creating a communicator allocates
- * control blocks, staging memory and events. This function does the same reduction as a
- * communicator in single-GPU emulation mode does, with the same kernel, but the only scratch memory
- * it touches is a fixed array that is part of the library image.
+ * control blocks, staging memory and events. This function is one launch of the kernel that a
+ * communicator uses for ranks that share a GPU (kernels/sm100/local_collectives.cu), which needs no
+ * memory but the caller's buffers.
  *
  * What it computes. `nranks` input buffers and `nranks` output buffers of `count` elements, all on
  * the current device. Every output receives the element-wise reduction (sum, avg, max, min; fp32
@@ -24,30 +24,15 @@
  * rejected, as is a count whose byte size overflows size_t. Work is enqueued on `stream`; the call
  * returns without waiting for it.
  *
- * Scratch. One control block per emulated rank (barrier flags, per-CTA epochs, abort word) in a
- * file-scope `static __device__` array of B2_NO_ALLOC_MAX_RANKS blocks, about 13 KiB each, roughly
- * 104 KiB in total. Every GPU on which the library is loaded holds that array until the process
- * exits, whether or not this function is ever called.
- *
  * Limits and errors. nranks must be between 1 and B2_NO_ALLOC_MAX_RANKS (8); larger values are
  * rejected with a message (see b2_last_error) and nothing is launched. count must be positive.
  * Return value: 0 on success, 2 for a rejected argument, 1 for a CUDA failure.
  *
- * Set-up. The first call on a device resolves the array's device address (with that device
- * current) and remembers it; do that first call before starting any stream capture on that device.
- * Later calls on the same device do no set-up.
+ * Sharing. Calls keep nothing between them: any number may run at once, on any streams, and any call
+ * may be captured into a graph.
  *
- * Sharing. All calls on one device use the same array, and the array keeps what the previous call
- * left in it. Each call therefore begins by clearing the array on `stream`. Two calls whose work
- * overlaps on the GPU (different streams without an ordering between them, or two host threads)
- * would race on the array: order them.
- *
- * Failure of a wait. The emulated ranks meet in barriers inside one cooperative launch, which the
- * driver only accepts when all of its blocks can be resident, so the bounded waits are not
- * expected to run out. If one does (after `B2_NO_ALLOC_WAIT_MS`), the kernel ends early and, when
- * `status_record` is not null, writes a 32-byte record there whose first 32-bit word is non-zero
- * (1 = timed out, 2 = aborted). `status_record` is caller-owned memory that the device can write
- * (device memory or mapped host memory), cleared by the caller beforehand; pass null to skip it.
+ * `status_record` is accepted for callers of earlier versions, whose kernel had waits that could run
+ * out; nothing is written to it.
  */
 #pragma once
 
@@ -58,7 +43,6 @@ extern "C" {
 #endif
 
 #define B2_NO_ALLOC_MAX_RANKS 8
-#define B2_NO_ALLOC_WAIT_MS 2000
 
 /* dtype: 0 float, 1 fp16, 2 bf16. redop: 0 sum, 1 avg, 2 max, 3 min. stream: a cudaStream_t. */
 int b2_local_all_reduce_no_alloc(const void* const* inputs, void* const* outputs, int nranks, size_t count, int dtype,

@@ -27,6 +27,7 @@ struct CallShape {
     bool output_multicast = false;    // output has a multicast alias (NVLS broadcast possible)
     bool staging_multicast = false;   // the staging arena has a multicast alias (staged NVLS possible)
     bool in_place = false;
+    bool one_device = false;     // all ranks' buffers live on one GPU and one stream orders them (emulated ranks)
     bool ring_only = false;      // transport without all-pairs peer access: ring is the only choice
     int max_ctas = 64;
 };

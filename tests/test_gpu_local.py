@@ -1,0 +1,83 @@
+"""Ranks that share one device, in one launch without waits (algo local, the choice for emulated ranks): lengths
+around the edges of packs, warps and tiles, aligned alike, misaligned alike, misaligned apart; blocks of
+reduce_scatter and all_gather whose ragged length moves every block's alignment. Compared with a plain PyTorch
+fp32 reference; elements on both sides of every output must stay as they were."""
+import pytest
+import torch
+
+import nano_nccl_b200 as nn
+
+pytestmark = pytest.mark.gpu
+
+TOL = {torch.float32: 1e-5, torch.float16: 1e-2, torch.bfloat16: 1e-1}
+# one element; around a 16- and a 32-byte pack; a warp's packs; a tile's (8 ranks: 256 packs of 32 bytes) and more than one tile
+COUNTS = [1, 7, 8, 9, 15, 16, 17, 255, 257, 511, 513, 2047, 2049, 4096, 4099, 16384 + 5, 70001]
+PAD = 64
+
+
+def buffers(ranks, numel, dtype, shifts, seed):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    raw = [torch.full((numel + 2 * PAD,), 7.0, device="cuda", dtype=dtype) for _ in range(ranks)]
+    views = [t[PAD + s:PAD + s + numel] for t, s in zip(raw, shifts)]
+    if seed:
+        for v in views:
+            v.normal_(generator=gen)
+    return raw, views
+
+
+def untouched(raw, views):
+    for t, v in zip(raw, views):
+        lo = (v.data_ptr() - t.data_ptr()) // t.element_size()
+        assert (t[:lo] == 7.0).all() and (t[lo + v.numel():] == 7.0).all()
+
+
+@pytest.mark.parametrize("ranks", range(2, 9))
+@pytest.mark.parametrize("dtype", list(TOL))
+def test_one_device_collectives_at_every_edge(ranks, dtype):
+    comm = nn.Communicator(devices=[0], loopback_ranks=ranks, wait_timeout_ms=2000)
+    try:
+        same, apart = [1] * ranks, [r % 3 for r in range(ranks)]
+        for k, count in enumerate(COUNTS):
+            op = ["sum", "avg", "max", "min"][k % 4]
+            for shifts_in, shifts_out in (([0] * ranks, [0] * ranks), (same, same), ([0] * ranks, same), (same, [0] * ranks), (apart, apart)):
+                _, ins = buffers(ranks, count, dtype, shifts_in, 100 + k)
+                raw, outs = buffers(ranks, count, dtype, shifts_out, 0)
+                comm.all_reduce(outs, ins, op=op)
+                assert comm.last_call()["algo"] == "local"
+                stack = torch.stack([t.float() for t in ins])
+                ref = {"sum": stack.sum(0), "avg": stack.sum(0) / ranks, "max": stack.max(0).values, "min": stack.min(0).values}[op]
+                for o in outs:
+                    assert (o.float() - ref).abs().max().item() <= TOL[dtype] * 2, (count, op, shifts_in, shifts_out)
+                    assert torch.equal(o, outs[0])
+                untouched(raw, outs)
+                _, ins = buffers(ranks, count * ranks, dtype, shifts_in, 200 + k)
+                raw, outs = buffers(ranks, count, dtype, shifts_out, 0)
+                comm.reduce_scatter(outs, ins, op=op)
+                stack = torch.stack([t.float() for t in ins])
+                ref = {"sum": stack.sum(0), "avg": stack.sum(0) / ranks, "max": stack.max(0).values, "min": stack.min(0).values}[op]
+                for r, o in enumerate(outs):
+                    assert (o.float() - ref[r * count:(r + 1) * count]).abs().max().item() <= TOL[dtype] * 2, (count, op, shifts_in, shifts_out)
+                untouched(raw, outs)
+                _, ins = buffers(ranks, count, dtype, shifts_in, 300 + k)
+                raw, outs = buffers(ranks, count * ranks, dtype, shifts_out, 0)
+                comm.all_gather(outs, ins)
+                for o in outs:
+                    assert torch.equal(o, torch.cat(ins)), (count, shifts_in, shifts_out)
+                untouched(raw, outs)
+        comm.check_async_error()
+    finally:
+        comm.close()
+
+
+def test_in_place_on_one_device_and_a_capped_grid():
+    comm = nn.Communicator(devices=[0], loopback_ranks=3, max_ctas=5, wait_timeout_ms=2000)
+    try:
+        for count in (17, 300003, 1 << 20):
+            _, ins = buffers(3, count, torch.float32, [0, 0, 0], 9)
+            ref = torch.stack(ins).sum(0)
+            comm.all_reduce(ins)
+            assert comm.last_call()["grid"] <= 5
+            for t in ins:
+                assert (t - ref).abs().max().item() <= 1e-5
+    finally:
+        comm.close()
