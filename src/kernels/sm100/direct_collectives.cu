@@ -31,6 +31,10 @@ template <typename A>
 __device__ __forceinline__ const A& select_args(const A& one) { return one; }
 template <typename A>
 __device__ __forceinline__ const A& select_args(const LoopPack<A>& all) { return all.r[blockIdx.y]; }
+template <typename A>
+constexpr bool kAllRanksHere = false;
+template <typename A>
+constexpr bool kAllRanksHere<LoopPack<A>> = true;
 
 // Copies the packs first, first+stripe, ... below len, four loads in flight per thread. One side is
 // the caller's own buffer (16-byte aligned at most), the other the staging arena.
@@ -117,7 +121,7 @@ reduce_kernel(const __grid_constant__ ParamT param) {
 
     // 2. Every rank's input is ready (and every rank's previous use of `out` is over).
     ++epoch;
-    if (!cta_barrier_all_ranks(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 1u, a.plan_hash)) return;
+    if (!cta_barrier_all_ranks<kAllRanksHere<ParamT>>(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 1u, a.plan_hash)) return;
 
     // 3. Reduce the own shard.
     {
@@ -205,7 +209,7 @@ reduce_kernel(const __grid_constant__ ParamT param) {
 
     // 4. Every rank has finished reading inputs and its stores to peers are visible.
     ++epoch;
-    if (!cta_barrier_all_ranks(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 2u)) return;
+    if (!cta_barrier_all_ranks<kAllRanksHere<ParamT>>(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 2u)) return;
 
     // 5. Staged output: copy what the same-numbered CTAs of all ranks stored into the arena.
     if (a.user_out != nullptr) {
@@ -246,7 +250,7 @@ gather_kernel(const __grid_constant__ ParamT param) {
         for (u64 j = first; j < a.len; j += stripe) store(stage, j, load(a.user_in, j));
     }
     ++epoch;
-    if (!cta_barrier_all_ranks(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 1u, a.plan_hash)) return;
+    if (!cta_barrier_all_ranks<kAllRanksHere<ParamT>>(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 1u, a.plan_hash)) return;
 
     if (a.mode == 0) {
         const u64 base = (u64)rank * a.out_stride;
@@ -284,7 +288,7 @@ gather_kernel(const __grid_constant__ ParamT param) {
     }
 
     ++epoch;
-    if (!cta_barrier_all_ranks(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 2u)) return;
+    if (!cta_barrier_all_ranks<kAllRanksHere<ParamT>>(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 2u)) return;
     if (threadIdx.x == 0) own->epoch[blockIdx.x] = epoch;
 }
 

@@ -24,6 +24,11 @@ __device__ __forceinline__ unsigned long long ld_relaxed_sys(const unsigned long
 __device__ __forceinline__ void st_release_sys(unsigned long long* p, unsigned long long v) {
     asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
+// The same between threads of ONE GPU (emulated ranks), whatever memory the word lies in. On B200 a release at
+// system scope takes 1.9 us in one CTA and 3.5-3.8 us when 16 or more CTAs do it, at GPU scope 0.55 us.
+__device__ __forceinline__ void st_release_gpu(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
 __device__ __forceinline__ void st_relaxed_sys(unsigned long long* p, unsigned long long v) {
     asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
@@ -101,6 +106,8 @@ __device__ __forceinline__ bool wait_at_least(const unsigned long long* flag, un
 // plan_hash != 0: CTA 0 also publishes the fingerprint of this launch's plan with the signal and
 // compares it with every peer's after the wait; a difference ends the collective on every rank
 // with kStatusPlanMismatch (the other CTAs leave through the abort word).
+// kOneGpu: every rank is part of this launch, so that GPU scope orders them all.
+template <bool kOneGpu>
 __device__ __forceinline__ bool cta_barrier_all_ranks(ControlBlock* const* ctrl, int rank, int nranks,
                                                       unsigned long long epoch, unsigned long long timeout_ns,
                                                       Status* status, unsigned int where,
@@ -111,7 +118,8 @@ __device__ __forceinline__ bool cta_barrier_all_ranks(ControlBlock* const* ctrl,
         const int p = threadIdx.x;
         const bool check = plan_hash != 0ull && blockIdx.x == 0;
         if (check) st_relaxed_sys(&ctrl[p]->plan_hash[rank], plan_hash);
-        st_release_sys(&ctrl[p]->barrier[blockIdx.x][rank], epoch);
+        if constexpr (kOneGpu) st_release_gpu(&ctrl[p]->barrier[blockIdx.x][rank], epoch);
+        else st_release_sys(&ctrl[p]->barrier[blockIdx.x][rank], epoch);
         ok = wait_at_least(&ctrl[rank]->barrier[blockIdx.x][p], epoch, ctrl[rank], timeout_ns,
                            status, ctrl, nranks, (unsigned)p, where)
                  ? 1 : 0;
