@@ -259,8 +259,14 @@ Communicator::Impl::Impl(const CommunicatorConfig& config, Bootstrap* bootstrap)
         // (8 GPUs: 11.7 GB/s with 4, 10.3 with 8, 9.2 with 16); network edges keep a proxy thread pair per channel.
         channels_ = resolved_ == TransportKind::P2p ? 32
                     : (resolved_ == TransportKind::Shm || resolved_ == TransportKind::Mixed) ? 4 : kDefaultChannels;
-        // Emulated ranks share one GPU and one cooperative launch: all their channel CTAs must be resident at once.
-        if (loopback_) channels_ = std::min(channels_, std::max(1, 64 / nranks_));
+        // Emulated ranks share one GPU and one cooperative launch: all their channel CTAs must be resident at once, one
+        // per SM. Over device memory more of them are faster up to there (4 ranks, 16 MiB: 108 us with 16 channels, 73
+        // with 32). Over host memory eight CTAs in all keep PCIe busy both ways (35 of the 38 GB/s that a copy from host
+        // to host reaches); more of them slow it down (8 ranks, 1 MiB: 555 us with one channel, 834 with four).
+        if (loopback_) {
+            const int ctas = resolved_ == TransportKind::P2p ? 128 : (resolved_ == TransportKind::Shm ? 8 : 64);
+            channels_ = std::min(channels_, std::max(1, ctas / nranks_));
+        }
     }
     channels_ = std::max(1, std::min(channels_, kMaxChannels));
     {

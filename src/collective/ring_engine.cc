@@ -234,10 +234,15 @@ std::string RingEngine::async_error() const { return state_->net ? state_->net->
 void RingEngine::launch(Collective collective, const CollectiveArgs& args) {
     State& s = *state_;
     const std::size_t esz = dtype_size(args.dtype);
-    bool wide = (args.count * esz) % 16 == 0;
+    // Whole vectors, and at the end of an all_reduce the elements that fill none. A ragged length still goes element by
+    // element between processes, where the choice must not depend on addresses that other ranks cannot see, and where
+    // emulated ranks have more CTAs than can be resident at once with the vector kernel's registers (one per SM).
+    const bool whole = (args.count * esz) % 16 == 0;
+    const bool crowded = s.cfg.loopback && s.cfg.nranks * s.cfg.channels > 128;
+    bool wide = whole || (collective == Collective::AllReduce && !s.bootstrap && !crowded);
     for (std::size_t i = 0; i < s.cfg.local.size(); ++i)
         wide &= ((reinterpret_cast<std::uintptr_t>(args.send_buffers[i]) | reinterpret_cast<std::uintptr_t>(args.recv_buffers[i])) & 15u) == 0;
-    if (s.bootstrap && !wide && (args.count * esz) % 16 == 0)
+    if (s.bootstrap && !wide && whole)
         throw std::invalid_argument("ring: buffers of a multi-process communicator must be 16-byte aligned");
     std::vector<dev::RingArgs> per(s.cfg.local.size());
     for (std::size_t i = 0; i < s.cfg.local.size(); ++i) {

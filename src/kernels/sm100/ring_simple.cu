@@ -3,9 +3,13 @@
 // One CTA per channel. Data moves in slices through per-edge FIFOs that live in the receiver's
 // memory (peer stores over NVLink) or in mapped host memory (SHM, socket and RDMA edges). Flow
 // control is two monotonically growing step counters per edge, published with st.release.sys and
-// polled with ld.acquire.sys; counters persist from launch to launch. The local operand of a
-// reduce slice is prefetched into shared memory with bulk asynchronous copies (TMA) that are
-// issued BEFORE the thread waits for the neighbour, so the local HBM read overlaps the wait.
+// polled with ld.acquire.sys; counters persist from launch to launch.
+//
+// Bound by the chain of slices: a rank can only work on what its neighbour has posted, so what counts is
+// the time from one post to the next. Inside a slice no barrier is left: every thread keeps kBatch vectors
+// of the FIFO and of the local input in flight in registers, and the first batch of the local input is
+// loaded BEFORE the wait for the neighbour. (The local input used to be staged by TMA through 32 KiB tiles
+// of shared memory, with three block barriers and four dependent FIFO loads per thread and tile.)
 //
 // Parity: nano-nccl src/kernels/ring_simple_kernel.cuh:1118-1237 (schedule 1170-1230:
 // direct_send, recv_reduce_send, recv_reduce_copy_send with the fused avg scale, recv_copy_send,
@@ -15,7 +19,6 @@
 #include "kernels/sm100/ring_simple.h"
 
 #include "kernels/sm100/sync.cuh"
-#include "kernels/sm100/tma.cuh"
 #include "kernels/sm100/vec.cuh"
 #include "sched/ring_geometry.h"
 
@@ -28,9 +31,8 @@ namespace {
 using u64 = unsigned long long;
 
 constexpr int kRingThreads = 512;
-constexpr unsigned kTileBytes = 32768;          // one TMA tile of the local operand
-constexpr unsigned kTileVecs = kTileBytes / 16;
-constexpr unsigned kMbarPolls = 1u << 24;       // bound on waiting for an own TMA copy
+constexpr int kBatch = 8;  // vectors in flight per thread and source: a 64 KiB slice at once
+constexpr unsigned kCreditThread = 64, kPostThread = 96;  // they publish; threads 0 and 32 poll
 
 enum SliceFlags : unsigned {
     kRecv = 1u,        // take the slice from the incoming FIFO
@@ -49,20 +51,14 @@ __device__ __forceinline__ uint4 ld16_volatile(const uint4* p) {
 
 struct ChannelState {
     RingChannel ch;
+    bool one_gpu;  // both neighbours run in this launch: their counters need GPU scope only
     u64 send_step;
     u64 recv_step;
 };
 
-struct Shared {
-    alignas(128) unsigned char tile[2][kTileBytes];
-    alignas(8) u64 mbar[2];
-    u64 base_steps[2];
-};
-
 // Waits of the two flow-control threads; the outcome is shared through smem.
-template <typename T>
-__device__ __forceinline__ bool wait_flags(const RingArgs& a, ChannelState& st, unsigned flags, Shared& sm,
-                                           u64& t_wait_recv, u64& t_wait_send) {
+__device__ __forceinline__ bool wait_flags(const RingArgs& a, ChannelState& st, unsigned flags, u64& t_wait_recv,
+                                           u64& t_wait_send) {
     int ok = 1;
     if ((flags & kRecv) && threadIdx.x == 0) {
         const u64 t0 = st.ch.stats ? global_timer_ns() : 0;
@@ -86,8 +82,7 @@ __device__ __forceinline__ bool wait_flags(const RingArgs& a, ChannelState& st, 
 
 // One slice: wait, move/combine `n` elements, publish. Returns false when a wait gave up.
 template <typename T, typename Op, bool kWide>
-__device__ bool run_slice(const RingArgs& a, ChannelState& st, Shared& sm, unsigned (&phase)[2], unsigned flags,
-                          const T* local_in, T* local_out, u64 n) {
+__device__ bool run_slice(const RingArgs& a, ChannelState& st, unsigned flags, const T* local_in, T* local_out, u64 n) {
     if (n == 0) {  // empty slice: neither side waits, posts or advances
         if (st.ch.stats && threadIdx.x == 0) atomicAdd(&st.ch.stats->empty_slices, 1ull);
         return true;
@@ -101,126 +96,115 @@ __device__ bool run_slice(const RingArgs& a, ChannelState& st, Shared& sm, unsig
     // sender BEFORE they are combined and forwarded: the slot is read into registers, the credit is
     // posted, and only then does the slice go on. On host-memory and network edges, where a credit
     // takes microseconds to arrive, this takes the consumer's own work off the sender's critical path.
+    // Inside one GPU the credit is there before the sender has used up its four slots, and the extra barrier and
+    // release only lengthen the slice (4 ranks, 64 KiB: 35.9 -> 32.2 us without).
     // Parity: the reference's early-credit path for slices of at most 4096 bytes
     // (src/kernels/ring_simple_kernel.cuh:486-583, 912-927).
     bool early = false;
-
     bool ok = true;
+    auto combine_element = [&](u64 i) {
+        float acc[1];
+        if (recv) {
+            Narrow<T>::unpack(Narrow<T>::load(fifo_in, i), acc);
+            if (local) acc[0] = Op::apply(Elem<T>::to_f(local_in[i]), acc[0]);
+        } else {
+            acc[0] = Elem<T>::to_f(local_in[i]);
+        }
+        if (scaled) acc[0] *= a.scale;
+        const T out = Elem<T>::from_f(acc[0]);
+        if (copy_out) local_out[i] = out;
+        if (send) fifo_out[i] = out;
+    };
     if constexpr (kWide) {
         constexpr int kElems = 16 / sizeof(T);
-        const u64 nvec = n / kElems;  // wide path: n is a whole number of vectors
-        const bool staged = local && recv;  // prefetch the local operand while waiting for the neighbour
-        const unsigned ntiles = staged ? (unsigned)((nvec + kTileVecs - 1) / kTileVecs) : 0;
-        auto issue = [&](unsigned t) {
-            const u64 v0 = (u64)t * kTileVecs;
-            const unsigned bytes = (unsigned)(((nvec - v0) < kTileVecs ? (nvec - v0) : kTileVecs) * 16);
-            mbar_arrive_expect_tx(&sm.mbar[t & 1], bytes);
-            tma_load_bulk(sm.tile[t & 1], reinterpret_cast<const uint4*>(local_in) + v0, bytes, &sm.mbar[t & 1]);
+        const u64 nvec = n / kElems;
+        const unsigned tail = (unsigned)(n - nvec * kElems);  // only the last slice of a ragged message has any
+        const uint4* in_v = reinterpret_cast<const uint4*>(local_in);
+        const uint4* fifo_v = reinterpret_cast<const uint4*>(fifo_in);
+        uint4 loc[kBatch];
+        auto load_local = [&](u64 v0) {
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u)
+                if (v0 + u * kRingThreads < nvec) loc[u] = ld16_stream(in_v + v0 + u * kRingThreads);
         };
-        if (staged && threadIdx.x == 0) issue(0);
-        ok = wait_flags<T>(a, st, flags, sm, t_wait_recv, t_wait_send);
-        if (!ok) {
-            // Leave only after the copy in flight has landed (bounded).
-            if (staged) mbar_wait_bounded(&sm.mbar[0], phase[0], kMbarPolls);
-            return false;
-        }
+        if (local) load_local(threadIdx.x);
+        ok = wait_flags(a, st, flags, t_wait_recv, t_wait_send);
+        if (!ok) return false;
         if (st.ch.stats && threadIdx.x == 0) t0 = global_timer_ns();
-        early = recv && nvec <= (u64)kRingThreads;
+        early = recv && !st.one_gpu && nvec <= (u64)kRingThreads && tail == 0;
         uint4 pre = make_uint4(0, 0, 0, 0);
         if (early) {
             int sink = 0;
             if (threadIdx.x < nvec) {
-                pre = ld16_volatile(reinterpret_cast<const uint4*>(fifo_in) + threadIdx.x);
+                pre = ld16_volatile(fifo_v + threadIdx.x);
                 sink = (pre.x ^ pre.y ^ pre.z ^ pre.w) == 0x5bd1e995u;  // a use of the value: the barrier below then follows the load's arrival
             }
             (void)__syncthreads_or(sink);  // every thread holds its part of the slot
-            if (threadIdx.x == 0) st_release_sys(st.ch.recv_head, st.recv_step + ring::kSliceSteps);
+            if (threadIdx.x == 0)
+                st.one_gpu ? st_release_gpu(st.ch.recv_head, st.recv_step + ring::kSliceSteps)
+                           : st_release_sys(st.ch.recv_head, st.recv_step + ring::kSliceSteps);
         }
-        auto combine_store = [&](u64 v, uint4 loc, bool have_loc) {
-            uint4 out;
-            if (recv) {
-                const uint4 r = early ? pre : ld16_volatile(reinterpret_cast<const uint4*>(fifo_in) + v);
-                if (have_loc || scaled) {
-                    float acc[kElems], f[kElems];
-                    Wide<T>::unpack(r, acc);
-                    if (have_loc) {
-                        Wide<T>::unpack(loc, f);
+        auto combine_store = [&](u64 v, const uint4& got, const uint4& mine) {
+            uint4 out = recv ? got : mine;
+            if (recv && (local || scaled)) {
+                float acc[kElems], f[kElems];
+                Wide<T>::unpack(got, acc);
+                if (local) {
+                    Wide<T>::unpack(mine, f);
 #pragma unroll
-                        for (int e = 0; e < kElems; ++e) acc[e] = Op::apply(f[e], acc[e]);
-                    }
-                    if (scaled) {
-#pragma unroll
-                        for (int e = 0; e < kElems; ++e) acc[e] *= a.scale;
-                    }
-                    out = Wide<T>::pack(acc);
-                } else {
-                    out = r;
+                    for (int e = 0; e < kElems; ++e) acc[e] = Op::apply(f[e], acc[e]);
                 }
-            } else {
-                out = loc;
+                if (scaled) {
+#pragma unroll
+                    for (int e = 0; e < kElems; ++e) acc[e] *= a.scale;
+                }
+                out = Wide<T>::pack(acc);
             }
             if (copy_out) st16(reinterpret_cast<uint4*>(local_out) + v, out);
             if (send) st16(reinterpret_cast<uint4*>(fifo_out) + v, out);
         };
-        if (staged) {
-            for (unsigned t = 0; t < ntiles; ++t) {
-                if (t + 1 < ntiles && threadIdx.x == 0) issue(t + 1);
-                const unsigned b = t & 1;
-                int got = mbar_wait_bounded(&sm.mbar[b], phase[b], kMbarPolls) ? 1 : 0;
-                phase[b] ^= 1u;
-                if (!__syncthreads_and(got)) {
-                    if (threadIdx.x == 0)
-                        report_failure(a.status, a.own_ctrl, nullptr, 0, kStatusTimeout, (unsigned)a.rank, 12u, st.recv_step, 0);
-                    if (t + 1 < ntiles) mbar_wait_bounded(&sm.mbar[b ^ 1], phase[b ^ 1], kMbarPolls);
-                    return false;
-                }
-                const u64 v0 = (u64)t * kTileVecs;
-                const u64 vend = (nvec - v0) < kTileVecs ? (nvec - v0) : kTileVecs;
-                const uint4* tile = reinterpret_cast<const uint4*>(sm.tile[b]);
-                for (u64 i = threadIdx.x; i < vend; i += kRingThreads) combine_store(v0 + i, tile[i], true);
-                __syncthreads();  // the tile may be refilled only after every thread has read it
-            }
+        if (early) {
+            if (threadIdx.x < nvec) combine_store(threadIdx.x, pre, loc[0]);
         } else {
-            for (u64 v = threadIdx.x; v < nvec; v += kRingThreads) {
-                uint4 loc = make_uint4(0, 0, 0, 0);
-                if (local) loc = ld16_stream(reinterpret_cast<const uint4*>(local_in) + v);
-                combine_store(v, loc, local);
+            for (u64 v0 = threadIdx.x; v0 < nvec; v0 += kBatch * kRingThreads) {
+                uint4 got[kBatch];
+                if (recv) {
+#pragma unroll
+                    for (int u = 0; u < kBatch; ++u)
+                        if (v0 + u * kRingThreads < nvec) got[u] = ld16_volatile(fifo_v + v0 + u * kRingThreads);
+                }
+                if (local && v0 != threadIdx.x) load_local(v0);
+#pragma unroll
+                for (int u = 0; u < kBatch; ++u)
+                    if (v0 + u * kRingThreads < nvec) combine_store(v0 + u * kRingThreads, got[u], loc[u]);
             }
+            if (threadIdx.x < tail) combine_element(nvec * kElems + threadIdx.x);
         }
     } else {
-        ok = wait_flags<T>(a, st, flags, sm, t_wait_recv, t_wait_send);
+        ok = wait_flags(a, st, flags, t_wait_recv, t_wait_send);
         if (!ok) return false;
         if (st.ch.stats && threadIdx.x == 0) t0 = global_timer_ns();
-        for (u64 i = threadIdx.x; i < n; i += kRingThreads) {
-            float acc[1];
-            if (recv) {
-                const T r = Narrow<T>::load(fifo_in, i);
-                Narrow<T>::unpack(r, acc);
-                if (local) acc[0] = Op::apply(Elem<T>::to_f(local_in[i]), acc[0]);
-            } else {
-                acc[0] = Elem<T>::to_f(local_in[i]);
-            }
-            if (scaled) acc[0] *= a.scale;
-            const T out = Elem<T>::from_f(acc[0]);
-            if (copy_out) local_out[i] = out;
-            if (send) fifo_out[i] = out;
-        }
+        for (u64 i = threadIdx.x; i < n; i += kRingThreads) combine_element(i);
     }
 
-    // Publish: all data stores of the CTA happen-before the counters (bar.sync, then release).
+    // Publish: all data stores of the CTA happen-before the counters (bar.sync, then release). Two warps that do
+    // not poll do it, so that the waits of the next slice begin while the releases are on their way.
     __syncthreads();
     u64 t1 = 0;
     if (st.ch.stats && threadIdx.x == 0) t1 = global_timer_ns();
     if (recv) {
-        if (!early && threadIdx.x == 0) st_release_sys(st.ch.recv_head, st.recv_step + ring::kSliceSteps);
+        if (!early && threadIdx.x == kCreditThread)
+            st.one_gpu ? st_release_gpu(st.ch.recv_head, st.recv_step + ring::kSliceSteps)
+                       : st_release_sys(st.ch.recv_head, st.recv_step + ring::kSliceSteps);
         st.recv_step += ring::kSliceSteps;
     }
     if (send) {
-        if (threadIdx.x == 32) {
+        if (threadIdx.x == kPostThread) {
             if (st.ch.send_sizes) {
                 st.ch.send_sizes[st.send_step % ring::kFifoSteps] = (unsigned)(n * sizeof(T));
             }
-            st_release_sys(st.ch.send_tail, st.send_step + ring::kSliceSteps);
+            st.one_gpu ? st_release_gpu(st.ch.send_tail, st.send_step + ring::kSliceSteps)
+                       : st_release_sys(st.ch.send_tail, st.send_step + ring::kSliceSteps);
         }
         st.send_step += ring::kSliceSteps;
     }
@@ -237,24 +221,21 @@ __device__ bool run_slice(const RingArgs& a, ChannelState& st, Shared& sm, unsig
 
 // A chunk travels as kSlicesPerChunk slices.
 template <typename T, typename Op, bool kWide>
-__device__ __forceinline__ bool run_chunk(const RingArgs& a, ChannelState& st, Shared& sm, unsigned (&phase)[2],
-                                          unsigned flags, const T* local_in, T* local_out, u64 n) {
+__device__ __forceinline__ bool run_chunk(const RingArgs& a, ChannelState& st, unsigned flags, const T* local_in,
+                                          T* local_out, u64 n) {
     const u64 sl = ring::slice_elems(n, sizeof(T), a.step_elems);
 #pragma unroll 1
     for (int s = 0; s < ring::kSlicesPerChunk; ++s) {
         const u64 off = (u64)s * sl;
         const u64 sn = ring::clamp_elems(sl, n, off);
-        if (!run_slice<T, Op, kWide>(a, st, sm, phase, flags, local_in ? local_in + off : nullptr,
-                                     local_out ? local_out + off : nullptr, sn))
-            return false;
+        if (!run_slice<T, Op, kWide>(a, st, flags, local_in + off, local_out + off, sn)) return false;
     }
     return true;
 }
 
 template <typename T, typename Op, bool kWide, typename ParamT>
-__global__ void __launch_bounds__(kRingThreads) ring_kernel(const __grid_constant__ ParamT param) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    Shared& sm = *reinterpret_cast<Shared*>(smem_raw);
+__global__ void __launch_bounds__(kRingThreads, kWide ? 1 : 2) ring_kernel(const __grid_constant__ ParamT param) {
+    __shared__ u64 base_steps[2];
     const RingArgs* ap;
     if constexpr (sizeof(ParamT) == sizeof(RingArgs)) ap = reinterpret_cast<const RingArgs*>(&param);
     else ap = reinterpret_cast<const RingArgs*>(&param) + blockIdx.y;
@@ -264,17 +245,15 @@ __global__ void __launch_bounds__(kRingThreads) ring_kernel(const __grid_constan
 
     ChannelState st;
     st.ch = a.channels[c];
+    // Network edges name an abort word: a host thread is at their other end.
+    st.one_gpu = sizeof(ParamT) != sizeof(RingArgs) && st.ch.abort_word == nullptr;
     if (threadIdx.x == 0) {
-        sm.base_steps[0] = *st.ch.send_base;
-        sm.base_steps[1] = *st.ch.recv_base;
-        mbar_init(&sm.mbar[0], 1);
-        mbar_init(&sm.mbar[1], 1);
-        mbar_fence_init();
+        base_steps[0] = *st.ch.send_base;
+        base_steps[1] = *st.ch.recv_base;
     }
     __syncthreads();
-    st.send_step = sm.base_steps[0];
-    st.recv_step = sm.base_steps[1];
-    unsigned phase[2] = {0u, 0u};
+    st.send_step = base_steps[0];
+    st.recv_step = base_steps[1];
 
     const T* in = static_cast<const T*>(a.input);
     T* out = static_cast<T*>(a.output);
@@ -283,58 +262,42 @@ __global__ void __launch_bounds__(kRingThreads) ring_kernel(const __grid_constan
     ring::Part part = ring::channel_part(a.count / kVecElems, c, a.nchannels);
     part.offset *= kVecElems;
     part.count *= kVecElems;
+    if (c == a.nchannels - 1) part.count += a.count % kVecElems;  // the rest of a ragged all_reduce
     bool ok = true;
     auto mod = [n](int v) { return ((v % n) + n) % n; };
 
-    if (a.collective == (int)Collective::AllReduce) {
-        const u64 cs = ring::all_reduce_chunk_elems(part.count, n, sizeof(T), a.step_elems);
-        for (u64 w0 = 0; ok && cs > 0 && w0 < part.count; w0 += cs * (u64)n) {
-            auto chunk = [&](int k, u64* off, u64* len) {
-                *off = w0 + (u64)k * cs;
-                *len = ring::clamp_elems(cs, part.count, *off);
-                *off += part.offset;
-            };
-            u64 off, len;
-            chunk(mod(r - 1), &off, &len);
-            ok = run_chunk<T, Op, kWide>(a, st, sm, phase, kLocal | kSend, in + off, nullptr, len);
-            for (int j = 2; ok && j < n; ++j) {
-                chunk(mod(r - j), &off, &len);
-                ok = run_chunk<T, Op, kWide>(a, st, sm, phase, kRecv | kLocal | kSend, in + off, nullptr, len);
+    // One schedule for the three collectives, so that the slice code exists once (four copies with their flags
+    // known at compile time spilled registers): windows of the part, in each of them `steps` chunks.
+    const bool reduces = a.collective != (int)Collective::AllGather, scatters = a.collective == (int)Collective::ReduceScatter;
+    const bool both = reduces && !scatters;  // all_reduce: n chunks per window, reduced on the way round and then passed on
+    const u64 cs = both ? ring::all_reduce_chunk_elems(part.count, n, sizeof(T), a.step_elems)
+                        : ring::block_chunk_elems(part.count, sizeof(T), a.step_elems);
+    const u64 window = both ? cs * (u64)n : cs;
+    const int steps = both ? 2 * n - 1 : n;
+    for (u64 w0 = 0; ok && cs > 0 && w0 < part.count; w0 += window) {
+#pragma unroll 1
+        for (int j = 1; ok && j <= steps; ++j) {
+            unsigned flags;
+            if (reduces) {
+                if (j == 1) flags = kLocal | kSend;
+                else if (j < n) flags = kRecv | kLocal | kSend;
+                else if (scatters) flags = kRecv | kLocal | kCopyOut | kScale;  // own block
+                else if (j == n) flags = kRecv | kLocal | kSend | kCopyOut | kScale;  // pivot: final value → output and onwards
+                else flags = j < steps ? kRecv | kSend | kCopyOut : kRecv | kCopyOut;
+            } else {
+                flags = j == 1 ? kLocal | kSend | kCopyOut : (j < n ? kRecv | kSend | kCopyOut : kRecv | kCopyOut);
             }
-            if (ok) {  // pivot: final value → output and onwards
-                chunk(r, &off, &len);
-                ok = run_chunk<T, Op, kWide>(a, st, sm, phase, kRecv | kLocal | kSend | kCopyOut | kScale, in + off, out + off, len);
+            const int k = mod(reduces ? r - j : r + 1 - j);  // chunk (all_reduce) or block
+            u64 at = w0, in_at, out_at;
+            if (both) {
+                at += (u64)k * cs;
+                in_at = out_at = part.offset + at;
+            } else {
+                const u64 here = part.offset + w0, block = (u64)k * a.count + here;
+                in_at = scatters ? block : here;
+                out_at = scatters ? here : block;
             }
-            for (int j = 1; ok && j < n - 1; ++j) {
-                chunk(mod(r - j), &off, &len);
-                ok = run_chunk<T, Op, kWide>(a, st, sm, phase, kRecv | kSend | kCopyOut, nullptr, out + off, len);
-            }
-            if (ok) {
-                chunk(mod(r + 1), &off, &len);
-                ok = run_chunk<T, Op, kWide>(a, st, sm, phase, kRecv | kCopyOut, nullptr, out + off, len);
-            }
-        }
-    } else if (a.collective == (int)Collective::ReduceScatter) {
-        const u64 cs = ring::block_chunk_elems(part.count, sizeof(T), a.step_elems);
-        for (u64 w0 = 0; ok && cs > 0 && w0 < part.count; w0 += cs) {
-            const u64 len = ring::clamp_elems(cs, part.count, w0);
-            auto blk = [&](int k) { return (u64)k * a.count + part.offset + w0; };
-            ok = run_chunk<T, Op, kWide>(a, st, sm, phase, kLocal | kSend, in + blk(mod(r - 1)), nullptr, len);
-            for (int j = 2; ok && j < n; ++j)
-                ok = run_chunk<T, Op, kWide>(a, st, sm, phase, kRecv | kLocal | kSend, in + blk(mod(r - j)), nullptr, len);
-            if (ok)
-                ok = run_chunk<T, Op, kWide>(a, st, sm, phase, kRecv | kLocal | kCopyOut | kScale, in + blk(r),
-                                             out + part.offset + w0, len);
-        }
-    } else {  // AllGather
-        const u64 cs = ring::block_chunk_elems(part.count, sizeof(T), a.step_elems);
-        for (u64 w0 = 0; ok && cs > 0 && w0 < part.count; w0 += cs) {
-            const u64 len = ring::clamp_elems(cs, part.count, w0);
-            auto blk = [&](int k) { return (u64)k * a.count + part.offset + w0; };
-            ok = run_chunk<T, Op, kWide>(a, st, sm, phase, kLocal | kSend | kCopyOut, in + part.offset + w0, out + blk(r), len);
-            for (int j = 1; ok && j < n - 1; ++j)
-                ok = run_chunk<T, Op, kWide>(a, st, sm, phase, kRecv | kSend | kCopyOut, nullptr, out + blk(mod(r - j)), len);
-            if (ok) ok = run_chunk<T, Op, kWide>(a, st, sm, phase, kRecv | kCopyOut, nullptr, out + blk(mod(r + 1)), len);
+            ok = run_chunk<T, Op, kWide>(a, st, flags, in + in_at, out + out_at, ring::clamp_elems(cs, part.count, at));
         }
     }
 
@@ -348,25 +311,17 @@ __global__ void __launch_bounds__(kRingThreads) ring_kernel(const __grid_constan
 
 template <typename T, typename Op, bool kWide>
 cudaError_t launch_ring_t(const RingArgs* args, const RingLaunch& cfg) {
-    const size_t smem = sizeof(Shared);
     dim3 grid(args[0].nchannels, cfg.loop_ranks > 0 ? cfg.loop_ranks : 1, 1);
     dim3 block(kRingThreads, 1, 1);
     if (cfg.loop_ranks > 0) {
         if (cfg.loop_ranks > kMaxRanks) return cudaErrorInvalidValue;
         LoopPack<RingArgs> pack;
         for (int i = 0; i < cfg.loop_ranks; ++i) pack.r[i] = args[i];
-        auto kernel = ring_kernel<T, Op, kWide, LoopPack<RingArgs>>;
-        cudaError_t st = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (st != cudaSuccess) return st;
         void* params[] = {&pack};
-        return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), grid, block, params, smem, cfg.stream);
+        return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(ring_kernel<T, Op, kWide, LoopPack<RingArgs>>), grid, block, params,
+                                           0, cfg.stream);
     }
-    auto kernel = ring_kernel<T, Op, kWide, RingArgs>;
-    // The attribute belongs to the current device's copy of the function: set it on every launch
-    // (a process may drive several GPUs).
-    cudaError_t st = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (st != cudaSuccess) return st;
-    kernel<<<grid, block, smem, cfg.stream>>>(args[0]);
+    ring_kernel<T, Op, kWide, RingArgs><<<grid, block, 0, cfg.stream>>>(args[0]);
     return cudaGetLastError();
 }
 

@@ -65,7 +65,7 @@ struct RingArgs {
     int nranks;
     int nchannels;
     int collective;  // b200ccl::Collective
-    int wide;        // 1: 16-byte accesses and TMA staging of local input are allowed
+    int wide;        // 1: 16-byte accesses (buffers, and every block of reduce_scatter and all_gather, 16-byte aligned)
 };
 
 }  // namespace b200ccl::dev
