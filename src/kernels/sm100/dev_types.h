@@ -100,6 +100,7 @@ struct CollArgs {
     int nranks;
     int shard_mode;     // ShardMode
     int store_all;      // 1 → store the reduced pack into every rank's `out`; 0 → own only
+    unsigned int tail;  // Whole/Split, unstaged: elements behind the last pack, too few for another one
 };
 
 // AllGather moves bytes only.

@@ -207,6 +207,20 @@ reduce_kernel(const __grid_constant__ ParamT param) {
         }
     }
 
+    // 3b. The elements of a ragged message that fill no pack, one per thread of CTA 0, in the last rank's shard.
+    if constexpr (!kNvls) {
+        if (a.tail != 0 && blockIdx.x == 0 && threadIdx.x < a.tail && (mode == kShardWhole || rank == n - 1)) {
+            const u64 e = a.len * kElems + threadIdx.x;
+            float acc = Elem<T>::to_f(Narrow<T>::load(a.in[0], e));
+            for (int p = 1; p < n; ++p) acc = Op::apply(acc, Elem<T>::to_f(Narrow<T>::load(a.in[p], e)));
+            if (a.scale != 1.0f) acc *= a.scale;
+            const T v = Elem<T>::from_f(acc);
+            if (a.store_all)
+                for (int q = 0; q < n; ++q) static_cast<T*>(a.out[q])[e] = v;
+            else static_cast<T*>(a.out[rank])[e] = v;
+        }
+    }
+
     // 4. Every rank has finished reading inputs and its stores to peers are visible.
     ++epoch;
     if (!cta_barrier_all_ranks<kAllRanksHere<ParamT>>(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 2u)) return;
