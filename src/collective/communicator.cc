@@ -157,7 +157,6 @@ private:
     sched::Tuning tuning_;
     sched::ProcessLayout layout_;
     sched::RingTransportPlan ring_plan_;
-    topo::TopologyReport topo_;
     std::vector<Local> local_;
     std::unique_ptr<mem::SymmetricAllocator> alloc_;
     std::unique_ptr<mem::SymmetricRegion> ctrl_;
@@ -251,7 +250,6 @@ Communicator::Impl::Impl(const CommunicatorConfig& config, Bootstrap* bootstrap)
         local_[i].device = loopback_ ? config.devices[0] : config.devices[i];
     }
 
-    topo_ = topo::discover(config.devices);
     resolve_transport();
     if (channels_ <= 0) {
         // One ring CTA moves about 8 GB/s over NVLink, so peer-memory rings want many channels (8 GPUs, 64 MiB:
@@ -298,7 +296,8 @@ Communicator::Impl::Impl(const CommunicatorConfig& config, Bootstrap* bootstrap)
         ctrl_ = alloc_->allocate(sizeof(dev::ControlBlock), "control");
         // Allocation is collective (and clears memory, which synchronises the device), so what the
         // small-message path needs exists before the first call rather than inside it.
-        if (nranks_ >= 2) ll_area_ = alloc_->allocate(kernels::ll_area_bytes(nranks_), "low-latency slots");
+        // Emulated ranks take that path only where the communicator was created for it.
+        if (nranks_ >= 2 && (!loopback_ || forced_algo_ == Algo::LowLatency)) ll_area_ = alloc_->allocate(kernels::ll_area_bytes(nranks_), "low-latency slots");
         // Between processes any call may need the staging arena (ordinary tensors of another process
         // cannot be addressed), and which call does is a per-rank fact: allocating it on first use
         // would leave a rank that needs it waiting, inside a collective allocation, for ranks that do not.
@@ -1245,7 +1244,11 @@ std::string Communicator::Impl::describe() const {
     else
         os << "memory: mapped host memory only (shm)\n";
     for (const auto& l : local_) os << "rank " << l.grank << ": device " << l.device << "\n";
-    os << topo_.text;
+    // Asked for here and not kept: bringing NVML up takes about 15 ms, most of what creating a communicator took.
+    std::vector<int> devices;
+    for (const auto& l : local_)
+        if (std::find(devices.begin(), devices.end(), l.device) == devices.end()) devices.push_back(l.device);
+    os << topo::discover(devices).text;
     os << ring_plan_.describe();
     return os.str();
 }
