@@ -6,7 +6,11 @@
 // polled with ld.acquire.sys; counters persist from launch to launch.
 //
 // Bound by the chain of slices: a rank can only work on what its neighbour has posted, so what counts is
-// the time from one post to the next. Inside a slice no barrier is left: every thread keeps kBatch vectors
+// the time from one post to the next. Where all ranks run in one launch over device memory, two groups of eight
+// warps take the slices in turn, so that one slice is moved while the other waits for its neighbour, for its loads
+// or for its release; shared memory hands the order of the posts from group to group (4 ranks: 64 KiB 37.6 -> 27.6
+// us, 16 MiB 65.8 -> 59.6 us). FIFOs in host memory keep one group: there each release waits for the other group's
+// writes over PCIe as well (4 ranks, 4 MiB: 724 us, 879 us with two). Inside a slice there is no barrier: every thread keeps kBatch vectors
 // of the FIFO and of the local input in flight in registers, and the first batch of the local input is
 // loaded BEFORE the wait for the neighbour. (The local input used to be staged by TMA through 32 KiB tiles
 // of shared memory, with three block barriers and four dependent FIFO loads per thread and tile.)
@@ -31,8 +35,8 @@ namespace {
 using u64 = unsigned long long;
 
 constexpr int kRingThreads = 512;
-constexpr int kBatch = 8;  // vectors in flight per thread and source: a 64 KiB slice at once
-constexpr unsigned kCreditThread = 64, kPostThread = 96;  // they publish; threads 0 and 32 poll
+constexpr int kBatch = 8;  // vectors in flight per thread and source
+constexpr unsigned kCreditThread = 64, kPostThread = 96;  // of a group: they publish; threads 0 and 32 poll
 
 enum SliceFlags : unsigned {
     kRecv = 1u,        // take the slice from the incoming FIFO
@@ -49,25 +53,82 @@ __device__ __forceinline__ uint4 ld16_volatile(const uint4* p) {
     return v;
 }
 
+// What the groups of a CTA share: up to which step each side has been published, and whether a group gave up.
+struct Turns {
+    u64 posted[2];  // 0: slices sent, 1: credits returned
+    unsigned failed;
+};
+
 struct ChannelState {
     RingChannel ch;
+    Turns* turns;
+    int group;
+    unsigned tid;      // within the group
+    unsigned slices;   // non-empty slices so far, of both groups
     bool one_gpu;  // both neighbours run in this launch: their counters need GPU scope only
     u64 send_step;
     u64 recv_step;
 };
 
+template <int kGroups>
+__device__ __forceinline__ void group_sync(int group) {
+    if constexpr (kGroups == 1) __syncthreads();
+    else asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(kRingThreads / kGroups) : "memory");
+}
+// Barrier of the group; true when `pred` holds in every thread.
+template <int kGroups>
+__device__ __forceinline__ bool group_sync_and(int group, bool pred) {
+    if constexpr (kGroups == 1) return __syncthreads_and(pred ? 1 : 0) != 0;
+    unsigned r;
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.and.pred q, %2, %3, p;\n selp.u32 %0, 1, 0, q;\n}\n"
+        : "=r"(r) : "r"(pred ? 1u : 0u), "r"(group + 1), "n"(kRingThreads / kGroups) : "memory");
+    return r != 0;
+}
+
+__device__ __forceinline__ u64 ld_acquire_turn(const u64* p) {
+    u64 v;
+    asm volatile("ld.acquire.cta.shared::cta.u64 %0, [%1];" : "=l"(v) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
+    return v;
+}
+template <int kGroups>
+__device__ __forceinline__ void st_release_turn(u64* p, u64 v) {
+    if constexpr (kGroups > 1)
+        asm volatile("st.release.cta.shared::cta.u64 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(p)), "l"(v) : "memory");
+}
+
+// Waits until every slice before `step` has been published; false when the other group gave up. The group that hands
+// over has released its slice before, so this group's release covers both.
+template <int kGroups>
+__device__ __forceinline__ bool wait_turn(const RingArgs& a, Turns& turns, int side, u64 step) {
+    if constexpr (kGroups == 1) return true;
+    u64 t0 = 0, waited = 0;
+    for (unsigned polls = 0;; ++polls) {
+        if (ld_acquire_turn(&turns.posted[side]) >= step) return true;
+        if (*static_cast<volatile unsigned*>(&turns.failed) != 0u) return false;
+        if ((polls & 0xffffu) == 0xffffu) {  // the other group's own waits end after timeout_ns
+            if (t0 == 0) t0 = global_timer_ns();
+            else if ((waited = global_timer_ns() - t0) > 2 * a.timeout_ns) break;
+        }
+    }
+    report_failure(a.status, a.own_ctrl, nullptr, 0, kStatusTimeout, (unsigned)a.rank, 12u, step, waited);
+    *static_cast<volatile unsigned*>(&turns.failed) = 1u;
+    return false;
+}
+
 // Waits of the two flow-control threads; the outcome is shared through smem.
+template <int kGroups>
 __device__ __forceinline__ bool wait_flags(const RingArgs& a, ChannelState& st, unsigned flags, u64& t_wait_recv,
                                            u64& t_wait_send) {
     int ok = 1;
-    if ((flags & kRecv) && threadIdx.x == 0) {
+    if ((flags & kRecv) && st.tid == 0) {
         const u64 t0 = st.ch.stats ? global_timer_ns() : 0;
         ok = wait_at_least(st.ch.recv_tail, st.recv_step + ring::kSliceSteps, a.own_ctrl, a.timeout_ns, a.status, nullptr,
                            0, (unsigned)((a.rank + a.nranks - 1) % a.nranks), 10u, st.ch.abort_word) ? 1 : 0;
         if (ok && st.ch.abort_word && ld_volatile_u32(st.ch.abort_word) != 0u) ok = 0;
         if (st.ch.stats) t_wait_recv += global_timer_ns() - t0;
     }
-    if ((flags & kSend) && threadIdx.x == 32) {
+    if ((flags & kSend) && st.tid == 32) {
         const u64 t0 = st.ch.stats ? global_timer_ns() : 0;
         // credit: head + kFifoSteps >= step + kSliceSteps
         const u64 want = st.send_step + ring::kSliceSteps >= (u64)ring::kFifoSteps
@@ -77,14 +138,24 @@ __device__ __forceinline__ bool wait_flags(const RingArgs& a, ChannelState& st, 
         if (ok && st.ch.abort_word && ld_volatile_u32(st.ch.abort_word) != 0u) ok = 0;
         if (st.ch.stats) t_wait_send += global_timer_ns() - t0;
     }
-    return __syncthreads_and(ok) != 0;
+    if constexpr (kGroups > 1) {
+        if (*static_cast<volatile unsigned*>(&st.turns->failed) != 0u) ok = 0;
+        if (!ok) *static_cast<volatile unsigned*>(&st.turns->failed) = 1u;
+    }
+    return group_sync_and<kGroups>(st.group, ok != 0);
 }
 
 // One slice: wait, move/combine `n` elements, publish. Returns false when a wait gave up.
-template <typename T, typename Op, bool kWide>
+template <typename T, typename Op, bool kWide, int kGroups>
 __device__ bool run_slice(const RingArgs& a, ChannelState& st, unsigned flags, const T* local_in, T* local_out, u64 n) {
+    constexpr int kGroupThreads = kRingThreads / kGroups;
     if (n == 0) {  // empty slice: neither side waits, posts or advances
-        if (st.ch.stats && threadIdx.x == 0) atomicAdd(&st.ch.stats->empty_slices, 1ull);
+        if (st.ch.stats && st.tid == 0) atomicAdd(&st.ch.stats->empty_slices, 1ull);
+        return true;
+    }
+    if (kGroups > 1 && (int)(st.slices++ % kGroups) != st.group) {  // the other group's
+        if (flags & kRecv) st.recv_step += ring::kSliceSteps;
+        if (flags & kSend) st.send_step += ring::kSliceSteps;
         return true;
     }
     const bool recv = flags & kRecv, send = flags & kSend, local = flags & kLocal, copy_out = flags & kCopyOut;
@@ -125,24 +196,26 @@ __device__ bool run_slice(const RingArgs& a, ChannelState& st, unsigned flags, c
         auto load_local = [&](u64 v0) {
 #pragma unroll
             for (int u = 0; u < kBatch; ++u)
-                if (v0 + u * kRingThreads < nvec) loc[u] = ld16_stream(in_v + v0 + u * kRingThreads);
+                if (v0 + u * kGroupThreads < nvec) loc[u] = ld16_stream(in_v + v0 + u * kGroupThreads);
         };
-        if (local) load_local(threadIdx.x);
-        ok = wait_flags(a, st, flags, t_wait_recv, t_wait_send);
+        if (local) load_local(st.tid);
+        ok = wait_flags<kGroups>(a, st, flags, t_wait_recv, t_wait_send);
         if (!ok) return false;
-        if (st.ch.stats && threadIdx.x == 0) t0 = global_timer_ns();
-        early = recv && !st.one_gpu && nvec <= (u64)kRingThreads && tail == 0;
+        if (st.ch.stats && st.tid == 0) t0 = global_timer_ns();
+        early = recv && !st.one_gpu && nvec <= (u64)kGroupThreads && tail == 0;
         uint4 pre = make_uint4(0, 0, 0, 0);
         if (early) {
             int sink = 0;
-            if (threadIdx.x < nvec) {
-                pre = ld16_volatile(fifo_v + threadIdx.x);
+            if (st.tid < nvec) {
+                pre = ld16_volatile(fifo_v + st.tid);
                 sink = (pre.x ^ pre.y ^ pre.z ^ pre.w) == 0x5bd1e995u;  // a use of the value: the barrier below then follows the load's arrival
             }
-            (void)__syncthreads_or(sink);  // every thread holds its part of the slot
-            if (threadIdx.x == 0)
-                st.one_gpu ? st_release_gpu(st.ch.recv_head, st.recv_step + ring::kSliceSteps)
-                           : st_release_sys(st.ch.recv_head, st.recv_step + ring::kSliceSteps);
+            // The group's __syncthreads_or(): every thread holds its part of the slot.
+            (void)group_sync_and<kGroups>(st.group, sink == 0);
+            if (st.tid == kCreditThread && wait_turn<kGroups>(a, *st.turns, 1, st.recv_step)) {
+                st_release_sys(st.ch.recv_head, st.recv_step + ring::kSliceSteps);
+                st_release_turn<kGroups>(&st.turns->posted[1], st.recv_step + ring::kSliceSteps);
+            }
         }
         auto combine_store = [&](u64 v, const uint4& got, const uint4& mine) {
             uint4 out = recv ? got : mine;
@@ -164,63 +237,66 @@ __device__ bool run_slice(const RingArgs& a, ChannelState& st, unsigned flags, c
             if (send) st16(reinterpret_cast<uint4*>(fifo_out) + v, out);
         };
         if (early) {
-            if (threadIdx.x < nvec) combine_store(threadIdx.x, pre, loc[0]);
+            if (st.tid < nvec) combine_store(st.tid, pre, loc[0]);
         } else {
-            for (u64 v0 = threadIdx.x; v0 < nvec; v0 += kBatch * kRingThreads) {
+            for (u64 v0 = st.tid; v0 < nvec; v0 += kBatch * kGroupThreads) {
                 uint4 got[kBatch];
                 if (recv) {
 #pragma unroll
                     for (int u = 0; u < kBatch; ++u)
-                        if (v0 + u * kRingThreads < nvec) got[u] = ld16_volatile(fifo_v + v0 + u * kRingThreads);
+                        if (v0 + u * kGroupThreads < nvec) got[u] = ld16_volatile(fifo_v + v0 + u * kGroupThreads);
                 }
-                if (local && v0 != threadIdx.x) load_local(v0);
+                if (local && v0 != st.tid) load_local(v0);
 #pragma unroll
                 for (int u = 0; u < kBatch; ++u)
-                    if (v0 + u * kRingThreads < nvec) combine_store(v0 + u * kRingThreads, got[u], loc[u]);
+                    if (v0 + u * kGroupThreads < nvec) combine_store(v0 + u * kGroupThreads, got[u], loc[u]);
             }
-            if (threadIdx.x < tail) combine_element(nvec * kElems + threadIdx.x);
+            if (st.tid < tail) combine_element(nvec * kElems + st.tid);
         }
     } else {
-        ok = wait_flags(a, st, flags, t_wait_recv, t_wait_send);
+        ok = wait_flags<kGroups>(a, st, flags, t_wait_recv, t_wait_send);
         if (!ok) return false;
-        if (st.ch.stats && threadIdx.x == 0) t0 = global_timer_ns();
-        for (u64 i = threadIdx.x; i < n; i += kRingThreads) combine_element(i);
+        if (st.ch.stats && st.tid == 0) t0 = global_timer_ns();
+        for (u64 i = st.tid; i < n; i += kGroupThreads) combine_element(i);
     }
 
-    // Publish: all data stores of the CTA happen-before the counters (bar.sync, then release). Two warps that do
-    // not poll do it, so that the waits of the next slice begin while the releases are on their way.
-    __syncthreads();
+    // Publish: all data stores of the group happen-before the counters (its __syncthreads(), then release), slice by
+    // slice in order. Two warps that do not poll do it.
+    group_sync<kGroups>(st.group);
     u64 t1 = 0;
-    if (st.ch.stats && threadIdx.x == 0) t1 = global_timer_ns();
+    if (st.ch.stats && st.tid == 0) t1 = global_timer_ns();
     if (recv) {
-        if (!early && threadIdx.x == kCreditThread)
+        if (!early && st.tid == kCreditThread && wait_turn<kGroups>(a, *st.turns, 1, st.recv_step)) {
             st.one_gpu ? st_release_gpu(st.ch.recv_head, st.recv_step + ring::kSliceSteps)
                        : st_release_sys(st.ch.recv_head, st.recv_step + ring::kSliceSteps);
+            st_release_turn<kGroups>(&st.turns->posted[1], st.recv_step + ring::kSliceSteps);
+        }
         st.recv_step += ring::kSliceSteps;
     }
     if (send) {
-        if (threadIdx.x == kPostThread) {
+        if (st.tid == kPostThread && wait_turn<kGroups>(a, *st.turns, 0, st.send_step)) {
             if (st.ch.send_sizes) {
                 st.ch.send_sizes[st.send_step % ring::kFifoSteps] = (unsigned)(n * sizeof(T));
             }
             st.one_gpu ? st_release_gpu(st.ch.send_tail, st.send_step + ring::kSliceSteps)
                        : st_release_sys(st.ch.send_tail, st.send_step + ring::kSliceSteps);
+            st_release_turn<kGroups>(&st.turns->posted[0], st.send_step + ring::kSliceSteps);
         }
         st.send_step += ring::kSliceSteps;
     }
-    if (st.ch.stats && threadIdx.x == 0) {
+    if (st.ch.stats && st.tid == 0) {
         RingTurnaroundStats* s = st.ch.stats;
         atomicAdd(&s->wait_recv_ns, t_wait_recv);
         atomicAdd(&s->compute_ns, t1 - t0);
         atomicAdd(&s->post_ns, global_timer_ns() - t1);
         atomicAdd(&s->slices, 1ull);
     }
-    if (st.ch.stats && threadIdx.x == 32 && t_wait_send) atomicAdd(&st.ch.stats->wait_send_ns, t_wait_send);
+    if (st.ch.stats && st.tid == 32 && t_wait_send) atomicAdd(&st.ch.stats->wait_send_ns, t_wait_send);
     return true;
 }
 
 // A chunk travels as kSlicesPerChunk slices.
-template <typename T, typename Op, bool kWide>
+template <typename T, typename Op, bool kWide, int kGroups>
 __device__ __forceinline__ bool run_chunk(const RingArgs& a, ChannelState& st, unsigned flags, const T* local_in,
                                           T* local_out, u64 n) {
     const u64 sl = ring::slice_elems(n, sizeof(T), a.step_elems);
@@ -228,14 +304,14 @@ __device__ __forceinline__ bool run_chunk(const RingArgs& a, ChannelState& st, u
     for (int s = 0; s < ring::kSlicesPerChunk; ++s) {
         const u64 off = (u64)s * sl;
         const u64 sn = ring::clamp_elems(sl, n, off);
-        if (!run_slice<T, Op, kWide>(a, st, flags, local_in + off, local_out + off, sn)) return false;
+        if (!run_slice<T, Op, kWide, kGroups>(a, st, flags, local_in + off, local_out + off, sn)) return false;
     }
     return true;
 }
 
-template <typename T, typename Op, bool kWide, typename ParamT>
+template <typename T, typename Op, bool kWide, int kGroups, typename ParamT>
 __global__ void __launch_bounds__(kRingThreads, kWide ? 1 : 2) ring_kernel(const __grid_constant__ ParamT param) {
-    __shared__ u64 base_steps[2];
+    __shared__ Turns turns;
     const RingArgs* ap;
     if constexpr (sizeof(ParamT) == sizeof(RingArgs)) ap = reinterpret_cast<const RingArgs*>(&param);
     else ap = reinterpret_cast<const RingArgs*>(&param) + blockIdx.y;
@@ -248,12 +324,18 @@ __global__ void __launch_bounds__(kRingThreads, kWide ? 1 : 2) ring_kernel(const
     // Network edges name an abort word: a host thread is at their other end.
     st.one_gpu = sizeof(ParamT) != sizeof(RingArgs) && st.ch.abort_word == nullptr;
     if (threadIdx.x == 0) {
-        base_steps[0] = *st.ch.send_base;
-        base_steps[1] = *st.ch.recv_base;
+        turns.posted[0] = *st.ch.send_base;
+        turns.posted[1] = *st.ch.recv_base;
+        turns.failed = 0u;
     }
     __syncthreads();
-    st.send_step = base_steps[0];
-    st.recv_step = base_steps[1];
+    st.turns = &turns;
+    st.group = (int)(threadIdx.x / (kRingThreads / kGroups));
+    st.tid = threadIdx.x % (kRingThreads / kGroups);
+    st.slices = 0;
+    st.send_step = turns.posted[0];
+    st.recv_step = turns.posted[1];
+    __syncthreads();  // every thread has read them before a group moves them on
 
     const T* in = static_cast<const T*>(a.input);
     T* out = static_cast<T*>(a.output);
@@ -297,12 +379,13 @@ __global__ void __launch_bounds__(kRingThreads, kWide ? 1 : 2) ring_kernel(const
                 in_at = scatters ? block : here;
                 out_at = scatters ? here : block;
             }
-            ok = run_chunk<T, Op, kWide>(a, st, flags, in + in_at, out + out_at, ring::clamp_elems(cs, part.count, at));
+            ok = run_chunk<T, Op, kWide, kGroups>(a, st, flags, in + in_at, out + out_at, ring::clamp_elems(cs, part.count, at));
         }
     }
 
     // Progress persists only when the whole schedule ran (an aborted launch leaves the
     // communicator poisoned, as in the reference, kernel:1186-1188).
+    ok = __syncthreads_and(ok && turns.failed == 0u) != 0;
     if (ok && threadIdx.x == 0) {
         *st.ch.send_base = st.send_step;
         *st.ch.recv_base = st.recv_step;
@@ -318,10 +401,11 @@ cudaError_t launch_ring_t(const RingArgs* args, const RingLaunch& cfg) {
         LoopPack<RingArgs> pack;
         for (int i = 0; i < cfg.loop_ranks; ++i) pack.r[i] = args[i];
         void* params[] = {&pack};
-        return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(ring_kernel<T, Op, kWide, LoopPack<RingArgs>>), grid, block, params,
-                                           0, cfg.stream);
+        const void* kernel = cfg.device_fifos ? reinterpret_cast<const void*>(ring_kernel<T, Op, kWide, 2, LoopPack<RingArgs>>)
+                                              : reinterpret_cast<const void*>(ring_kernel<T, Op, kWide, 1, LoopPack<RingArgs>>);
+        return cudaLaunchCooperativeKernel(kernel, grid, block, params, 0, cfg.stream);
     }
-    ring_kernel<T, Op, kWide, RingArgs><<<grid, block, 0, cfg.stream>>>(args[0]);
+    ring_kernel<T, Op, kWide, 1, RingArgs><<<grid, block, 0, cfg.stream>>>(args[0]);
     return cudaGetLastError();
 }
 
