@@ -49,6 +49,7 @@ struct LocalArgs {
     unsigned char nranks;
     unsigned char outs;  // outputs that a segment writes: all of them, or (1) out[s] only
     unsigned char kind;  // Collective
+    unsigned char in_align;  // 16 or 32: what the inputs' addresses agree on
     // Segment s lies s * count elements into every input (reduce_scatter) or every output (all_gather), which reads in[s] only.
     __device__ __forceinline__ u64 in_step(unsigned elem) const { return kind == (int)Collective::ReduceScatter ? count * elem : 0; }
     __device__ __forceinline__ u64 out_step(unsigned elem) const { return kind == (int)Collective::AllGather ? count * elem : 0; }
@@ -95,13 +96,14 @@ __device__ __forceinline__ void reduce_one(const LocalArgs& a, unsigned seg, u64
     for (int q = 0; q < a.outs; ++q) reinterpret_cast<T*>(a.out[a.outs == 1 ? seg : q] + out_off)[e] = v;
 }
 
-// kPack 32: inputs and outputs are aligned alike. kPack 16: outputs may be aligned differently from inputs.
-template <typename T, typename Op, int N, int kPack, int kPerThread>
+// kShift false: inputs and outputs are all aligned alike, modulo 32. kShift true: the inputs are aligned alike modulo
+// 32 or (in_align 16) modulo 16, and so are the outputs, but differently.
+template <typename T, typename Op, int N, bool kShift, int kPerThread>
 __global__ void __launch_bounds__(kThreads, N <= 2 ? 4 : (N <= 4 ? 3 : 2)) local_kernel(const __grid_constant__ LocalArgs a) {
-    using P = std::conditional_t<kPack == 32, Wide32<T>, Wide<T>>;
-    using Raw = typename P::Raw;
-    constexpr int kElems = P::kElems;
-    constexpr int U = kPerThread / kPack;
+    using P = Wide32<T>;
+    constexpr int kElems = P::kElems, kHalf = kElems / 2;
+    constexpr int U = kPerThread / 32;
+    static_assert(N > 1 || !kShift);  // copies: local_shift_copy_kernel
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const bool scaled = a.scale != 1.0f;
@@ -109,8 +111,9 @@ __global__ void __launch_bounds__(kThreads, N <= 2 ? 4 : (N <= 4 ? 3 : 2)) local
         const unsigned seg = t / a.tiles, tile = t - seg * a.tiles;
         const u64 in_off = seg * a.in_step(sizeof(T)), out_off = seg * a.out_step(sizeof(T));
         const char* src0 = a.first_in(seg) + in_off;
-        const unsigned skew = (unsigned)(reinterpret_cast<std::uintptr_t>(src0) & (kPack - 1));
-        const unsigned before = ((unsigned)kPack - skew) & (kPack - 1);  // bytes until the inputs are aligned
+        const unsigned cut = kShift ? a.in_align : 32u;
+        const unsigned skew = (unsigned)(reinterpret_cast<std::uintptr_t>(src0) & (cut - 1u));
+        const unsigned before = (cut - skew) & (cut - 1u);  // bytes until the inputs are aligned
         const u64 head = before / sizeof(T) < a.count ? before / sizeof(T) : a.count;
         const u64 packs = (a.count - head) / kElems;
         if (tile == 0) {
@@ -120,18 +123,23 @@ __global__ void __launch_bounds__(kThreads, N <= 2 ? 4 : (N <= 4 ? 3 : 2)) local
         }
         const u64 in_body = in_off + before, out_body = out_off + before;
         const u64 i0 = (u64)tile * (kThreads * U) + threadIdx.x;
-        Raw r[U][N];
+        const unsigned lane = threadIdx.x & 31u;
+        // Bytes by which the outputs are past the inputs' alignment.
+        const unsigned m = kShift ? (unsigned)(reinterpret_cast<std::uintptr_t>(a.out[a.outs == 1 ? seg : 0] + out_body) & 15u) : 0u;
+        auto body = [&](int p) { return (N == 1 ? src0 - in_off : a.in[p]) + in_body; };
+        Raw32 r[U][N];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            if (i0 + u * kThreads < packs) {
+            const u64 i = i0 + u * kThreads;
+            if (i < packs) {
 #pragma unroll
-                for (int p = 0; p < N; ++p) r[u][p] = P::load((N == 1 ? src0 - in_off : a.in[p]) + in_body, i0 + u * kThreads);
+                for (int p = 0; p < N; ++p) r[u][p] = kShift && cut == 16u ? P::load_user(body(p), i) : P::load(body(p), i);
             }
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const u64 i = i0 + u * kThreads;
-            Raw v = r[u][0];
+            Raw32 v = r[u][0];
             if constexpr (N > 1) {
                 float acc[kElems];
                 P::unpack(r[u][0], acc);
@@ -148,37 +156,101 @@ __global__ void __launch_bounds__(kThreads, N <= 2 ? 4 : (N <= 4 ? 3 : 2)) local
                 }
                 v = P::pack(acc);
             }
-            if constexpr (kPack == 32) {
+            if constexpr (!kShift) {
                 if (i < packs)
                     for (int q = 0; q < a.outs; ++q) P::store(a.out[a.outs == 1 ? seg : q] + out_body, i, v);
+            } else if (m == 0) {
+                if (i < packs)
+                    for (int q = 0; q < a.outs; ++q) P::store_user(a.out[a.outs == 1 ? seg : q] + out_body, i, v);
             } else {
-                const unsigned m = (unsigned)(reinterpret_cast<std::uintptr_t>(a.out[a.outs == 1 ? seg : 0] + out_body) & 15u);
-                if (m == 0) {
-                    if (i < packs)
-                        for (int q = 0; q < a.outs; ++q) P::store(a.out[a.outs == 1 ? seg : q] + out_body, i, v);
-                } else {
-                    // The aligned vector that starts s bytes into this lane's pack ends m bytes into the next lane's.
-                    const unsigned s = 16u - m, lane = threadIdx.x & 31u;
-                    uint4 next;
-                    next.x = __shfl_down_sync(0xffffffffu, v.x, 1);
-                    next.y = __shfl_down_sync(0xffffffffu, v.y, 1);
-                    next.z = __shfl_down_sync(0xffffffffu, v.z, 1);
-                    next.w = __shfl_down_sync(0xffffffffu, v.w, 1);
-                    if (i < packs) {
-                        const bool last = lane == 31u || i + 1 >= packs;
-                        const uint4 w = shift_pair(v, next, s);
-                        T elems[kElems];
-                        *reinterpret_cast<uint4*>(elems) = v;
-                        for (int q = 0; q < a.outs; ++q) {
-                            char* dst = a.out[a.outs == 1 ? seg : q] + out_body + i * 16ull;
-                            if (!last) st16(reinterpret_cast<uint4*>(dst + s), w);
-                            if (lane == 0u || last) {
+                // The aligned vectors start s bytes into each half of the lane's pack; the second one ends m bytes into the
+                // next lane's pack. The two ends of the warp are stored element by element. (With 16-byte packs, twice the
+                // shuffles and ends: reduce_scatter, 3 ranks, 22 MB blocks of odd length 51.0 us, now 42.0; aligned 40.1.)
+                const unsigned s = 16u - m;
+                uint4 next;
+                next.x = __shfl_down_sync(0xffffffffu, v.lo.x, 1);
+                next.y = __shfl_down_sync(0xffffffffu, v.lo.y, 1);
+                next.z = __shfl_down_sync(0xffffffffu, v.lo.z, 1);
+                next.w = __shfl_down_sync(0xffffffffu, v.lo.w, 1);
+                if (i < packs) {
+                    const bool first = lane == 0u, last = lane == 31u || i + 1 >= packs;
+                    const uint4 w0 = shift_pair(v.lo, v.hi, s), w1 = shift_pair(v.hi, next, s);
+                    T ends[kElems];
+                    *reinterpret_cast<uint4*>(ends) = v.lo;
+                    *reinterpret_cast<uint4*>(ends + kHalf) = v.hi;
+                    for (int q = 0; q < a.outs; ++q) {
+                        char* dst = a.out[a.outs == 1 ? seg : q] + out_body + i * 32ull;
+                        st16(reinterpret_cast<uint4*>(dst + s), w0);
+                        if (!last) st16(reinterpret_cast<uint4*>(dst + 16 + s), w1);
+                        if (first) {
 #pragma unroll
-                                for (int e = 0; e < kElems; ++e)
-                                    if (e * sizeof(T) < s ? lane == 0u : last) reinterpret_cast<T*>(dst)[e] = elems[e];
-                            }
+                            for (int e = 0; e < kHalf; ++e)
+                                if (e * sizeof(T) < s) reinterpret_cast<T*>(dst)[e] = ends[e];
+                        }
+                        if (last) {
+#pragma unroll
+                            for (int e = 0; e < kHalf; ++e)
+                                if (e * sizeof(T) >= s) reinterpret_cast<T*>(dst + 16)[e] = ends[kHalf + e];
                         }
                     }
+                }
+            }
+        }
+    }
+}
+
+// Copies whose outputs are aligned differently from their inputs. Stores are most of the traffic of an all_gather, so
+// a warp stores 512 contiguous bytes at a time: 16-byte packs, and lane 31 loads the pack behind the warp's last one
+// (6 ranks, 8 MB blocks of odd length: 56.0 us; 64.9 us when the warp's ends are stored element by element, 67.9 us
+// with 32-byte packs, whose two stores per lane touch every other 16 bytes).
+template <typename T>
+__global__ void __launch_bounds__(kThreads, 4) local_shift_copy_kernel(const __grid_constant__ LocalArgs a) {
+    constexpr int kElems = 16 / sizeof(T), U = kBytes / 16;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (unsigned t = blockIdx.x; t < a.tiles * a.segments; t += gridDim.x) {
+        const unsigned seg = t / a.tiles, tile = t - seg * a.tiles;
+        const u64 out_off = seg * a.out_step(sizeof(T));
+        const char* src0 = a.first_in(seg);
+        const unsigned before = (16u - (unsigned)(reinterpret_cast<std::uintptr_t>(src0) & 15u)) & 15u;
+        const u64 head = before / sizeof(T) < a.count ? before / sizeof(T) : a.count;
+        const u64 packs = (a.count - head) / kElems, tail0 = head + packs * kElems;
+        if (tile == 0)
+            for (u64 e = threadIdx.x; e < head + (a.count - tail0); e += kThreads)
+                reduce_one<T, OpAdd, 1>(a, seg, 0, out_off, e < head ? e : tail0 + (e - head));
+        const uint4* src = reinterpret_cast<const uint4*>(src0 + before);
+        const u64 out_body = out_off + before, i0 = (u64)tile * (kThreads * U) + threadIdx.x;
+        const unsigned lane = threadIdx.x & 31u;
+        const unsigned m = (unsigned)(reinterpret_cast<std::uintptr_t>(a.out[0] + out_body) & 15u), s = 16u - m;
+        uint4 v[U], beyond[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const u64 i = i0 + u * kThreads;
+            v[u] = beyond[u] = make_uint4(0, 0, 0, 0);
+            if (i < packs) v[u] = ld16_stream(src + i);
+            if (m != 0 && lane == 31u && i + 1 < packs) beyond[u] = ld16_stream(src + i + 1);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const u64 i = i0 + u * kThreads;
+            uint4 next;
+            next.x = __shfl_down_sync(0xffffffffu, v[u].x, 1);
+            next.y = __shfl_down_sync(0xffffffffu, v[u].y, 1);
+            next.z = __shfl_down_sync(0xffffffffu, v[u].z, 1);
+            next.w = __shfl_down_sync(0xffffffffu, v[u].w, 1);
+            if (lane == 31u) next = beyond[u];
+            if (i >= packs) continue;
+            const uint4 w = m == 0 ? v[u] : shift_pair(v[u], next, s);
+            const bool first = m != 0 && i == 0, last = m != 0 && i + 1 >= packs;
+            T ends[kElems];
+            *reinterpret_cast<uint4*>(ends) = v[u];
+            for (int q = 0; q < a.outs; ++q) {
+                char* dst = a.out[q] + out_body + i * 16ull;
+                if (!last) st16(reinterpret_cast<uint4*>(m == 0 ? dst : dst + s), w);
+                if (first || last) {
+#pragma unroll
+                    for (int e = 0; e < kElems; ++e)
+                        if (e * sizeof(T) < s ? first : last) reinterpret_cast<T*>(dst)[e] = ends[e];
                 }
             }
         }
@@ -201,12 +273,12 @@ __global__ void __launch_bounds__(kThreads) local_scalar_kernel(const __grid_con
 
 struct Plan {
     LocalArgs args;
-    int pack = 0;  // 32, 16 or 0 (element by element)
+    enum { kElements, kAlike, kShifted } how = kElements;
     int max_ctas = 0;  // 0: one CTA per tile
     cudaStream_t stream = nullptr;
 };
 
-cudaError_t start(void (*kernel)(LocalArgs), const Plan& p, u64 work, LocalLaunch* made) {
+cudaError_t start(void (*kernel)(LocalArgs), const Plan& p, u64 work, int elem_bytes, LocalLaunch* made) {
     const u64 grid = p.max_ctas > 0 ? std::min<u64>(work, (u64)p.max_ctas) : work;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3((unsigned)grid, 1, 1);
@@ -219,29 +291,26 @@ cudaError_t start(void (*kernel)(LocalArgs), const Plan& p, u64 work, LocalLaunc
     config.numAttrs = 1;
     made->grid = (int)grid;
     made->block = kThreads;
-    made->pack_bytes = p.pack;
+    made->pack_bytes = p.how == Plan::kElements ? elem_bytes : 32;
     return cudaLaunchKernelEx(&config, kernel, p.args);
 }
 
-template <typename T, typename Op, int N, int kPack, int kPerThread = kBytes>
-cudaError_t start_packed(Plan& p, LocalLaunch* made) {
+template <typename T, int kPerThread = kBytes>
+cudaError_t start_tiles(void (*kernel)(LocalArgs), Plan& p, LocalLaunch* made) {
     constexpr u64 tile = (u64)kThreads * (kPerThread / sizeof(T));
     const u64 tiles = (p.args.count + tile - 1) / tile;
     if (tiles * p.args.segments > 0x7fffffffull) return cudaErrorInvalidValue;
     p.args.tiles = (unsigned)tiles;
-    return start(local_kernel<T, Op, N, kPack, kPerThread>, p, tiles * p.args.segments, made);
+    return start(kernel, p, tiles * p.args.segments, (int)sizeof(T), made);
 }
 
 template <typename T, typename Op>
 cudaError_t start_op(Plan& p, LocalLaunch* made) {
-    if (p.pack == 0) {
-        made->pack_bytes = (int)sizeof(T);
-        p.pack = (int)sizeof(T);
-        return start(local_scalar_kernel<T, Op>, p, std::min<u64>((p.args.count + kThreads - 1) / kThreads, 0x7fffffffull), made);
-    }
+    if (p.how == Plan::kElements)
+        return start(local_scalar_kernel<T, Op>, p, std::min<u64>((p.args.count + kThreads - 1) / kThreads, 0x7fffffffull), (int)sizeof(T), made);
     switch (p.args.nranks) {
 #define B2_LOCAL_N(n) \
-    case n: return p.pack == 32 ? start_packed<T, Op, n, 32>(p, made) : start_packed<T, Op, n, 16>(p, made);
+    case n: return start_tiles<T>(p.how == Plan::kAlike ? local_kernel<T, Op, n, false, kBytes> : local_kernel<T, Op, n, true, kBytes>, p, made);
         B2_LOCAL_N(2)
         B2_LOCAL_N(3)
         B2_LOCAL_N(4)
@@ -256,9 +325,9 @@ cudaError_t start_op(Plan& p, LocalLaunch* made) {
 
 // Copies: two-byte elements serve every type.
 cudaError_t start_copy(Plan& p, LocalLaunch* made) {
-    if (p.pack == 32 && p.args.nranks == 1) return start_packed<__half, OpAdd, 1, 32, kCopyBytes>(p, made);
-    if (p.pack == 32) return start_packed<__half, OpAdd, 1, 32>(p, made);
-    if (p.pack == 16) return start_packed<__half, OpAdd, 1, 16>(p, made);
+    if (p.how == Plan::kAlike && p.args.nranks == 1) return start_tiles<__half, kCopyBytes>(local_kernel<__half, OpAdd, 1, false, kCopyBytes>, p, made);
+    if (p.how == Plan::kAlike) return start_tiles<__half>(local_kernel<__half, OpAdd, 1, false, kBytes>, p, made);
+    if (p.how == Plan::kShifted) return start_tiles<__half>(local_shift_copy_kernel<__half>, p, made);
     return start_op<__half, OpAdd>(p, made);
 }
 
@@ -300,8 +369,9 @@ cudaError_t launch_local(const LocalCall& call, LocalLaunch* made) {
         out_bits |= reinterpret_cast<std::uintptr_t>(call.out[r]) ^ out0;
     }
     const std::uintptr_t steps = a.segments > 1 ? bytes : 0;
-    if (((in_bits | out_bits | (in0 ^ out0) | steps) & 31u) == 0) p.pack = 32;
-    else if (((in_bits | out_bits) & 15u) == 0) p.pack = 16;
+    if (((in_bits | out_bits | (in0 ^ out0) | steps) & 31u) == 0) p.how = Plan::kAlike;
+    else if (((in_bits | out_bits) & 15u) == 0) p.how = Plan::kShifted;
+    a.in_align = (in_bits & 31u) == 0 ? 32 : 16;
     p.max_ctas = call.max_ctas;
     p.stream = call.stream;
     if (copies) return start_copy(p, made);

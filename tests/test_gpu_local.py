@@ -36,10 +36,11 @@ def untouched(raw, views):
 def test_one_device_collectives_at_every_edge(ranks, dtype):
     comm = nn.Communicator(devices=[0], loopback_ranks=ranks, wait_timeout_ms=2000)
     try:
-        same, apart = [1] * ranks, [r % 3 for r in range(ranks)]
+        half = 16 // torch.empty(0, dtype=dtype).element_size()  # 16 bytes: aligned alike modulo 16 only
+        same, apart, halves = [1] * ranks, [r % 3 for r in range(ranks)], [half * (r % 2) + 1 for r in range(ranks)]
         for k, count in enumerate(COUNTS):
             op = ["sum", "avg", "max", "min"][k % 4]
-            for shifts_in, shifts_out in (([0] * ranks, [0] * ranks), (same, same), ([0] * ranks, same), (same, [0] * ranks), (apart, apart)):
+            for shifts_in, shifts_out in (([0] * ranks, [0] * ranks), (same, same), ([0] * ranks, same), (same, [0] * ranks), (apart, apart), (halves, [0] * ranks)):
                 _, ins = buffers(ranks, count, dtype, shifts_in, 100 + k)
                 raw, outs = buffers(ranks, count, dtype, shifts_out, 0)
                 comm.all_reduce(outs, ins, op=op)
