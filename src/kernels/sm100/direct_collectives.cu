@@ -62,7 +62,7 @@ __device__ __forceinline__ void copy_stripes(void* dst, u64 dst0, const void* sr
 // Packs in flight per thread and peer: fewer ranks, or narrower packs, leave room for more.
 template <int N, int kPackBytes>
 struct UnrollFor {
-    static constexpr int k16 = N == 0 ? 1 : (N >= 8 ? 1 : (N >= 4 ? 2 : (N >= 2 ? 4 : 8)));
+    static constexpr int k16 = N == 0 ? 1 : (N >= 8 ? 1 : (N >= 4 ? 2 : 4));
     static constexpr int value = kPackBytes == 32 ? (k16 > 1 ? k16 / 2 : 1) : k16;
 };
 
@@ -334,7 +334,6 @@ cudaError_t launch_reduce_n(int nranks, const ParamT& param, const LaunchConfig&
         return launch(reduce_kernel<T, Op, 0, PackT, false, ParamT>, param, cfg);
     } else {
         switch (nranks) {
-            case 1: return launch(reduce_kernel<T, Op, 1, PackT, false, ParamT>, param, cfg);
             case 2: return launch(reduce_kernel<T, Op, 2, PackT, false, ParamT>, param, cfg);
             case 4: return launch(reduce_kernel<T, Op, 4, PackT, false, ParamT>, param, cfg);
             case 8: return launch(reduce_kernel<T, Op, 8, PackT, false, ParamT>, param, cfg);
