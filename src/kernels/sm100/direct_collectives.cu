@@ -121,7 +121,7 @@ reduce_kernel(const __grid_constant__ ParamT param) {
 
     // 2. Every rank's input is ready (and every rank's previous use of `out` is over).
     ++epoch;
-    if (!cta_barrier_all_ranks<kAllRanksHere<ParamT>>(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 1u, a.plan_hash)) return;
+    if (!cta_barrier_all_ranks<kAllRanksHere<ParamT>>(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 1u, a.plan_hash, a.user_in == nullptr)) return;
 
     // 3. Reduce the own shard.
     {
@@ -264,7 +264,7 @@ gather_kernel(const __grid_constant__ ParamT param) {
         for (u64 j = first; j < a.len; j += stripe) store(stage, j, load(a.user_in, j));
     }
     ++epoch;
-    if (!cta_barrier_all_ranks<kAllRanksHere<ParamT>>(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 1u, a.plan_hash)) return;
+    if (!cta_barrier_all_ranks<kAllRanksHere<ParamT>>(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 1u, a.plan_hash, a.user_in == nullptr)) return;
 
     if (a.mode == 0) {
         const u64 base = (u64)rank * a.out_stride;
