@@ -257,7 +257,32 @@ __device__ bool run_slice(const RingArgs& a, ChannelState& st, unsigned flags, c
         ok = wait_flags<kGroups>(a, st, flags, t_wait_recv, t_wait_send);
         if (!ok) return false;
         if (st.ch.stats && st.tid == 0) t0 = global_timer_ns();
-        for (u64 i = st.tid; i < n; i += kGroupThreads) combine_element(i);
+        // More than one element per thread: in batches as well (all_gather of 8 ranks, 500001 bf16: 229 us one by one, 134
+        // us; a few hundred elements are faster one by one).
+        if (n <= (u64)kGroupThreads) {
+            if (st.tid < n) combine_element(st.tid);
+        } else {
+            for (u64 i0 = st.tid; i0 < n; i0 += kBatch * kGroupThreads) {
+                T got[kBatch], mine[kBatch];
+#pragma unroll
+                for (int u = 0; u < kBatch; ++u) {
+                    const u64 i = i0 + u * kGroupThreads;
+                    if (recv && i < n) got[u] = Narrow<T>::load(fifo_in, i);
+                    if (local && i < n) mine[u] = local_in[i];
+                }
+#pragma unroll
+                for (int u = 0; u < kBatch; ++u) {
+                    const u64 i = i0 + u * kGroupThreads;
+                    if (i >= n) continue;
+                    float acc = Elem<T>::to_f(recv ? got[u] : mine[u]);
+                    if (recv && local) acc = Op::apply(Elem<T>::to_f(mine[u]), acc);
+                    if (scaled) acc *= a.scale;
+                    const T out = Elem<T>::from_f(acc);
+                    if (copy_out) local_out[i] = out;
+                    if (send) fifo_out[i] = out;
+                }
+            }
+        }
     }
 
     // Publish: all data stores of the group happen-before the counters (its __syncthreads(), then release), slice by
