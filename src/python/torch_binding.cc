@@ -2,8 +2,8 @@
 //
 // A call on eight ranks looks at sixteen tensors (type, place, layout, length, address) and eight
 // streams. Through Python attributes and ctypes a 4 KiB call took 40 us of host time, over ten times what
-// its kernel takes; with these checks native and one completion event instead of eight it takes 5 us
-// (one rank, 8 KiB: 9.3 -> 2.8 us). The module knows the C interface only by two addresses handed over in
+// its kernel takes; with these checks native and one completion event instead of eight it takes 3.3 us
+// (one rank, 8 KiB: 9.4 -> 2.9 us). The module knows the C interface only by two addresses handed over in
 // bind(), so whichever build of the library the process loaded is the one that runs.
 //
 // The reference library (nano-nccl) has no Python layer; its C++ calls
