@@ -27,3 +27,23 @@ def test_installed_package_is_usable_from_another_project(native_build, tmp_path
     env = dict(os.environ, LD_LIBRARY_PATH=str(prefix / "lib") + ":" + os.environ.get("LD_LIBRARY_PATH", ""))
     proc = subprocess.run([str(build / "app")], capture_output=True, text=True, env=env, timeout=120)
     assert proc.returncode == 0 and "consumer ok bf16 avg" in proc.stdout, proc.stdout + proc.stderr
+
+
+def test_a_python_without_torch_does_not_stop_the_build(tmp_path):
+    """The C++ library needs no Python: where none has torch the Python part is left out, unless it was asked for."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-m", "venv", "--without-pip", str(tmp_path / "bare")], check=True, capture_output=True)
+    env = dict(os.environ, PYTHONNOUSERSITE="1")
+    env.pop("PYTHONPATH", None)
+    env.setdefault("CUDACXX", "/usr/local/cuda/bin/nvcc")
+    configure = ["cmake", "-S", root, "-B", str(tmp_path / "build"), "-G", "Ninja", "-DB200CCL_BUILD_TESTS=OFF",
+                 f"-DPython3_EXECUTABLE={tmp_path / 'bare' / 'bin' / 'python'}"]
+    p = subprocess.run(configure, capture_output=True, text=True, env=env, timeout=300)
+    assert p.returncode == 0 and "Python communicator left out" in p.stdout, p.stdout + p.stderr
+    text = (tmp_path / "build" / "build.ninja").read_text()
+    assert "libb200ccl.so" in text and "_b200ccl_torch" not in text
+    p = subprocess.run([*configure, "-DB200CCL_BUILD_PYTHON=ON"], capture_output=True, text=True, env=env, timeout=300)
+    assert p.returncode != 0 and "B200CCL_BUILD_PYTHON=ON" in p.stderr, p.stdout + p.stderr
