@@ -6,6 +6,7 @@ The shared library is built in-tree (nano_nccl_b200/lib/) by ``__graft_entry__.b
 import ctypes
 import importlib.util
 import os
+import re
 
 _LIB = None
 _NATIVE = None
@@ -102,14 +103,22 @@ def load_native_calls():
     load() returns. Like the library it is built in-tree, and nothing stands in for it."""
     global _NATIVE
     if _NATIVE is None:
-        import torch  # noqa: F401  (the module needs torch's libraries in the process)
+        import torch  # the module needs torch's libraries in the process
 
         path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "_b200ccl_torch.so")
         if not os.path.exists(path):
             raise ImportError(f"{path} is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'`")
         spec = importlib.util.spec_from_file_location("_b200ccl_torch", path)
         module = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(module)
+        rebuild = "build it again with the torch that runs: `python -c 'import __graft_entry__ as g; g.build()'`"
+        try:
+            spec.loader.exec_module(module)
+        except ImportError as e:
+            raise ImportError(f"{path} does not load beside torch {torch.__version__} ({e}); {rebuild}") from e
+        # It reads tensors through torch's C++ structures, which change from release to release.
+        running = re.match(r"\d+(\.\d+)*", torch.__version__)  # without "a0", ".dev..." and "+cu..."
+        if running is None or module.torch_version != running.group():
+            raise ImportError(f"{path} was built for torch {module.torch_version}, this is torch {torch.__version__}; {rebuild}")
         lib = load()
         address = [ctypes.cast(f, ctypes.c_void_p).value for f in (lib.b2_collective, lib.b2_last_error)]
         module.bind(address[0], address[1], B200CclError)

@@ -14,6 +14,7 @@
 #include <ATen/core/Tensor.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/version.h>
 
 #include "b200ccl/types.h"
 
@@ -300,6 +301,11 @@ PyMODINIT_FUNC PyInit__b200ccl_torch() {
     PyObject* type = PyType_FromSpec(&caller_spec);
     if (type == nullptr || PyModule_AddObject(m, "Caller", type) < 0) {
         Py_XDECREF(type);
+        Py_DECREF(m);
+        return nullptr;
+    }
+    // The calls read torch's own structures: whoever loads the module compares this with the torch that runs.
+    if (PyModule_AddStringConstant(m, "torch_version", TORCH_VERSION) < 0) {
         Py_DECREF(m);
         return nullptr;
     }

@@ -4,6 +4,7 @@ import ctypes
 
 import pytest
 
+from conftest import ROOT
 from nano_nccl_b200 import _lib
 
 
@@ -178,3 +179,19 @@ def test_tuning_file_from_tuner_tables():
                       "twoshot_max_ctas": 48}
     text = format_tuning(values, "synthetic")
     assert "ll_max_bytes = 2048\n" in text and text.startswith("# b200ccl tuning file")
+
+
+@pytest.mark.parametrize("version,fits", [(None, True), ("2.10.0+cu128", False), ("1.0.0", False), ("nightly", False)])
+def test_native_calls_are_tied_to_the_torch_they_were_built_for(native_build, version, fits):
+    import subprocess
+    import sys
+    code = ("import torch\n" + (f"torch.__version__ = {version!r}\n" if version else "") +
+            "from nano_nccl_b200 import _lib\n"
+            "try:\n    _lib.load_native_calls()\n    print('LOADED')\n"
+            "except ImportError as e:\n    print('REFUSED', e)\n")
+    p = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=240)
+    assert p.returncode == 0, p.stderr
+    if fits:
+        assert p.stdout.strip() == "LOADED"
+    else:
+        assert p.stdout.startswith("REFUSED") and "built for torch" in p.stdout and version in p.stdout
