@@ -213,6 +213,7 @@ Communicator::Impl::Impl(const CommunicatorConfig& config, Bootstrap* bootstrap)
     if (config.max_ctas > 0) {  // an explicit cap applies to every algorithm
         tuning_.max_ctas = tuning_.nvls_max_ctas = tuning_.nvls_staged_max_ctas = tuning_.twoshot_max_ctas =
             std::min(config.max_ctas, dev::kMaxCtas);
+        tuning_.one_device_max_ctas = config.max_ctas;
     }
 
     // Rank layout: ranks are contiguous per process, in bootstrap order

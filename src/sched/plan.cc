@@ -97,7 +97,7 @@ Tuning tuning_from_text(const std::string& text, const Tuning& base, const std::
                 throw std::invalid_argument(where + "rank count in '" + key + "' must be 2.." + std::to_string(kMaxRanks));
             t.oneshot_max_bytes[n] = bytes;
         } else if (key == "nvls_min_bytes") t.nvls_min_bytes = bytes;
-        else if (key == "max_ctas") t.max_ctas = std::max(as_int, 1);
+        else if (key == "max_ctas") t.max_ctas = t.one_device_max_ctas = std::max(as_int, 1);
         else if (key == "nvls_max_ctas") t.nvls_max_ctas = t.nvls_staged_max_ctas = std::max(as_int, 1);
         else if (key == "nvls_staged_max_ctas") t.nvls_staged_max_ctas = std::max(as_int, 1);
         else if (key == "twoshot_max_ctas") t.twoshot_max_ctas = std::max(as_int, 1);
@@ -141,6 +141,7 @@ Tuning tuning_from_env() {
     if (env::get("B200CCL_MAX_CTAS")) {
         t.max_ctas = static_cast<int>(env::get_int("B200CCL_MAX_CTAS", t.max_ctas));
         t.nvls_max_ctas = t.nvls_staged_max_ctas = t.twoshot_max_ctas = t.max_ctas;  // an explicit cap applies to every algorithm
+        t.one_device_max_ctas = std::max(t.max_ctas, 1);
     }
     if (env::get("B200CCL_NVLS_MAX_CTAS"))
         t.nvls_max_ctas = t.nvls_staged_max_ctas = static_cast<int>(env::get_int("B200CCL_NVLS_MAX_CTAS", t.nvls_max_ctas));
@@ -214,16 +215,16 @@ Plan make_plan(const CallShape& s, Algo forced, const Tuning& t) {
     if (s.nranks > 1 && s.one_device && (forced == Algo::Auto || forced == Algo::Local)) {
         // Ranks that share a device need none of the waiting that the peer kernels do between GPUs, at any size:
         // 4 KiB on 8 ranks in 3.5 us against 40 us, 64 MiB 158 us against 172 us. Those kernels still run there when they are asked for
-        // by name. A cap on CTAs counts only where it is tighter than the default.
+        // by name. Of caps on CTAs only one that somebody asked for counts: the default is made for kernels whose CTAs loop.
         p.algo = Algo::Local;
-        p.grid = cap < default_tuning().max_ctas ? cap : 0;  // 0: no cap
+        p.grid = t.one_device_max_ctas;  // 0: no cap
         return p;
     }
     if (s.nranks == 1) {
         // One rank: every collective is a copy of `count` elements, which the one-device kernel does at any
         // length and alignment (reported as one-shot where it is no whole number of aligned 16-byte packs).
         p.algo = s.wide ? Algo::Copy : Algo::OneShot;
-        p.grid = cap < default_tuning().max_ctas ? cap : 0;
+        p.grid = t.one_device_max_ctas;
         return p;
     }
 

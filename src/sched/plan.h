@@ -51,6 +51,7 @@ struct Tuning {
     std::size_t oneshot_max_bytes[kMaxRanks + 1];  // per nranks: AllReduce sizes up to this use one-shot
     std::size_t nvls_min_bytes = 0;                // NVLS from this size up (when available)
     int max_ctas = 128;                            // hard cap for every algorithm (B200CCL_MAX_CTAS)
+    int one_device_max_ctas = 0;                   // the cap that somebody asked for, of any size; 0: nobody did (one-device kernel)
     int nvls_max_ctas = 64;                        // more CTAs than this slowed the multimem kernels down
     int nvls_staged_max_ctas = 64;                 // when the same CTAs also copy the message in and out of the arena
     int twoshot_max_ctas = 128;

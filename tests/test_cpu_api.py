@@ -124,6 +124,25 @@ def test_cta_cap_from_the_environment(lib, monkeypatch):
     assert cfg.max_ctas == 0 and cfg.enable_nvls == 1
 
 
+@pytest.mark.parametrize("nranks", [1, 4])
+def test_cta_cap_of_ranks_that_share_a_device(lib, monkeypatch, tmp_path, nranks):
+    # A cap that somebody asked for holds at any value, the default of the kernels that loop (128) does not apply.
+    WIDE, RD, WR, ONE_DEVICE = 1, 2, 4, 256
+    for var in ("B200CCL_MAX_CTAS", "B200CCL_TUNING_FILE"):
+        monkeypatch.delenv(var, raising=False)
+    assert _plan(lib, 0, 1 << 24, WIDE | RD | WR | ONE_DEVICE, nranks=nranks)[1][1] == 0
+    for asked in (1, 5, 127, 128, 129, 160, 4096):
+        monkeypatch.setenv("B200CCL_MAX_CTAS", str(asked))
+        for flags in (RD | WR | ONE_DEVICE, WIDE | RD | WR | ONE_DEVICE):
+            rc, p = _plan(lib, 0, 1 << 24, flags, nranks=nranks)
+            assert rc == 0 and p[1] == asked
+    monkeypatch.delenv("B200CCL_MAX_CTAS")
+    path = tmp_path / "b200.tuning"
+    path.write_text("max_ctas = 128\n")
+    monkeypatch.setenv("B200CCL_TUNING_FILE", str(path))
+    assert _plan(lib, 0, 1 << 24, WIDE | RD | WR | ONE_DEVICE, nranks=nranks)[1][1] == 128
+
+
 def test_tuning_file(lib, monkeypatch, tmp_path):
     WIDE, RD, WR, IMC, OMC, WORD = 1, 2, 4, 8, 16, 128
     path = tmp_path / "b200.tuning"

@@ -82,3 +82,21 @@ def test_in_place_on_one_device_and_a_capped_grid():
                 assert (t - ref).abs().max().item() <= 1e-5
     finally:
         comm.close()
+
+
+@pytest.mark.parametrize("ranks", [1, 8])
+@pytest.mark.parametrize("cap", [1, 128, 160, 1000])
+def test_a_cap_on_ctas_holds_at_any_value(ranks, cap):
+    comm = nn.Communicator(devices=[0], loopback_ranks=ranks if ranks > 1 else 0, max_ctas=cap, wait_timeout_ms=2000)
+    try:
+        for count in (1 << 20, (1 << 20) + 3):
+            ins = [torch.full((count,), float(r + 1), device="cuda") for r in range(ranks)]
+            for shift in (0, 1):  # 1: outputs that start one element past the inputs' alignment
+                outs = [torch.zeros(count + 1, device="cuda")[shift:shift + count] for _ in range(ranks)]
+                comm.all_reduce(outs, ins)
+                torch.cuda.synchronize()
+                assert 1 <= comm.last_call()["grid"] <= cap
+                assert all((o == ranks * (ranks + 1) / 2).all() for o in outs)
+        comm.check_async_error()
+    finally:
+        comm.close()
