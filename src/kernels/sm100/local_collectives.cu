@@ -327,7 +327,11 @@ cudaError_t start_op(Plan& p, LocalLaunch* made) {
 cudaError_t start_copy(Plan& p, LocalLaunch* made) {
     if (p.how == Plan::kAlike && p.args.nranks == 1) return start_tiles<__half, kCopyBytes>(local_kernel<__half, OpAdd, 1, false, kCopyBytes>, p, made);
     if (p.how == Plan::kAlike) return start_tiles<__half>(local_kernel<__half, OpAdd, 1, false, kBytes>, p, made);
-    if (p.how == Plan::kShifted) return start_tiles<__half>(local_shift_copy_kernel<__half>, p, made);
+    if (p.how == Plan::kShifted) {
+        const cudaError_t st = start_tiles<__half>(local_shift_copy_kernel<__half>, p, made);
+        made->pack_bytes = 16;
+        return st;
+    }
     return start_op<__half, OpAdd>(p, made);
 }
 

@@ -222,8 +222,8 @@ Plan make_plan(const CallShape& s, Algo forced, const Tuning& t) {
     }
     if (s.nranks == 1) {
         // One rank: every collective is a copy of `count` elements, which the one-device kernel does at any
-        // length and alignment (reported as one-shot where it is no whole number of aligned 16-byte packs).
-        p.algo = s.wide ? Algo::Copy : Algo::OneShot;
+        // length and alignment.
+        p.algo = Algo::Copy;
         p.grid = t.one_device_max_ctas;
         return p;
     }

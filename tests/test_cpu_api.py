@@ -61,6 +61,9 @@ def test_planner(lib):
     assert rc == 0 and p[4] == 1 and p[2] == 1  # else pulls from the staged inputs
     rc, p = _plan(lib, 0, 1 << 20, WIDE, forced=3)
     assert rc == 2 and b"nvls" in lib.b2_last_error()
+    for flags in (0, RD | WR, WIDE | RD | WR):
+        rc, p = _plan(lib, 0, 4097, flags, nranks=1)
+        assert rc == 0 and p[0] == 6  # one rank: a copy at any length and alignment
 
 
 def test_planner_low_latency(lib, monkeypatch):

@@ -45,7 +45,7 @@ def test_single_rank_collectives_are_copies(one_rank, dtype):
     assert torch.equal(y, keep) and torch.equal(z, keep) and torch.equal(x, keep)
 
 
-def test_single_rank_unaligned_buffers_take_the_element_path(one_rank):
+def test_single_rank_unaligned_buffers_are_copied_too(one_rank):
     comm = one_rank
     base = torch.randn(1 << 16, device="cuda")
     x = base[1:4098]  # 4 bytes past a 16-byte boundary, 4097 elements
@@ -53,7 +53,8 @@ def test_single_rank_unaligned_buffers_take_the_element_path(one_rank):
     comm.all_reduce(y, x, op="min")
     torch.cuda.synchronize()
     comm.check_async_error()
-    assert comm.last_call()["algo"] == "oneshot" and not comm.last_call()["vectorized"]
+    assert comm.last_call()["algo"] == "copy" and not comm.last_call()["vectorized"]
+    assert comm.last_call()["pack_bytes"] == 16  # shifted from the inputs' alignment to the outputs'
     assert torch.equal(y, x)
 
 
