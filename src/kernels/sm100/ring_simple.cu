@@ -168,7 +168,9 @@ __device__ bool run_slice(const RingArgs& a, ChannelState& st, unsigned flags, c
     // posted, and only then does the slice go on. On host-memory and network edges, where a credit
     // takes microseconds to arrive, this takes the consumer's own work off the sender's critical path.
     // Inside one GPU the credit is there before the sender has used up its four slots, and the extra barrier and
-    // release only lengthen the slice (4 ranks, 64 KiB: 35.9 -> 32.2 us without).
+    // release only lengthen the slice (4 ranks, 64 KiB: 35.9 -> 32.2 us without). Two groups run inside one GPU only and
+    // so never take this path; their instances keep the branch because the compiler lays out the slice loop worse without
+    // it (2 ranks, 16 MiB: 39.1 us with the branch, 41.1 us without; 4 ranks: 58.6 and 59.7 us).
     // Parity: the reference's early-credit path for slices of at most 4096 bytes
     // (src/kernels/ring_simple_kernel.cuh:486-583, 912-927).
     bool early = false;

@@ -63,12 +63,16 @@ def test_step_counters_use_system_scope_release_acquire():
     sync = read(os.path.join(KERNELS, "sync.cuh"))
     assert "ld.acquire.sys.global.u64" in sync and "st.release.sys.global.u64" in sync
     ring = read(os.path.join(KERNELS, "ring_simple.cu"))
-    # data stores of the whole CTA are ordered before the counter by a block barrier, then release
-    publish = ring[ring.index("// Publish:"):]
-    assert publish.index("__syncthreads()") < publish.index("st_release_sys(st.ch.recv_head") < publish.index("st_release_sys(st.ch.send_tail")
+    # data stores of the whole group are ordered before the counter by its barrier, then release (comments count for nothing)
+    code = lambda text: re.sub(r"//[^\n]*", "", text)
+    barriers = code(ring[ring.index("void group_sync("):ring.index("u64 ld_acquire_turn")])
+    assert "__syncthreads();" in barriers and "bar.sync %0" in barriers
+    assert "return __syncthreads_and(" in barriers and "bar.red.and.pred" in barriers
+    publish = code(ring[ring.index("// Publish:"):])
+    assert publish.index("group_sync<kGroups>(") < publish.index("st_release_sys(st.ch.recv_head") < publish.index("st_release_sys(st.ch.send_tail")
     # the early credit of small slices is posted only after every thread holds its part of the slot
-    early = ring[ring.index("if (early) {"):ring.index("auto combine_store")]
-    assert early.index("ld16_volatile(") < early.index("__syncthreads_or(") < early.index("st_release_sys(st.ch.recv_head")
+    early = code(ring[ring.index("if (early) {"):ring.index("auto combine_store")])
+    assert early.index("ld16_volatile(") < early.index("group_sync_and<kGroups>(") < early.index("st_release_sys(st.ch.recv_head")
 
 
 def test_low_latency_kernel_waits_are_bounded_and_flags_travel_with_the_data():
