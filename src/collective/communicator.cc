@@ -1224,7 +1224,7 @@ void Communicator::Impl::launch_all_gather(const CollectiveArgs& args, const sch
 std::string Communicator::Impl::describe() const {
     std::ostringstream os;
     os << "b200ccl communicator: " << nranks_ << " ranks, " << local_.size() << " local"
-       << (loopback_ ? " (loopback emulation)" : "") << (multiprocess_ ? " (multi-process)" : "") << "\n";
+       << (loopback_ ? (dev::kRanksShareGpu ? " (loopback emulation)" : " (loopback emulation, synchronised as on GPUs of their own)") : "") << (multiprocess_ ? " (multi-process)" : "") << "\n";
     os << "transport: requested " << transport_name(requested_) << ", resolved " << transport_name(resolved_) << "\n";
     if (alloc_)
         os << "memory: " << (alloc_->uses_vmm() ? "virtual memory management" : "cudaMalloc + peer access")

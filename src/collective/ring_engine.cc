@@ -272,7 +272,7 @@ void RingEngine::launch(Collective collective, const CollectiveArgs& args) {
         DeviceGuard guard(s.cfg.local[0].device);
         cfg.stream = args.streams[0];
         cfg.loop_ranks = s.cfg.nranks;
-        cfg.device_fifos = !s.net && s.host_fifo.empty();
+        cfg.device_fifos = dev::kRanksShareGpu && !s.net && s.host_fifo.empty();
         B2_CUDA(kernels::launch_ring(args.dtype, args.redop, per.data(), cfg));
     } else {
         for (std::size_t i = 0; i < s.cfg.local.size(); ++i) {

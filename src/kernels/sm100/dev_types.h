@@ -19,6 +19,15 @@ constexpr int kLlCtas = 8;                  // the low-latency kernel always run
 constexpr unsigned kLlMaxBytes = 128u << 10; // largest message it takes
 constexpr unsigned kLlMaxWords = kLlMaxBytes / 4;
 
+// Emulated ranks are part of one launch on one GPU: they order their stores at GPU scope, and their plans cannot differ.
+// In the checking build they do what ranks on GPUs of their own do instead (system scope, plan fingerprints, a ring of
+// one group of warps that returns credits early), so that one GPU can run those paths. Numbers never come from it.
+#if defined(B200CCL_DEBUG_BOUNDS)
+constexpr bool kRanksShareGpu = false;
+#else
+constexpr bool kRanksShareGpu = true;
+#endif
+
 // Per-rank control block. It lives in symmetric memory: every rank can store into every other
 // rank's block; each rank polls only its own.
 struct ControlBlock {

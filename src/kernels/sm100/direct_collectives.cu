@@ -34,7 +34,7 @@ __device__ __forceinline__ const A& select_args(const LoopPack<A>& all) { return
 template <typename A>
 constexpr bool kAllRanksHere = false;
 template <typename A>
-constexpr bool kAllRanksHere<LoopPack<A>> = true;
+constexpr bool kAllRanksHere<LoopPack<A>> = kRanksShareGpu;
 
 // Copies the packs first, first+stripe, ... below len, four loads in flight per thread. One side is
 // the caller's own buffer (16-byte aligned at most), the other the staging arena.

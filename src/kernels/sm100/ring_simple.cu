@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(kRingThreads, kWide ? 1 : 2) ring_kernel(const
     ChannelState st;
     st.ch = a.channels[c];
     // Network edges name an abort word: a host thread is at their other end.
-    st.one_gpu = sizeof(ParamT) != sizeof(RingArgs) && st.ch.abort_word == nullptr;
+    st.one_gpu = kRanksShareGpu && sizeof(ParamT) != sizeof(RingArgs) && st.ch.abort_word == nullptr;
     if (threadIdx.x == 0) {
         turns.posted[0] = *st.ch.send_base;
         turns.posted[1] = *st.ch.recv_base;

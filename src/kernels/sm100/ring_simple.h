@@ -75,7 +75,7 @@ namespace b200ccl::kernels {
 struct RingLaunch {
     cudaStream_t stream = nullptr;
     int loop_ranks = 0;  // >0: one cooperative launch plays that many ranks (args[0..loop_ranks))
-    bool device_fifos = false;  // every FIFO and counter lies in device memory
+    bool device_fifos = false;  // every FIFO and counter lies in the memory of the one GPU (two groups of warps)
 };
 
 // Launches one CTA per channel (512 threads). `args` points to one struct, or loop_ranks structs.

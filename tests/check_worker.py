@@ -4,6 +4,8 @@ socket-fault — a send proxy closes its socket after two slices: the ring kerne
                waits, the error must name the edge, and the communicator must refuse new work;
 bounds       — the host is told to pass extents that are too short: the kernel must record the
                first bad index, skip those accesses and still run to its end;
+separate-gpus — emulated ranks synchronise as ranks on GPUs of their own do: the ring's early credit and single
+               group of warps at system scope, the peer kernels' barriers with their plan fingerprints;
 canary       — the staging arena sits between two pages of canary bytes: they survive staged
                collectives, and a byte overwritten from the host is reported."""
 import os
@@ -12,6 +14,43 @@ import sys
 import torch
 
 import nano_nccl_b200 as nn
+
+
+def reference(ins, op):
+    stack = torch.stack([t.float() for t in ins])
+    return {"sum": stack.sum(0), "avg": stack.sum(0) / len(ins), "max": stack.max(0).values, "min": stack.min(0).values}[op]
+
+
+def separate_gpus():
+    """Every algorithm that a job on several GPUs may take, several calls in a row: lengths of one early-credit slice, of many
+    slices and ragged ones for the ring; around the packs for the peer kernels; all three collectives."""
+    cases = [("ring", t, c, r) for t, c in (("auto", 4), ("auto", 0), ("shm", 4)) for r in (2, 3, 8)]
+    cases += [(a, "auto", 0, r) for a in ("oneshot", "twoshot", "ll") for r in (2, 3, 8)]
+    for algo, transport, channels, ranks in cases:
+        comm = nn.Communicator(devices=[0], loopback_ranks=ranks, algo=algo, transport=transport, channels=channels, wait_timeout_ms=3000)
+        assert "as on GPUs of their own" in comm.describe()
+        for dtype, tol in ((torch.float32, 1e-5), (torch.bfloat16, 2e-1)):  # bf16: the ring rounds once per hop, sums to 30
+            counts = [1024, 4096, 16384, 2048, 4096, 1024, 8192] * 3 + ([1 << 15, 6] if algo == "ll" else [(1 << 20) + 8, 300001, 7])
+            for i, count in enumerate(counts):
+                op = ["sum", "avg", "max", "min"][i % 4]
+                gen = torch.Generator(device="cuda").manual_seed(900 + i)
+                ins = [torch.randn(count, device="cuda", generator=gen).to(dtype) for _ in range(ranks)]
+                outs = [torch.full_like(t, float("nan")) for t in ins]
+                comm.all_reduce(outs, ins, op=op)
+                assert comm.last_call()["algo"] == algo
+                for o in outs:
+                    assert (o.float() - reference(ins, op)).abs().max().item() <= tol, (algo, transport, ranks, count, op)
+            for block in () if algo == "ll" else (2048, 1 << 17, 1001, 3):
+                ins = [torch.randn(block * ranks, device="cuda").to(dtype) for _ in range(ranks)]
+                shards = [torch.empty(block, device="cuda", dtype=dtype) for _ in range(ranks)]
+                full = [torch.empty(block * ranks, device="cuda", dtype=dtype) for _ in range(ranks)]
+                comm.reduce_scatter(shards, ins, op="max")
+                comm.all_gather(full, shards)
+                most = reference(ins, "max").to(dtype)
+                assert all(torch.equal(f, most) for f in full), (algo, transport, ranks, block)
+        torch.cuda.synchronize()
+        comm.check_async_error()
+        comm.close()
 
 
 def main():
@@ -62,6 +101,8 @@ def main():
             assert (o[:good] - ref[:good]).abs().max().item() <= 1e-5
             assert (o[good:] == -7.0).all()
         comm.close()
+    elif mode == "separate-gpus":
+        separate_gpus()
     elif mode == "canary":
         smash = os.environ.pop("B200CCL_DEBUG_SMASH_CANARY", None)
         comm = nn.Communicator(devices=[0], loopback_ranks=4, algo="pipeline", wait_timeout_ms=3000, staging_bytes=8 << 20)

@@ -32,6 +32,11 @@ def test_device_index_checks_record_and_skip():
     assert rc == 0 and "WORKER OK" in out, out
 
 
+def test_emulated_ranks_synchronise_as_on_gpus_of_their_own():
+    rc, out = run("separate-gpus")
+    assert rc == 0 and "WORKER OK" in out, out
+
+
 def test_canary_pages_around_the_staging_arena():
     rc, out = run("canary")
     assert rc == 0 and "WORKER OK" in out, out

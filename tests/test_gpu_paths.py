@@ -172,10 +172,12 @@ def test_staged_pipeline_all_reduce(ranks, dtype):
 
 
 @pytest.mark.parametrize("ranks", [2, 4, 8])
-@pytest.mark.parametrize("transport", ["auto", "shm"])
+@pytest.mark.parametrize("transport", ["auto", "shm", "socket"])
 def test_ring_small_slices_return_their_credit_early(ranks, transport):
-    # Messages whose slices hold at most one 16-byte vector per thread take the early-credit path
-    # of the ring kernel (slot read into registers, credit posted, then combined and forwarded).
+    # Messages whose slices hold at most one 16-byte vector per thread. Over network edges, as between
+    # GPUs, they take the early-credit path of the ring kernel (slot read into registers, credit posted,
+    # then combined and forwarded); emulated ranks over device or host memory return the credit with the
+    # slice (the checking build has them return it early, tests/test_gpu_check_build.py).
     # Many calls in a row reuse every FIFO slot several times, so a credit posted too early would
     # let the sender overwrite a slot that is still being read and corrupt a later call.
     comm = nn.Communicator(devices=[0], loopback_ranks=ranks, algo="ring", transport=transport, channels=4, wait_timeout_ms=3000)
