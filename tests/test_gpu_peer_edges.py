@@ -41,3 +41,42 @@ def test_peer_kernels_around_their_packs(algo, ranks, dtype):
         comm.check_async_error()
     finally:
         comm.close()
+
+
+@pytest.mark.parametrize("ranks", [2, 3, 8])
+@pytest.mark.parametrize("dtype", list(TOL))
+def test_peer_reduce_scatter_and_all_gather_around_their_packs(ranks, dtype):
+    # Blocks of every rank behind one another (reduce_kernel) and each rank's block into every output (gather_kernel): whole
+    # packs, lengths that put every block on another alignment (4- and 2-byte accesses), buffers that start off a pack.
+    comm = nn.Communicator(devices=[0], loopback_ranks=ranks, algo="oneshot", wait_timeout_ms=2000)
+    try:
+        esz = torch.empty(0, dtype=dtype).element_size()
+        for k, block in enumerate([1, 2, 7, 8, 9, 16, 31, 256, 257, 1021, 4096, 4099, 65536 // esz, 65536 // esz + 2, 300001, 1 << 19]):
+            for shift in (0, 1, 4 // esz):
+                op = ["sum", "avg", "max", "min"][k % 4]
+                gen = torch.Generator(device="cuda").manual_seed(800 + k)
+                ins = [torch.randn(block * ranks + 32, device="cuda", generator=gen).to(dtype)[16 + shift:16 + shift + block * ranks] for _ in range(ranks)]
+                raw = [torch.full((block + 64,), 7.0, device="cuda", dtype=dtype) for _ in range(ranks)]
+                outs = [t[16 + shift:16 + shift + block] for t in raw]
+                comm.reduce_scatter(outs, ins, op=op)
+                assert comm.last_call()["algo"] == "oneshot"
+                # added in rank order in fp32 and rounded once, so that a reference can match every bit
+                acc = ins[0].float()
+                for t in ins[1:]:
+                    acc = acc + t.float() if op in ("sum", "avg") else (torch.maximum if op == "max" else torch.minimum)(acc, t.float())
+                if op == "avg":
+                    acc = acc * torch.tensor(1.0, device="cuda").div(ranks)
+                expect = acc.to(dtype)
+                for r, (t, o) in enumerate(zip(raw, outs)):
+                    assert torch.equal(o, expect[r * block:(r + 1) * block]), (block, shift, op)
+                    assert (t[:16 + shift] == 7.0).all() and (t[16 + shift + block:] == 7.0).all(), (block, shift)
+                raw = [torch.full((block * ranks + 64,), 7.0, device="cuda", dtype=dtype) for _ in range(ranks)]
+                full = [t[16 + shift:16 + shift + block * ranks] for t in raw]
+                comm.all_gather(full, outs)
+                assert comm.last_call()["algo"] == "oneshot"
+                for t, o in zip(raw, full):
+                    assert torch.equal(o, expect), (block, shift)
+                    assert (t[:16 + shift] == 7.0).all() and (t[16 + shift + block * ranks:] == 7.0).all(), (block, shift)
+        comm.check_async_error()
+    finally:
+        comm.close()
