@@ -1,5 +1,6 @@
 """Native programs on a GPU: the command-line benchmark in single-GPU emulation must verify every
-element (#wrong = 0, exit status 0) for each collective, algorithm and dtype, and the smoke entry."""
+element (#wrong = 0, exit status 0) for each collective, algorithm and dtype, and the smoke entry.
+Without --algo the emulated ranks take the one-device kernel; the peer kernels are asked for by name."""
 import pytest
 
 from conftest import run_native
@@ -17,6 +18,11 @@ pytestmark = pytest.mark.gpu
     ["--collective", "all_reduce", "--nranks", "4", "--transport", "shm"],
     ["--collective", "all_reduce", "--nranks", "4", "--graph"],
     ["--collective", "all_gather", "--nranks", "2", "--graph", "--symmetric"],
+    ["--collective", "all_reduce", "--nranks", "4", "--algo", "twoshot", "--symmetric"],
+    ["--collective", "all_reduce", "--nranks", "4", "--algo", "oneshot", "--graph"],
+    ["--collective", "all_reduce", "--nranks", "8", "--algo", "twoshot", "--graph"],
+    ["--collective", "reduce_scatter", "--nranks", "8", "--algo", "oneshot", "--dtype", "bf16", "--graph"],
+    ["--collective", "all_gather", "--nranks", "2", "--algo", "oneshot", "--graph", "--symmetric"],
 ])
 def test_bench_cli_verifies(native_build, args):
     proc = run_native("b200ccl_collective_bench", "--loopback", *args, "-b", "1024", "-e", "4194304", "-f", "64", "-w", "1", "-n",
