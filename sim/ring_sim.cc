@@ -3,9 +3,11 @@
 #include "core/datagen.h"
 #include "sched/ring_geometry.h"
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <cmath>
+#include <condition_variable>
 #include <memory>
 #include <mutex>
 #include <thread>
@@ -45,13 +47,53 @@ float apply(RedOp op, float a, float b) {
 
 enum : unsigned { kRecv = 1, kLocal = 2, kSend = 4, kCopyOut = 8, kScale = 16 };
 
+// Barrier of one group of lanes; says whether `ok` held in all of them.
+class GroupBarrier {
+public:
+    explicit GroupBarrier(int lanes) : lanes_(lanes) {}
+    bool meet(bool ok) {
+        if (lanes_ == 1) return ok;
+        std::unique_lock<std::mutex> lock(mu_);
+        all_ = all_ && ok;
+        if (++arrived_ == lanes_) {
+            arrived_ = 0;
+            result_ = all_;
+            all_ = true;
+            ++generation_;
+            cv_.notify_all();
+            return result_;
+        }
+        const u64 mine = generation_;
+        cv_.wait(lock, [&] { return generation_ != mine; });
+        return result_;  // the next meeting cannot end before this lane arrives at it
+    }
+
+private:
+    std::mutex mu_;
+    std::condition_variable cv_;
+    const int lanes_;
+    int arrived_ = 0;
+    bool all_ = true, result_ = true;
+    u64 generation_ = 0;
+};
+
+// What the groups of one (rank, channel) share during a call.
+struct Cta {
+    std::atomic<u64> posted[2];  // 0: slices sent, 1: credits returned
+    std::atomic<bool> failed{false};
+    std::vector<std::unique_ptr<GroupBarrier>> barrier;
+};
+
 class Worker {
 public:
-    Worker(Shared& sh, int rank, int channel) : sh_(sh), r_(rank), c_(channel) {
+    Worker(Shared& sh, Cta& cta, int rank, int channel, int group, int lane, u64 send_step, u64 recv_step)
+        : sh_(sh), cta_(cta), r_(rank), c_(channel), group_(group), lane_(lane), send_step_(send_step), recv_step_(recv_step) {
         const int n = sh.cfg->nranks, C = sh.cfg->channels;
         out_edge_ = sh.edges[r_ * C + c_].get();
         in_edge_ = sh.edges[((r_ + n - 1) % n) * C + c_].get();
     }
+    u64 send_step() const { return send_step_; }
+    u64 recv_step() const { return recv_step_; }
 
     void run() {
         const RingSimConfig& cfg = *sh_.cfg;
@@ -148,57 +190,107 @@ private:
         return true;
     }
 
+    bool has_role(int role) const { return lane_ == role % sh_.cfg->lanes; }
+
+    // Waits until every slice before `step` has been published; false when the other group gave up.
+    bool wait_turn(int side, u64 step) {
+        if (sh_.cfg->groups == 1 || sh_.cfg->skip_turns) return true;
+        const auto t0 = Clock::now();
+        for (unsigned polls = 1;; ++polls) {
+            if (cta_.posted[side].load(std::memory_order_acquire) >= step) return true;
+            if (cta_.failed.load(std::memory_order_relaxed)) return false;
+            if ((polls & 255u) == 0) {
+                if (std::chrono::duration<double, std::milli>(Clock::now() - t0).count() > 2 * sh_.cfg->wait_timeout_ms) {
+                    cta_.failed.store(true, std::memory_order_relaxed);
+                    return false;
+                }
+                std::this_thread::yield();
+            }
+        }
+    }
+    void publish(int side, std::atomic<u64>& counter, u64 step) {
+        if (!wait_turn(side, step)) return;
+        counter.store(step + ring::kSliceSteps, std::memory_order_release);
+        cta_.posted[side].store(step + ring::kSliceSteps, std::memory_order_release);
+    }
+
     bool run_slice(unsigned flags, const float* local_in, float* local_out, std::size_t n) {
         if (n == 0) {
-            sh_.empty.fetch_add(1, std::memory_order_relaxed);
+            if (group_ == 0 && lane_ == 0) sh_.empty.fetch_add(1, std::memory_order_relaxed);
             return true;
         }
         const RingSimConfig& cfg = *sh_.cfg;
-        if (cfg.stall_rank == r_ && static_cast<long long>(done_) >= cfg.stall_after_slices) return false;  // this rank "dies"
-        const int nr = cfg.nranks;
+        if (cfg.stall_rank == r_ && static_cast<long long>(slices_) >= cfg.stall_after_slices) return false;  // this rank "dies"
         const bool recv = flags & kRecv, send = flags & kSend, local = flags & kLocal, copy_out = flags & kCopyOut;
+        if (static_cast<int>(slices_++ % static_cast<u64>(cfg.groups)) != group_) {  // the other group's
+            if (recv) recv_step_ += ring::kSliceSteps;
+            if (send) send_step_ += ring::kSliceSteps;
+            return true;
+        }
+        GroupBarrier& group = *cta_.barrier[group_];
+        const int nr = cfg.nranks;
         const float scale = (flags & kScale) && cfg.redop == RedOp::Avg ? 1.0f / nr : 1.0f;
-        if (recv && !wait(in_edge_->tail, recv_step_ + ring::kSliceSteps, (r_ + nr - 1) % nr, recv_step_)) return false;
-        if (send) {
+        bool ok = true;
+        if (recv && has_role(0)) ok = wait(in_edge_->tail, recv_step_ + ring::kSliceSteps, (r_ + nr - 1) % nr, recv_step_);
+        if (ok && send && has_role(1)) {
             const u64 want = send_step_ + ring::kSliceSteps >= static_cast<u64>(ring::kFifoSteps)
                                  ? send_step_ + ring::kSliceSteps - ring::kFifoSteps : 0;
-            if (!wait(out_edge_->head, want, (r_ + 1) % nr, send_step_)) return false;
+            ok = wait(out_edge_->head, want, (r_ + 1) % nr, send_step_);
         }
+        if (cta_.failed.load(std::memory_order_relaxed)) ok = false;
+        if (!ok) cta_.failed.store(true, std::memory_order_relaxed);
+        if (!group.meet(ok)) return false;
         const float* fin = recv ? in_edge_->fifo.data() + ring::slot_offset(recv_step_, sh_.step_elems) : nullptr;
         float* fout = send ? out_edge_->fifo.data() + ring::slot_offset(send_step_, sh_.step_elems) : nullptr;
-        for (std::size_t i = 0; i < n; ++i) {
+        const bool early = cfg.groups == 1 && recv && n <= cfg.early_credit_elems;
+        if (early) {
+            held_.clear();
+            for (std::size_t i = lane_; i < n; i += cfg.lanes) held_.push_back(fin[i]);
+            group.meet(true);  // every lane holds its part of the slot
+            if (has_role(2)) publish(1, in_edge_->head, recv_step_);
+        }
+        if (cfg.slow_group == group_ && (cfg.slow_rank < 0 || cfg.slow_rank == r_)) std::this_thread::sleep_for(std::chrono::microseconds(100));
+        std::size_t k = 0;
+        for (std::size_t i = lane_; i < n; i += cfg.lanes) {
             float v;
-            if (recv) v = local ? apply(cfg.redop, local_in[i], fin[i]) : fin[i];
-            else v = local_in[i];
+            if (recv) {
+                const float got = early ? held_[k++] : fin[i];
+                v = local ? apply(cfg.redop, local_in[i], got) : got;
+            } else {
+                v = local_in[i];
+            }
             if (scale != 1.0f) v *= scale;
             if (copy_out) local_out[i] = v;
             if (send) fout[i] = v;
         }
+        group.meet(true);
         if (recv) {
-            in_edge_->head.store(recv_step_ + ring::kSliceSteps, std::memory_order_release);
+            if (!early && has_role(2)) publish(1, in_edge_->head, recv_step_);
             recv_step_ += ring::kSliceSteps;
         }
         if (send) {
-            out_edge_->tail.store(send_step_ + ring::kSliceSteps, std::memory_order_release);
+            if (has_role(3)) publish(0, out_edge_->tail, send_step_);
             send_step_ += ring::kSliceSteps;
         }
-        ++done_;
-        sh_.slices.fetch_add(1, std::memory_order_relaxed);
+        if (lane_ == 0) sh_.slices.fetch_add(1, std::memory_order_relaxed);
         return true;
     }
 
     Shared& sh_;
-    int r_, c_;
+    Cta& cta_;
+    int r_, c_, group_, lane_;
     Edge* out_edge_ = nullptr;
     Edge* in_edge_ = nullptr;
-    u64 send_step_ = 0, recv_step_ = 0, done_ = 0;
+    u64 send_step_, recv_step_, slices_ = 0;
+    std::vector<float> held_;
 };
 
 }  // namespace
 
 RingSimResult run_ring_sim(const RingSimConfig& cfg) {
     RingSimResult result;
-    if (cfg.nranks < 2 || cfg.nranks > kMaxRanks || cfg.channels < 1 || cfg.channels > kMaxChannels || cfg.count == 0) {
+    if (cfg.nranks < 2 || cfg.nranks > kMaxRanks || cfg.channels < 1 || cfg.channels > kMaxChannels || cfg.count == 0 ||
+        cfg.groups < 1 || cfg.groups > 2 || cfg.lanes < 1 || cfg.lanes > 4 || cfg.calls < 1) {
         result.message = "bad simulator configuration";
         result.wrong = -1;
         return result;
@@ -221,14 +313,35 @@ RingSimResult run_ring_sim(const RingSimConfig& cfg) {
         sh.output[r].assign(out_count, std::nanf(""));
         for (std::size_t i = 0; i < in_count; ++i) sh.input[r][i] = datagen::uniform_pm1(static_cast<std::uint64_t>(r), r, i);
     }
-    std::vector<Worker> workers;
-    workers.reserve(static_cast<std::size_t>(n) * C);
-    for (int r = 0; r < n; ++r)
-        for (int c = 0; c < C; ++c) workers.emplace_back(sh, r, c);
     const auto t0 = Clock::now();
-    std::vector<std::thread> threads;
-    for (auto& w : workers) threads.emplace_back([&w] { w.run(); });
-    for (auto& t : threads) t.join();
+    std::vector<u64> send_base(static_cast<std::size_t>(n) * C, 0), recv_base(send_base);
+    for (int call = 0; call < cfg.calls && !result.timed_out; ++call) {
+        std::vector<std::unique_ptr<Cta>> ctas;
+        std::vector<Worker> workers;
+        workers.reserve(static_cast<std::size_t>(n) * C * cfg.groups * cfg.lanes);
+        for (int r = 0; r < n; ++r) {
+            for (int c = 0; c < C; ++c) {
+                const int at = r * C + c;
+                ctas.emplace_back(new Cta());
+                ctas.back()->posted[0] = send_base[at];
+                ctas.back()->posted[1] = recv_base[at];
+                for (int g = 0; g < cfg.groups; ++g) {
+                    ctas.back()->barrier.emplace_back(new GroupBarrier(cfg.lanes));
+                    for (int l = 0; l < cfg.lanes; ++l) workers.emplace_back(sh, *ctas.back(), r, c, g, l, send_base[at], recv_base[at]);
+                }
+            }
+        }
+        if (call > 0)
+            for (auto& o : sh.output) std::fill(o.begin(), o.end(), std::nanf(""));
+        std::vector<std::thread> threads;
+        for (auto& w : workers) threads.emplace_back([&w] { w.run(); });
+        for (auto& t : threads) t.join();
+        const std::size_t per_cta = static_cast<std::size_t>(cfg.groups) * cfg.lanes;
+        for (int at = 0; at < n * C; ++at) {
+            send_base[at] = workers[at * per_cta].send_step();
+            recv_base[at] = workers[at * per_cta].recv_step();
+        }
+    }
     result.seconds = std::chrono::duration<double>(Clock::now() - t0).count();
     result.slices = sh.slices.load();
     result.empty_slices = sh.empty.load();

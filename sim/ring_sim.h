@@ -1,6 +1,12 @@
-// CPU-only simulator of the ring + Simple protocol: every (rank, channel) pair is a host thread
-// that runs the same schedule as the device kernel (same geometry header), with FIFOs in host
-// memory and step counters as std::atomic with release/acquire ordering. It needs no GPU.
+// CPU-only simulator of the ring + Simple protocol: every (rank, channel) pair is a host thread, or
+// `groups` x `lanes` of them, that runs the same schedule as the device kernel (same geometry header),
+// with FIFOs in host memory and step counters as std::atomic with release/acquire ordering. It needs no GPU.
+//
+// A lane stands for the device threads of one role (lane 0 polls the incoming counter, 1 the outgoing
+// one, 2 returns credits, 3 posts slices; all of them move data), a group for the warps that take every
+// groups-th slice, with their barrier. Two groups hand the order of their posts over through shared
+// memory (`Turns` in src/kernels/sm100/ring_simple.cu): that word is an atomic here, FIFOs and buffers
+// are plain memory, so that a missing hand-over is a data race and a wrong result.
 //
 // Uses: (1) an oracle and timing baseline for the plumbing (4 ranks, 4 channels, 1 Mi floats per
 // rank, values uniform[-1,1) from seed = rank); (2) a place to run the flag protocol under a
@@ -28,6 +34,13 @@ struct RingSimConfig {
     double wait_timeout_ms = 5000.0;
     int stall_rank = -1;                   // failure injection: this rank stops ...
     long long stall_after_slices = 0;      // ... after this many slices (on every channel)
+    int groups = 1;                        // 2: as emulated ranks over device memory, alternating slices
+    int lanes = 1;                         // threads per group, 1 to 4
+    std::size_t early_credit_elems = 0;    // one group: slices of at most this many elements return their slot early
+    int calls = 1;                         // launches in a row; the steps carry on, as on the device
+    int slow_group = -1;                   // this group dawdles over every slice, on every rank ...
+    int slow_rank = -1;                    // ... or on this one only
+    bool skip_turns = false;               // plants a mistake: groups post without waiting for their turn
 };
 
 struct RingSimResult {
