@@ -161,7 +161,7 @@ private:
     std::unique_ptr<mem::SymmetricRegion> stage_;
     std::unique_ptr<mem::SymmetricRegion> pipe_flags_;  // dev::PipeFlags per rank, allocated with the arena
     std::vector<dev::PipeStats*> pipe_stats_;           // per local rank, device memory (B200CCL_PIPELINE_STATS=1)
-    std::unique_ptr<mem::SymmetricRegion> ll_area_;  // receive slots of the low-latency kernel (first use)
+    std::unique_ptr<mem::SymmetricRegion> ll_area_;  // receive slots of the low-latency kernel (allocated with the communicator)
     // A window is a buffer that exists on every rank and that every rank can address: a symmetric
     // allocation (with a multicast alias where available) or a registered ordinary buffer.
     struct Window {
@@ -251,14 +251,15 @@ Communicator::Impl::Impl(const CommunicatorConfig& config, Bootstrap* bootstrap)
 
     resolve_transport();
     if (channels_ <= 0) {
-        // One ring CTA moves about 8 GB/s over NVLink, so peer-memory rings want many channels (8 GPUs, 64 MiB:
-        // 272 GB/s with 32, 193 with 16); host-memory edges are limited by the host path and do best with few
+        // One ring CTA moved about 8 GB/s over NVLink, so peer-memory rings want many channels (8 GPUs, 64 MiB:
+        // 272 GB/s with 32, 193 with 16, measured with a kernel that staged the local operand in shared memory; the
+        // present one has not run across NVLink); host-memory edges are limited by the host path and do best with few
         // (8 GPUs: 11.7 GB/s with 4, 10.3 with 8, 9.2 with 16); network edges keep a proxy thread pair per channel.
         channels_ = resolved_ == TransportKind::P2p ? 32
                     : (resolved_ == TransportKind::Shm || resolved_ == TransportKind::Mixed) ? 4 : kDefaultChannels;
         // Emulated ranks share one GPU and one cooperative launch: all their channel CTAs must be resident at once, one
         // per SM. Over device memory more of them are faster up to there (4 ranks, 16 MiB: 108 us with 16 channels, 73
-        // with 32). Over host memory eight CTAs in all keep PCIe busy both ways (35 of the 38 GB/s that a copy from host
+        // with 32). Over host memory eight CTAs in all keep PCIe busy both ways (35 of the 40 GB/s that a copy from host
         // to host reaches); more of them slow it down (8 ranks, 1 MiB: 555 us with one channel, 834 with four).
         if (loopback_) {
             const int ctas = resolved_ == TransportKind::P2p ? 128 : (resolved_ == TransportKind::Shm ? 8 : 64);

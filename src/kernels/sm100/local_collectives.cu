@@ -56,7 +56,7 @@ struct LocalArgs {
     __device__ __forceinline__ const char* first_in(unsigned seg) const { return in[kind == (int)Collective::AllGather ? seg : 0]; }
 };
 // Launching a kernel takes 1.9-2.0 us of host time when the size of its parameters, modulo 64, lies in (16, 32], and
-// 2.25-2.5 us otherwise, at any size from 24 to 2848 bytes (CUDA 12.9, driver 580).
+// 2.2-2.5 us otherwise, at any size from 16 to 2848 bytes (CUDA 12.9, driver 580).
 static_assert(sizeof(LocalArgs) % 64 > 16 && sizeof(LocalArgs) % 64 <= 32);
 
 // Bytes in flight per thread and input. A copy from one buffer to one buffer wants more (one rank, 64 MiB: 21.6 us

@@ -10,10 +10,11 @@
 // warps take the slices in turn, so that one slice is moved while the other waits for its neighbour, for its loads
 // or for its release; shared memory hands the order of the posts from group to group (4 ranks: 64 KiB 37.6 -> 27.6
 // us, 16 MiB 65.8 -> 59.6 us). FIFOs in host memory keep one group: there each release waits for the other group's
-// writes over PCIe as well (4 ranks, 4 MiB: 724 us, 879 us with two). Inside a slice there is no barrier: every
-// thread keeps kBatch vectors of the FIFO and of the local input in flight in registers, and the first batch of the
-// local input is loaded BEFORE the wait for the neighbour. (The local input used to be staged by TMA through 32 KiB
-// tiles of shared memory, with three block barriers and four dependent FIFO loads per thread and tile.)
+// writes over PCIe as well (4 ranks, 4 MiB: 724 us, 879 us with two). While a slice is moved there is no barrier (one
+// comes before an early credit, see run_slice): every thread keeps kBatch vectors of the FIFO and of the local input in
+// flight in registers, and the first batch of the local input is loaded BEFORE the wait for the neighbour. (The local
+// input used to be staged by TMA through 32 KiB tiles of shared memory, with three block barriers and four dependent
+// FIFO loads per thread and tile.)
 //
 // Parity: nano-nccl src/kernels/ring_simple_kernel.cuh:1118-1237 (schedule 1170-1230:
 // direct_send, recv_reduce_send, recv_reduce_copy_send with the fused avg scale, recv_copy_send,
@@ -375,8 +376,9 @@ __global__ void __launch_bounds__(kRingThreads, kWide ? 1 : 2) ring_kernel(const
     bool ok = true;
     auto mod = [n](int v) { return ((v % n) + n) % n; };
 
-    // One schedule for the three collectives, so that the slice code exists once (four copies with their flags
-    // known at compile time spilled registers): windows of the part, in each of them `steps` chunks.
+    // One schedule for the three collectives, so that the slice code exists once: windows of the part, in each of them
+    // `steps` chunks. (Four copies with their flags known at compile time spilled registers; the one copy spills up to 24
+    // bytes in the 16-byte instances and 48 to 72 in the element ones, which are held to 64 registers.)
     const bool reduces = a.collective != (int)Collective::AllGather, scatters = a.collective == (int)Collective::ReduceScatter;
     const bool both = reduces && !scatters;  // all_reduce: n chunks per window, reduced on the way round and then passed on
     const u64 cs = both ? ring::all_reduce_chunk_elems(part.count, n, sizeof(T), a.step_elems)

@@ -104,7 +104,8 @@ __device__ __forceinline__ bool wait_at_least(const unsigned long long* flag, un
 
 // Barrier among the CTAs with the same blockIdx.x on every rank. Thread p signals rank p and
 // waits for rank p. Everything the CTA stored before the call is visible to every rank's CTA
-// after it (release on the signal, acquire on the poll, bar.sync on both sides).
+// after it (release on the signal, acquire on the poll, bar.sync on both sides), except where the caller says
+// that it has stored nothing (`nothing_stored`, below).
 // Returns false (to every thread of the CTA) when the wait gave up.
 // plan_hash != 0: CTA 0 also publishes the fingerprint of this launch's plan with the signal and
 // compares it with every peer's after the wait; a difference ends the collective on every rank

@@ -1,7 +1,7 @@
-"""GPU tests of single code paths on ONE device: the single-rank copy kernel (TMA bulk copies), the
-256-bit and 128-bit variants of the peer two-shot loop, fp32 accumulation of 16-bit inputs shown by a
-case that 16-bit accumulation gets wrong, and the plan fingerprint that the first barrier compares.
-Numerics are compared with a plain PyTorch fp32 reference. Every device wait is bounded."""
+"""GPU tests of single code paths on ONE device: one rank, whose collectives are copies, the 256-bit and
+128-bit variants of the peer two-shot loop, fp32 accumulation of 16-bit inputs shown by a case that 16-bit
+accumulation gets wrong, the tile pipeline, and small slices of the ring. Numerics are compared with a plain
+PyTorch fp32 reference. Every device wait is bounded."""
 import pytest
 import torch
 
@@ -21,8 +21,8 @@ def one_rank():
 def test_single_rank_collectives_are_copies(one_rank, dtype):
     comm = one_rank
     esz = torch.empty(0, dtype=dtype).element_size()
-    # one 16-byte pack; less than a tile; exactly one tile; a ragged last tile; more tiles than the
-    # ring of shared-memory slots holds per CTA; enough for every SM to loop
+    # one 16-byte pack; less than a tile (256 threads x 128 bytes); exactly one tile; a ragged last tile; several; as
+    # many as a large message has
     for nbytes in (16, 48, 32768, 32768 + 16, 7 * 32768 + 4096, (64 << 20) + 16):
         numel = nbytes // esz
         x = torch.randn(numel, device="cuda").to(dtype)
