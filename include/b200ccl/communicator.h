@@ -75,6 +75,9 @@ public:
     Communicator& operator=(Communicator&&) noexcept;
     ~Communicator();
 
+    // Asynchronous on the given streams. Calls run in the order in which they are made: one on another stream than the
+    // call before waits (on the device) for that call, and for nothing else that either stream holds. Between a call
+    // that is captured into a graph and one that is not, the caller orders them.
     void all_reduce(const CollectiveArgs& args);
     void reduce_scatter(const CollectiveArgs& args);
     void all_gather(const CollectiveArgs& args);
