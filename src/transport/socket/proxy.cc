@@ -75,10 +75,9 @@ void SendProxy::loop() {
             const std::size_t slot = step % fifo_.slot_count;
             const unsigned int bytes = fifo_.slot_sizes[slot];
             if (bytes > inc * fifo_.slot_bytes) throw std::runtime_error("slice larger than its FIFO slots");
-            if (fail_after_ != 0 && slices_.load() >= fail_after_) {
-                connection_.reset();
+            // run() records the failure before it ends the connection, so that the peer's echo is never the first one.
+            if (fail_after_ != 0 && slices_.load() >= fail_after_)
                 throw std::runtime_error("injected socket failure after " + std::to_string(fail_after_) + " slices");
-            }
             send_slice(connection_.get(), fifo_.data + slot * fifo_.slot_bytes, bytes);
             step += inc;
             step_.store(step, std::memory_order_release);
