@@ -126,6 +126,9 @@ private:
     void launch_all_gather(const CollectiveArgs& args, const sched::Plan& plan, bool wide,
                            const Located* in_loc, const Located* out_loc);
     void fill_common(dev::CollArgs& a, const Local& l) const;
+    // Emulated ranks whose direct kernels need one set of arguments: the first rank's, with every rank's buffers.
+    bool one_launch() const { return loopback_ && dev::kRanksShareGpu; }
+    int direct_grid(int planned) const;
     void launch_reduce_ranks(const CollectiveArgs& args, std::vector<dev::CollArgs>& per_rank, int pack_bytes,
                              bool nvls, int grid);
     void launch_gather_ranks(const CollectiveArgs& args, std::vector<dev::GatherArgs>& per_rank, int grid);
@@ -698,19 +701,25 @@ void Communicator::Impl::fill_common(dev::CollArgs& a, const Local& l) const {
     a.nranks = nranks_;
 }
 
+// CTAs per rank of a direct kernel that was planned with `planned` of them. Flags have a row per CTA, and emulated ranks that
+// meet over flags are one cooperative launch, all of it resident; those that need not meet run in any number.
+int Communicator::Impl::direct_grid(int planned) const {
+    if (one_launch()) return planned;
+    return std::min({planned, dev::kMaxCtas, loopback_ ? std::max(1, 128 / nranks_) : dev::kMaxCtas});
+}
+
 void Communicator::Impl::launch_reduce_ranks(const CollectiveArgs& args, std::vector<dev::CollArgs>& per_rank,
                                              int pack_bytes, bool nvls, int grid) {
     kernels::LaunchConfig cfg;
-    cfg.grid = std::min(grid, dev::kMaxCtas);
-    cfg.block = tuning_.block_threads;
+    cfg.grid = direct_grid(grid);
+    cfg.block = one_launch() ? tuning_.one_device_block_threads : tuning_.block_threads;
     cfg.nvls_unroll = tuning_.nvls_unroll;
-    if (loopback_) cfg.grid = std::min(cfg.grid, std::max(1, 128 / nranks_));  // one cooperative launch: keep it resident
     for (auto& a : per_rank) {
         // Everything that must be equal on every rank for the kernels to meet: a rank that planned
         // differently (another buffer kind, alignment or size) is told so by the first barrier.
         a.plan_hash = plan_fingerprint({static_cast<unsigned long long>(last_.collective), static_cast<unsigned long long>(last_.algo),
                                         static_cast<unsigned long long>(cfg.grid), static_cast<unsigned long long>(pack_bytes),
-                                        a.len, static_cast<unsigned long long>(a.shard_mode), static_cast<unsigned long long>(a.store_all), a.tail,
+                                        a.len, static_cast<unsigned long long>(a.shard_mode), static_cast<unsigned long long>(a.store_all), a.tail, a.head,
                                         a.user_in != nullptr, a.user_out != nullptr, static_cast<unsigned long long>(args.dtype),
                                         static_cast<unsigned long long>(args.redop), nvls});
     }
@@ -742,9 +751,8 @@ void Communicator::Impl::launch_reduce_ranks(const CollectiveArgs& args, std::ve
 void Communicator::Impl::launch_gather_ranks(const CollectiveArgs& args, std::vector<dev::GatherArgs>& per_rank,
                                              int grid) {
     kernels::LaunchConfig cfg;
-    cfg.grid = std::min(grid, dev::kMaxCtas);
-    cfg.block = tuning_.block_threads;
-    if (loopback_) cfg.grid = std::min(cfg.grid, std::max(1, 128 / nranks_));
+    cfg.grid = direct_grid(grid);
+    cfg.block = one_launch() ? tuning_.one_device_block_threads : tuning_.block_threads;
     for (auto& a : per_rank)
         a.plan_hash = plan_fingerprint({static_cast<unsigned long long>(Collective::AllGather), static_cast<unsigned long long>(cfg.grid),
                                         a.len, a.out_stride, static_cast<unsigned long long>(a.mode),
@@ -1070,7 +1078,8 @@ void Communicator::Impl::launch_all_reduce(const CollectiveArgs& args, const sch
     // one common offset; a single process sees every pointer. (Shard boundaries are counted in
     // packs, so all ranks must use the same pack.)
     const bool staged = plan.stage_in || plan.stage_out;
-    bool wide32 = packs && tuning_.wide32 && plan.algo == Algo::TwoShot && (!staged || (args.count * esz) % 32 == 0);
+    const bool may_wide32 = tuning_.wide32 && (plan.algo == Algo::TwoShot || (loopback_ && oneshot)) && (!staged || (args.count * esz) % 32 == 0);
+    bool wide32 = packs && may_wide32;
     auto aligned32 = [](const void* p) { return (reinterpret_cast<std::uintptr_t>(p) & 31u) == 0; };
     if (wide32 && !plan.stage_in) {
         if (in_win != nullptr) wide32 = aligned32(static_cast<const char*>(windows_[in_win[0].region].ptr[0]) + in_win[0].offset);
@@ -1080,16 +1089,31 @@ void Communicator::Impl::launch_all_reduce(const CollectiveArgs& args, const sch
         if (out_win != nullptr) wide32 = aligned32(static_cast<const char*>(windows_[out_win[0].region].ptr[0]) + out_win[0].offset);
         else for (const void* p : args.recv_buffers) wide32 = wide32 && aligned32(p);
     }
+    // Buffers that are all misaligned alike (x[1:] of aligned tensors), where one process sees them: the elements before the
+    // first 16-byte boundary are taken one by one like those behind the last pack (two-shot, 4 ranks, 32 MiB: 223 us when every element went that way, 41 us, as aligned).
+    std::size_t head = 0;
+    if (direct && !staged && !packs) {
+        std::uintptr_t differ = 0;
+        const auto first = reinterpret_cast<std::uintptr_t>(args.send_buffers[0]);
+        for (const void* p : args.send_buffers) differ |= reinterpret_cast<std::uintptr_t>(p) ^ first;
+        for (const void* p : args.recv_buffers) differ |= reinterpret_cast<std::uintptr_t>(p) ^ first;
+        const std::size_t before = (32 - (first & 31u)) & 31u, before16 = before & 15u;
+        if ((differ & 15u) == 0 && args.count * esz >= 32 + before) {
+            packs = true;
+            wide32 = may_wide32 && (differ & 31u) == 0;
+            head = (wide32 ? before : before16) / esz;
+        }
+    }
     const std::size_t pack = wide32 ? 32 : (packs ? 16 : esz);
-    const std::size_t total_packs = args.count * esz / pack;
-    const std::size_t tail = (args.count * esz - total_packs * pack) / esz;  // not 0 only in an unstaged call, which is one launch
+    const std::size_t total_packs = (args.count - head) * esz / pack;
+    const std::size_t tail = ((args.count - head) * esz - total_packs * pack) / esz;  // not 0 only in an unstaged call, which is one launch
     const std::size_t cap_packs = staged ? staging_half_ / pack : std::max<std::size_t>(total_packs, 1);
 
     for (std::size_t done = 0; done < std::max<std::size_t>(total_packs, 1); done += cap_packs) {
         const std::size_t len = std::min(cap_packs, total_packs - done);
-        const std::size_t off = done * pack;
-        std::vector<dev::CollArgs> per(local_.size());
-        for (std::size_t i = 0; i < local_.size(); ++i) {
+        const std::size_t off = head * esz + done * pack;
+        std::vector<dev::CollArgs> per(one_launch() ? 1 : local_.size());
+        for (std::size_t i = 0; i < per.size(); ++i) {
             dev::CollArgs& a = per[i];
             fill_common(a, local_[i]);
             a.len = len;
@@ -1109,10 +1133,15 @@ void Communicator::Impl::launch_all_reduce(const CollectiveArgs& args, const sch
                     a.out[p] = static_cast<char*>(windows_[out_win[i].region].ptr[p]) + out_win[i].offset + off;
                 else if (direct) a.out[p] = static_cast<char*>(args.recv_buffers[p]) + off;
             }
-            if (oneshot) a.out[local_[i].grank] = static_cast<char*>(args.recv_buffers[i]) + off;
+            // Outputs that only their own rank writes.
+            if (oneshot) {
+                if (one_launch()) for (int p = 0; p < nranks_; ++p) a.out[p] = static_cast<char*>(args.recv_buffers[p]) + off;
+                else a.out[local_[i].grank] = static_cast<char*>(args.recv_buffers[i]) + off;
+            }
             if (plan.stage_in) a.user_in = static_cast<const char*>(args.send_buffers[i]) + off;
             if (plan.stage_out) a.user_out = static_cast<char*>(args.recv_buffers[i]) + off;
             a.tail = static_cast<unsigned>(tail);
+            a.head = static_cast<unsigned>(head);
             a.in_extent = a.out_extent = len;  // what in[p] and out[p] address, in packs (checking builds compare against it)
 #if defined(B200CCL_DEBUG_BOUNDS)
             // Test hook of the checking build: pretend the buffers are this many packs shorter, as a
@@ -1143,8 +1172,8 @@ void Communicator::Impl::launch_reduce_scatter(const CollectiveArgs& args, const
     for (std::size_t done = 0; done < block_packs; done += cap_packs) {
         const std::size_t len = std::min(cap_packs, block_packs - done);
         const std::size_t off = done * pack;
-        std::vector<dev::CollArgs> per(local_.size());
-        for (std::size_t i = 0; i < local_.size(); ++i) {
+        std::vector<dev::CollArgs> per(one_launch() ? 1 : local_.size());
+        for (std::size_t i = 0; i < per.size(); ++i) {
             dev::CollArgs& a = per[i];
             fill_common(a, local_[i]);
             a.len = len;
@@ -1159,7 +1188,8 @@ void Communicator::Impl::launch_reduce_scatter(const CollectiveArgs& args, const
                     a.in[p] = static_cast<const char*>(windows_[in_win[i].region].ptr[p]) + in_win[i].offset + off;
                 else if (direct) a.in[p] = static_cast<const char*>(args.send_buffers[p]) + off;
             }
-            a.out[local_[i].grank] = static_cast<char*>(args.recv_buffers[i]) + off;
+            if (one_launch()) for (int p = 0; p < nranks_; ++p) a.out[p] = static_cast<char*>(args.recv_buffers[p]) + off;
+            else a.out[local_[i].grank] = static_cast<char*>(args.recv_buffers[i]) + off;
             a.in_extent = a.in_stride * static_cast<std::size_t>(nranks_ - 1) + len;
             a.out_extent = len;
             if (plan.stage_in) a.user_in = static_cast<const char*>(args.send_buffers[i]) + off;
@@ -1187,8 +1217,8 @@ void Communicator::Impl::launch_all_gather(const CollectiveArgs& args, const sch
     for (std::size_t done = 0; done < block_packs; done += cap_packs) {
         const std::size_t len = std::min(cap_packs, block_packs - done);
         const std::size_t off = done * pack;
-        std::vector<dev::GatherArgs> per(local_.size());
-        for (std::size_t i = 0; i < local_.size(); ++i) {
+        std::vector<dev::GatherArgs> per(one_launch() ? 1 : local_.size());
+        for (std::size_t i = 0; i < per.size(); ++i) {
             dev::GatherArgs& a = per[i];
             std::memset(&a, 0, sizeof(a));
             for (int p = 0; p < nranks_; ++p) a.ctrl[p] = static_cast<dev::ControlBlock*>(ctrl_->rank_ptr(p));
@@ -1212,7 +1242,8 @@ void Communicator::Impl::launch_all_gather(const CollectiveArgs& args, const sch
                     else if (direct) a.out[p] = static_cast<char*>(args.recv_buffers[p]) + off;
                 }
             }
-            if (plan.gather_mode != 1) a.in[local_[i].grank] = static_cast<const char*>(args.send_buffers[i]) + off;
+            if (plan.gather_mode == 0 && one_launch()) for (int p = 0; p < nranks_; ++p) a.in[p] = static_cast<const char*>(args.send_buffers[p]) + off;
+            else if (plan.gather_mode != 1) a.in[local_[i].grank] = static_cast<const char*>(args.send_buffers[i]) + off;
             if (plan.gather_mode != 0) a.out[local_[i].grank] = static_cast<char*>(args.recv_buffers[i]) + off;
             if (plan.stage_in) a.user_in = static_cast<const char*>(args.send_buffers[i]) + off;
             if (plan.gather_mode == 2)

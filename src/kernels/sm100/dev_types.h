@@ -19,9 +19,10 @@ constexpr int kLlCtas = 8;                  // the low-latency kernel always run
 constexpr unsigned kLlMaxBytes = 128u << 10; // largest message it takes
 constexpr unsigned kLlMaxWords = kLlMaxBytes / 4;
 
-// Emulated ranks are part of one launch on one GPU: they order their stores at GPU scope, and their plans cannot differ.
-// In the checking build they do what ranks on GPUs of their own do instead (system scope, plan fingerprints, a ring of
-// one group of warps that returns credits early), so that one GPU can run those paths. Numbers never come from it.
+// Emulated ranks are part of one launch on one GPU: their plans cannot differ, those of the direct kernels need not wait for
+// one another, and those of the ring order their stores at GPU scope. In the checking build they do what ranks on GPUs of
+// their own do instead (flags at system scope, plan fingerprints, a ring of one group of warps that returns credits early), so
+// that one GPU can run those paths. Numbers never come from it.
 #if defined(B200CCL_DEBUG_BOUNDS)
 constexpr bool kRanksShareGpu = false;
 #else
@@ -110,6 +111,7 @@ struct CollArgs {
     int shard_mode;     // ShardMode
     int store_all;      // 1 → store the reduced pack into every rank's `out`; 0 → own only
     unsigned int tail;  // Whole/Split, unstaged: elements behind the last pack, too few for another one
+    unsigned int head;  // likewise: elements before the first pack, where all buffers are misaligned alike; in[] and out[] point behind them
 };
 
 // AllGather moves bytes only.
@@ -150,6 +152,13 @@ struct LlArgs {
 template <typename A>
 struct LoopPack {
     A r[kMaxRanks];
+};
+
+// What emulated ranks of the direct kernels share: the same buffers, no flags; the rank is blockIdx.y. A launch is fastest with parameters of this size, modulo 64 (see local_collectives.cu).
+template <typename A>
+struct OneGpu {
+    A a;
+    char pad[(24 + 64 - sizeof(A) % 64) % 64];
 };
 
 }  // namespace b200ccl::dev

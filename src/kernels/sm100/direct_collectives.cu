@@ -17,6 +17,8 @@
 #include "kernels/sm100/sync.cuh"
 #include "kernels/sm100/vec.cuh"
 
+#include <type_traits>
+
 namespace b200ccl::kernels {
 
 using namespace b200ccl::dev;
@@ -25,16 +27,60 @@ namespace {
 
 using u64 = unsigned long long;
 
-// A kernel parameter is either one rank's arguments, or (loopback emulation) the arguments of
-// every emulated rank, of which the CTA picks the one of rank blockIdx.y.
+// A kernel parameter is one rank's arguments, or what all emulated ranks share (OneGpu), or, in the checking build, the
+// arguments of every emulated rank (LoopPack), of which the CTA picks the one of rank blockIdx.y.
 template <typename A>
 __device__ __forceinline__ const A& select_args(const A& one) { return one; }
 template <typename A>
 __device__ __forceinline__ const A& select_args(const LoopPack<A>& all) { return all.r[blockIdx.y]; }
 template <typename A>
+__device__ __forceinline__ const A& select_args(const OneGpu<A>& all) { return all.a; }
+template <typename A>
 constexpr bool kAllRanksHere = false;
 template <typename A>
-constexpr bool kAllRanksHere<LoopPack<A>> = kRanksShareGpu;
+constexpr bool kAllRanksHere<OneGpu<A>> = true;
+
+// Emulated ranks are part of one launch: what it finds in memory is every rank's input and its end is every rank's, and no
+// rank reads what another one writes (rank r alone reads and writes shard r). So they have nothing to meet for; the launch
+// need not be cooperative nor resident all at once, a rank has one CTA for every 8 KiB that it stores to each output, and the launch is a programmatic
+// dependent of the one before. As one cooperative launch of CTAs that stayed and met over flags, kernels also followed one
+// another only every 2.05 us. Meeting in thread block clusters (1 x ranks) costs little in small calls, but leaves too few
+// loads in flight in large ones. bf16 two-shot, us before / in clusters of 512 threads / now: 4 ranks, 4 KiB 6.1 / 3.1 / 3.1,
+// 2 MiB 8.2 / 5.7 / 3.7, 8 MiB 16.4 / 14.4 / 11.7 (5.7 TB/s), 256 MiB 346 / 337 / 311 (6.9 TB/s); 8 ranks, 8 MiB 28.5 / 32.5 / 22.5, 256 MiB
+// 649 / 870 / 625; one-shot, which is bound by reading every input once per rank through L2: 8 ranks, 4 MiB 36.6 / 71.2 / 23.0.
+
+// Starts a call, behind the launch before it.
+template <typename ParamT>
+__device__ __forceinline__ void begin_call() {
+    if constexpr (kAllRanksHere<ParamT>) {
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
+}
+
+// Where ranks on GPUs of their own meet over flags; `epoch` counts the meetings. False when a wait gave up.
+template <typename ParamT, typename A>
+__device__ __forceinline__ bool meet(const A& a, int rank, int n, u64& epoch, unsigned where, u64 plan_hash) {
+    if constexpr (kAllRanksHere<ParamT>) {
+        return true;
+    } else {
+        ++epoch;
+        return cta_barrier_all_ranks(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, where, plan_hash);
+    }
+}
+
+// How many meetings this CTA has been through.
+template <typename ParamT>
+__device__ __forceinline__ u64 read_epoch(const ControlBlock* own) {
+    if constexpr (kAllRanksHere<ParamT>) {
+        return 0;
+    } else {
+        __shared__ u64 s_epoch;
+        if (threadIdx.x == 0) s_epoch = own->epoch[blockIdx.x];
+        __syncthreads();
+        return s_epoch;
+    }
+}
 
 // Copies the packs first, first+stripe, ... below len, four loads in flight per thread. One side is
 // the caller's own buffer (16-byte aligned at most), the other the staging arena.
@@ -85,18 +131,17 @@ reduce_kernel(const __grid_constant__ ParamT param) {
     using Raw = typename P::Raw;
     constexpr int kElems = P::kElems;
     constexpr int NN = N > 0 ? N : kMaxRanks;
-    // For the multimem variant the N slot carries the unroll factor (the rank count is a run-time value there).
-    constexpr int kU = kNvls ? (N > 0 ? N : 4) : UnrollFor<N, P::kBytes>::value;
+    // For the multimem variant the N slot carries the unroll factor (the rank count is a run-time value there). Emulated ranks
+    // take 32 bytes per thread and peer, or 16 from five ranks up where those are the packs.
+    constexpr int kU = kNvls ? (N > 0 ? N : 4) : (kAllRanksHere<ParamT> ? (P::kBytes == 16 && N <= 4 ? 2 : 1) : UnrollFor<N, P::kBytes>::value);
 
-    __shared__ u64 s_epoch;
     const CollArgs& a = select_args(param);
+    begin_call<ParamT>();
 
     const int n = (N > 0 && !kNvls) ? N : a.nranks;
-    const int rank = a.rank;
-    ControlBlock* own = a.ctrl[rank];
-    if (threadIdx.x == 0) s_epoch = own->epoch[blockIdx.x];
-    __syncthreads();
-    u64 epoch = s_epoch;
+    const int rank = kAllRanksHere<ParamT> ? (int)blockIdx.y : a.rank;
+    ControlBlock* own = kAllRanksHere<ParamT> ? nullptr : a.ctrl[rank];
+    u64 epoch = read_epoch<ParamT>(own);
 
     const u64 stripe = (u64)gridDim.x * blockDim.x;
     const u64 first = (u64)blockIdx.x * blockDim.x + threadIdx.x;
@@ -120,8 +165,7 @@ reduce_kernel(const __grid_constant__ ParamT param) {
     }
 
     // 2. Every rank's input is ready (and every rank's previous use of `out` is over).
-    ++epoch;
-    if (!cta_barrier_all_ranks<kAllRanksHere<ParamT>>(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 1u, a.plan_hash, a.user_in == nullptr)) return;
+    if (!meet<ParamT>(a, rank, n, epoch, 1u, a.plan_hash)) return;
 
     // 3. Reduce the own shard.
     {
@@ -207,23 +251,24 @@ reduce_kernel(const __grid_constant__ ParamT param) {
         }
     }
 
-    // 3b. The elements of a ragged message that fill no pack, one per thread of CTA 0, in the last rank's shard.
+    // 3b. The elements of a ragged or misaligned message that fill no pack, one per thread of CTA 0, in the last rank's shard.
     if constexpr (!kNvls) {
-        if (a.tail != 0 && blockIdx.x == 0 && threadIdx.x < a.tail && (mode == kShardWhole || rank == n - 1)) {
-            const u64 e = a.len * kElems + threadIdx.x;
-            float acc = Elem<T>::to_f(Narrow<T>::load(a.in[0], e));
-            for (int p = 1; p < n; ++p) acc = Op::apply(acc, Elem<T>::to_f(Narrow<T>::load(a.in[p], e)));
+        const unsigned ends = a.head + a.tail;  // at most 14 + 15
+        if (ends != 0 && blockIdx.x == 0 && threadIdx.x < ends && (mode == kShardWhole || rank == n - 1)) {
+            const u64 e = threadIdx.x < a.head ? threadIdx.x : a.len * kElems + threadIdx.x;
+            auto first = [&](const void* base) { return static_cast<const T*>(base) - a.head; };
+            float acc = Elem<T>::to_f(Narrow<T>::load(first(a.in[0]), e));
+            for (int p = 1; p < n; ++p) acc = Op::apply(acc, Elem<T>::to_f(Narrow<T>::load(first(a.in[p]), e)));
             if (a.scale != 1.0f) acc *= a.scale;
             const T v = Elem<T>::from_f(acc);
             if (a.store_all)
-                for (int q = 0; q < n; ++q) static_cast<T*>(a.out[q])[e] = v;
-            else static_cast<T*>(a.out[rank])[e] = v;
+                for (int q = 0; q < n; ++q) const_cast<T*>(first(a.out[q]))[e] = v;
+            else const_cast<T*>(first(a.out[rank]))[e] = v;
         }
     }
 
     // 4. Every rank has finished reading inputs and its stores to peers are visible.
-    ++epoch;
-    if (!cta_barrier_all_ranks<kAllRanksHere<ParamT>>(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 2u)) return;
+    if (!meet<ParamT>(a, rank, n, epoch, 2u, 0ull)) return;
 
     // 5. Staged output: copy what the same-numbered CTAs of all ranks stored into the arena.
     if (a.user_out != nullptr) {
@@ -232,7 +277,7 @@ reduce_kernel(const __grid_constant__ ParamT param) {
             copy_stripes<P, false>(a.user_out, lo, a.out[rank], lo, first, len, stripe);
         }
     }
-    if (threadIdx.x == 0) own->epoch[blockIdx.x] = epoch;
+    if (!kAllRanksHere<ParamT> && threadIdx.x == 0) own->epoch[blockIdx.x] = epoch;
 }
 
 // AllGather: bytes only. push: store the own block into every rank's output; pull: load every
@@ -240,13 +285,11 @@ reduce_kernel(const __grid_constant__ ParamT param) {
 template <typename RawT, typename ParamT>
 __global__ void __launch_bounds__(kBlockThreads)
 gather_kernel(const __grid_constant__ ParamT param) {
-    __shared__ u64 s_epoch;
     const GatherArgs& a = select_args(param);
-    const int n = a.nranks, rank = a.rank;
-    ControlBlock* own = a.ctrl[rank];
-    if (threadIdx.x == 0) s_epoch = own->epoch[blockIdx.x];
-    __syncthreads();
-    u64 epoch = s_epoch;
+    begin_call<ParamT>();
+    const int n = a.nranks, rank = kAllRanksHere<ParamT> ? (int)blockIdx.y : a.rank;
+    ControlBlock* own = kAllRanksHere<ParamT> ? nullptr : a.ctrl[rank];
+    u64 epoch = read_epoch<ParamT>(own);
     const u64 stripe = (u64)gridDim.x * blockDim.x;
     const u64 first = (u64)blockIdx.x * blockDim.x + threadIdx.x;
     constexpr bool kWide = sizeof(RawT) == 16;
@@ -263,8 +306,7 @@ gather_kernel(const __grid_constant__ ParamT param) {
         void* stage = const_cast<void*>(a.in[rank]);
         for (u64 j = first; j < a.len; j += stripe) store(stage, j, load(a.user_in, j));
     }
-    ++epoch;
-    if (!cta_barrier_all_ranks<kAllRanksHere<ParamT>>(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 1u, a.plan_hash, a.user_in == nullptr)) return;
+    if (!meet<ParamT>(a, rank, n, epoch, 1u, a.plan_hash)) return;
 
     if (a.mode == 0) {
         const u64 base = (u64)rank * a.out_stride;
@@ -301,20 +343,44 @@ gather_kernel(const __grid_constant__ ParamT param) {
         }
     }
 
-    ++epoch;
-    if (!cta_barrier_all_ranks<kAllRanksHere<ParamT>>(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 2u)) return;
-    if (threadIdx.x == 0) own->epoch[blockIdx.x] = epoch;
+    if (!meet<ParamT>(a, rank, n, epoch, 2u, 0ull)) return;
+    if (!kAllRanksHere<ParamT> && threadIdx.x == 0) own->epoch[blockIdx.x] = epoch;
 }
 
 // ---- launch helpers ------------------------------------------------------------------------
+
+template <typename A>
+using EmulatedRanks = std::conditional_t<kRanksShareGpu, OneGpu<A>, LoopPack<A>>;
+
+// Nothing is staged on one GPU.
+template <typename A>
+bool fill(OneGpu<A>& all, const A* args, int) {
+    all.a = args[0];
+    return args[0].user_in == nullptr;
+}
+template <typename A>
+bool fill(LoopPack<A>& all, const A* args, int ranks) {
+    for (int r = 0; r < ranks; ++r) all.r[r] = args[r];
+    return true;
+}
 
 template <typename ParamT>
 cudaError_t launch(void (*kernel)(ParamT), const ParamT& param, const LaunchConfig& cfg) {
     dim3 grid(cfg.grid, cfg.loop_ranks > 0 ? cfg.loop_ranks : 1, 1);
     dim3 block(cfg.block, 1, 1);
-    if (cfg.loop_ranks > 0) {
-        // The emulated ranks wait for one another inside one launch: all CTAs must be resident,
-        // which a cooperative launch checks.
+    if constexpr (kAllRanksHere<ParamT>) {
+        cudaLaunchAttribute attrs[1];
+        attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attrs[0].val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t config = {};
+        config.gridDim = grid;
+        config.blockDim = block;
+        config.stream = cfg.stream;
+        config.attrs = attrs;
+        config.numAttrs = 1;
+        return cudaLaunchKernelEx(&config, kernel, param);
+    } else if (cfg.loop_ranks > 0) {
+        // Emulated ranks that wait for one another over flags: all CTAs must be resident, which a cooperative launch checks.
         void* params[] = {const_cast<ParamT*>(&param)};
         return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), grid, block, params, 0,
                                            cfg.stream);
@@ -333,6 +399,15 @@ cudaError_t launch_reduce_n(int nranks, const ParamT& param, const LaunchConfig&
     } else if constexpr (PackT<T>::kBytes < 16) {
         return launch(reduce_kernel<T, Op, 0, PackT, false, ParamT>, param, cfg);
     } else {
+        if constexpr (kAllRanksHere<ParamT>) {
+            switch (nranks) {
+                case 3: return launch(reduce_kernel<T, Op, 3, PackT, false, ParamT>, param, cfg);
+                case 5: return launch(reduce_kernel<T, Op, 5, PackT, false, ParamT>, param, cfg);
+                case 6: return launch(reduce_kernel<T, Op, 6, PackT, false, ParamT>, param, cfg);
+                case 7: return launch(reduce_kernel<T, Op, 7, PackT, false, ParamT>, param, cfg);
+                default: break;
+            }
+        }
         switch (nranks) {
             case 2: return launch(reduce_kernel<T, Op, 2, PackT, false, ParamT>, param, cfg);
             case 4: return launch(reduce_kernel<T, Op, 4, PackT, false, ParamT>, param, cfg);
@@ -365,9 +440,9 @@ cudaError_t launch_reduce_t(RedOp op, int pack_bytes, bool nvls, const CollArgs*
     const int n = args[0].nranks;
     if (cfg.loop_ranks > 0) {
         if (nvls || cfg.loop_ranks > kMaxRanks) return cudaErrorInvalidValue;
-        LoopPack<CollArgs> pack;
-        for (int r = 0; r < cfg.loop_ranks; ++r) pack.r[r] = args[r];
-        return launch_reduce_pack<T>(op, pack_bytes, n, pack, cfg);
+        EmulatedRanks<CollArgs> all;
+        if (!fill(all, args, cfg.loop_ranks)) return cudaErrorInvalidValue;
+        return launch_reduce_pack<T>(op, pack_bytes, n, all, cfg);
     }
     if (nvls) {
         if (pack_bytes != 16 || (op != RedOp::Sum && op != RedOp::Avg)) return cudaErrorInvalidValue;
@@ -380,9 +455,9 @@ template <typename RawT>
 cudaError_t launch_gather_t(const GatherArgs* args, const LaunchConfig& cfg) {
     if (cfg.loop_ranks > 0) {
         if (cfg.loop_ranks > kMaxRanks) return cudaErrorInvalidValue;
-        LoopPack<GatherArgs> pack;
-        for (int r = 0; r < cfg.loop_ranks; ++r) pack.r[r] = args[r];
-        return launch(gather_kernel<RawT, LoopPack<GatherArgs>>, pack, cfg);
+        EmulatedRanks<GatherArgs> all;
+        if (!fill(all, args, cfg.loop_ranks)) return cudaErrorInvalidValue;
+        return launch(gather_kernel<RawT, EmulatedRanks<GatherArgs>>, all, cfg);
     }
     return launch(gather_kernel<RawT, GatherArgs>, args[0], cfg);
 }

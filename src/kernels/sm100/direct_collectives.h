@@ -9,11 +9,11 @@
 namespace b200ccl::kernels {
 
 struct LaunchConfig {
-    int grid = 1;    // CTAs per rank (≤ dev::kMaxCtas)
+    int grid = 1;    // CTAs per rank (≤ dev::kMaxCtas where ranks meet over flags)
     int block = dev::kBlockThreads;
     cudaStream_t stream = nullptr;
-    // Loopback emulation: one cooperative launch plays `loop_ranks` ranks (blockIdx.y = rank)
-    // and `args` points to that many argument structs. 0 → normal launch of args[0].
+    // Loopback emulation: one launch plays `loop_ranks` ranks (blockIdx.y = rank), with the tables of args[0] for all of them.
+    // (Checking build: a cooperative launch, `args` points to one struct per rank.) 0 → normal launch of args[0].
     int loop_ranks = 0;
     int nvls_unroll = 2;  // multimem loads in flight per thread (1, 2, 4 or 8)
 };

@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(kThreads, 1) pipeline_kernel(const __grid_cons
 
     // Every rank is inside this call (so nobody still uses the arena for an earlier one) and
     // launched it with the same plan.
-    if (!cta_barrier_all_ranks<false>(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 50u, a.plan_hash)) return;
+    if (!cta_barrier_all_ranks(a.ctrl, rank, n, epoch, a.timeout_ns, a.status, 50u, a.plan_hash)) return;
 
     const u64 total_tiles = (a.bytes + a.tile_bytes - 1) / a.tile_bytes;
     const u64 K = cta < total_tiles ? (total_tiles - cta + gridDim.x - 1) / gridDim.x : 0;  // tiles cta, cta + grid, ...

@@ -29,9 +29,6 @@ __device__ __forceinline__ void st_release_sys(unsigned long long* p, unsigned l
 __device__ __forceinline__ void st_release_gpu(unsigned long long* p, unsigned long long v) {
     asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-__device__ __forceinline__ void st_relaxed_gpu(unsigned long long* p, unsigned long long v) {
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
 __device__ __forceinline__ void st_relaxed_sys(unsigned long long* p, unsigned long long v) {
     asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
@@ -104,31 +101,22 @@ __device__ __forceinline__ bool wait_at_least(const unsigned long long* flag, un
 
 // Barrier among the CTAs with the same blockIdx.x on every rank. Thread p signals rank p and
 // waits for rank p. Everything the CTA stored before the call is visible to every rank's CTA
-// after it (release on the signal, acquire on the poll, bar.sync on both sides), except where the caller says
-// that it has stored nothing (`nothing_stored`, below).
+// after it (release on the signal, acquire on the poll, bar.sync on both sides).
 // Returns false (to every thread of the CTA) when the wait gave up.
 // plan_hash != 0: CTA 0 also publishes the fingerprint of this launch's plan with the signal and
 // compares it with every peer's after the wait; a difference ends the collective on every rank
 // with kStatusPlanMismatch (the other CTAs leave through the abort word).
-// kOneGpu: every rank is part of this launch, so that GPU scope orders them all; and what the launch found in memory is
-// every rank's anyway, so that a CTA which has stored nothing yet (`nothing_stored`) need not release anything (two-shot
-// of 8 ranks, 4 KiB: 8.6 us, 6.8 us without the release; 4 ranks, 8 MiB: 17.5 and 17.2 us). Their plans come from one
-// host call and cannot differ: no fingerprints.
-template <bool kOneGpu>
 __device__ __forceinline__ bool cta_barrier_all_ranks(ControlBlock* const* ctrl, int rank, int nranks,
                                                       unsigned long long epoch, unsigned long long timeout_ns,
                                                       Status* status, unsigned int where,
-                                                      unsigned long long plan_hash = 0ull,
-                                                      bool nothing_stored = false) {
+                                                      unsigned long long plan_hash = 0ull) {
     __syncthreads();
     int ok = 1;
     if (threadIdx.x < (unsigned)nranks) {
         const int p = threadIdx.x;
-        const bool check = !kOneGpu && plan_hash != 0ull && blockIdx.x == 0;
+        const bool check = plan_hash != 0ull && blockIdx.x == 0;
         if (check) st_relaxed_sys(&ctrl[p]->plan_hash[rank], plan_hash);
-        if (kOneGpu && nothing_stored) st_relaxed_gpu(&ctrl[p]->barrier[blockIdx.x][rank], epoch);
-        else if (kOneGpu) st_release_gpu(&ctrl[p]->barrier[blockIdx.x][rank], epoch);
-        else st_release_sys(&ctrl[p]->barrier[blockIdx.x][rank], epoch);
+        st_release_sys(&ctrl[p]->barrier[blockIdx.x][rank], epoch);
         ok = wait_at_least(&ctrl[rank]->barrier[blockIdx.x][p], epoch, ctrl[rank], timeout_ns,
                            status, ctrl, nranks, (unsigned)p, where)
                  ? 1 : 0;

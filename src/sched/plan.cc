@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <fstream>
+#include <limits>
 #include <sstream>
 #include <stdexcept>
 
@@ -100,16 +101,16 @@ Tuning tuning_from_text(const std::string& text, const Tuning& base, const std::
         else if (key == "max_ctas") t.max_ctas = t.one_device_max_ctas = std::max(as_int, 1);
         else if (key == "nvls_max_ctas") t.nvls_max_ctas = t.nvls_staged_max_ctas = std::max(as_int, 1);
         else if (key == "nvls_staged_max_ctas") t.nvls_staged_max_ctas = std::max(as_int, 1);
-        else if (key == "twoshot_max_ctas") t.twoshot_max_ctas = std::max(as_int, 1);
+        else if (key == "twoshot_max_ctas") t.twoshot_max_ctas = t.one_device_twoshot_max_ctas = std::max(as_int, 1);
         else if (key == "nvls_unroll") t.nvls_unroll = as_int;
-        else if (key == "bytes_per_cta") t.bytes_per_cta = std::max<std::size_t>(bytes, 1);
+        else if (key == "bytes_per_cta") t.bytes_per_cta = t.one_device_bytes_per_cta = std::max<std::size_t>(bytes, 1);
         else if (key == "oneshot_bytes_per_cta") t.oneshot_bytes_per_cta = std::max<std::size_t>(bytes, 1);
         else if (key == "ll_max_bytes") t.ll_max_bytes = t.ll_max_bytes_upto4 = std::min(bytes, kLlPlanMaxBytes);
         else if (key == "ll_max_bytes_upto4") t.ll_max_bytes_upto4 = std::min(bytes, kLlPlanMaxBytes);
         else if (key == "wide32") t.wide32 = bytes != 0;
         else if (key == "block_threads") {
             if (as_int < 32 || as_int > 512 || as_int % 32 != 0) throw std::invalid_argument(where + "block_threads must be a multiple of 32 between 32 and 512");
-            t.block_threads = as_int;
+            t.block_threads = t.one_device_block_threads = as_int;
         }
         else if (key == "pipeline_min_bytes") t.pipeline_min_bytes = t.pipeline_min_bytes_upto4 = bytes;
         else if (key == "pipeline_min_bytes_upto4") t.pipeline_min_bytes_upto4 = bytes;
@@ -146,7 +147,7 @@ Tuning tuning_from_env() {
     if (env::get("B200CCL_NVLS_MAX_CTAS"))
         t.nvls_max_ctas = t.nvls_staged_max_ctas = static_cast<int>(env::get_int("B200CCL_NVLS_MAX_CTAS", t.nvls_max_ctas));
     t.nvls_unroll = static_cast<int>(env::get_int("B200CCL_NVLS_UNROLL", t.nvls_unroll));
-    t.bytes_per_cta = env::get_bytes("B200CCL_BYTES_PER_CTA", t.bytes_per_cta);
+    if (env::get("B200CCL_BYTES_PER_CTA")) t.bytes_per_cta = t.one_device_bytes_per_cta = env::get_bytes("B200CCL_BYTES_PER_CTA", 0);
     t.oneshot_bytes_per_cta = env::get_bytes("B200CCL_ONESHOT_BYTES_PER_CTA", t.oneshot_bytes_per_cta);
     if (env::get("B200CCL_LL_MAX_BYTES"))
         t.ll_max_bytes = t.ll_max_bytes_upto4 = std::min<std::size_t>(env::get_bytes("B200CCL_LL_MAX_BYTES", 0), kLlPlanMaxBytes);
@@ -154,6 +155,7 @@ Tuning tuning_from_env() {
     t.block_threads = static_cast<int>(env::get_int("B200CCL_BLOCK_THREADS", t.block_threads, "NANO_NCCL_BLOCK_THREADS"));
     if (t.block_threads < 32 || t.block_threads > 512 || t.block_threads % 32 != 0)
         throw std::invalid_argument("B200CCL_BLOCK_THREADS must be a multiple of 32 between 32 and 512");
+    if (env::get("B200CCL_BLOCK_THREADS") || env::get("NANO_NCCL_BLOCK_THREADS")) t.one_device_block_threads = t.block_threads;
     if (env::get("B200CCL_PIPELINE_MIN_BYTES"))
         t.pipeline_min_bytes = t.pipeline_min_bytes_upto4 = env::get_bytes("B200CCL_PIPELINE_MIN_BYTES", 0);
     t.pipeline_nvls_unroll = std::max(1, static_cast<int>(env::get_int("B200CCL_PIPELINE_NVLS_UNROLL", t.pipeline_nvls_unroll)));
@@ -170,8 +172,8 @@ std::size_t message_bytes(const CallShape& s) {
 
 namespace {
 
-int grid_for(std::size_t bytes_this_rank_handles, const Tuning& t, int cap, std::size_t per_cta = 0) {
-    const std::size_t per = std::max<std::size_t>(per_cta ? per_cta : t.bytes_per_cta, 1);
+int grid_for(std::size_t bytes_this_rank_handles, int cap, std::size_t per_cta) {
+    const std::size_t per = std::max<std::size_t>(per_cta, 1);
     std::size_t g = (bytes_this_rank_handles + per - 1) / per;
     g = std::max<std::size_t>(g, 1);
     return static_cast<int>(std::min<std::size_t>(g, static_cast<std::size_t>(std::max(cap, 1))));
@@ -199,7 +201,11 @@ bool nvls_usable(const CallShape& s) {
 
 Plan make_plan(const CallShape& s, Algo forced, const Tuning& t) {
     Plan p;
-    const int cap = std::max(1, std::min(s.max_ctas > 0 ? s.max_ctas : t.max_ctas, t.max_ctas));
+    // Ranks on one device need no CTA to stay and loop: of caps only one that somebody asked for counts.
+    const int no_cap = std::numeric_limits<int>::max();
+    const int cap = s.one_device ? (t.one_device_max_ctas > 0 ? t.one_device_max_ctas : no_cap)
+                                 : std::max(1, std::min(s.max_ctas > 0 ? s.max_ctas : t.max_ctas, t.max_ctas));
+    const std::size_t per_cta = s.one_device ? t.one_device_bytes_per_cta : t.bytes_per_cta;
     const std::size_t bytes = message_bytes(s);
     const std::size_t esz = dtype_size(s.dtype);
 
@@ -246,7 +252,7 @@ Plan make_plan(const CallShape& s, Algo forced, const Tuning& t) {
             p.gather_mode = 1;
             p.stage_in = !s.peers_read_input;
         }
-        p.grid = grid_for(s.count * esz * (p.gather_mode == 1 ? s.nranks : 1), t, cap);
+        p.grid = grid_for(s.count * esz * (p.gather_mode == 1 ? s.nranks : 1), cap, per_cta);
         return p;
     }
 
@@ -254,7 +260,7 @@ Plan make_plan(const CallShape& s, Algo forced, const Tuning& t) {
         p.algo = (forced == Algo::Nvls || (forced == Algo::Auto && nvls_ok && bytes >= t.nvls_min_bytes))
                      ? Algo::Nvls : Algo::OneShot;
         p.stage_in = p.algo != Algo::Nvls && !s.peers_read_input;
-        p.grid = grid_for(s.count * esz * (p.stage_in ? s.nranks : 1), t, cap);
+        p.grid = grid_for(s.count * esz * (p.stage_in ? s.nranks : 1), cap, per_cta);
         return p;
     }
 
@@ -312,20 +318,19 @@ Plan make_plan(const CallShape& s, Algo forced, const Tuning& t) {
         // A staged call also copies the whole message in and out with these CTAs, which wants more of them than
         // the switch does (8 ranks, 64 MiB plain: 224 us on 64 CTAs, 236 us on 48).
         const bool staged = p.stage_in || p.stage_out;
-        p.grid = grid_for(bytes / s.nranks * (staged ? s.nranks : 1), t,
-                          std::min(cap, staged ? std::max(t.nvls_max_ctas, t.nvls_staged_max_ctas) : t.nvls_max_ctas));
+        p.grid = grid_for(bytes / s.nranks * (staged ? s.nranks : 1),
+                          std::min(cap, staged ? std::max(t.nvls_max_ctas, t.nvls_staged_max_ctas) : t.nvls_max_ctas), t.bytes_per_cta);
     } else if (algo == Algo::OneShot) {
         p.stage_in = !s.peers_read_input;
-        p.grid = grid_for(bytes, t, cap, t.oneshot_bytes_per_cta);
+        p.grid = grid_for(bytes, cap, t.oneshot_bytes_per_cta);
     } else {
         p.stage_in = !s.peers_read_input;
         p.stage_out = !s.peers_write_output;
         // Staging works on (input arena, output arena) pairs: if either side is staged the
         // kernel still reads/writes the other side in place.
-        // The bytes per CTA are what hides the latency of NVLink; emulated ranks read their own GPU's memory, where more
-        // CTAs with less each are faster (8 ranks, 300001 bf16: 10.9 us with 3 CTAs per rank, 8.5 us with 16).
-        p.grid = grid_for(bytes / s.nranks * (p.stage_in || p.stage_out ? s.nranks : 1), t, std::min(cap, t.twoshot_max_ctas),
-                          s.one_device ? std::max<std::size_t>(t.bytes_per_cta / 8, 1) : 0);
+        // The bytes per CTA are what hides the latency of NVLink.
+        const int most = s.one_device ? (t.one_device_twoshot_max_ctas > 0 ? t.one_device_twoshot_max_ctas : no_cap) : t.twoshot_max_ctas;
+        p.grid = grid_for(bytes / s.nranks * (p.stage_in || p.stage_out ? s.nranks : 1), std::min(cap, most), per_cta);
     }
     return p;
 }

@@ -51,7 +51,13 @@ struct Tuning {
     std::size_t oneshot_max_bytes[kMaxRanks + 1];  // per nranks: AllReduce sizes up to this use one-shot
     std::size_t nvls_min_bytes = 0;                // NVLS from this size up (when available)
     int max_ctas = 128;                            // hard cap for every algorithm (B200CCL_MAX_CTAS)
-    int one_device_max_ctas = 0;                   // the cap that somebody asked for, of any size; 0: nobody did (one-device kernel)
+    int one_device_max_ctas = 0;                   // the cap that somebody asked for, of any size; 0: nobody did (ranks on one device)
+    int one_device_twoshot_max_ctas = 0;           // likewise for two-shot alone (tuning file: twoshot_max_ctas)
+    // Ranks on one device have a CTA for every 32 bytes per thread (all of it is one batch of loads) unless somebody asks for
+    // other CTAs. Two-shot with 512 / 256 / 128 threads: 4 ranks, 8 MiB 11.9 / 11.7 / 11.7 us, 8 ranks, 8 MiB 23.7 / 22.5 / 22.0
+    // us, 512 KiB 4.9 / 3.4 / 3.5 us, 256 MiB 626 / 625 / 625 us; with 256 threads and 64 bytes per thread 12.7, 24.8, 4.8 and 631 us.
+    int one_device_block_threads = 256;
+    std::size_t one_device_bytes_per_cta = 8u << 10;
     int nvls_max_ctas = 64;                        // more CTAs than this slowed the multimem kernels down
     int nvls_staged_max_ctas = 64;                 // when the same CTAs also copy the message in and out of the arena
     int twoshot_max_ctas = 128;

@@ -176,6 +176,30 @@ def test_tuning_file(lib, monkeypatch, tmp_path):
     assert rc == 2 and b"cannot be read" in lib.b2_last_error()
 
 
+def test_planner_peer_kernels_on_one_device(lib, tmp_path, monkeypatch):
+    WIDE, RD, WR, ONE = 1, 2, 4, 256
+    for var in ("B200CCL_TUNING_FILE", "B200CCL_MAX_CTAS", "B200CCL_BLOCK_THREADS", "B200CCL_BYTES_PER_CTA", "B200CCL_ONESHOT_BYTES_PER_CTA"):
+        monkeypatch.delenv(var, raising=False)
+    count = 1 << 24  # 64 MiB of float32, 8 MiB per shard
+    rc, p = _plan(lib, 0, count, WIDE | RD | WR | ONE, forced=2)
+    assert rc == 0 and p[0] == 2 and p[1] == 1024 and p[2] == 0  # two-shot: a CTA for every 8 KiB of a shard
+    rc, p = _plan(lib, 0, count, WIDE | RD | WR | ONE, forced=1)
+    assert rc == 0 and p[0] == 1 and p[1] == 8192
+    rc, p = _plan(lib, 1, count // 8, WIDE | RD | WR | ONE, forced=1)
+    assert rc == 0 and p[1] == 1024
+    rc, p = _plan(lib, 0, count, WIDE | RD | WR, forced=2)
+    assert rc == 0 and p[1] == 128  # GPUs of their own: CTAs that loop, as before
+    path = tmp_path / "one.tuning"
+    path.write_text("twoshot_max_ctas = 24\n")
+    monkeypatch.setenv("B200CCL_TUNING_FILE", str(path))
+    rc, p = _plan(lib, 0, count, WIDE | RD | WR | ONE, forced=2)
+    assert p[1] == 24
+    monkeypatch.setenv("B200CCL_MAX_CTAS", "5")
+    for forced in (1, 2):
+        rc, p = _plan(lib, 0, count, WIDE | RD | WR | ONE, forced=forced)
+        assert p[1] == 5
+
+
 def test_tuning_file_from_tuner_tables():
     import json
     import os

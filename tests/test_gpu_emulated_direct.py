@@ -1,0 +1,63 @@
+"""One-shot and two-shot of emulated ranks (one launch, a CTA for every few KiB): buffers that are all misaligned alike, around
+the packs and the CTAs' shares, for every rank count; bit for bit against a sum in rank order in fp32, rounded once."""
+import pytest
+import torch
+
+import nano_nccl_b200 as nn
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("algo", ["oneshot", "twoshot"])
+@pytest.mark.parametrize("ranks", [2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_buffers_misaligned_alike(algo, ranks, dtype):
+    comm = nn.Communicator(devices=[0], loopback_ranks=ranks, algo=algo, wait_timeout_ms=2000)
+    try:
+        esz = torch.empty(0, dtype=dtype).element_size()
+        gen = torch.Generator(device="cuda").manual_seed(ranks)
+        share = 8192 // esz  # what one CTA of 256 threads takes at a time
+        counts = [1, 16 // esz, 32 // esz, 48 // esz - 1, 62 // esz, 64 // esz + 1, 257, share * ranks - 1, share * ranks + 33, 3 * share * ranks + 5]
+        for k, count in enumerate(counts):
+            for shift in (1, 5, 16 // esz + 1, 32 // esz - 1):
+                op = ["sum", "avg", "max", "min"][(k + shift) % 4]
+                ins = [torch.randn(count + 64, device="cuda", generator=gen).to(dtype)[shift:shift + count] for _ in range(ranks)]
+                raw = [torch.full((count + 64,), 7.0, device="cuda", dtype=dtype) for _ in range(ranks)]
+                outs = [t[shift:shift + count] for t in raw]
+                if algo == "twoshot" and k % 2:  # in place
+                    for t, o in zip(ins, outs):
+                        o.copy_(t)
+                    comm.all_reduce(outs, outs, op=op)
+                else:
+                    comm.all_reduce(outs, ins, op=op)
+                assert comm.last_call()["algo"] == algo
+                acc = ins[0].float()
+                for t in ins[1:]:
+                    acc = acc + t.float() if op in ("sum", "avg") else (torch.maximum if op == "max" else torch.minimum)(acc, t.float())
+                if op == "avg":
+                    acc = acc * torch.tensor(1.0, device="cuda").div(ranks)
+                expect = acc.to(dtype)
+                for t, o in zip(raw, outs):
+                    assert torch.equal(o, expect), (count, shift, op)
+                    assert (t[:shift] == 7.0).all() and (t[shift + count:] == 7.0).all(), (count, shift, op)
+        comm.check_async_error()
+    finally:
+        comm.close()
+
+
+@pytest.mark.parametrize("algo", ["oneshot", "twoshot"])
+def test_buffers_misaligned_differently_and_a_capped_grid(algo):
+    # Not all alike modulo 16: element by element. And CTAs that loop, where the caller caps their number.
+    comm = nn.Communicator(devices=[0], loopback_ranks=3, algo=algo, max_ctas=2, wait_timeout_ms=2000)
+    try:
+        gen = torch.Generator(device="cuda").manual_seed(5)
+        for shifts, count in (((1, 2, 3), 30001), ((1, 1, 1), 100003), ((8, 8, 8), 100000), ((0, 0, 8), 4099)):
+            ins = [torch.randn(count + 16, device="cuda", generator=gen).bfloat16()[s:s + count] for s in shifts]
+            outs = [torch.zeros(count + 16, device="cuda", dtype=torch.bfloat16)[s:s + count] for s in shifts]
+            comm.all_reduce(outs, ins)
+            assert comm.last_call()["grid"] <= 2
+            expect = (ins[0].float() + ins[1].float() + ins[2].float()).bfloat16()
+            for o in outs:
+                assert torch.equal(o, expect), (shifts, count)
+    finally:
+        comm.close()
