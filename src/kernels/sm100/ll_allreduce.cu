@@ -52,50 +52,60 @@ struct Word<__nv_bfloat16> {
     static __device__ __forceinline__ unsigned pack(const float (&f)[2]) { return f2_to_b2(f[0], f[1]); }
 };
 
-template <typename T, typename Op, typename ParamT>
-__global__ void __launch_bounds__(kBlockThreads) ll_kernel(const __grid_constant__ ParamT param) {
-    const LlArgs* ap;
-    if constexpr (sizeof(ParamT) == sizeof(LlArgs)) ap = reinterpret_cast<const LlArgs*>(&param);
-    else ap = reinterpret_cast<const LlArgs*>(&param) + blockIdx.y;
-    const LlArgs& a = *ap;
+constexpr unsigned kWordsAtATime = kLlCtas * kBlockThreads;  // words that the CTAs of a rank take at a time
+
+// One rank's part of the exchange, kBatch words per thread at a time; false when a wait gave up.
+template <typename T, typename Op, int kBatch>
+__device__ __forceinline__ bool exchange(const LlArgs& a, u64 call) {
+    static_assert(kBatch * kMaxRanks <= 32, "pending words are bits of one register");
     const int n = a.nranks, rank = a.rank;
-    // Every thread reads the CTA's call counter; thread 0 writes it back at the end.
-    const u64 call = a.own_ctrl->ll_epoch[blockIdx.x] + 1;
     const unsigned flag = static_cast<unsigned>(call % 0xffffffffull) + 1u;  // never 0: a zeroed area matches no call
     const u64 parity = call & 1ull;
     const unsigned* in = static_cast<const unsigned*>(a.in);
     unsigned* out = static_cast<unsigned*>(a.out);
-    const unsigned stride = kLlCtas * kBlockThreads;
     const unsigned first = blockIdx.x * kBlockThreads + threadIdx.x;
 
     // 1. Publish: word w of this rank goes to slot (parity, rank, w) of every rank.
-    for (unsigned w = first; w < a.nwords; w += stride) {
-        const unsigned v = in[w];
-        const u64 slot = (parity * (u64)n + (u64)rank) * kLlMaxWords + w;
+    for (unsigned w0 = first; w0 < a.nwords; w0 += kWordsAtATime * kBatch) {
+        unsigned v[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+            if (w0 + u * kWordsAtATime < a.nwords) v[u] = in[w0 + u * kWordsAtATime];
+        const u64 slot = (parity * (u64)n + (u64)rank) * kLlMaxWords + w0;
         for (int k = 0; k < n; ++k) {
             int q = rank + k;
             if (q >= n) q -= n;
-            st_slot(a.area[q] + slot, v, flag);
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u)
+                if (w0 + u * kWordsAtATime < a.nwords) st_slot(a.area[q] + slot + u * kWordsAtATime, v[u], flag);
         }
     }
-    // 2. Collect: the slots of all sources are loaded together (n loads in flight), then only the
-    //    sources whose call number has not arrived yet are polled again; combine in rank order.
+    // 2. Collect: the slots of all sources and of kBatch words are loaded together, then only those whose call number
+    //    has not arrived yet are polled again; combine in rank order.
     bool ok = true;
-    const u64 t0 = global_timer_ns();
+    u64 t0 = 0;
     const u64* own_area = a.area[rank] + parity * (u64)n * kLlMaxWords;
-    for (unsigned w = first; ok && w < a.nwords; w += stride) {
-        uint2 v[kMaxRanks];
-        unsigned pending = (1u << n) - 1u;
+    for (unsigned w0 = first; ok && w0 < a.nwords; w0 += kWordsAtATime * kBatch) {
+        uint2 v[kBatch][kMaxRanks];
+        unsigned pending = 0u;  // bit u * kMaxRanks + p: word u of rank p
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+            if (w0 + u * kWordsAtATime < a.nwords) pending |= ((1u << n) - 1u) << (u * kMaxRanks);
         unsigned polls = 0;
         while (pending != 0u) {
 #pragma unroll
-            for (int p = 0; p < kMaxRanks; ++p)
-                if (pending & (1u << p)) v[p] = ld_slot(own_area + (u64)p * kLlMaxWords + w);
+            for (int u = 0; u < kBatch; ++u)
 #pragma unroll
-            for (int p = 0; p < kMaxRanks; ++p)
-                if ((pending & (1u << p)) && v[p].y == flag) pending &= ~(1u << p);
+                for (int p = 0; p < kMaxRanks; ++p)
+                    if (pending & (1u << (u * kMaxRanks + p))) v[u][p] = ld_slot(own_area + (u64)p * kLlMaxWords + w0 + u * kWordsAtATime);
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u)
+#pragma unroll
+                for (int p = 0; p < kMaxRanks; ++p)
+                    if ((pending & (1u << (u * kMaxRanks + p))) && v[u][p].y == flag) pending &= ~(1u << (u * kMaxRanks + p));
             if (pending != 0u && (++polls & 255u) == 0u) {
-                const unsigned who = (unsigned)(__ffs((int)pending) - 1);
+                if (t0 == 0) t0 = global_timer_ns();
+                const unsigned who = (unsigned)(__ffs((int)pending) - 1) % kMaxRanks;
                 if (ld_volatile_u32(&a.own_ctrl->abort_flag) != 0u) {
                     report_failure(a.status, a.own_ctrl, nullptr, 0, kStatusAborted, who, 20u, call, global_timer_ns() - t0);
                     ok = false;
@@ -110,28 +120,44 @@ __global__ void __launch_bounds__(kBlockThreads) ll_kernel(const __grid_constant
             }
         }
         if (!ok) break;
-        float acc[Word<T>::kLanes];
-        Word<T>::unpack(v[0].x, acc);
 #pragma unroll
-        for (int p = 1; p < kMaxRanks; ++p) {
-            if (p < n) {
-                float f[Word<T>::kLanes];
-                Word<T>::unpack(v[p].x, f);
+        for (int u = 0; u < kBatch; ++u) {
+            if (w0 + u * kWordsAtATime >= a.nwords) break;
+            float acc[Word<T>::kLanes];
+            Word<T>::unpack(v[u][0].x, acc);
 #pragma unroll
-                for (int e = 0; e < Word<T>::kLanes; ++e) acc[e] = Op::apply(acc[e], f[e]);
+            for (int p = 1; p < kMaxRanks; ++p) {
+                if (p < n) {
+                    float f[Word<T>::kLanes];
+                    Word<T>::unpack(v[u][p].x, f);
+#pragma unroll
+                    for (int e = 0; e < Word<T>::kLanes; ++e) acc[e] = Op::apply(acc[e], f[e]);
+                }
             }
-        }
-        if (a.scale != 1.0f) {
+            if (a.scale != 1.0f) {
 #pragma unroll
-            for (int e = 0; e < Word<T>::kLanes; ++e) acc[e] *= a.scale;
+                for (int e = 0; e < Word<T>::kLanes; ++e) acc[e] *= a.scale;
+            }
+            out[w0 + u * kWordsAtATime] = Word<T>::pack(acc);
         }
-        out[w] = Word<T>::pack(acc);
     }
+    return ok;
+}
+
+template <typename T, typename Op, int kBatch, typename ParamT>
+__global__ void __launch_bounds__(kBlockThreads) ll_kernel(const __grid_constant__ ParamT param) {
+    const LlArgs* ap;
+    if constexpr (sizeof(ParamT) == sizeof(LlArgs)) ap = reinterpret_cast<const LlArgs*>(&param);
+    else ap = reinterpret_cast<const LlArgs*>(&param) + blockIdx.y;
+    const LlArgs& a = *ap;
+    // Every thread reads the CTA's call counter; thread 0 writes it back at the end.
+    const u64 call = a.own_ctrl->ll_epoch[blockIdx.x] + 1;
+    const bool ok = exchange<T, Op, kBatch>(a, call);
     // A CTA whose wait gave up leaves its counter alone: the communicator is poisoned anyway.
     if (__syncthreads_and(ok ? 1 : 0) && threadIdx.x == 0) a.own_ctrl->ll_epoch[blockIdx.x] = call;
 }
 
-template <typename T, typename Op>
+template <typename T, typename Op, int kBatch>
 cudaError_t launch_ll_t(const LlArgs* args, int loop_ranks, cudaStream_t stream) {
     dim3 grid(kLlCtas, loop_ranks > 0 ? loop_ranks : 1, 1), block(kBlockThreads, 1, 1);
     if (loop_ranks > 0) {
@@ -139,19 +165,27 @@ cudaError_t launch_ll_t(const LlArgs* args, int loop_ranks, cudaStream_t stream)
         LoopPack<LlArgs> pack;
         for (int r = 0; r < loop_ranks; ++r) pack.r[r] = args[r];
         void* params[] = {&pack};
-        return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(ll_kernel<T, Op, LoopPack<LlArgs>>), grid, block, params, 0, stream);
+        return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(ll_kernel<T, Op, kBatch, LoopPack<LlArgs>>), grid, block, params, 0, stream);
     }
-    ll_kernel<T, Op, LlArgs><<<grid, block, 0, stream>>>(args[0]);
+    ll_kernel<T, Op, kBatch, LlArgs><<<grid, block, 0, stream>>>(args[0]);
     return cudaGetLastError();
+}
+
+// Above 16 KiB a thread has several words. One at a time, each took a round trip to the slots (emulated ranks, 128 KiB: 2 ranks
+// 10.2 -> 8.2 us, 4 ranks 12.3 -> 10.2, 8 ranks 14.2 -> 12.3); the batch costs registers (89 against 40) and branches, which a
+// message of one word per thread feels (8 ranks, 1 KiB: 4.1 us, 4.4 with the batched kernel).
+template <typename T, typename Op>
+cudaError_t launch_ll_size(const LlArgs* args, int loop_ranks, cudaStream_t stream) {
+    return args[0].nwords <= kWordsAtATime ? launch_ll_t<T, Op, 1>(args, loop_ranks, stream) : launch_ll_t<T, Op, 4>(args, loop_ranks, stream);
 }
 
 template <typename T>
 cudaError_t launch_ll_op(RedOp op, const LlArgs* args, int loop_ranks, cudaStream_t stream) {
     switch (op) {
         case RedOp::Sum:
-        case RedOp::Avg: return launch_ll_t<T, OpAdd>(args, loop_ranks, stream);
-        case RedOp::Max: return launch_ll_t<T, OpMax>(args, loop_ranks, stream);
-        case RedOp::Min: return launch_ll_t<T, OpMin>(args, loop_ranks, stream);
+        case RedOp::Avg: return launch_ll_size<T, OpAdd>(args, loop_ranks, stream);
+        case RedOp::Max: return launch_ll_size<T, OpMax>(args, loop_ranks, stream);
+        case RedOp::Min: return launch_ll_size<T, OpMin>(args, loop_ranks, stream);
     }
     return cudaErrorInvalidValue;
 }

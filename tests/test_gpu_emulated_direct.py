@@ -61,3 +61,28 @@ def test_buffers_misaligned_differently_and_a_capped_grid(algo):
                 assert torch.equal(o, expect), (shifts, count)
     finally:
         comm.close()
+
+
+@pytest.mark.parametrize("ranks", [2, 3, 8])
+def test_low_latency_batches_of_words(ranks):
+    # One word per thread up to 16 KiB, four at a time above: both sides of that line, a ragged batch, and the largest message;
+    # long and short messages in turn, so that slots of both kinds of call are used again.
+    comm = nn.Communicator(devices=[0], loopback_ranks=ranks, algo="ll", wait_timeout_ms=2000)
+    try:
+        gen = torch.Generator(device="cuda").manual_seed(3)
+        for k, words in enumerate([4096, 4097, 5, 16384, 16385, 4095, 16383, 32768, 1, 32767, 12289]):
+            ins = [torch.randn(words * 2, device="cuda", generator=gen).half() for _ in range(ranks)]
+            outs = [torch.empty_like(t) for t in ins]
+            op = ["sum", "avg", "max", "min"][k % 4]
+            comm.all_reduce(outs, ins, op=op)
+            assert comm.last_call()["algo"] == "ll"
+            acc = ins[0].float()
+            for t in ins[1:]:
+                acc = acc + t.float() if op in ("sum", "avg") else (torch.maximum if op == "max" else torch.minimum)(acc, t.float())
+            if op == "avg":
+                acc = acc * torch.tensor(1.0, device="cuda").div(ranks)
+            for o in outs:
+                assert torch.equal(o, acc.half()), (words, op)
+        comm.check_async_error()
+    finally:
+        comm.close()
