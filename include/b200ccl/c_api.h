@@ -103,7 +103,8 @@ int b2_ll_sim(const long long cfg[8], const size_t* call_words, int ncalls, doub
 
 /* Single-GPU self-tests of the signalling primitives (bounded; they cannot hang the device).
  * kind 0: a wait on a flag nothing sets must time out; kind 1: the host raises the abort word
- * while a kernel waits. out = {wait_ok, status_code, where, abort_raised}; *waited_ms as measured
+ * while a kernel waits; kind 2: the wait on an mbarrier of a thread block cluster that nobody arrives on must time out.
+ * out = {wait_ok, status_code, where, abort_raised}; *waited_ms as measured
  * on the device. */
 int b2_selftest_wait(int kind, int device, double timeout_ms, int out[4], double* waited_ms);
 /* A kernel writes a payload then releases a counter in mapped host memory; the host acquires the

@@ -286,7 +286,8 @@ int b2_ring_sim(const long long cfg[6], size_t count, size_t fifo_bytes, double 
 
 int b2_selftest_wait(int kind, int device, double timeout_ms, int out[4], double* waited_ms) {
     return guarded([&] {
-        const kernels::SelfTestResult r = kind == 0 ? kernels::selftest_wait_timeout(device, timeout_ms)
+        const kernels::SelfTestResult r = kind == 0   ? kernels::selftest_wait_timeout(device, timeout_ms)
+                                          : kind == 2 ? kernels::selftest_cluster_wait_timeout(device, timeout_ms)
                                                     : kernels::selftest_abort(device, timeout_ms);
         out[0] = r.wait_ok;
         out[1] = static_cast<int>(r.status_code);

@@ -155,6 +155,7 @@ private:
     std::size_t staging_half_ = 0;
     std::size_t stage_guard_ = 0;  // bytes of canary before and after the arena (checking builds), else 0
     int channels_ = kDefaultChannels;
+    bool channels_asked_for_ = false;
     sched::Tuning tuning_;
     sched::ProcessLayout layout_;
     sched::RingTransportPlan ring_plan_;
@@ -212,6 +213,7 @@ Communicator::Impl::Impl(const CommunicatorConfig& config, Bootstrap* bootstrap)
     staging_half_ = std::max<std::size_t>(staging_half_ / 4096 * 4096, 4096);
     // 0: decided below, once the transport is known.
     channels_ = config.channels > 0 ? config.channels : static_cast<int>(env::get_int("B200CCL_NCHANNELS", 0, "NANO_NCCL_NCHANNELS"));
+    channels_asked_for_ = channels_ > 0;
     tuning_ = sched::tuning_from_env();
     if (config.max_ctas > 0) {  // an explicit cap applies to every algorithm
         tuning_.max_ctas = tuning_.nvls_max_ctas = tuning_.nvls_staged_max_ctas = tuning_.twoshot_max_ctas =
@@ -261,8 +263,8 @@ Communicator::Impl::Impl(const CommunicatorConfig& config, Bootstrap* bootstrap)
         channels_ = resolved_ == TransportKind::P2p ? 32
                     : (resolved_ == TransportKind::Shm || resolved_ == TransportKind::Mixed) ? 4 : kDefaultChannels;
         // Emulated ranks share one GPU and one cooperative launch: all their channel CTAs must be resident at once, one
-        // per SM. Over device memory more of them are faster up to there (4 ranks, 16 MiB: 108 us with 16 channels, 73
-        // with 32). Over host memory eight CTAs in all keep PCIe busy both ways (35 of the 40 GB/s that a copy from host
+        // per SM. Over device memory these channels count only where ring_simple.cu plays them (else clusters do, as many as
+        // fit). Over host memory eight CTAs in all keep PCIe busy both ways (35 of the 40 GB/s that a copy from host
         // to host reaches); more of them slow it down (8 ranks, 1 MiB: 555 us with one channel, 834 with four).
         if (loopback_) {
             const int ctas = resolved_ == TransportKind::P2p ? 128 : (resolved_ == TransportKind::Shm ? 8 : 64);
@@ -868,6 +870,7 @@ void Communicator::Impl::run(Collective collective, const CollectiveArgs& args) 
             RingEngineConfig rc;
             rc.nranks = nranks_;
             rc.channels = channels_;
+            rc.channels_asked_for = channels_asked_for_;
             rc.timeout_ns = timeout_ns_;
             rc.edge_kinds = ring_plan_.edge_kinds;
             rc.loopback = loopback_;
@@ -881,7 +884,7 @@ void Communicator::Impl::run(Collective collective, const CollectiveArgs& args) 
                 DeviceGuard guard(local_[i].device);
                 wait_previous(local_[i], args.streams[i]);
             }
-            ring_->launch(collective, args);
+            last_.grid = ring_->launch(collective, args);
             for (std::size_t i = 0; i < launches_per_call(); ++i) {
                 DeviceGuard guard(local_[i].device);
                 record_done(local_[i], args.streams[i]);
@@ -892,7 +895,6 @@ void Communicator::Impl::run(Collective collective, const CollectiveArgs& args) 
             poison(std::string("ring launch failed: ") + e.what());
             throw;
         }
-        last_.grid = ring_->channels();
         last_.block = ring_->block_threads();
         return;
     }

@@ -4,10 +4,12 @@
 #include "core/check.h"
 #include "core/env.h"
 #include "core/numa.h"
+#include "kernels/sm100/ring_cluster.h"
 #include "kernels/sm100/ring_simple.h"
 #include "sched/ring_geometry.h"
 #include "transport/net_edge.h"
 
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <stdexcept>
@@ -34,6 +36,7 @@ struct RingEngine::State {
     std::vector<std::vector<dev::RingChannel>> wiring;   // per local rank: [channels], host copy
     std::vector<DeviceBuffer<dev::RingChannel>> tables;  // per local rank: [channels]
     MappedBuffer<dev::RingTurnaroundStats> stats;        // [local rank][channel], optional
+    int clusters = 0;  // > 0: emulated ranks whose slices go through distributed shared memory, in at most that many clusters
 };
 
 namespace {
@@ -124,6 +127,14 @@ RingEngine::RingEngine(const RingEngineConfig& config, mem::SymmetricAllocator* 
         s.net = transport::create_net_edges(nc, bootstrap);
     }
     if (env::get_bool("B200CCL_RING_TURNAROUND", false)) s.stats.reset(config.local.size() * C);
+
+    // Ranks that share a GPU, and no host memory or network between them. (The counters of ring_simple.cu are the ones that
+    // the turnaround statistics are taken at.)
+    if (config.loopback && dev::kRanksShareGpu && !net && !any_shm && s.stats.get() == nullptr) {
+        DeviceGuard guard(config.local[0].device);
+        s.clusters = kernels::ring_cluster_capacity(n);
+        if (config.channels_asked_for) s.clusters = std::min(s.clusters, C);
+    }
 
     auto ctrl_of = [&](int grank) -> dev::ControlBlock* {
         if (symmetric) return static_cast<dev::ControlBlock*>(ctrl->rank_ptr(grank));
@@ -234,8 +245,38 @@ int RingEngine::channels() const { return state_->cfg.channels; }
 int RingEngine::block_threads() const { return kernels::ring_block_threads(); }
 std::string RingEngine::async_error() const { return state_->net ? state_->net->first_error() : std::string(); }
 
-void RingEngine::launch(Collective collective, const CollectiveArgs& args) {
+int RingEngine::launch_clusters(Collective collective, const CollectiveArgs& args) {
     State& s = *state_;
+    const std::size_t esz = dtype_size(args.dtype);
+    dev::RingClusterArgs a;
+    std::memset(&a, 0, sizeof(a));
+    std::uintptr_t differ = 0;
+    const auto first = reinterpret_cast<std::uintptr_t>(args.send_buffers[0]);
+    for (int r = 0; r < s.cfg.nranks; ++r) {
+        a.in[r] = args.send_buffers[r];
+        a.out[r] = args.recv_buffers[r];
+        a.ctrl[r] = s.ctrl != nullptr ? static_cast<dev::ControlBlock*>(s.ctrl->rank_ptr(r)) : s.own_ctrl[r].get();
+        a.status[r] = s.cfg.status[r];
+        differ |= (reinterpret_cast<std::uintptr_t>(a.in[r]) ^ first) | (reinterpret_cast<std::uintptr_t>(a.out[r]) ^ first);
+    }
+    a.count = args.count;
+    a.timeout_ns = s.cfg.timeout_ns;
+    a.scale = args.redop == RedOp::Avg ? 1.0f / static_cast<float>(s.cfg.nranks) : 1.0f;
+    a.nranks = s.cfg.nranks;
+    a.collective = static_cast<int>(collective);
+    // 16-byte accesses: an all_reduce of buffers that are aligned alike; the blocks of the others must all be aligned.
+    const bool alike = (differ & 15u) == 0;
+    const bool wide = alike && (collective == Collective::AllReduce || ((first & 15u) == 0 && (args.count * esz) % 16 == 0));
+    if (wide) a.lead = static_cast<unsigned>((first & 15u) / esz);
+    int used = 0;
+    DeviceGuard guard(s.cfg.local[0].device);
+    B2_CUDA(kernels::launch_ring_cluster(args.dtype, args.redop, wide, a, s.clusters, args.streams[0], &used));
+    return used;
+}
+
+int RingEngine::launch(Collective collective, const CollectiveArgs& args) {
+    State& s = *state_;
+    if (s.clusters > 0) return launch_clusters(collective, args);
     const std::size_t esz = dtype_size(args.dtype);
     // Whole vectors, and at the end of an all_reduce the elements that fill none. A ragged length still goes element by
     // element between processes, where the choice must not depend on addresses that other ranks cannot see, and where
@@ -281,6 +322,7 @@ void RingEngine::launch(Collective collective, const CollectiveArgs& args) {
             B2_CUDA(kernels::launch_ring(args.dtype, args.redop, &per[i], cfg));
         }
     }
+    return s.cfg.channels;
 }
 
 }  // namespace b200ccl

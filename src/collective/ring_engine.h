@@ -23,6 +23,7 @@ namespace b200ccl {
 struct RingEngineConfig {
     int nranks = 0;
     int channels = kDefaultChannels;
+    bool channels_asked_for = false;  // by the caller; else the count is a default
     unsigned long long timeout_ns = 0;
     // Kind of every directed ring edge e -> (e + 1) % nranks: P2p (FIFO in the receiver's device
     // memory, counters in device memory of the rank that polls them), Shm (FIFO and counters in
@@ -45,7 +46,7 @@ public:
     RingEngine(const RingEngineConfig& config, mem::SymmetricAllocator* alloc, const mem::SymmetricRegion* ctrl,
                Bootstrap* bootstrap);
     ~RingEngine();
-    void launch(Collective collective, const CollectiveArgs& args);
+    int launch(Collective collective, const CollectiveArgs& args);  // CTAs per rank
     int channels() const;
     int block_threads() const;
     std::string async_error() const;  // first proxy/transport failure, "" when none
@@ -55,6 +56,7 @@ public:
 
 private:
     struct State;
+    int launch_clusters(Collective collective, const CollectiveArgs& args);
     std::unique_ptr<State> state_;
 };
 

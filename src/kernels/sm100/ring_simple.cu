@@ -5,6 +5,9 @@
 // control is two monotonically growing step counters per edge, published with st.release.sys and
 // polled with ld.acquire.sys; counters persist from launch to launch.
 //
+// Emulated ranks over device memory run ring_cluster.cu; this kernel plays them only where the turnaround statistics are
+// asked for, where host memory or a network lies between them, and in the checking build.
+//
 // Bound by the chain of slices: a rank can only work on what its neighbour has posted, so what counts is
 // the time from one post to the next. Where all ranks run in one launch over device memory, two groups of eight
 // warps take the slices in turn, so that one slice is moved while the other waits for its neighbour, for its loads

@@ -1,6 +1,7 @@
 // Small self-tests of the signalling primitives, callable on any single GPU. None of them can
 // hang or fault the device: every wait is bounded and ends with a status record.
 //   * wait timeout: a warp waits for a flag that nothing sets; the wait must run out and say so.
+//   * cluster wait timeout: the same for the wait on an mbarrier of a thread block cluster.
 //   * abort: the host raises the abort word while a warp waits; the wait must end as "aborted".
 //   * publication: a kernel writes a payload and then releases a step counter in mapped host
 //     memory; a host thread that acquires the counter must already see the payload.
@@ -14,6 +15,7 @@
 
 #include "core/check.h"
 #include "kernels/sm100/sync.cuh"
+#include "kernels/sm100/tma.cuh"
 
 #include <chrono>
 #include <cstring>
@@ -36,6 +38,20 @@ __global__ void wait_kernel(const unsigned long long* flag, unsigned long long w
         const bool ok = wait_at_least(flag, want, own, timeout_ns, status, ctrl, 1, 0u, 99u);
         *ok_out = ok ? 1 : 0;
     }
+}
+
+// The same for a wait on an mbarrier that nobody arrives on (one warp, as in ring_cluster.cu).
+__global__ void cluster_wait_kernel(ControlBlock* own, Status* status, unsigned long long timeout_ns, int* ok_out) {
+    __shared__ unsigned long long bar;
+    __shared__ unsigned failed;
+    if (threadIdx.x == 0) {
+        mbar_init(&bar, 1u);
+        failed = 0u;
+    }
+    __syncwarp();
+    const bool ok = wait_cluster_phase(smem_addr(&bar), 0u, &failed, own, timeout_ns, status, 0u, 97u, 1ull);
+    drain_cluster_phase(smem_addr(&bar), 0u);
+    if (threadIdx.x == 0) *ok_out = ok || failed == 0u ? 1 : 0;
 }
 
 __global__ void publish_kernel(unsigned int* payload, int n, unsigned long long* step, unsigned long long value) {
@@ -120,6 +136,20 @@ SelfTestResult selftest_wait_timeout(int device, double timeout_ms) {
     unsigned int abort_seen = 0;
     B2_CUDA(cudaMemcpy(&abort_seen, &s.ctrl->abort_flag, sizeof(abort_seen), cudaMemcpyDeviceToHost));
     r.abort_raised = abort_seen != 0;
+    return r;
+}
+
+SelfTestResult selftest_cluster_wait_timeout(int device, double timeout_ms) {
+    DeviceGuard guard(device);
+    Scratch s;
+    cluster_wait_kernel<<<1, 32, 0, s.stream>>>(s.ctrl, s.status, static_cast<unsigned long long>(timeout_ms * 1e6), s.ok);
+    B2_CUDA(cudaGetLastError());
+    B2_CUDA(cudaStreamSynchronize(s.stream));
+    SelfTestResult r;
+    r.wait_ok = *s.ok;
+    r.status_code = s.status->code;
+    r.waited_ms = static_cast<double>(s.status->waited_ns) * 1e-6;
+    r.where = s.status->where;
     return r;
 }
 

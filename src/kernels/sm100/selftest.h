@@ -12,6 +12,7 @@ struct SelfTestResult {
 };
 
 SelfTestResult selftest_wait_timeout(int device, double timeout_ms);
+SelfTestResult selftest_cluster_wait_timeout(int device, double timeout_ms);
 SelfTestResult selftest_abort(int device, double timeout_ms);
 bool selftest_publication(int device, int rounds);
 // Device-side "send" of `slices` slices into a mapped host FIFO with no proxy thread: the host plays

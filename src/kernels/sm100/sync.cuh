@@ -99,6 +99,50 @@ __device__ __forceinline__ bool wait_at_least(const unsigned long long* flag, un
     }
 }
 
+// Whether the phase of parity `parity` of an mbarrier in this CTA's shared memory is over; what other CTAs of the cluster stored
+// before it is visible then. Every lane of the warp calls it and gets the same answer, after a microsecond at most.
+__device__ __forceinline__ bool cluster_phase_over(unsigned bar, unsigned parity) {
+    unsigned done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, 1000;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    return __all_sync(0xffffffffu, done != 0u) != 0;
+}
+
+// Waits for that phase. False (in every lane) after `timeout_ns`, or when the local abort flag or `failed` (shared memory:
+// another warp of the cluster gave up) is set; `failed` is set then.
+__device__ __forceinline__ bool wait_cluster_phase(unsigned bar, unsigned parity, unsigned* failed, ControlBlock* own,
+                                                   unsigned long long timeout_ns, Status* status, unsigned int peer,
+                                                   unsigned int where, unsigned long long step) {
+    if (cluster_phase_over(bar, parity)) return true;
+    unsigned long long t0 = 0;
+    for (unsigned polls = 1;; ++polls) {
+        if (cluster_phase_over(bar, parity)) return true;
+        if ((polls & 63u) != 0u) continue;
+        const unsigned long long now = global_timer_ns();
+        if (t0 == 0) t0 = now;
+        const bool late = now - t0 > timeout_ns;
+        const bool told = *static_cast<volatile unsigned*>(failed) != 0u || ld_volatile_u32(&own->abort_flag) != 0u;
+        if (__any_sync(0xffffffffu, late || told)) {
+            if ((threadIdx.x & 31u) == 0u) {
+                *static_cast<volatile unsigned*>(failed) = 1u;
+                report_failure(status, own, nullptr, 0, told ? kStatusAborted : kStatusTimeout, peer, where, step, now - t0);
+            }
+            return false;
+        }
+    }
+}
+
+// Gives a phase that may still come a tenth of a millisecond to do so (after a failure: what was sent lands before its
+// receiver ends).
+__device__ __forceinline__ void drain_cluster_phase(unsigned bar, unsigned parity) {
+    const unsigned long long t0 = global_timer_ns();
+    for (unsigned polls = 0; polls < 1000000u; ++polls) {
+        const bool late = global_timer_ns() - t0 > 100000ull;
+        if (cluster_phase_over(bar, parity) || __any_sync(0xffffffffu, late)) return;
+    }
+}
+
 // Barrier among the CTAs with the same blockIdx.x on every rank. Thread p signals rank p and
 // waits for rank p. Everything the CTA stored before the call is visible to every rank's CTA
 // after it (release on the signal, acquire on the poll, bar.sync on both sides).
