@@ -65,32 +65,34 @@ __device__ __forceinline__ bool exchange(const LlArgs& a, u64 call) {
     unsigned* out = static_cast<unsigned*>(a.out);
     const unsigned first = blockIdx.x * kBlockThreads + threadIdx.x;
 
+    auto has = [&](unsigned w0, int u) { return u == 0 || w0 + u * kWordsAtATime < a.nwords; };  // the loops see to the first one
+
     // 1. Publish: word w of this rank goes to slot (parity, rank, w) of every rank.
     for (unsigned w0 = first; w0 < a.nwords; w0 += kWordsAtATime * kBatch) {
         unsigned v[kBatch];
 #pragma unroll
         for (int u = 0; u < kBatch; ++u)
-            if (w0 + u * kWordsAtATime < a.nwords) v[u] = in[w0 + u * kWordsAtATime];
+            if (has(w0, u)) v[u] = in[w0 + u * kWordsAtATime];
         const u64 slot = (parity * (u64)n + (u64)rank) * kLlMaxWords + w0;
         for (int k = 0; k < n; ++k) {
             int q = rank + k;
             if (q >= n) q -= n;
 #pragma unroll
             for (int u = 0; u < kBatch; ++u)
-                if (w0 + u * kWordsAtATime < a.nwords) st_slot(a.area[q] + slot + u * kWordsAtATime, v[u], flag);
+                if (has(w0, u)) st_slot(a.area[q] + slot + u * kWordsAtATime, v[u], flag);
         }
     }
     // 2. Collect: the slots of all sources and of kBatch words are loaded together, then only those whose call number
     //    has not arrived yet are polled again; combine in rank order.
     bool ok = true;
-    u64 t0 = 0;
+    const u64 t0 = global_timer_ns();
     const u64* own_area = a.area[rank] + parity * (u64)n * kLlMaxWords;
     for (unsigned w0 = first; ok && w0 < a.nwords; w0 += kWordsAtATime * kBatch) {
         uint2 v[kBatch][kMaxRanks];
         unsigned pending = 0u;  // bit u * kMaxRanks + p: word u of rank p
 #pragma unroll
         for (int u = 0; u < kBatch; ++u)
-            if (w0 + u * kWordsAtATime < a.nwords) pending |= ((1u << n) - 1u) << (u * kMaxRanks);
+            if (has(w0, u)) pending |= ((1u << n) - 1u) << (u * kMaxRanks);
         unsigned polls = 0;
         while (pending != 0u) {
 #pragma unroll
@@ -104,7 +106,6 @@ __device__ __forceinline__ bool exchange(const LlArgs& a, u64 call) {
                 for (int p = 0; p < kMaxRanks; ++p)
                     if ((pending & (1u << (u * kMaxRanks + p))) && v[u][p].y == flag) pending &= ~(1u << (u * kMaxRanks + p));
             if (pending != 0u && (++polls & 255u) == 0u) {
-                if (t0 == 0) t0 = global_timer_ns();
                 const unsigned who = (unsigned)(__ffs((int)pending) - 1) % kMaxRanks;
                 if (ld_volatile_u32(&a.own_ctrl->abort_flag) != 0u) {
                     report_failure(a.status, a.own_ctrl, nullptr, 0, kStatusAborted, who, 20u, call, global_timer_ns() - t0);
@@ -122,7 +123,7 @@ __device__ __forceinline__ bool exchange(const LlArgs& a, u64 call) {
         if (!ok) break;
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) {
-            if (w0 + u * kWordsAtATime >= a.nwords) break;
+            if (!has(w0, u)) break;
             float acc[Word<T>::kLanes];
             Word<T>::unpack(v[u][0].x, acc);
 #pragma unroll
@@ -171,12 +172,12 @@ cudaError_t launch_ll_t(const LlArgs* args, int loop_ranks, cudaStream_t stream)
     return cudaGetLastError();
 }
 
-// Above 16 KiB a thread has several words. One at a time, each took a round trip to the slots (emulated ranks, 128 KiB: 2 ranks
-// 10.2 -> 8.2 us, 4 ranks 12.3 -> 10.2, 8 ranks 14.2 -> 12.3); the batch costs registers (89 against 40) and branches, which a
-// message of one word per thread feels (8 ranks, 1 KiB: 4.1 us, 4.4 with the batched kernel).
+// One word at a time, each takes a round trip to the slots (emulated ranks, 128 KiB, one at a time -> four: 2 ranks 10.2 -> 8.2 us,
+// 4 ranks 12.3 -> 10.2, 8 ranks 14.3 -> 12.3). But a batch that is not full only costs its registers (91 against 40) and
+// conditions: 20000 bytes, 2 ranks 4.6 -> 6.1 us, 8 ranks 6.2 -> 6.8; level at 40000 and 70000 bytes. So from four full words up.
 template <typename T, typename Op>
 cudaError_t launch_ll_size(const LlArgs* args, int loop_ranks, cudaStream_t stream) {
-    return args[0].nwords <= kWordsAtATime ? launch_ll_t<T, Op, 1>(args, loop_ranks, stream) : launch_ll_t<T, Op, 4>(args, loop_ranks, stream);
+    return args[0].nwords <= 4 * kWordsAtATime ? launch_ll_t<T, Op, 1>(args, loop_ranks, stream) : launch_ll_t<T, Op, 4>(args, loop_ranks, stream);
 }
 
 template <typename T>

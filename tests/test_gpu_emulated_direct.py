@@ -65,7 +65,7 @@ def test_buffers_misaligned_differently_and_a_capped_grid(algo):
 
 @pytest.mark.parametrize("ranks", [2, 3, 8])
 def test_low_latency_batches_of_words(ranks):
-    # One word per thread up to 16 KiB, four at a time above: both sides of that line, a ragged batch, and the largest message;
+    # One word per thread at a time up to 64 KiB, four above: both sides of that line, a ragged batch, and the largest message;
     # long and short messages in turn, so that slots of both kinds of call are used again.
     comm = nn.Communicator(devices=[0], loopback_ranks=ranks, algo="ll", wait_timeout_ms=2000)
     try:
