@@ -222,6 +222,8 @@ int b2_make_plan(int collective, int dtype, int redop, int nranks, size_t count,
         s.ring_only = flags & 64u;
         s.word_aligned = flags & 128u;
         s.one_device = flags & 256u;
+        s.host_exchange = flags & 512u;
+        s.aligned = flags & 1024u;
         s.max_ctas = 0;  // the tuning decides
         const sched::Plan p = sched::make_plan(s, static_cast<Algo>(forced_algo), sched::tuning_from_env());
         if (!p.error.empty()) throw std::invalid_argument(p.error);

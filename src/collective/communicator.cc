@@ -13,6 +13,7 @@
 #include "b200ccl/communicator.h"
 
 #include "b200ccl/bootstrap.h"
+#include "collective/host_exchange.h"
 #include "collective/ring_engine.h"
 #include "collective/validate.h"
 #include "core/check.h"
@@ -133,6 +134,9 @@ private:
                              bool nvls, int grid);
     void launch_gather_ranks(const CollectiveArgs& args, std::vector<dev::GatherArgs>& per_rank, int grid);
     void launch_low_latency(const CollectiveArgs& args);
+    void ensure_ring();
+    void ensure_host_exchange();
+    void launch_through_host(Collective collective, const CollectiveArgs& args);
     void launch_on_one_device(Collective collective, const CollectiveArgs& args, int max_ctas);
     void launch_pipeline(const CollectiveArgs& args, const sched::Plan& plan);
     bool direct_peer_pointers() const { return loopback_ || (!multiprocess_ && resolved_ == TransportKind::P2p); }
@@ -178,6 +182,7 @@ private:
     std::vector<Window> windows_;
     mem::GroupDesc group_;
     std::unique_ptr<RingEngine> ring_;
+    std::unique_ptr<HostExchange> host_exchange_;
     CallInfo last_;
     mutable std::string latched_;
 };
@@ -487,6 +492,7 @@ Communicator::Impl::~Impl() {
         }
     }
     ring_.reset();
+    host_exchange_.reset();
     windows_.clear();
     pipe_flags_.reset();
     stage_.reset();
@@ -830,6 +836,7 @@ void Communicator::Impl::run(Collective collective, const CollectiveArgs& args) 
     shape.nranks = nranks_;
     shape.count = args.count;
     shape.wide = wide;
+    shape.aligned = aligned;
     shape.word_aligned = (args.count * esz) % 4 == 0 && args.count > 0;
     for (std::size_t i = 0; i < local_.size(); ++i)
         shape.word_aligned &= reinterpret_cast<std::uintptr_t>(args.send_buffers[i]) % 4 == 0 &&
@@ -841,6 +848,8 @@ void Communicator::Impl::run(Collective collective, const CollectiveArgs& args) 
     shape.output_multicast = out_sym && windows_[out_loc[0].region].mc != nullptr;
     shape.one_device = loopback_;
     shape.ring_only = resolved_ != TransportKind::P2p;  // shm, mixed, socket, rdma: only the ring crosses those edges
+    // Emulated ranks that were given host memory as their transport, and no number of channels, which only a ring has.
+    shape.host_exchange = one_launch() && resolved_ == TransportKind::Shm && !channels_asked_for_;
     shape.max_ctas = tuning_.max_ctas;
     shape.staging_multicast = alloc_ && alloc_->multicast_supported() && (!stage_ || stage_->multicast_ptr() != nullptr);
     sched::Plan plan = sched::make_plan(shape, forced_algo_, tuning_);
@@ -865,20 +874,17 @@ void Communicator::Impl::run(Collective collective, const CollectiveArgs& args) 
               args.count, dtype_name(args.dtype), redop_name(args.redop), algo_name(plan.algo), plan.grid,
               plan.stage_in, plan.stage_out, wide);
 
+    if (shape.host_exchange) {
+        // Both, whichever the first call takes: a later call of the other kind may be part of a capture, which survives no allocation.
+        ensure_host_exchange();
+        ensure_ring();
+    }
+    if (plan.through_host) {
+        launch_through_host(collective, args);
+        return;
+    }
     if (plan.algo == Algo::Ring) {
-        if (!ring_) {
-            RingEngineConfig rc;
-            rc.nranks = nranks_;
-            rc.channels = channels_;
-            rc.channels_asked_for = channels_asked_for_;
-            rc.timeout_ns = timeout_ns_;
-            rc.edge_kinds = ring_plan_.edge_kinds;
-            rc.loopback = loopback_;
-            if (resolved_ == TransportKind::Socket || resolved_ == TransportKind::Rdma) rc.net_kind = resolved_;
-            for (const auto& l : local_) rc.local.push_back({l.grank, l.device});
-            for (const auto& l : local_) rc.status.push_back(l.status);
-            ring_.reset(new RingEngine(rc, alloc_.get(), ctrl_.get(), bootstrap_));
-        }
+        ensure_ring();
         try {
             for (std::size_t i = 0; i < launches_per_call(); ++i) {
                 DeviceGuard guard(local_[i].device);
@@ -917,6 +923,42 @@ void Communicator::Impl::run(Collective collective, const CollectiveArgs& args) 
         case Collective::ReduceScatter: launch_reduce_scatter(args, plan, wide, in_sym ? in_loc.data() : nullptr); break;
         case Collective::AllGather: launch_all_gather(args, plan, wide, in_sym ? in_loc.data() : nullptr, out_sym ? out_loc.data() : nullptr); break;
     }
+}
+
+void Communicator::Impl::ensure_ring() {
+    if (ring_) return;
+    RingEngineConfig rc;
+    rc.nranks = nranks_;
+    rc.channels = channels_;
+    rc.channels_asked_for = channels_asked_for_;
+    rc.timeout_ns = timeout_ns_;
+    rc.edge_kinds = ring_plan_.edge_kinds;
+    rc.loopback = loopback_;
+    if (resolved_ == TransportKind::Socket || resolved_ == TransportKind::Rdma) rc.net_kind = resolved_;
+    for (const auto& l : local_) rc.local.push_back({l.grank, l.device});
+    for (const auto& l : local_) rc.status.push_back(l.status);
+    ring_.reset(new RingEngine(rc, alloc_.get(), ctrl_.get(), bootstrap_));
+}
+
+void Communicator::Impl::ensure_host_exchange() {
+    if (host_exchange_) return;
+    std::vector<dev::Status*> status;
+    for (const auto& l : local_) status.push_back(l.status);
+    host_exchange_.reset(new HostExchange(nranks_, local_[0].device, timeout_ns_, std::move(status)));
+}
+
+// Emulated ranks over host memory. One launch, tracked by the first rank's event.
+void Communicator::Impl::launch_through_host(Collective collective, const CollectiveArgs& args) {
+    try {
+        DeviceGuard guard(local_[0].device);
+        wait_previous(local_[0], args.streams[0]);
+        last_.grid = host_exchange_->launch(collective, args);
+        record_done(local_[0], args.streams[0]);
+    } catch (const std::exception& e) {
+        poison(std::string("launch failed: ") + e.what());
+        throw;
+    }
+    last_.block = dev::kBlockThreads;
 }
 
 // All ranks on one device: emulated ranks, or a single one.

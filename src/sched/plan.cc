@@ -197,6 +197,28 @@ bool nvls_usable(const CallShape& s) {
     return false;
 }
 
+// Emulated ranks over host memory: two-shot (host_exchange.cu) or the ring. Two-shot has two hops instead of 2(n-1), writes less and
+// reads as much, but waits longer for every hop of a long message. us, ring / two-shot, one B200:
+//   all_reduce      2 ranks 32 KiB 39 / 22, 512 KiB 61 / 56, 1 MiB 94 / 95, 8 MiB 546 / 604; 3 ranks 1 MiB 162 / 149, 2 MiB 268 / 274;
+//                   4 ranks 4 KiB 97 / 23, 1 MiB 241 / 198, 8 MiB 1399 / 1371; 8 ranks 2 KiB 200 / 34, 8 MiB 3172 / 2873
+//   all_gather      (block) 2 ranks 128 KiB 29 / 27, 256 KiB 36 / 37; 3 ranks 128 KiB 52 / 44, 1 MiB 219 / 231; 4 ranks 1 MiB 392 / 388;
+//                   8 ranks 1 MiB 1648 / 1395
+//   reduce_scatter  (block) 2 ranks 2 KiB 25 / 20, 32 KiB 24 / 27; 3 ranks 32 KiB 39 / 35, 128 KiB 52 / 59; 7 ranks 32 KiB 120 / 95, 128 KiB
+//                   229 / 253; 8 ranks 128 KiB 294 / 274, 512 KiB 852 / 868: what it reads and writes is the ring's
+//   Where the ring would go element by element (views that start off a vector, ragged blocks) two-shot is ahead at any size:
+//   all_reduce, 4 ranks, 4 MiB 1318 / 708; blocks of 1 MiB, 2 ranks 157 / 145 (reduce_scatter) and 163 / 123, 8 ranks 2957 / 1924 and 3171 / 1406.
+bool exchange_pays(const CallShape& s) {
+    const bool ring_by_element = !s.wide && !(s.collective == Collective::AllReduce && s.aligned);
+    if (ring_by_element) return true;
+    const std::size_t bytes = s.count * dtype_size(s.dtype);  // the message or a block
+    switch (s.collective) {
+        case Collective::AllReduce: return s.nranks >= 4 || bytes <= (s.nranks == 3 ? 1u << 20 : 512u << 10);
+        case Collective::AllGather: return s.nranks >= 4 || bytes <= 128u << 10;
+        case Collective::ReduceScatter: return bytes <= (s.nranks == 2 ? 4u << 10 : (s.nranks < 8 ? 32u << 10 : 128u << 10));
+    }
+    return false;
+}
+
 }  // namespace
 
 Plan make_plan(const CallShape& s, Algo forced, const Tuning& t) {
@@ -209,6 +231,12 @@ Plan make_plan(const CallShape& s, Algo forced, const Tuning& t) {
     const std::size_t bytes = message_bytes(s);
     const std::size_t esz = dtype_size(s.dtype);
 
+    if (s.ring_only && s.host_exchange && forced == Algo::Auto && exchange_pays(s)) {
+        p.algo = Algo::TwoShot;
+        p.through_host = p.stage_in = p.stage_out = true;
+        p.grid = 0;  // sized by the launch
+        return p;
+    }
     if (s.ring_only || forced == Algo::Ring) {
         p.algo = Algo::Ring;
         p.grid = 0;  // the ring path sizes itself by channels

@@ -20,6 +20,7 @@ struct CallShape {
     int nranks = 1;
     std::size_t count = 0;       // the API's `count`
     bool wide = false;           // every pointer 16-byte aligned and every block a multiple of 16 bytes
+    bool aligned = false;        // every pointer 16-byte aligned
     bool word_aligned = false;   // every pointer 4-byte aligned and the message a multiple of 4 bytes
     bool peers_read_input = false;    // peers can load this call's input directly
     bool peers_write_output = false;  // peers can store into this call's output directly
@@ -29,6 +30,7 @@ struct CallShape {
     bool in_place = false;
     bool one_device = false;     // all ranks' buffers live on one GPU and one stream orders them (emulated ranks)
     bool ring_only = false;      // transport without all-pairs peer access: ring is the only choice
+    bool host_exchange = false;  // likewise, but ranks on one device may exchange through host memory without a ring
     int max_ctas = 64;
 };
 
@@ -42,6 +44,7 @@ struct Plan {
     // goes through the switch (multimem) or over plain peer loads and stores.
     std::size_t tile_bytes = 0;
     bool pipe_nvls = false;
+    bool through_host = false;  // two-shot over host memory
     std::string error;    // non-empty → the request cannot be satisfied (forced algo impossible)
 };
 

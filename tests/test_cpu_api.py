@@ -200,6 +200,29 @@ def test_planner_peer_kernels_on_one_device(lib, tmp_path, monkeypatch):
         assert p[1] == 5
 
 
+def test_planner_emulated_ranks_over_host_memory(lib):
+    WIDE, RING, ONE, HOST, ALIGNED = 1, 64, 256, 512, 1024
+    base = RING | ONE | HOST
+
+    def algo(coll, count, flags, nranks, forced=0):
+        rc, p = _plan(lib, coll, count, flags, nranks=nranks, forced=forced)
+        assert rc == 0
+        return p[0]
+
+    ring, twoshot = algo(0, 1024, RING | ONE | WIDE | ALIGNED, 4), 2  # not allowed: the ring
+    assert ring != twoshot
+    for n in (4, 5, 8):
+        assert algo(0, 1 << 24, base | WIDE | ALIGNED, n) == twoshot and algo(2, 1 << 20, base | WIDE | ALIGNED, n) == twoshot
+    for n, most in ((2, 128 << 10), (3, 256 << 10)):  # floats
+        assert algo(0, most, base | WIDE | ALIGNED, n) == twoshot and algo(0, most + 4, base | WIDE | ALIGNED, n) == ring
+        assert algo(0, most + 1, base | ALIGNED, n) == ring and algo(0, most + 1, base, n) == twoshot  # ragged; off a vector
+        assert algo(2, 32 << 10, base | WIDE | ALIGNED, n) == twoshot and algo(2, (32 << 10) + 4, base | WIDE | ALIGNED, n) == ring
+    for n, most in ((2, 1 << 10), (3, 8 << 10), (7, 8 << 10), (8, 32 << 10)):
+        assert algo(1, most, base | WIDE | ALIGNED, n) == twoshot and algo(1, most + 4, base | WIDE | ALIGNED, n) == ring
+        assert algo(1, most + 1, base | ALIGNED, n) == twoshot and algo(2, 1 << 22, base | ALIGNED, n) == twoshot  # ragged blocks
+    assert algo(0, 1024, base | WIDE | ALIGNED, 8, forced=4) == ring  # asked for by name
+
+
 def test_tuning_file_from_tuner_tables():
     import json
     import os
