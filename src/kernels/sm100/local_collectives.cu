@@ -18,8 +18,8 @@
 //
 // Lengths and addresses need no alignment beyond the element's. Packs are cut where the INPUTS are aligned; the
 // elements before the first and after the last pack of a segment are handled one by one by the CTA of its first
-// tile. Where the outputs are aligned differently (blocks of a ragged reduce_scatter or all_gather), results
-// move between neighbouring lanes by shuffle so that the stores are aligned 16-byte vectors all the same.
+// tile. Where the outputs are aligned differently (blocks of a ragged reduce_scatter or all_gather), bytes move
+// between neighbouring lanes by shuffle so that loads and stores are aligned vectors all the same.
 #include "kernels/sm100/local_collectives.h"
 
 #include "kernels/sm100/dev_types.h"
@@ -49,7 +49,7 @@ struct LocalArgs {
     unsigned char nranks;
     unsigned char outs;  // outputs that a segment writes: all of them, or (1) out[s] only
     unsigned char kind;  // Collective
-    unsigned char in_align;  // 16 or 32: what the inputs' addresses agree on
+    unsigned char align;  // 16 or 32: what the inputs' addresses (shifted copies: the outputs') agree on
     // Segment s lies s * count elements into every input (reduce_scatter) or every output (all_gather), which reads in[s] only.
     __device__ __forceinline__ u64 in_step(unsigned elem) const { return kind == (int)Collective::ReduceScatter ? count * elem : 0; }
     __device__ __forceinline__ u64 out_step(unsigned elem) const { return kind == (int)Collective::AllGather ? count * elem : 0; }
@@ -97,7 +97,7 @@ __device__ __forceinline__ void reduce_one(const LocalArgs& a, unsigned seg, u64
 }
 
 // kShift false: inputs and outputs are all aligned alike, modulo 32. kShift true: the inputs are aligned alike modulo
-// 32 or (in_align 16) modulo 16, and so are the outputs, but differently.
+// 32 or (align 16) modulo 16, and so are the outputs, but differently.
 template <typename T, typename Op, int N, bool kShift, int kPerThread>
 __global__ void __launch_bounds__(kThreads, N <= 2 ? 4 : (N <= 4 ? 3 : 2)) local_kernel(const __grid_constant__ LocalArgs a) {
     using P = Wide32<T>;
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kThreads, N <= 2 ? 4 : (N <= 4 ? 3 : 2)) local
         const unsigned seg = t / a.tiles, tile = t - seg * a.tiles;
         const u64 in_off = seg * a.in_step(sizeof(T)), out_off = seg * a.out_step(sizeof(T));
         const char* src0 = a.first_in(seg) + in_off;
-        const unsigned cut = kShift ? a.in_align : 32u;
+        const unsigned cut = kShift ? a.align : 32u;
         const unsigned skew = (unsigned)(reinterpret_cast<std::uintptr_t>(src0) & (cut - 1u));
         const unsigned before = (cut - skew) & (cut - 1u);  // bytes until the inputs are aligned
         const u64 head = before / sizeof(T) < a.count ? before / sizeof(T) : a.count;
@@ -199,59 +199,62 @@ __global__ void __launch_bounds__(kThreads, N <= 2 ? 4 : (N <= 4 ? 3 : 2)) local
     }
 }
 
-// Copies whose outputs are aligned differently from their inputs. Stores are most of the traffic of an all_gather, so
-// a warp stores 512 contiguous bytes at a time: 16-byte packs, and lane 31 loads the pack behind the warp's last one
-// (6 ranks, 8 MB blocks of odd length: 56.0 us; 64.9 us when the warp's ends are stored element by element, 67.9 us
-// with 32-byte packs, whose two stores per lane touch every other 16 bytes).
+// Copies whose outputs are aligned differently from their inputs. Stores are most of the traffic of an all_gather, so packs
+// of 32 bytes are cut where the OUTPUTS are aligned and the shift is on the loads: every store is a whole sector. (Cut at the
+// inputs, neighbouring warps shared sectors, which L2 had to merge. all_gather, bf16, blocks of odd length, us: 8 ranks, 100 KB 6.9
+// -> 3.0, 4.2 MB 52.2 -> 48.4, 12 MB 143.7 -> 137.2; 4 ranks, 4.2 MB 15.7 -> 14.7; aligned blocks of 4.2 MB 47.0 and 14.4.) A pack's
+// bytes begin `skew` bytes into an aligned vector of the input; the third vector that it touches is the next lane's first.
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 4) local_shift_copy_kernel(const __grid_constant__ LocalArgs a) {
-    constexpr int kElems = 16 / sizeof(T), U = kBytes / 16;
+    constexpr u64 kPack = 32;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (unsigned t = blockIdx.x; t < a.tiles * a.segments; t += gridDim.x) {
         const unsigned seg = t / a.tiles, tile = t - seg * a.tiles;
-        const u64 out_off = seg * a.out_step(sizeof(T));
+        const u64 out_off = seg * a.out_step(sizeof(T)), bytes = a.count * sizeof(T);
         const char* src0 = a.first_in(seg);
-        const unsigned before = (16u - (unsigned)(reinterpret_cast<std::uintptr_t>(src0) & 15u)) & 15u;
-        const u64 head = before / sizeof(T) < a.count ? before / sizeof(T) : a.count;
-        const u64 packs = (a.count - head) / kElems, tail0 = head + packs * kElems;
+        const unsigned cut = a.align;  // 32 or 16: what the outputs agree on
+        u64 before = (cut - (unsigned)(reinterpret_cast<std::uintptr_t>(a.out[0] + out_off) & (cut - 1u))) & (cut - 1u);
+        const unsigned skew = (unsigned)(reinterpret_cast<std::uintptr_t>(src0 + before) & 15u);
+        if (before < skew) before += cut;  // the first vector lies within the input
+        u64 packs = bytes > before ? (bytes - before) / kPack : 0;
+        if (skew != 0 && packs != 0 && before - skew + packs * kPack + 16 > bytes) --packs;  // and so does the last
+        const u64 head = (before < bytes ? before : bytes) / sizeof(T), tail0 = head + packs * (kPack / sizeof(T));
         if (tile == 0)
             for (u64 e = threadIdx.x; e < head + (a.count - tail0); e += kThreads)
                 reduce_one<T, OpAdd, 1>(a, seg, 0, out_off, e < head ? e : tail0 + (e - head));
-        const uint4* src = reinterpret_cast<const uint4*>(src0 + before);
-        const u64 out_body = out_off + before, i0 = (u64)tile * (kThreads * U) + threadIdx.x;
+        const uint4* src = reinterpret_cast<const uint4*>(src0 + before - skew);
+        const u64 i = (u64)tile * kThreads + threadIdx.x;
         const unsigned lane = threadIdx.x & 31u;
-        const unsigned m = (unsigned)(reinterpret_cast<std::uintptr_t>(a.out[0] + out_body) & 15u), s = 16u - m;
-        uint4 v[U], beyond[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const u64 i = i0 + u * kThreads;
-            v[u] = beyond[u] = make_uint4(0, 0, 0, 0);
-            if (i < packs) v[u] = ld16_stream(src + i);
-            if (m != 0 && lane == 31u && i + 1 < packs) beyond[u] = ld16_stream(src + i + 1);
+        uint4 w0 = make_uint4(0, 0, 0, 0), w1 = w0, w2;
+        Raw32 v;
+        if (i < packs) {
+            w0 = ld16_stream(src + 2 * i);
+            w1 = ld16_stream(src + 2 * i + 1);
         }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const u64 i = i0 + u * kThreads;
-            uint4 next;
-            next.x = __shfl_down_sync(0xffffffffu, v[u].x, 1);
-            next.y = __shfl_down_sync(0xffffffffu, v[u].y, 1);
-            next.z = __shfl_down_sync(0xffffffffu, v[u].z, 1);
-            next.w = __shfl_down_sync(0xffffffffu, v[u].w, 1);
-            if (lane == 31u) next = beyond[u];
-            if (i >= packs) continue;
-            const uint4 w = m == 0 ? v[u] : shift_pair(v[u], next, s);
-            const bool first = m != 0 && i == 0, last = m != 0 && i + 1 >= packs;
-            T ends[kElems];
-            *reinterpret_cast<uint4*>(ends) = v[u];
-            for (int q = 0; q < a.outs; ++q) {
-                char* dst = a.out[q] + out_body + i * 16ull;
-                if (!last) st16(reinterpret_cast<uint4*>(m == 0 ? dst : dst + s), w);
-                if (first || last) {
-#pragma unroll
-                    for (int e = 0; e < kElems; ++e)
-                        if (e * sizeof(T) < s ? first : last) reinterpret_cast<T*>(dst)[e] = ends[e];
-                }
+        if (skew != 0) {
+            uint4 beyond = make_uint4(0, 0, 0, 0);
+            const bool last = lane == 31u || i + 1 >= packs;
+            if (i < packs && last) beyond = ld16_stream(src + 2 * i + 2);
+            w2.x = __shfl_down_sync(0xffffffffu, w0.x, 1);
+            w2.y = __shfl_down_sync(0xffffffffu, w0.y, 1);
+            w2.z = __shfl_down_sync(0xffffffffu, w0.z, 1);
+            w2.w = __shfl_down_sync(0xffffffffu, w0.w, 1);
+            if (last) w2 = beyond;
+            v.lo = shift_pair(w0, w1, skew);
+            v.hi = shift_pair(w1, w2, skew);
+        } else {
+            v.lo = w0;
+            v.hi = w1;
+        }
+        if (i >= packs) continue;
+        for (int q = 0; q < a.outs; ++q) {
+            char* dst = a.out[q] + out_off + before + i * kPack;
+            if (cut == 32u) {
+                st32(dst, v);
+            } else {
+                st16(reinterpret_cast<uint4*>(dst), v.lo);
+                st16(reinterpret_cast<uint4*>(dst) + 1, v.hi);
             }
         }
     }
@@ -375,7 +378,7 @@ cudaError_t launch_local(const LocalCall& call, LocalLaunch* made) {
     const std::uintptr_t steps = a.segments > 1 ? bytes : 0;
     if (((in_bits | out_bits | (in0 ^ out0) | steps) & 31u) == 0) p.how = Plan::kAlike;
     else if (((in_bits | out_bits) & 15u) == 0) p.how = Plan::kShifted;
-    a.in_align = (in_bits & 31u) == 0 ? 32 : 16;
+    a.align = ((copies ? out_bits : in_bits) & 31u) == 0 ? 32 : 16;
     p.max_ctas = call.max_ctas;
     p.stream = call.stream;
     if (copies) return start_copy(p, made);
