@@ -7,7 +7,7 @@
 // kernel before it.
 //
 // Layout of the work: a call is cut into segments that share one set of addresses (all_reduce: one;
-// reduce_scatter: one per output block; all_gather: one per input), a segment into tiles of kThreads packs, and
+// reduce_scatter: one per output block; all_gather: one per input), a segment into tiles of one pack per thread, and
 // there is one CTA per tile. CTAs start in order and live for one load and one store phase, which keeps the
 // window of addresses in flight narrow and the DRAM on reads, then on writes. Measured against CTAs that stay
 // and loop (one or two per SM, interleaved or contiguous, 16- to 256-byte windows per thread, and TMA bulk
@@ -37,7 +37,8 @@ namespace {
 
 using u64 = unsigned long long;
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 256;  // or half of that, see start_tiles()
+constexpr u64 kSms = 148;
 
 struct LocalArgs {
     const char* in[kMaxRanks];
@@ -98,12 +99,15 @@ __device__ __forceinline__ void reduce_one(const LocalArgs& a, unsigned seg, u64
 
 // kShift false: inputs and outputs are all aligned alike, modulo 32. kShift true: the inputs are aligned alike modulo
 // 32 or (align 16) modulo 16, and so are the outputs, but differently.
-template <typename T, typename Op, int N, bool kShift, int kPerThread>
+// kSize: threads of a CTA, 0 where the launch says (copies know it when they are compiled: all_gather, 4 ranks, 1 MiB blocks 4.2 us,
+// 4.3 without).
+template <typename T, typename Op, int N, bool kShift, int kPerThread, int kSize = 0>
 __global__ void __launch_bounds__(kThreads, N <= 2 ? 4 : (N <= 4 ? 3 : 2)) local_kernel(const __grid_constant__ LocalArgs a) {
     using P = Wide32<T>;
     constexpr int kElems = P::kElems, kHalf = kElems / 2;
     constexpr int U = kPerThread / 32;
     static_assert(N > 1 || !kShift);  // copies: local_shift_copy_kernel
+    const unsigned threads = kSize != 0 ? kSize : blockDim.x;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const bool scaled = a.scale != 1.0f;
@@ -118,11 +122,11 @@ __global__ void __launch_bounds__(kThreads, N <= 2 ? 4 : (N <= 4 ? 3 : 2)) local
         const u64 packs = (a.count - head) / kElems;
         if (tile == 0) {
             const u64 tail0 = head + packs * kElems;
-            for (u64 e = threadIdx.x; e < head + (a.count - tail0); e += kThreads)
+            for (u64 e = threadIdx.x; e < head + (a.count - tail0); e += threads)
                 reduce_one<T, Op, N>(a, seg, in_off, out_off, e < head ? e : tail0 + (e - head));
         }
         const u64 in_body = in_off + before, out_body = out_off + before;
-        const u64 i0 = (u64)tile * (kThreads * U) + threadIdx.x;
+        const u64 i0 = (u64)tile * (threads * U) + threadIdx.x;
         const unsigned lane = threadIdx.x & 31u;
         // Bytes by which the outputs are past the inputs' alignment.
         const unsigned m = kShift ? (unsigned)(reinterpret_cast<std::uintptr_t>(a.out[a.outs == 1 ? seg : 0] + out_body) & 15u) : 0u;
@@ -130,7 +134,7 @@ __global__ void __launch_bounds__(kThreads, N <= 2 ? 4 : (N <= 4 ? 3 : 2)) local
         Raw32 r[U][N];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const u64 i = i0 + u * kThreads;
+            const u64 i = i0 + u * threads;
             if (i < packs) {
 #pragma unroll
                 for (int p = 0; p < N; ++p) r[u][p] = kShift && cut == 16u ? P::load_user(body(p), i) : P::load(body(p), i);
@@ -138,7 +142,7 @@ __global__ void __launch_bounds__(kThreads, N <= 2 ? 4 : (N <= 4 ? 3 : 2)) local
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const u64 i = i0 + u * kThreads;
+            const u64 i = i0 + u * threads;
             Raw32 v = r[u][0];
             if constexpr (N > 1) {
                 float acc[kElems];
@@ -207,6 +211,7 @@ __global__ void __launch_bounds__(kThreads, N <= 2 ? 4 : (N <= 4 ? 3 : 2)) local
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 4) local_shift_copy_kernel(const __grid_constant__ LocalArgs a) {
     constexpr u64 kPack = 32;
+    const unsigned threads = blockDim.x;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (unsigned t = blockIdx.x; t < a.tiles * a.segments; t += gridDim.x) {
@@ -221,10 +226,10 @@ __global__ void __launch_bounds__(kThreads, 4) local_shift_copy_kernel(const __g
         if (skew != 0 && packs != 0 && before - skew + packs * kPack + 16 > bytes) --packs;  // and so does the last
         const u64 head = (before < bytes ? before : bytes) / sizeof(T), tail0 = head + packs * (kPack / sizeof(T));
         if (tile == 0)
-            for (u64 e = threadIdx.x; e < head + (a.count - tail0); e += kThreads)
+            for (u64 e = threadIdx.x; e < head + (a.count - tail0); e += threads)
                 reduce_one<T, OpAdd, 1>(a, seg, 0, out_off, e < head ? e : tail0 + (e - head));
         const uint4* src = reinterpret_cast<const uint4*>(src0 + before - skew);
-        const u64 i = (u64)tile * kThreads + threadIdx.x;
+        const u64 i = (u64)tile * threads + threadIdx.x;
         const unsigned lane = threadIdx.x & 31u;
         uint4 w0 = make_uint4(0, 0, 0, 0), w1 = w0, w2;
         Raw32 v;
@@ -263,11 +268,12 @@ __global__ void __launch_bounds__(kThreads, 4) local_shift_copy_kernel(const __g
 // Inputs (or outputs) that are not aligned alike among themselves: one element per access.
 template <typename T, typename Op>
 __global__ void __launch_bounds__(kThreads) local_scalar_kernel(const __grid_constant__ LocalArgs a) {
+    const unsigned threads = blockDim.x;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (unsigned seg = 0; seg < a.segments; ++seg) {
         const u64 in_off = seg * a.in_step(sizeof(T)), out_off = seg * a.out_step(sizeof(T));
-        for (u64 e = (u64)blockIdx.x * kThreads + threadIdx.x; e < a.count; e += (u64)gridDim.x * kThreads) {
+        for (u64 e = (u64)blockIdx.x * threads + threadIdx.x; e < a.count; e += (u64)gridDim.x * threads) {
             if (a.nranks == 1 || a.kind == (int)Collective::AllGather) reduce_one<T, Op, 1>(a, seg, in_off, out_off, e);
             else reduce_one<T, Op, 0>(a, seg, in_off, out_off, e);
         }
@@ -278,6 +284,7 @@ struct Plan {
     LocalArgs args;
     enum { kElements, kAlike, kShifted } how = kElements;
     int max_ctas = 0;  // 0: one CTA per tile
+    int threads = kThreads;
     cudaStream_t stream = nullptr;
 };
 
@@ -285,7 +292,7 @@ cudaError_t start(void (*kernel)(LocalArgs), const Plan& p, u64 work, int elem_b
     const u64 grid = p.max_ctas > 0 ? std::min<u64>(work, (u64)p.max_ctas) : work;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3((unsigned)grid, 1, 1);
-    config.blockDim = dim3(kThreads, 1, 1);
+    config.blockDim = dim3(p.threads, 1, 1);
     config.stream = p.stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -293,18 +300,25 @@ cudaError_t start(void (*kernel)(LocalArgs), const Plan& p, u64 work, int elem_b
     config.attrs = attr;
     config.numAttrs = 1;
     made->grid = (int)grid;
-    made->block = kThreads;
+    made->block = p.threads;
     made->pack_bytes = p.how == Plan::kElements ? elem_bytes : 32;
     return cudaLaunchKernelEx(&config, kernel, p.args);
 }
 
+// half: the instance for half as many threads, where that is another one.
 template <typename T, int kPerThread = kBytes>
-cudaError_t start_tiles(void (*kernel)(LocalArgs), Plan& p, LocalLaunch* made) {
-    constexpr u64 tile = (u64)kThreads * (kPerThread / sizeof(T));
-    const u64 tiles = (p.args.count + tile - 1) / tile;
+cudaError_t start_tiles(void (*kernel)(LocalArgs), Plan& p, LocalLaunch* made, void (*half)(LocalArgs) = nullptr) {
+    // Half as many threads where a grid of kThreads leaves SMs idle or with one CTA beside two: an SM stores no faster than its
+    // L1 passes on (us, 256 -> 128 threads: all_reduce, 8 ranks, 512 KiB 4.4 -> 3.0, 1 MiB 4.8 -> 4.3, 2 MiB, 256 CTAs, 6.1 -> 6.2; 6 ranks, 1 MiB
+    // 3.8 -> 3.2; one rank, 4 MiB 3.6 -> 2.6; all_gather, 8 ranks, blocks of 200 KB 6.1 -> 3.8, of 512 KiB, 512 CTAs, 7.4 -> 7.5). And in
+    // a reduce_scatter, which loads most of what it moves (4 ranks, 1 MiB blocks 4.0 -> 3.4; 8 ranks, 2 MiB 23.5 -> 23.3).
+    const bool scatters = p.args.kind == (int)Collective::ReduceScatter;
+    const auto tiles_of = [&](int threads) { const u64 tile = (u64)threads * (kPerThread / sizeof(T)); return (p.args.count + tile - 1) / tile; };
+    if (2 * tiles_of(kThreads) * p.args.segments < 3 * kSms || (scatters && p.args.nranks >= 4)) p.threads = kThreads / 2;
+    const u64 tiles = tiles_of(p.threads);
     if (tiles * p.args.segments > 0x7fffffffull) return cudaErrorInvalidValue;
     p.args.tiles = (unsigned)tiles;
-    return start(kernel, p, tiles * p.args.segments, (int)sizeof(T), made);
+    return start(p.threads != kThreads && half != nullptr ? half : kernel, p, tiles * p.args.segments, (int)sizeof(T), made);
 }
 
 template <typename T, typename Op>
@@ -328,8 +342,9 @@ cudaError_t start_op(Plan& p, LocalLaunch* made) {
 
 // Copies: two-byte elements serve every type.
 cudaError_t start_copy(Plan& p, LocalLaunch* made) {
-    if (p.how == Plan::kAlike && p.args.nranks == 1) return start_tiles<__half, kCopyBytes>(local_kernel<__half, OpAdd, 1, false, kCopyBytes>, p, made);
-    if (p.how == Plan::kAlike) return start_tiles<__half>(local_kernel<__half, OpAdd, 1, false, kBytes>, p, made);
+    if (p.how == Plan::kAlike && p.args.nranks == 1) return start_tiles<__half, kCopyBytes>(local_kernel<__half, OpAdd, 1, false, kCopyBytes, kThreads>, p, made,
+                                                                                                   local_kernel<__half, OpAdd, 1, false, kCopyBytes, kThreads / 2>);
+    if (p.how == Plan::kAlike) return start_tiles<__half>(local_kernel<__half, OpAdd, 1, false, kBytes, kThreads>, p, made, local_kernel<__half, OpAdd, 1, false, kBytes, kThreads / 2>);
     if (p.how == Plan::kShifted) {
         const cudaError_t st = start_tiles<__half>(local_shift_copy_kernel<__half>, p, made);
         made->pack_bytes = 16;

@@ -107,3 +107,34 @@ def test_a_cap_on_ctas_holds_at_any_value(ranks, cap):
         comm.check_async_error()
     finally:
         comm.close()
+
+
+@pytest.mark.parametrize("ranks", [1, 2, 3, 5, 8])
+@pytest.mark.parametrize("collective", ["all_reduce", "reduce_scatter", "all_gather"])
+def test_both_sizes_of_cta_around_their_tiles(ranks, collective):
+    # 128 threads up to three CTAs for two SMs of what 256 would take, and in a reduce_scatter of four ranks and more; tiles of
+    # 4096 or 2048 elements here (one rank: 16384 or 8192). Around that line and around a tile's end, three alignments.
+    comm = nn.Communicator(devices=[0], loopback_ranks=ranks, wait_timeout_ms=2000) if ranks > 1 else nn.Communicator(devices=[0], wait_timeout_ms=2000)
+    try:
+        tile = 4096 if ranks > 1 else 16384
+        segments = 1 if collective == "all_reduce" or ranks == 1 else ranks
+        line = 222 // segments * tile
+        for k, count in enumerate([line - tile - 1, line, line + 1, line + tile, line + tile + 2049, 3 * line + 16]):
+            for s_in, s_out in ((0, 0), (1, 1), (0, 3)):
+                n_in = count * (ranks if collective == "reduce_scatter" else 1)
+                n_out = count * (ranks if collective == "all_gather" else 1)
+                _, ins = buffers(ranks, n_in, torch.bfloat16, [s_in] * ranks, 500 + k)
+                raw, outs = buffers(ranks, n_out, torch.bfloat16, [s_out] * ranks, 0)
+                a, b = (outs, ins) if ranks > 1 else (outs[0], ins[0])
+                if collective == "all_gather":
+                    comm.all_gather(a, b)
+                    expect = [torch.cat(ins)] * ranks
+                else:
+                    (comm.all_reduce if collective == "all_reduce" else comm.reduce_scatter)(a, b, op="avg")
+                    full = reference(ins, "avg")
+                    expect = [full] * ranks if collective == "all_reduce" else [full[r * count:(r + 1) * count] for r in range(ranks)]
+                for o, e in zip(outs, expect):
+                    assert torch.equal(o, e), (count, s_in, s_out)
+                untouched(raw, outs)
+    finally:
+        comm.close()
