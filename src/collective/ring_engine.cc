@@ -242,7 +242,7 @@ RingEngine::~RingEngine() {
 }
 
 int RingEngine::channels() const { return state_->cfg.channels; }
-int RingEngine::block_threads() const { return kernels::ring_block_threads(); }
+int RingEngine::block_threads() const { return state_->clusters > 0 ? kernels::ring_cluster_threads() : kernels::ring_block_threads(); }
 std::string RingEngine::async_error() const { return state_->net ? state_->net->first_error() : std::string(); }
 
 int RingEngine::launch_clusters(Collective collective, const CollectiveArgs& args) {

@@ -8,15 +8,17 @@
 // returned by an arrival on an mbarrier of the sender. Nothing is fenced and no counter is polled in global memory.
 //
 // Every warp is a ring of its own (a unit): it talks to the warps of the same index in the neighbours' CTAs only, so that
-// there is no barrier in the loop, and sixteen warps hide one another's hops (0.35 us for a slice of 512 bytes). The local
+// there is no barrier in the loop, and an SM's sixteen warps hide one another's hops (0.35 us for a slice of 512 bytes). They
+// come as four CTAs of four warps: a cluster lies within one GPC, and of small CTAs more clusters fit (8 ranks, one CTA of 16 warps
+// per SM 15 clusters on 120 SMs, now 71 that fill 142: 64 MiB 301 -> 259 us; 7 ranks 292 -> 230; two CTAs of 8 warps 275 and 240). The local
 // input of the next step is loaded before the wait for the neighbour. A slice is 1, 2, 4 or 8 rows of 32 vectors; the message is
 // cut so that all slices but its last ones are full and move without a condition per vector.
 //
 // Bound by the hops up to about 1 MiB, then by distributed shared memory (4.0-4.4 TB/s into neighbours, 5.3 in pairs; st.async,
 // plain remote stores and bulk copies alike). float sum, us with FIFOs in global memory and two groups of eight warps -> here: 4
-// ranks, 4 KiB 22.4 -> 7.8, 1 MiB 28.9 -> 10.2, 16 MiB 58.6 -> 37.0, 64 MiB 199 -> 130; 2 ranks, 64 MiB 133 -> 51; 8 ranks, 4 KiB 36.9 ->
-// 12.3, 64 MiB 407 -> 301; bf16, 4 ranks, 16 MiB of views that start off a vector 219 -> 40, reduce_scatter in ragged blocks of 4 MiB
-// 128 -> 33. Slots of 3 slices instead of 2, 32 warps of 4 rows or 12 of 8 are slower.
+// ranks, 4 KiB 22.4 -> 7.7, 1 MiB 28.9 -> 10.2, 16 MiB 58.6 -> 35.6, 64 MiB 199 -> 125; 2 ranks, 64 MiB 133 -> 51; 8 ranks, 4 KiB 36.9 ->
+// 12.7, 64 MiB 407 -> 259; bf16, 4 ranks, 16 MiB of views that start off a vector 219 -> 38, reduce_scatter in ragged blocks of 4 MiB
+// 128 -> 32. Slots of 3 slices instead of 2, or slices of 4 rows for all sizes, are slower.
 //
 // Every wait is bounded. The launch is cooperative, as all launches whose CTAs wait for one another.
 #include "kernels/sm100/ring_cluster.h"
@@ -37,7 +39,7 @@ namespace {
 
 using u64 = unsigned long long;
 
-constexpr int kWarps = 16, kThreads = kWarps * 32;
+constexpr int kWarps = 4, kThreads = kWarps * 32, kCtasPerSm = 4;
 constexpr int kSlots = 2;                 // slices that a unit's FIFO holds
 constexpr unsigned kRowBytes = 32 * 16;   // what a warp moves at a time
 // Rows of a slice (kRows below): 8 move most, fewer keep more warps busy in small messages.
@@ -82,7 +84,7 @@ __device__ __forceinline__ void cluster_sync() {
 }
 
 template <typename T, typename Op, bool kWide, int kRows>
-__global__ void __launch_bounds__(kThreads, 1) ring_cluster_kernel(const __grid_constant__ RingClusterArgs a) {
+__global__ void __launch_bounds__(kThreads, kCtasPerSm) ring_cluster_kernel(const __grid_constant__ RingClusterArgs a) {
     constexpr int kElems = 16 / sizeof(T);
     constexpr unsigned kRow = 32u * kElems, kSlice = kRows * kRow, kSliceBytes = kRows * kRowBytes;  // elements, elements, bytes
     extern __shared__ __align__(128) unsigned char fifo[];
@@ -376,8 +378,10 @@ Kernel pick_op(RedOp op, bool wide, int rows) {
 
 }  // namespace
 
+int ring_cluster_threads() { return kThreads; }
+
 int ring_cluster_capacity(int nranks) {
-    const Kernel kernel = pick<float, OpAdd>(true, kMostRows);  // every instance runs one CTA per SM: its FIFOs fill shared memory
+    const Kernel kernel = pick<float, OpAdd>(true, kMostRows);  // every instance runs kCtasPerSm: its FIFOs and registers see to that
     int clusters = 0;
     cudaLaunchAttribute attrs[2];
     const cudaLaunchConfig_t config = configure(nranks, 1, nullptr, attrs);

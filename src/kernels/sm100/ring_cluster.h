@@ -29,6 +29,7 @@ namespace b200ccl::kernels {
 
 // Clusters of `nranks` CTAs that are resident at once on the current device; 0 when it cannot be told.
 int ring_cluster_capacity(int nranks);
+int ring_cluster_threads();
 
 // One cooperative launch of at most `clusters` clusters. wide: 16-byte accesses (all_reduce: buffers aligned alike modulo 16, args.lead
 // elements past it; reduce_scatter and all_gather: buffers and every block 16-byte aligned), else element by element.
