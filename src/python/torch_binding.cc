@@ -69,7 +69,8 @@ struct Side {
     ~Side() { Py_XDECREF(held); }
 
     bool read(PyObject* obj) {
-        if (THPVariable_Check(obj)) {
+        // (Whether a list is a tensor is asked of the tensor class, which takes as long as looking at five tensors.)
+        if (!PyList_CheckExact(obj) && !PyTuple_CheckExact(obj) && THPVariable_Check(obj)) {
             single = true;
             size = 1;
             item[0] = obj;
