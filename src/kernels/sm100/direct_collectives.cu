@@ -412,7 +412,9 @@ cudaError_t launch_reduce_n(int nranks, const ParamT& param, const LaunchConfig&
             case 2: return launch(reduce_kernel<T, Op, 2, PackT, false, ParamT>, param, cfg);
             case 4: return launch(reduce_kernel<T, Op, 4, PackT, false, ParamT>, param, cfg);
             case 8: return launch(reduce_kernel<T, Op, 8, PackT, false, ParamT>, param, cfg);
-            default: return launch(reduce_kernel<T, Op, 0, PackT, false, ParamT>, param, cfg);
+            default:
+                if constexpr (kAllRanksHere<ParamT>) return cudaErrorInvalidValue;
+                else return launch(reduce_kernel<T, Op, 0, PackT, false, ParamT>, param, cfg);
         }
     }
 }
