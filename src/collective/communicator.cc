@@ -1002,7 +1002,6 @@ void Communicator::Impl::launch_low_latency(const CollectiveArgs& args) {
             a.area[p] = static_cast<unsigned long long*>(ll_area_->rank_ptr(p));
             a.ctrl[p] = static_cast<dev::ControlBlock*>(ctrl_->rank_ptr(p));
         }
-        a.own_ctrl = a.ctrl[local_[i].grank];
         a.status = local_[i].status;
         a.timeout_ns = timeout_ns_;
         a.nwords = static_cast<unsigned>(args.count * dtype_size(args.dtype) / 4);

@@ -138,8 +138,7 @@ struct LlArgs {
     const void* in;              // local input (any device memory of this rank)
     void* out;                   // local output
     unsigned long long* area[kMaxRanks];  // every rank's receive area
-    ControlBlock* own_ctrl;
-    ControlBlock* ctrl[kMaxRanks];        // to raise every rank's abort word when a wait runs out
+    ControlBlock* ctrl[kMaxRanks];        // the own one, and to raise every rank's abort word when a wait runs out
     Status* status;
     unsigned long long timeout_ns;
     unsigned int nwords;         // 4-byte words in the message

@@ -14,6 +14,9 @@
 #include "kernels/sm100/sync.cuh"
 #include "kernels/sm100/vec.cuh"
 
+#include <cstdint>
+#include <type_traits>
+
 namespace b200ccl::kernels {
 
 using namespace b200ccl::dev;
@@ -54,20 +57,27 @@ struct Word<__nv_bfloat16> {
 
 constexpr unsigned kWordsAtATime = kLlCtas * kBlockThreads;  // words that the CTAs of a rank take at a time
 
-// One rank's part of the exchange, kBatch words per thread at a time; false when a wait gave up.
-template <typename T, typename Op, int kBatch>
-__device__ __forceinline__ bool exchange(const LlArgs& a, u64 call) {
-    static_assert(kBatch * kMaxRanks <= 32, "pending words are bits of one register");
-    const int n = a.nranks, rank = a.rank;
-    const unsigned flag = static_cast<unsigned>(call % 0xffffffffull) + 1u;  // never 0: a zeroed area matches no call
-    const u64 parity = call & 1ull;
+// Emulated ranks: what they share. The rank is blockIdx.y.
+struct LlOneGpuArgs {
+    const void* in[kMaxRanks];
+    void* out[kMaxRanks];
+    u64* area[kMaxRanks];
+    ControlBlock* ctrl[kMaxRanks];
+    Status* status;
+    u64 timeout_ns;
+    unsigned nwords;
+    float scale;
+    int nranks;
+    int pad;
+};
+static_assert(sizeof(LlOneGpuArgs) % 64 > 16 && sizeof(LlOneGpuArgs) % 64 <= 32);  // launches fastest, see local_collectives.cu
+
+// 1. Publish, kBatch words per thread at a time. Between GPUs: word w of this rank goes to slot (parity, rank, w) of every rank.
+template <int kBatch>
+__device__ __forceinline__ void publish(const LlArgs& a, int rank, u64 parity, unsigned flag, unsigned first) {
+    const int n = a.nranks;
     const unsigned* in = static_cast<const unsigned*>(a.in);
-    unsigned* out = static_cast<unsigned*>(a.out);
-    const unsigned first = blockIdx.x * kBlockThreads + threadIdx.x;
-
     auto has = [&](unsigned w0, int u) { return u == 0 || w0 + u * kWordsAtATime < a.nwords; };  // the loops see to the first one
-
-    // 1. Publish: word w of this rank goes to slot (parity, rank, w) of every rank.
     for (unsigned w0 = first; w0 < a.nwords; w0 += kWordsAtATime * kBatch) {
         unsigned v[kBatch];
 #pragma unroll
@@ -82,6 +92,52 @@ __device__ __forceinline__ bool exchange(const LlArgs& a, u64 call) {
                 if (has(w0, u)) st_slot(a.area[q] + slot + u * kWordsAtATime, v[u], flag);
         }
     }
+}
+
+// Emulated ranks: the thread that will collect a word for this rank stores every rank's word into this rank's slots itself. The
+// same stores in all, but a thread only ever waits for its own: no CTA waits for another one, and the launch is a plain
+// programmatic dependent of the one before instead of a cooperative one. Not in place: see outputs_overlap_inputs(). (A thread that did so for every rank at once,
+// ranks^2 slots, was slower from five ranks up: 8 ranks, 16 KiB 10.1 us.) Cooperative -> now: 2 ranks, 1 KiB 4.3 -> 3.1 us, 128 KiB 10.2 -> 7.2;
+// 8 ranks, 1 KiB 4.5 -> 3.3, 16 KiB 6.1 -> 3.4, 64 KiB 8.2 -> 6.7, 128 KiB 14.3 -> 11.4.
+template <int kBatch>
+__device__ __forceinline__ void publish(const LlOneGpuArgs& a, int rank, u64 parity, unsigned flag, unsigned first) {
+    const int n = a.nranks;
+    u64* own_area = a.area[rank] + parity * (u64)n * kLlMaxWords;
+    auto has = [&](unsigned w0, int u) { return u == 0 || w0 + u * kWordsAtATime < a.nwords; };
+    for (unsigned w0 = first; w0 < a.nwords; w0 += kWordsAtATime * kBatch) {
+        unsigned v[kBatch][kMaxRanks];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+#pragma unroll
+            for (int p = 0; p < kMaxRanks; ++p)
+                if (p < n && has(w0, u)) v[u][p] = static_cast<const unsigned*>(a.in[p])[w0 + u * kWordsAtATime];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+#pragma unroll
+            for (int p = 0; p < kMaxRanks; ++p)
+                if (p < n && has(w0, u)) st_slot(own_area + (u64)p * kLlMaxWords + w0 + u * kWordsAtATime, v[u][p], flag);
+    }
+}
+
+template <typename A>
+__device__ __forceinline__ unsigned* output(const A& a, int rank) {
+    if constexpr (std::is_same_v<A, LlOneGpuArgs>) return static_cast<unsigned*>(a.out[rank]);
+    else return static_cast<unsigned*>(a.out);
+}
+
+// One rank's part of the exchange; false when a wait gave up.
+template <typename T, typename Op, int kBatch, typename A>
+__device__ __forceinline__ bool exchange(const A& a, int rank, u64 call) {
+    static_assert(kBatch * kMaxRanks <= 32, "pending words are bits of one register");
+    const int n = a.nranks;
+    const unsigned flag = static_cast<unsigned>(call % 0xffffffffull) + 1u;  // never 0: a zeroed area matches no call
+    const u64 parity = call & 1ull;
+    unsigned* out = output(a, rank);
+    ControlBlock* own = a.ctrl[rank];
+    const unsigned first = blockIdx.x * kBlockThreads + threadIdx.x;
+    auto has = [&](unsigned w0, int u) { return u == 0 || w0 + u * kWordsAtATime < a.nwords; };
+
+    publish<kBatch>(a, rank, parity, flag, first);
     // 2. Collect: the slots of all sources and of kBatch words are loaded together, then only those whose call number
     //    has not arrived yet are polled again; combine in rank order.
     bool ok = true;
@@ -107,14 +163,14 @@ __device__ __forceinline__ bool exchange(const LlArgs& a, u64 call) {
                     if ((pending & (1u << (u * kMaxRanks + p))) && v[u][p].y == flag) pending &= ~(1u << (u * kMaxRanks + p));
             if (pending != 0u && (++polls & 255u) == 0u) {
                 const unsigned who = (unsigned)(__ffs((int)pending) - 1) % kMaxRanks;
-                if (ld_volatile_u32(&a.own_ctrl->abort_flag) != 0u) {
-                    report_failure(a.status, a.own_ctrl, nullptr, 0, kStatusAborted, who, 20u, call, global_timer_ns() - t0);
+                if (ld_volatile_u32(&own->abort_flag) != 0u) {
+                    report_failure(a.status, own, nullptr, 0, kStatusAborted, who, 20u, call, global_timer_ns() - t0);
                     ok = false;
                     break;
                 }
                 const u64 waited = global_timer_ns() - t0;
                 if (waited > a.timeout_ns) {
-                    report_failure(a.status, a.own_ctrl, a.ctrl, n, kStatusTimeout, who, 20u, call, waited);
+                    report_failure(a.status, own, a.ctrl, n, kStatusTimeout, who, 20u, call, waited);
                     ok = false;
                     break;
                 }
@@ -145,24 +201,72 @@ __device__ __forceinline__ bool exchange(const LlArgs& a, u64 call) {
     return ok;
 }
 
+template <typename A>
+__device__ __forceinline__ const A& select_args(const A& a) { return a; }
+template <typename A>
+__device__ __forceinline__ const A& select_args(const LoopPack<A>& all) { return all.r[blockIdx.y]; }
+
 template <typename T, typename Op, int kBatch, typename ParamT>
 __global__ void __launch_bounds__(kBlockThreads) ll_kernel(const __grid_constant__ ParamT param) {
-    const LlArgs* ap;
-    if constexpr (sizeof(ParamT) == sizeof(LlArgs)) ap = reinterpret_cast<const LlArgs*>(&param);
-    else ap = reinterpret_cast<const LlArgs*>(&param) + blockIdx.y;
-    const LlArgs& a = *ap;
+    constexpr bool kOneGpu = std::is_same_v<ParamT, LlOneGpuArgs>;
+    if constexpr (kOneGpu) {
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
+    const auto& a = select_args(param);
+    int rank;
+    if constexpr (kOneGpu) rank = (int)blockIdx.y;
+    else rank = a.rank;
     // Every thread reads the CTA's call counter; thread 0 writes it back at the end.
-    const u64 call = a.own_ctrl->ll_epoch[blockIdx.x] + 1;
-    const bool ok = exchange<T, Op, kBatch>(a, call);
+    ControlBlock* own = a.ctrl[rank];
+    const u64 call = own->ll_epoch[blockIdx.x] + 1;
+    const bool ok = exchange<T, Op, kBatch>(a, rank, call);
     // A CTA whose wait gave up leaves its counter alone: the communicator is poisoned anyway.
-    if (__syncthreads_and(ok ? 1 : 0) && threadIdx.x == 0) a.own_ctrl->ll_epoch[blockIdx.x] = call;
+    if (__syncthreads_and(ok ? 1 : 0) && threadIdx.x == 0) own->ll_epoch[blockIdx.x] = call;
+}
+
+// Whether an output overlaps an input, its own rank's (a call in place) or another one's. The thread that writes a word of it knows
+// that every rank has read that word only where the ranks wait for one another.
+bool outputs_overlap_inputs(const LlArgs* args, int ranks) {
+    const std::uintptr_t bytes = 4ull * args[0].nwords;
+    for (int q = 0; q < ranks; ++q)
+        for (int r = 0; r < ranks; ++r) {
+            const auto out = reinterpret_cast<std::uintptr_t>(args[q].out), in = reinterpret_cast<std::uintptr_t>(args[r].in);
+            if (out < in + bytes && in < out + bytes) return true;
+        }
+    return false;
 }
 
 template <typename T, typename Op, int kBatch>
-cudaError_t launch_ll_t(const LlArgs* args, int loop_ranks, cudaStream_t stream) {
+cudaError_t launch_ll_t(const LlArgs* args, int loop_ranks, cudaStream_t stream, bool waiting) {
     dim3 grid(kLlCtas, loop_ranks > 0 ? loop_ranks : 1, 1), block(kBlockThreads, 1, 1);
+    if (loop_ranks > kMaxRanks) return cudaErrorInvalidValue;
     if (loop_ranks > 0) {
-        if (loop_ranks > kMaxRanks) return cudaErrorInvalidValue;
+        if (!waiting) {
+            LlOneGpuArgs a = {};
+            for (int r = 0; r < loop_ranks; ++r) {
+                a.in[r] = args[r].in;
+                a.out[r] = args[r].out;
+                a.area[r] = args[0].area[r];
+                a.ctrl[r] = args[0].ctrl[r];
+            }
+            a.status = args[0].status;
+            a.timeout_ns = args[0].timeout_ns;
+            a.nwords = args[0].nwords;
+            a.scale = args[0].scale;
+            a.nranks = loop_ranks;
+            cudaLaunchAttribute attrs[1];
+            attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attrs[0].val.programmaticStreamSerializationAllowed = 1;
+            cudaLaunchConfig_t config = {};
+            config.gridDim = grid;
+            config.blockDim = block;
+            config.stream = stream;
+            config.attrs = attrs;
+            config.numAttrs = 1;
+            return cudaLaunchKernelEx(&config, ll_kernel<T, Op, kBatch, LlOneGpuArgs>, a);
+        }
+        // Ranks that wait for one another: all CTAs must be resident, which a cooperative launch checks.
         LoopPack<LlArgs> pack;
         for (int r = 0; r < loop_ranks; ++r) pack.r[r] = args[r];
         void* params[] = {&pack};
@@ -172,12 +276,16 @@ cudaError_t launch_ll_t(const LlArgs* args, int loop_ranks, cudaStream_t stream)
     return cudaGetLastError();
 }
 
-// One word at a time, each takes a round trip to the slots (emulated ranks, 128 KiB, one at a time -> four: 2 ranks 10.2 -> 8.2 us,
-// 4 ranks 12.3 -> 10.2, 8 ranks 14.3 -> 12.3). But a batch that is not full only costs its registers (91 against 40) and
-// conditions: 20000 bytes, 2 ranks 4.6 -> 6.1 us, 8 ranks 6.2 -> 6.8; level at 40000 and 70000 bytes. So from four full words up.
+// One word at a time, each takes a round trip to the slots; but a batch that is not full costs its registers (91 or 124 against 40)
+// and conditions. Ranks that wait for one another (as emulated ranks did; us, one at a time / four): 20000 bytes, 2 ranks 4.6 / 6.1,
+// 8 ranks 6.2 / 6.8; level at 40000 and 70000 bytes; 128 KiB, 8 ranks 14.3 / 12.3. So from four full words up. Emulated ranks as they are
+// now: 32 KiB, 2 ranks 3.2 / 4.3, 4 ranks 4.3 / 4.4, 6 ranks 6.3 / 4.7, 8 ranks 7.3 / 5.2; 64 KiB, 2 ranks 4.9 / 4.6, 8 ranks 12.6 / 6.7.
 template <typename T, typename Op>
 cudaError_t launch_ll_size(const LlArgs* args, int loop_ranks, cudaStream_t stream) {
-    return args[0].nwords <= 4 * kWordsAtATime ? launch_ll_t<T, Op, 1>(args, loop_ranks, stream) : launch_ll_t<T, Op, 4>(args, loop_ranks, stream);
+    const bool waiting = !kRanksShareGpu || loop_ranks == 0 || outputs_overlap_inputs(args, loop_ranks);
+    const unsigned singles = waiting ? 4u : (loop_ranks <= 5 ? 2u : 1u);
+    return args[0].nwords <= singles * kWordsAtATime ? launch_ll_t<T, Op, 1>(args, loop_ranks, stream, waiting)
+                                                     : launch_ll_t<T, Op, 4>(args, loop_ranks, stream, waiting);
 }
 
 template <typename T>

@@ -65,12 +65,13 @@ def test_buffers_misaligned_differently_and_a_capped_grid(algo):
 
 @pytest.mark.parametrize("ranks", [2, 3, 8])
 def test_low_latency_batches_of_words(ranks):
-    # One word per thread at a time up to 64 KiB, four above: both sides of that line, a ragged batch, and the largest message;
+    # One word per thread at a time up to 16 KiB (32 KiB up to five ranks), four above: both sides of that line, a ragged batch, and
+    # the largest message;
     # long and short messages in turn, so that slots of both kinds of call are used again.
     comm = nn.Communicator(devices=[0], loopback_ranks=ranks, algo="ll", wait_timeout_ms=2000)
     try:
         gen = torch.Generator(device="cuda").manual_seed(3)
-        for k, words in enumerate([4096, 4097, 5, 16384, 16385, 4095, 16383, 32768, 1, 32767, 12289]):
+        for k, words in enumerate([4096, 4097, 5, 8192, 8193, 16384, 16385, 4095, 16383, 32768, 1, 32767, 12289]):
             ins = [torch.randn(words * 2, device="cuda", generator=gen).half() for _ in range(ranks)]
             outs = [torch.empty_like(t) for t in ins]
             op = ["sum", "avg", "max", "min"][k % 4]
@@ -83,6 +84,33 @@ def test_low_latency_batches_of_words(ranks):
                 acc = acc * torch.tensor(1.0, device="cuda").div(ranks)
             for o in outs:
                 assert torch.equal(o, acc.half()), (words, op)
+        comm.check_async_error()
+    finally:
+        comm.close()
+
+
+@pytest.mark.parametrize("ranks", [2, 8])
+@pytest.mark.parametrize("rotate", [0, 1])
+def test_low_latency_outputs_that_are_inputs(ranks, rotate):
+    # In place, or into the next rank's input: a word is only overwritten when every rank has read it. Calls of both kinds in turn
+    # share slots and counters.
+    comm = nn.Communicator(devices=[0], loopback_ranks=ranks, algo="ll", wait_timeout_ms=2000)
+    try:
+        gen = torch.Generator(device="cuda").manual_seed(4)
+        wrong = torch.zeros((), device="cuda", dtype=torch.int64)
+        for k in range(60):
+            words = (32768, 4096, 20000)[k % 3]
+            ins = [torch.randn(words, device="cuda", generator=gen) for _ in range(ranks)]
+            expect = torch.stack(ins).sum(0) if ranks == 2 else torch.stack(ins).max(0).values
+            op = "sum" if ranks == 2 else "max"
+            apart = [torch.empty_like(t) for t in ins]
+            comm.all_reduce(apart, ins, op=op)
+            outs = ins[rotate:] + ins[:rotate]
+            comm.all_reduce(outs, ins, op=op)
+            assert comm.last_call()["algo"] == "ll"
+            for o in outs + apart:
+                wrong += (o != expect).sum()
+        assert wrong.item() == 0
         comm.check_async_error()
     finally:
         comm.close()
