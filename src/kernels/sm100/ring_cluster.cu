@@ -5,7 +5,7 @@
 // hand-over is a release and an acquire of step counters, which takes 3.4 us per hop on one B200 (1.2 to release, 1 to see
 // the counter, 1.2 to load the slice). Here the CTAs of a channel, one per rank, are a thread block cluster: the receiver's
 // memory is its shared memory, a slice goes there with st.async, whose bytes an mbarrier of the receiver counts, and a slot is
-// returned by an arrival on an mbarrier of the sender. Nothing is fenced and no counter is polled in global memory.
+// returned by an arrival on an mbarrier of the sender, behind a fence for shared memory only. No counter is polled in global memory.
 //
 // Every warp is a ring of its own (a unit): it talks to the warps of the same index in the neighbours' CTAs only, so that
 // there is no barrier in the loop, and an SM's sixteen warps hide one another's hops (0.35 us for a slice of 512 bytes). They
@@ -16,9 +16,9 @@
 //
 // Bound by the hops up to about 1 MiB, then by distributed shared memory (4.0-4.4 TB/s into neighbours, 5.3 in pairs; st.async,
 // plain remote stores and bulk copies alike). float sum, us with FIFOs in global memory and two groups of eight warps -> here: 4
-// ranks, 4 KiB 22.4 -> 7.7, 1 MiB 28.9 -> 10.2, 16 MiB 58.6 -> 35.6, 64 MiB 199 -> 125; 2 ranks, 64 MiB 133 -> 51; 8 ranks, 4 KiB 36.9 ->
-// 12.7, 64 MiB 407 -> 259; bf16, 4 ranks, 16 MiB of views that start off a vector 219 -> 38, reduce_scatter in ragged blocks of 4 MiB
-// 128 -> 32. Slots of 3 slices instead of 2, or slices of 4 rows for all sizes, are slower.
+// ranks, 4 KiB 22.4 -> 8.2, 1 MiB 28.9 -> 10.2, 16 MiB 58.6 -> 35.8, 64 MiB 199 -> 124; 2 ranks, 64 MiB 133 -> 51; 8 ranks, 4 KiB 36.9 ->
+// 12.3, 64 MiB 407 -> 261; bf16, 4 ranks, 16 MiB of views that start off a vector 219 -> 39, reduce_scatter in ragged blocks of 4 MiB
+// 128 -> 31. Slots of 3 slices instead of 2, or slices of 4 rows for all sizes, are slower.
 //
 // Every wait is bounded. The launch is cooperative, as all launches whose CTAs wait for one another.
 #include "kernels/sm100/ring_cluster.h"
@@ -74,8 +74,16 @@ __device__ __forceinline__ void st_slot16(unsigned remote, const uint4& v, unsig
 __device__ __forceinline__ void announce(unsigned remote_bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(remote_bar), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void return_slot(unsigned remote_bar) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
+// Hands a slot of this CTA back to the rank that fills it, whose wait acquires at cluster scope. What the warp has read from the slot
+// before is ordered before everything that rank does after its wait: __syncwarp() orders the lanes' reads before the fence, and the
+// fence releases at cluster scope what was done to this CTA's shared memory. It does not wait for the stores to the output, as an arrival
+// that releases everything does (float sum, us, here / so: 4 ranks, 4 KiB 8.2 / 10.3, 16 MiB 35.8 / 43.0; 8 ranks, 64 MiB 261 / 319).
+__device__ __forceinline__ void return_slot(unsigned remote_bar, unsigned lane) {
+    __syncwarp();
+    if (lane == 0) {
+        asm volatile("fence.release.sync_restrict::shared::cta.cluster;" ::: "memory");
+        asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
+    }
 }
 
 __device__ __forceinline__ void cluster_sync() {
@@ -234,18 +242,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) ring_cluster_kernel(cons
                     got[u] = Wide<T>::pack(acc);
                 }
             }
-            // The slot is returned when every lane holds its part of it: the vote needs the loaded values. An arrival that follows
-            // the loads in program order only was seen to overtake them (a row of a slice replaced by that of the slice two
-            // later, in one of 100 all_gathers); one that releases at cluster scope waits for the stores to the output as
-            // well (4 ranks, 16 MiB: 45.0 us instead of 37.1).
-            unsigned seen = 0;
-#pragma unroll
-            for (int u = 0; u < kRows; ++u) {
-                if (over(u)) break;
-                if (has(u)) seen ^= got[u].x;
-            }
-            const unsigned who = __any_sync(0xffffffffu, seen == 0x5bd1e995u) ? 1u : 0u;  // either lane will do
-            if (lane == who) return_slot(prev_empty + slot * 8u);
+            return_slot(prev_empty + slot * 8u, lane);
             ++received;
         } else {
 #pragma unroll

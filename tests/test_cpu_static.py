@@ -145,3 +145,21 @@ def test_transport_kinds_and_parser_contract():
     parse = types_cc[types_cc.index("bool parse_transport"):]
     parse = parse[:parse.index("\n}\n")]
     assert '"rdma"' in parse and '"socket"' not in parse and '"mixed"' not in parse
+
+
+def test_a_ring_slot_in_a_cluster_is_returned_by_a_release_that_reaches_the_cluster():
+    # What a rank has read from its FIFO is ordered before the next slice by the memory model, not by the timing of the loads: the
+    # lanes' reads come before a release at cluster scope (the sender's wait acquires at that scope), and nothing is inferred from values.
+    ring = re.sub(r"//[^\n]*", "", read(os.path.join(KERNELS, "ring_cluster.cu")))
+    give_back = ring[ring.index("void return_slot("):]
+    give_back = give_back[:give_back.index("\n}\n")]
+    assert give_back.index("__syncwarp();") < give_back.index("mbarrier.arrive.")
+    restricted = "fence.release.sync_restrict::shared::cta.cluster;" in give_back and "mbarrier.arrive.relaxed.cluster.shared::cluster" in give_back
+    assert restricted or "mbarrier.arrive.release.cluster.shared::cluster" in give_back
+    if restricted:
+        assert give_back.index("fence.release.") < give_back.index("mbarrier.arrive.")
+    assert ring.index("got[u] = ld_slot16(") < ring.index("return_slot(prev_empty")
+    for arrival in re.findall(r"mbarrier\.arrive[\w.:]*shared::cluster", ring):
+        assert ".cluster.shared::cluster" in arrival, f"{arrival}: an arrival in another CTA names its scope"
+    sync = read(os.path.join(KERNELS, "sync.cuh"))
+    assert "mbarrier.try_wait.parity.acquire.cluster" in sync

@@ -144,3 +144,28 @@ def test_wait_in_a_cluster_reports_instead_of_hanging():
     assert out[0] == 0 and out[1] == 1 and out[2] == 97
     assert 45.0 <= waited.value <= 1000.0
     assert torch.ones(4, device="cuda").sum().item() == 4
+
+
+@pytest.mark.parametrize("ranks", [2, 4, 8])
+def test_slots_of_reducing_steps_are_not_filled_before_they_are_read(ranks):
+    # As above for all_reduce and reduce_scatter, whose receiving steps also combine; with max every element names its place.
+    comm = nn.Communicator(devices=[0], loopback_ranks=ranks, algo="ring", wait_timeout_ms=2000)
+    try:
+        for count in (1 << 20, (1 << 20) + 5):
+            ins = [torch.arange(count, device="cuda", dtype=torch.float32) * ranks + (r + count) % ranks for r in range(ranks)]
+            most = torch.stack(ins).max(0).values
+            block = count // ranks
+            outs = [torch.empty(count, device="cuda") for _ in range(ranks)]
+            shards = [torch.empty(block, device="cuda") for _ in range(ranks)]
+            parts = [t[:block * ranks] for t in ins]
+            wrong = torch.zeros((), device="cuda", dtype=torch.int64)
+            for _ in range(100):
+                comm.all_reduce(outs, ins, op="max")
+                comm.reduce_scatter(shards, parts, op="max")
+                for o in outs:
+                    wrong += (o != most).sum()
+                wrong += (torch.cat(shards) != most[:block * ranks]).sum()
+            assert wrong.item() == 0
+        comm.check_async_error()
+    finally:
+        comm.close()
