@@ -59,8 +59,8 @@ struct CollectiveArgs {
 struct CallInfo {
     Collective collective = Collective::AllReduce;
     Algo algo = Algo::Auto;
-    int grid = 0;
-    int block = 0;
+    int grid = 0;   // CTAs per rank; ring: channels
+    int block = 0;  // threads of a CTA; ring: of a channel, which may be several CTAs of every rank
     bool staged_in = false;   // input went through the staging arena
     bool staged_out = false;  // output went through the staging arena
     bool vectorized = false;  // every buffer and block is a whole number of aligned 16-byte packs (pack_bytes says what was moved)

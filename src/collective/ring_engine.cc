@@ -133,7 +133,9 @@ RingEngine::RingEngine(const RingEngineConfig& config, mem::SymmetricAllocator* 
     if (config.loopback && dev::kRanksShareGpu && !net && !any_shm && s.stats.get() == nullptr) {
         DeviceGuard guard(config.local[0].device);
         s.clusters = kernels::ring_cluster_capacity(n);
-        if (config.channels_asked_for) s.clusters = std::min(s.clusters, C);
+        // A channel keeps its meaning, an SM of every rank (4 ranks, 16 MiB, 16 channels: 45 us; 125 us with a cluster each, 85 us in
+        // ring_simple.cu).
+        if (config.channels_asked_for) s.clusters = std::min(s.clusters, C * kernels::ring_clusters_per_channel());
     }
 
     auto ctrl_of = [&](int grank) -> dev::ControlBlock* {
@@ -242,7 +244,9 @@ RingEngine::~RingEngine() {
 }
 
 int RingEngine::channels() const { return state_->cfg.channels; }
-int RingEngine::block_threads() const { return state_->clusters > 0 ? kernels::ring_cluster_threads() : kernels::ring_block_threads(); }
+int RingEngine::block_threads() const {
+    return state_->clusters > 0 ? kernels::ring_cluster_threads() * kernels::ring_clusters_per_channel() : kernels::ring_block_threads();
+}
 std::string RingEngine::async_error() const { return state_->net ? state_->net->first_error() : std::string(); }
 
 int RingEngine::launch_clusters(Collective collective, const CollectiveArgs& args) {
@@ -271,7 +275,8 @@ int RingEngine::launch_clusters(Collective collective, const CollectiveArgs& arg
     int used = 0;
     DeviceGuard guard(s.cfg.local[0].device);
     B2_CUDA(kernels::launch_ring_cluster(args.dtype, args.redop, wide, a, s.clusters, args.streams[0], &used));
-    return used;
+    const int per_channel = kernels::ring_clusters_per_channel();
+    return (used + per_channel - 1) / per_channel;
 }
 
 int RingEngine::launch(Collective collective, const CollectiveArgs& args) {

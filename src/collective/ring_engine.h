@@ -46,7 +46,7 @@ public:
     RingEngine(const RingEngineConfig& config, mem::SymmetricAllocator* alloc, const mem::SymmetricRegion* ctrl,
                Bootstrap* bootstrap);
     ~RingEngine();
-    int launch(Collective collective, const CollectiveArgs& args);  // CTAs per rank
+    int launch(Collective collective, const CollectiveArgs& args);  // channels of the call
     int channels() const;
     int block_threads() const;
     std::string async_error() const;  // first proxy/transport failure, "" when none

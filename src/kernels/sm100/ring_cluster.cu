@@ -376,6 +376,7 @@ Kernel pick_op(RedOp op, bool wide, int rows) {
 }  // namespace
 
 int ring_cluster_threads() { return kThreads; }
+int ring_clusters_per_channel() { return kCtasPerSm; }
 
 int ring_cluster_capacity(int nranks) {
     const Kernel kernel = pick<float, OpAdd>(true, kMostRows);  // every instance runs kCtasPerSm: its FIFOs and registers see to that

@@ -29,7 +29,9 @@ namespace b200ccl::kernels {
 
 // Clusters of `nranks` CTAs that are resident at once on the current device; 0 when it cannot be told.
 int ring_cluster_capacity(int nranks);
-int ring_cluster_threads();
+int ring_cluster_threads();  // of a CTA
+// Clusters that make a channel: as many warps of every rank as a channel of ring_simple.cu has, on as many SMs.
+int ring_clusters_per_channel();
 
 // One cooperative launch of at most `clusters` clusters. wide: 16-byte accesses (all_reduce: buffers aligned alike modulo 16, args.lead
 // elements past it; reduce_scatter and all_gather: buffers and every block 16-byte aligned), else element by element.

@@ -169,3 +169,20 @@ def test_slots_of_reducing_steps_are_not_filled_before_they_are_read(ranks):
         comm.check_async_error()
     finally:
         comm.close()
+
+
+@pytest.mark.parametrize("channels", [1, 3, 32])
+def test_a_channel_has_the_threads_of_a_whole_cta(channels):
+    # A channel that somebody asks for is 512 threads of every rank, however many clusters make it up.
+    comm = nn.Communicator(devices=[0], loopback_ranks=4, algo="ring", channels=channels, wait_timeout_ms=2000)
+    try:
+        for count in (1, 1 << 20, (1 << 22) + 3):
+            ins = [torch.randn(count, device="cuda") for _ in range(4)]
+            outs = [torch.empty_like(t) for t in ins]
+            comm.all_reduce(outs, ins, op="max")
+            info = comm.last_call()
+            assert info["algo"] == "ring" and 1 <= info["grid"] <= channels and info["block"] == 512
+            assert all(torch.equal(o, torch.stack(ins).max(0).values) for o in outs)
+        assert info["grid"] == channels
+    finally:
+        comm.close()
