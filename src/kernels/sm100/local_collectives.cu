@@ -312,9 +312,11 @@ cudaError_t start_tiles(void (*kernel)(LocalArgs), Plan& p, LocalLaunch* made, v
     // L1 passes on (us, 256 -> 128 threads: all_reduce, 8 ranks, 512 KiB 4.4 -> 3.0, 1 MiB 4.8 -> 4.3, 2 MiB, 256 CTAs, 6.1 -> 6.2; 6 ranks, 1 MiB
     // 3.8 -> 3.2; one rank, 4 MiB 3.6 -> 2.6; all_gather, 8 ranks, blocks of 200 KB 6.1 -> 3.8, of 512 KiB, 512 CTAs, 7.4 -> 7.5). And in
     // a reduce_scatter, which loads most of what it moves (4 ranks, 1 MiB blocks 4.0 -> 3.4; 8 ranks, 2 MiB 23.5 -> 23.3).
+    // Not where the caller caps the CTAs below that number: those that there are then loop, and half of them would be missing.
     const bool scatters = p.args.kind == (int)Collective::ReduceScatter;
     const auto tiles_of = [&](int threads) { const u64 tile = (u64)threads * (kPerThread / sizeof(T)); return (p.args.count + tile - 1) / tile; };
-    if (2 * tiles_of(kThreads) * p.args.segments < 3 * kSms || (scatters && p.args.nranks >= 4)) p.threads = kThreads / 2;
+    const bool capped = p.max_ctas > 0 && tiles_of(kThreads / 2) * p.args.segments > (u64)p.max_ctas;
+    if (!capped && (2 * tiles_of(kThreads) * p.args.segments < 3 * kSms || (scatters && p.args.nranks >= 4))) p.threads = kThreads / 2;
     const u64 tiles = tiles_of(p.threads);
     if (tiles * p.args.segments > 0x7fffffffull) return cudaErrorInvalidValue;
     p.args.tiles = (unsigned)tiles;

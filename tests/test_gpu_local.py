@@ -138,3 +138,35 @@ def test_both_sizes_of_cta_around_their_tiles(ranks, collective):
                 untouched(raw, outs)
     finally:
         comm.close()
+
+
+@pytest.mark.parametrize("ranks", [1, 4, 8])
+def test_a_cap_on_ctas_does_not_halve_their_threads(ranks):
+    # CTAs of 128 threads are for calls that start as many of them as they like; a capped call whose CTAs loop keeps 256.
+    comm = nn.Communicator(devices=[0], loopback_ranks=ranks if ranks > 1 else 0, max_ctas=8, wait_timeout_ms=2000)
+    try:
+        for count, threads in ((2000, 128), ((1 << 17) + 3, 256)):
+            ins = [torch.randn(count * ranks, device="cuda") for _ in range(ranks)]
+            outs = [torch.empty(count, device="cuda") for _ in range(ranks)]
+            full = [torch.empty(count * ranks, device="cuda") for _ in range(ranks)]
+            if ranks == 1:
+                comm.all_reduce(outs[0], ins[0])
+                assert torch.equal(outs[0], ins[0])
+            else:
+                comm.reduce_scatter(outs, ins, op="max")
+                most = torch.stack(ins).max(0).values
+                assert all(torch.equal(o, most[r * count:(r + 1) * count]) for r, o in enumerate(outs))
+                if threads == 256:
+                    assert comm.last_call()["block"] == threads
+                comm.all_gather(full, outs)
+                assert all(torch.equal(f, most) for f in full)
+                if threads == 256:
+                    assert comm.last_call()["block"] == threads
+                comm.all_reduce(full, ins, op="max")
+                assert all(torch.equal(f, most) for f in full)
+            info = comm.last_call()
+            assert info["grid"] <= 8
+            if threads == 256 or ranks == 1:
+                assert info["block"] == threads, (count, info)
+    finally:
+        comm.close()
