@@ -130,9 +130,10 @@ private:
     // Emulated ranks whose direct kernels need one set of arguments: the first rank's, with every rank's buffers.
     bool one_launch() const { return loopback_ && dev::kRanksShareGpu; }
     int direct_grid(int planned) const;
+    int direct_threads(const sched::Plan& plan) const;
     void launch_reduce_ranks(const CollectiveArgs& args, std::vector<dev::CollArgs>& per_rank, int pack_bytes,
-                             bool nvls, int grid);
-    void launch_gather_ranks(const CollectiveArgs& args, std::vector<dev::GatherArgs>& per_rank, int grid);
+                             bool nvls, const sched::Plan& plan);
+    void launch_gather_ranks(const CollectiveArgs& args, std::vector<dev::GatherArgs>& per_rank, const sched::Plan& plan);
     void launch_low_latency(const CollectiveArgs& args);
     void ensure_ring();
     void ensure_host_exchange();
@@ -716,11 +717,17 @@ int Communicator::Impl::direct_grid(int planned) const {
     return std::min({planned, dev::kMaxCtas, loopback_ ? std::max(1, 128 / nranks_) : dev::kMaxCtas});
 }
 
+// Small CTAs where there are as many as it takes; where they are fewer and loop (a cap, a share that somebody asked for), each has
+// the threads that it has between GPUs.
+int Communicator::Impl::direct_threads(const sched::Plan& plan) const {
+    return one_launch() && !plan.loops ? tuning_.one_device_block_threads : tuning_.block_threads;
+}
+
 void Communicator::Impl::launch_reduce_ranks(const CollectiveArgs& args, std::vector<dev::CollArgs>& per_rank,
-                                             int pack_bytes, bool nvls, int grid) {
+                                             int pack_bytes, bool nvls, const sched::Plan& plan) {
     kernels::LaunchConfig cfg;
-    cfg.grid = direct_grid(grid);
-    cfg.block = one_launch() ? tuning_.one_device_block_threads : tuning_.block_threads;
+    cfg.grid = direct_grid(plan.grid);
+    cfg.block = direct_threads(plan);
     cfg.nvls_unroll = tuning_.nvls_unroll;
     for (auto& a : per_rank) {
         // Everything that must be equal on every rank for the kernels to meet: a rank that planned
@@ -757,10 +764,10 @@ void Communicator::Impl::launch_reduce_ranks(const CollectiveArgs& args, std::ve
 }
 
 void Communicator::Impl::launch_gather_ranks(const CollectiveArgs& args, std::vector<dev::GatherArgs>& per_rank,
-                                             int grid) {
+                                             const sched::Plan& plan) {
     kernels::LaunchConfig cfg;
-    cfg.grid = direct_grid(grid);
-    cfg.block = one_launch() ? tuning_.one_device_block_threads : tuning_.block_threads;
+    cfg.grid = direct_grid(plan.grid);
+    cfg.block = direct_threads(plan);
     for (auto& a : per_rank)
         a.plan_hash = plan_fingerprint({static_cast<unsigned long long>(Collective::AllGather), static_cast<unsigned long long>(cfg.grid),
                                         a.len, a.out_stride, static_cast<unsigned long long>(a.mode),
@@ -1199,7 +1206,7 @@ void Communicator::Impl::launch_all_reduce(const CollectiveArgs& args, const sch
             }
         }
         last_.pack_bytes = static_cast<int>(pack);
-        launch_reduce_ranks(args, per, static_cast<int>(pack), nvls, plan.grid);
+        launch_reduce_ranks(args, per, static_cast<int>(pack), nvls, plan);
     }
 }
 
@@ -1238,7 +1245,7 @@ void Communicator::Impl::launch_reduce_scatter(const CollectiveArgs& args, const
             if (plan.stage_in) a.user_in = static_cast<const char*>(args.send_buffers[i]) + off;
             if (nvls) a.mc_in = static_cast<const char*>(windows_[in_win[i].region].mc) + in_win[i].offset + off;
         }
-        launch_reduce_ranks(args, per, static_cast<int>(pack), nvls, plan.grid);
+        launch_reduce_ranks(args, per, static_cast<int>(pack), nvls, plan);
     }
 }
 
@@ -1292,7 +1299,7 @@ void Communicator::Impl::launch_all_gather(const CollectiveArgs& args, const sch
             if (plan.gather_mode == 2)
                 a.mc_out = static_cast<char*>(windows_[out_win[i].region].mc) + out_win[i].offset + off;
         }
-        launch_gather_ranks(args, per, plan.grid);
+        launch_gather_ranks(args, per, plan);
     }
 }
 

@@ -49,12 +49,17 @@ constexpr bool kAllRanksHere<OneGpu<A>> = true;
 // 2 MiB 8.2 / 5.7 / 3.7, 8 MiB 16.4 / 14.4 / 11.7 (5.7 TB/s), 256 MiB 346 / 337 / 311 (6.9 TB/s); 8 ranks, 8 MiB 28.5 / 32.5 / 22.5, 256 MiB
 // 649 / 870 / 625; one-shot, which is bound by reading every input once per rank through L2: 8 ranks, 4 MiB 36.6 / 71.2 / 23.0.
 
-// Starts a call, behind the launch before it.
+// Starts a call, behind the launch before it, on `bytes` of the rank's share. The next launch may come at once; where a rank has fewer
+// CTAs than take 32 bytes per thread (the caller caps them), only when this one runs: else several launches wait on the SMs, and
+// those of one come to lie two on an SM with others idle (two-shot, 4 ranks, 8 MiB, 16 CTAs each: 15.5 us, 23.4 us when the next comes at
+// once).
 template <typename ParamT>
-__device__ __forceinline__ void begin_call() {
+__device__ __forceinline__ void begin_call(u64 bytes) {
     if constexpr (kAllRanksHere<ParamT>) {
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        const bool loops = (u64)gridDim.x * blockDim.x * 32 < bytes;
+        if (!loops) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (loops) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
 }
 
@@ -132,13 +137,14 @@ reduce_kernel(const __grid_constant__ ParamT param) {
     constexpr int kElems = P::kElems;
     constexpr int NN = N > 0 ? N : kMaxRanks;
     // For the multimem variant the N slot carries the unroll factor (the rank count is a run-time value there). Emulated ranks
-    // take 32 bytes per thread and peer, or 16 from five ranks up where those are the packs.
-    constexpr int kU = kNvls ? (N > 0 ? N : 4) : (kAllRanksHere<ParamT> ? (P::kBytes == 16 && N <= 4 ? 2 : 1) : UnrollFor<N, P::kBytes>::value);
+    // take 32 bytes per thread and peer, or 16 from five ranks up where those are the packs; two ranks 64, for CTAs that loop
+    // (8 MiB in 2 CTAs each 99.8 -> 89.0 us; without a cap 5.6 us either way).
+    constexpr int kU = kNvls ? (N > 0 ? N : 4) : (kAllRanksHere<ParamT> ? ((P::kBytes == 16 && N <= 4) || N == 2 ? 2 : 1) : UnrollFor<N, P::kBytes>::value);
 
     const CollArgs& a = select_args(param);
-    begin_call<ParamT>();
-
     const int n = (N > 0 && !kNvls) ? N : a.nranks;
+    begin_call<ParamT>((a.shard_mode == kShardSplit ? a.len / n : a.len) * P::kBytes);
+
     const int rank = kAllRanksHere<ParamT> ? (int)blockIdx.y : a.rank;
     ControlBlock* own = kAllRanksHere<ParamT> ? nullptr : a.ctrl[rank];
     u64 epoch = read_epoch<ParamT>(own);
@@ -286,7 +292,7 @@ template <typename RawT, typename ParamT>
 __global__ void __launch_bounds__(kBlockThreads)
 gather_kernel(const __grid_constant__ ParamT param) {
     const GatherArgs& a = select_args(param);
-    begin_call<ParamT>();
+    begin_call<ParamT>(a.len * sizeof(RawT));
     const int n = a.nranks, rank = kAllRanksHere<ParamT> ? (int)blockIdx.y : a.rank;
     ControlBlock* own = kAllRanksHere<ParamT> ? nullptr : a.ctrl[rank];
     u64 epoch = read_epoch<ParamT>(own);

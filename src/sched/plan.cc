@@ -227,6 +227,11 @@ Plan make_plan(const CallShape& s, Algo forced, const Tuning& t) {
     const int no_cap = std::numeric_limits<int>::max();
     const int cap = s.one_device ? (t.one_device_max_ctas > 0 ? t.one_device_max_ctas : no_cap)
                                  : std::max(1, std::min(s.max_ctas > 0 ? s.max_ctas : t.max_ctas, t.max_ctas));
+    // Whether CTAs of one_device_block_threads, 32 bytes per thread, go over a share more than once.
+    const auto loops = [&](std::size_t share, int grid) {
+        const std::size_t at_once = static_cast<std::size_t>(t.one_device_block_threads) * 32;
+        return s.one_device && share > static_cast<std::size_t>(grid) * at_once;
+    };
     const std::size_t per_cta = s.one_device ? t.one_device_bytes_per_cta : t.bytes_per_cta;
     const std::size_t bytes = message_bytes(s);
     const std::size_t esz = dtype_size(s.dtype);
@@ -280,7 +285,9 @@ Plan make_plan(const CallShape& s, Algo forced, const Tuning& t) {
             p.gather_mode = 1;
             p.stage_in = !s.peers_read_input;
         }
-        p.grid = grid_for(s.count * esz * (p.gather_mode == 1 ? s.nranks : 1), cap, per_cta);
+        const std::size_t share = s.count * esz * (p.gather_mode == 1 ? s.nranks : 1);
+        p.grid = grid_for(share, cap, per_cta);
+        p.loops = loops(share, p.grid);
         return p;
     }
 
@@ -288,7 +295,9 @@ Plan make_plan(const CallShape& s, Algo forced, const Tuning& t) {
         p.algo = (forced == Algo::Nvls || (forced == Algo::Auto && nvls_ok && bytes >= t.nvls_min_bytes))
                      ? Algo::Nvls : Algo::OneShot;
         p.stage_in = p.algo != Algo::Nvls && !s.peers_read_input;
-        p.grid = grid_for(s.count * esz * (p.stage_in ? s.nranks : 1), cap, per_cta);
+        const std::size_t share = s.count * esz * (p.stage_in ? s.nranks : 1);
+        p.grid = grid_for(share, cap, per_cta);
+        p.loops = loops(share, p.grid);
         return p;
     }
 
@@ -351,6 +360,7 @@ Plan make_plan(const CallShape& s, Algo forced, const Tuning& t) {
     } else if (algo == Algo::OneShot) {
         p.stage_in = !s.peers_read_input;
         p.grid = grid_for(bytes, cap, t.oneshot_bytes_per_cta);
+        p.loops = loops(bytes, p.grid);
     } else {
         p.stage_in = !s.peers_read_input;
         p.stage_out = !s.peers_write_output;
@@ -358,7 +368,9 @@ Plan make_plan(const CallShape& s, Algo forced, const Tuning& t) {
         // kernel still reads/writes the other side in place.
         // The bytes per CTA are what hides the latency of NVLink.
         const int most = s.one_device ? (t.one_device_twoshot_max_ctas > 0 ? t.one_device_twoshot_max_ctas : no_cap) : t.twoshot_max_ctas;
-        p.grid = grid_for(bytes / s.nranks * (p.stage_in || p.stage_out ? s.nranks : 1), std::min(cap, most), per_cta);
+        const std::size_t share = bytes / s.nranks * (p.stage_in || p.stage_out ? s.nranks : 1);
+        p.grid = grid_for(share, std::min(cap, most), per_cta);
+        p.loops = loops(share, p.grid);
     }
     return p;
 }

@@ -44,6 +44,7 @@ struct Plan {
     // goes through the switch (multimem) or over plain peer loads and stores.
     std::size_t tile_bytes = 0;
     bool pipe_nvls = false;
+    bool loops = false;         // direct kernels of ranks on one device: fewer CTAs than take the whole share at once
     bool through_host = false;  // two-shot over host memory
     std::string error;    // non-empty → the request cannot be satisfied (forced algo impossible)
 };
@@ -59,6 +60,7 @@ struct Tuning {
     // Ranks on one device have a CTA for every 32 bytes per thread (all of it is one batch of loads) unless somebody asks for
     // other CTAs. Two-shot with 512 / 256 / 128 threads: 4 ranks, 8 MiB 11.9 / 11.7 / 11.7 us, 8 ranks, 8 MiB 23.7 / 22.5 / 22.0
     // us, 512 KiB 4.9 / 3.4 / 3.5 us, 256 MiB 626 / 625 / 625 us; with 256 threads and 64 bytes per thread 12.7, 24.8, 4.8 and 631 us.
+    // CTAs that are fewer than that and loop have block_threads (8 MiB, 8 CTAs per rank, 256 / 512 threads: 2 ranks 47 / 25 us, 8 ranks 42 / 30).
     int one_device_block_threads = 256;
     std::size_t one_device_bytes_per_cta = 8u << 10;
     int nvls_max_ctas = 64;                        // more CTAs than this slowed the multimem kernels down

@@ -114,3 +114,41 @@ def test_low_latency_outputs_that_are_inputs(ranks, rotate):
         comm.check_async_error()
     finally:
         comm.close()
+
+
+@pytest.mark.parametrize("algo", ["oneshot", "twoshot"])
+@pytest.mark.parametrize("ranks", [2, 3, 8])
+def test_ctas_that_loop_have_the_threads_of_a_whole_cta(algo, ranks):
+    # A cap below what a call would take: 512 threads, shares of one, two and three rounds, and calls that read what the one before
+    # wrote (the next launch may already wait on the SMs). Without a cap 256 threads.
+    caps = {c: nn.Communicator(devices=[0], loopback_ranks=ranks, algo=algo, max_ctas=c, wait_timeout_ms=2000) for c in (2, 0)}
+    try:
+        gen = torch.Generator(device="cuda").manual_seed(11)
+        parts = ranks if algo == "twoshot" else 1  # what the CTAs of a rank share: 8 KiB each without a cap
+        for rounds in (2, 4, 5, 6):
+            count = rounds * 2 * 4096 * parts + (3 if rounds == 5 else 0)
+            for cap, comm in caps.items():
+                ins = [torch.randn(count, device="cuda", generator=gen).bfloat16() for _ in range(ranks)]
+                a, b = ([torch.zeros_like(t) for t in ins] for _ in range(2))
+                comm.all_reduce(a, ins, op="avg")
+                info = comm.last_call()
+                assert info["algo"] == algo and info["block"] == (512 if cap else 256) and (not cap or info["grid"] == cap), info
+                comm.all_reduce(b, a, op="max")
+                comm.all_reduce(a, b, op="min")
+                acc = ins[0].float()
+                for t in ins[1:]:
+                    acc = acc + t.float()
+                expect = (acc * torch.tensor(1.0, device="cuda").div(ranks)).bfloat16()
+                for o in a + b:
+                    assert torch.equal(o, expect), (rounds, cap)
+                blocks = [torch.zeros(count // ranks, device="cuda", dtype=torch.bfloat16) for _ in range(ranks)]
+                whole = [torch.zeros(count // ranks * ranks, device="cuda", dtype=torch.bfloat16) for _ in range(ranks)]
+                comm.reduce_scatter(blocks, [t[:count // ranks * ranks] for t in a], op="max")
+                comm.all_gather(whole, blocks)
+                for o in whole:
+                    assert torch.equal(o, expect[:o.numel()]), (rounds, cap)
+        for comm in caps.values():
+            comm.check_async_error()
+    finally:
+        for comm in caps.values():
+            comm.close()
