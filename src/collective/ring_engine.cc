@@ -200,6 +200,7 @@ RingEngine::RingEngine(const RingEngineConfig& config, mem::SymmetricAllocator* 
         s.tables.emplace_back(config.local[i].device, static_cast<std::size_t>(C));
         DeviceGuard guard(config.local[i].device);
         B2_CUDA(cudaMemcpy(s.tables.back().get(), table.data(), sizeof(dev::RingChannel) * C, cudaMemcpyHostToDevice));
+        B2_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // the copy of pageable memory may still be under way
         s.wiring.push_back(std::move(table));
     }
     if (s.net) s.net->start();

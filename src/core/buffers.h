@@ -34,10 +34,12 @@ public:
         device_ = device;
         count_ = count;
     }
+    // Done when it returns: cudaMemset is not, and the streams that calls come on need not wait for the default stream.
     void zero() {
         if (!ptr_) return;
         DeviceGuard guard(device_);
         B2_CUDA(cudaMemset(ptr_, 0, count_ * sizeof(T)));
+        B2_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     }
     T* get() const { return ptr_; }
     std::size_t count() const { return count_; }

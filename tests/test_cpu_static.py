@@ -163,3 +163,19 @@ def test_a_ring_slot_in_a_cluster_is_returned_by_a_release_that_reaches_the_clus
         assert ".cluster.shared::cluster" in arrival, f"{arrival}: an arrival in another CTA names its scope"
     sync = read(os.path.join(KERNELS, "sync.cuh"))
     assert "mbarrier.try_wait.parity.acquire.cluster" in sync
+
+
+def test_memory_that_is_cleared_or_filled_at_set_up_is_ready_when_the_call_returns():
+    # Calls come on streams that do not wait for the default stream, where cudaMemset and copies of pageable memory are still under
+    # way when they return: counters of a kernel that waits must not be cleared under it.
+    code = lambda text: re.sub(r"//[^\n]*", "", text)
+    zero = code(read(os.path.join(ROOT, "src", "core", "buffers.h")))
+    zero = zero[zero.index("void zero()"):]
+    zero = zero[:zero.index("T* get()")]
+    assert zero.index("cudaMemset(") < zero.index("cudaStreamSynchronize(cudaStreamLegacy)")
+    ring = code(read(os.path.join(ROOT, "src", "collective", "ring_engine.cc")))
+    fill = ring[ring.index("cudaMemcpy(s.tables"):]
+    assert "cudaStreamSynchronize(cudaStreamLegacy)" in fill[:fill.index("s.wiring.push_back")]
+    regions = code(read(os.path.join(ROOT, "src", "mem", "symmetric.cc")))
+    fill = regions[regions.index("cudaMemset(region->rank_va_"):]
+    assert fill.index("cudaDeviceSynchronize()") < fill.index("barrier()")

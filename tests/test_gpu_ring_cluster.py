@@ -186,3 +186,25 @@ def test_a_channel_has_the_threads_of_a_whole_cta(channels):
         assert info["grid"] == channels
     finally:
         comm.close()
+
+
+def test_a_captured_ring():
+    comm = nn.Communicator(devices=[0], loopback_ranks=4, algo="ring", wait_timeout_ms=2000)
+    try:
+        ins = [torch.randn(100003, device="cuda") for _ in range(4)]
+        outs, again = ([torch.empty_like(t) for t in ins] for _ in range(2))
+        comm.all_reduce(outs, ins, op="max")
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            comm.all_reduce(outs, ins, op="max")
+            comm.all_reduce(again, outs, op="min")
+        for _ in range(3):
+            for t in ins:
+                t.normal_()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert all(torch.equal(o, torch.stack(ins).max(0).values) for o in outs + again)
+        comm.check_async_error()
+    finally:
+        comm.close()
