@@ -268,12 +268,11 @@ __global__ void __launch_bounds__(kThreads, 4) local_shift_copy_kernel(const __g
 // Inputs (or outputs) that are not aligned alike among themselves: one element per access.
 template <typename T, typename Op>
 __global__ void __launch_bounds__(kThreads) local_scalar_kernel(const __grid_constant__ LocalArgs a) {
-    const unsigned threads = blockDim.x;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (unsigned seg = 0; seg < a.segments; ++seg) {
         const u64 in_off = seg * a.in_step(sizeof(T)), out_off = seg * a.out_step(sizeof(T));
-        for (u64 e = (u64)blockIdx.x * threads + threadIdx.x; e < a.count; e += (u64)gridDim.x * threads) {
+        for (u64 e = (u64)blockIdx.x * kThreads + threadIdx.x; e < a.count; e += (u64)gridDim.x * kThreads) {
             if (a.nranks == 1 || a.kind == (int)Collective::AllGather) reduce_one<T, Op, 1>(a, seg, in_off, out_off, e);
             else reduce_one<T, Op, 0>(a, seg, in_off, out_off, e);
         }
