@@ -161,6 +161,7 @@ private:
     std::size_t stage_guard_ = 0;  // bytes of canary before and after the arena (checking builds), else 0
     int channels_ = kDefaultChannels;
     bool channels_asked_for_ = false;
+    bool ring_asked_for_ = false;  // by a number of channels, a FIFO size or the ring's statistics
     sched::Tuning tuning_;
     sched::ProcessLayout layout_;
     sched::RingTransportPlan ring_plan_;
@@ -261,6 +262,9 @@ Communicator::Impl::Impl(const CommunicatorConfig& config, Bootstrap* bootstrap)
     }
 
     resolve_transport();
+    if (resolved_ == TransportKind::Shm)
+        ring_asked_for_ = channels_asked_for_ || env::get("B200CCL_FIFO_BUFF_BYTES", "NANO_NCCL_FIFO_BUFF_BYTES") ||
+                          env::get_bool("B200CCL_RING_TURNAROUND", false);
     if (channels_ <= 0) {
         // One ring CTA moved about 8 GB/s over NVLink, so peer-memory rings want many channels (8 GPUs, 64 MiB:
         // 272 GB/s with 32, 193 with 16, measured with a kernel that staged the local operand in shared memory; the
@@ -855,8 +859,8 @@ void Communicator::Impl::run(Collective collective, const CollectiveArgs& args) 
     shape.output_multicast = out_sym && windows_[out_loc[0].region].mc != nullptr;
     shape.one_device = loopback_;
     shape.ring_only = resolved_ != TransportKind::P2p;  // shm, mixed, socket, rdma: only the ring crosses those edges
-    // Emulated ranks that were given host memory as their transport, and no number of channels, which only a ring has.
-    shape.host_exchange = one_launch() && resolved_ == TransportKind::Shm && !channels_asked_for_;
+    // Emulated ranks that were given host memory as their transport, and nothing that only a ring has.
+    shape.host_exchange = one_launch() && resolved_ == TransportKind::Shm && forced_algo_ == Algo::Auto && !ring_asked_for_;
     shape.max_ctas = tuning_.max_ctas;
     shape.staging_multicast = alloc_ && alloc_->multicast_supported() && (!stage_ || stage_->multicast_ptr() != nullptr);
     sched::Plan plan = sched::make_plan(shape, forced_algo_, tuning_);

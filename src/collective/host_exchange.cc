@@ -21,6 +21,7 @@ HostExchange::HostExchange(int nranks, int device, unsigned long long timeout_ns
     tiles_.zero();
     ctrl_.reset(device, static_cast<std::size_t>(nranks));
     ctrl_.zero();
+    log_info("host exchange: %zu bytes of parts, %zu of results", kernels::host_parts_bytes(nranks), kernels::host_results_bytes(nranks));
 }
 
 int HostExchange::launch(Collective collective, const CollectiveArgs& args) {

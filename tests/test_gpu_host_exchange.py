@@ -1,12 +1,17 @@
 """Two-shot of emulated ranks over host memory (transport shm), around its rows of 512 bytes, its growing and shrinking tiles and the
 lines where the planner turns to the ring; views that start off a vector; every collective in turn on one communicator, so
 that slots of one kind of call are used by the next. Sums are added in rank order in fp32 and rounded once: bit for bit."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
 import nano_nccl_b200 as nn
 
 pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def combine(ins, op):
@@ -99,5 +104,96 @@ def test_channels_asked_for_mean_a_ring():
         outs = [torch.empty_like(t) for t in ins]
         comm.all_reduce(outs, ins, op="max")
         assert comm.last_call()["algo"] == "ring" and torch.equal(outs[3], combine(ins, "max"))
+    finally:
+        comm.close()
+
+
+SHM_CALLS = """
+import torch, nano_nccl_b200 as nn
+comm = nn.Communicator(devices=[0], loopback_ranks=4, transport="shm", algo=ALGO, wait_timeout_ms=3000)
+ins = [torch.randn(1000, device="cuda") for _ in range(4)]
+outs = [torch.empty_like(t) for t in ins]
+comm.all_reduce(outs, ins, op="max")
+assert all(torch.equal(o, torch.stack(ins).max(0).values) for o in outs)
+comm.check_async_error()
+print("ALGO", comm.last_call()["algo"])
+comm.close()
+"""
+
+
+@pytest.mark.parametrize("algo, env, expect", [
+    ("auto", {}, "twoshot"),
+    ("ring", {}, "ring"),
+    ("auto", {"B200CCL_RING_TURNAROUND": "1"}, "ring"),
+    ("auto", {"B200CCL_RING_TURNAROUND": "0"}, "twoshot"),
+    ("auto", {"B200CCL_FIFO_BUFF_BYTES": "1M"}, "ring"),
+    ("auto", {"NANO_NCCL_FIFO_BUFF_BYTES": "1M"}, "ring"),
+])
+def test_what_only_a_ring_has_means_a_ring_and_no_other_memory(algo, env, expect):
+    # The ring by name, its statistics or the size of its FIFOs: the ring runs, the statistics count its slices, and the up to 37 MiB of
+    # host memory of the other way are not allocated.
+    full = dict(os.environ, PYTHONPATH=ROOT, B200CCL_DEBUG="INFO", **env)
+    p = subprocess.run([sys.executable, "-c", f"ALGO = {algo!r}\n" + SHM_CALLS], env=full, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True,
+                       timeout=240)
+    assert p.returncode == 0 and f"ALGO {expect}" in p.stdout, p.stdout
+    assert ("host exchange:" in p.stdout) == (expect == "twoshot"), p.stdout
+    if env.get("B200CCL_RING_TURNAROUND") == "1":
+        slices = [int(line.split(" slices=")[1].split()[0]) for line in p.stdout.splitlines() if line.startswith("ring turnaround")]
+        assert len(slices) >= 4 and sum(slices) > 0, p.stdout
+
+
+def algo_of(collective, ranks, bytes_, wide, aligned):
+    # The lines of the planner, written out once more (bytes of the message, or of a block).
+    if not wide and not (collective == "all_reduce" and aligned):
+        return "twoshot"
+    most = {"all_reduce": {2: 512 << 10, 3: 1 << 20}.get(ranks), "all_gather": 128 << 10 if ranks < 4 else None,
+            "reduce_scatter": {2: 4 << 10, 8: 128 << 10}.get(ranks, 32 << 10)}[collective]
+    return "twoshot" if most is None or bytes_ <= most else "ring"
+
+
+@pytest.mark.parametrize("ranks", [2, 3, 4, 7, 8])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_each_way_is_taken_where_the_planner_draws_the_line_and_is_right(ranks, dtype):
+    # Both sides of every line, aligned and not: the expected algorithm runs; max is exact in both; sums bit for bit in two-shot and within
+    # one rounding per hop in the ring.
+    comm = nn.Communicator(devices=[0], loopback_ranks=ranks, transport="shm", wait_timeout_ms=3000)
+    eps = {torch.float32: 2.0 ** -24, torch.bfloat16: 2.0 ** -8}[dtype]
+    esz = torch.empty(0, dtype=dtype).element_size()
+    gen = torch.Generator(device="cuda").manual_seed(70 + ranks)
+
+    def compare(got, ins, op, algo):
+        if algo == "twoshot" or op == "max":
+            assert torch.equal(got, combine(ins, op))
+        else:
+            stack = torch.stack([t.double() for t in ins])
+            assert ((got.double() - stack.sum(0)).abs() <= 1.01 * (ranks + 1) * eps * stack.abs().sum(0) + 1e-7).all()
+
+    try:
+        seen = set()
+        for size in (4 << 10, 32 << 10, 128 << 10, 512 << 10, 1 << 20):
+            for extra in (0, 16):
+                for shift in (0, 1):
+                    count = (size + extra) // esz
+                    aligned = shift == 0
+                    for op in ("sum", "max"):
+                        ins = [torch.randn(count + shift, device="cuda", generator=gen).to(dtype)[shift:] for _ in range(ranks)]
+                        outs = [torch.empty(count + shift, device="cuda", dtype=dtype)[shift:] for _ in range(ranks)]
+                        comm.all_reduce(outs, ins, op=op)
+                        algo = algo_of("all_reduce", ranks, count * esz, aligned, aligned)
+                        seen.add(algo)
+                        assert comm.last_call()["algo"] == algo, (size, extra, shift)
+                        for o in outs:
+                            compare(o, ins, op, algo)
+                        whole = [torch.randn(count * ranks + shift, device="cuda", generator=gen).to(dtype)[shift:] for _ in range(ranks)]
+                        comm.reduce_scatter(outs, whole, op=op)
+                        algo = algo_of("reduce_scatter", ranks, count * esz, aligned, aligned)
+                        assert comm.last_call()["algo"] == algo, (size, extra, shift)
+                        for r, o in enumerate(outs):
+                            compare(o, [t[r * count:(r + 1) * count] for t in whole], op, algo)
+                        comm.all_gather(whole, outs)
+                        assert comm.last_call()["algo"] == algo_of("all_gather", ranks, count * esz, aligned, aligned), (size, extra, shift)
+                        assert all(torch.equal(t, torch.cat(outs)) for t in whole)
+        assert "twoshot" in seen and (ranks > 3 or "ring" in seen)
+        comm.check_async_error()
     finally:
         comm.close()
