@@ -69,7 +69,8 @@ int b2_collective(b2_comm* comm, int collective, const void* const* send, void* 
 /* What the last call resolved to: algo, grid, block, staged_in, staged_out, vectorized, pack_bytes. */
 int b2_comm_last_call(const b2_comm* comm, int out[7]);
 /* Ring wiring of one local rank's channel: send_fifo, recv_fifo, send_tail, send_head, recv_tail,
- * recv_head, send_base, recv_base. Fails until a ring collective has run. */
+ * recv_head, send_base, recv_base. Fails until a ring collective has run. The FIFOs are null where ranks
+ * share a GPU and hand slices over in shared memory. */
 int b2_comm_ring_channel(const b2_comm* comm, int local_rank, int channel, const void* out[8]);
 /* Where an address lives, from cudaPointerGetAttributes: out[0] = 0 unknown, 1 host (pinned or
  * mapped), 2 device, 3 managed; out[1] = the device that owns it (for host memory: the device whose

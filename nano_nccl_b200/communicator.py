@@ -113,7 +113,8 @@ class Communicator:
                 "staged_out": bool(out[4]), "vectorized": bool(out[5]), "pack_bytes": out[6]}
 
     def ring_channel(self, local_rank=0, channel=0):
-        """Addresses one local rank's ring channel is wired to (after a ring collective has run)."""
+        """Addresses one local rank's ring channel is wired to (after a ring collective has run); a FIFO
+        of ranks that share a GPU and hand slices over in shared memory is 0."""
         out = (ctypes.c_void_p * 8)()
         _lib.check(self._lib.b2_comm_ring_channel(self._handle, int(local_rank), int(channel), out))
         names = ("send_fifo", "recv_fifo", "send_tail", "send_head", "recv_tail", "recv_head", "send_base", "recv_base")

@@ -82,12 +82,25 @@ RingEngine::RingEngine(const RingEngineConfig& config, mem::SymmetricAllocator* 
     if (s.fifo_bytes < quantum || s.fifo_bytes % quantum != 0)
         throw std::invalid_argument("FIFO size must be a positive multiple of " + std::to_string(quantum) + " bytes");
 
+    if (env::get_bool("B200CCL_RING_TURNAROUND", false)) s.stats.reset(config.local.size() * C);
+
+    // Ranks that share a GPU, and no host memory or network between them: the FIFOs lie in distributed shared memory, and none
+    // in global memory is made. (The counters of ring_simple.cu are the ones that the turnaround statistics are taken at.)
+    if (config.loopback && dev::kRanksShareGpu && !net && !any_shm && s.stats.get() == nullptr) {
+        DeviceGuard guard(config.local[0].device);
+        s.clusters = kernels::ring_cluster_capacity(n);
+        // A channel keeps its meaning, an SM of every rank (4 ranks, 16 MiB, 16 channels: 45 us; 125 us with a cluster each, 85 us in
+        // ring_simple.cu).
+        if (config.channels_asked_for) s.clusters = std::min(s.clusters, C * kernels::ring_clusters_per_channel());
+    }
+    const bool device_fifos = s.clusters == 0;
+
     if (!symmetric && (bootstrap != nullptr || net))
         throw std::invalid_argument("a ring that leaves this process needs peer-mapped memory");
 
     if (symmetric) {
         // Every rank's incoming FIFOs in one symmetric region (unused by a rank whose incoming edge is SHM).
-        if (any_p2p || net) s.fifo_region = alloc->allocate(static_cast<std::size_t>(C) * s.fifo_bytes, "ring-fifo");
+        if (device_fifos && (any_p2p || net)) s.fifo_region = alloc->allocate(static_cast<std::size_t>(C) * s.fifo_bytes, "ring-fifo");
     } else {
         for (const auto& l : config.local) {
             s.own_ctrl.emplace_back(l.device, 1);
@@ -101,7 +114,7 @@ RingEngine::RingEngine(const RingEngineConfig& config, mem::SymmetricAllocator* 
             const int src = local_index_of(config, e), dst = local_index_of(config, (e + 1) % n);
             if (src < 0 || dst < 0) throw std::invalid_argument("ring edge without a local endpoint");
             if (!config.loopback) enable_pair(config.local[src].device, config.local[dst].device);
-            s.dev_fifo[dst].reset(config.local[dst].device, static_cast<std::size_t>(C) * s.fifo_bytes);
+            if (device_fifos) s.dev_fifo[dst].reset(config.local[dst].device, static_cast<std::size_t>(C) * s.fifo_bytes);
         }
     }
     if (any_shm) {
@@ -126,23 +139,12 @@ RingEngine::RingEngine(const RingEngineConfig& config, mem::SymmetricAllocator* 
         nc.all_edges = bootstrap == nullptr;  // single process: every edge loops through the transport
         s.net = transport::create_net_edges(nc, bootstrap);
     }
-    if (env::get_bool("B200CCL_RING_TURNAROUND", false)) s.stats.reset(config.local.size() * C);
-
-    // Ranks that share a GPU, and no host memory or network between them. (The counters of ring_simple.cu are the ones that
-    // the turnaround statistics are taken at.)
-    if (config.loopback && dev::kRanksShareGpu && !net && !any_shm && s.stats.get() == nullptr) {
-        DeviceGuard guard(config.local[0].device);
-        s.clusters = kernels::ring_cluster_capacity(n);
-        // A channel keeps its meaning, an SM of every rank (4 ranks, 16 MiB, 16 channels: 45 us; 125 us with a cluster each, 85 us in
-        // ring_simple.cu).
-        if (config.channels_asked_for) s.clusters = std::min(s.clusters, C * kernels::ring_clusters_per_channel());
-    }
-
     auto ctrl_of = [&](int grank) -> dev::ControlBlock* {
         if (symmetric) return static_cast<dev::ControlBlock*>(ctrl->rank_ptr(grank));
         return s.own_ctrl[local_index_of(config, grank)].get();
     };
     auto fifo_of = [&](int grank, int c) -> char* {
+        if (!device_fifos) return nullptr;
         char* base = symmetric ? static_cast<char*>(s.fifo_region->rank_ptr(grank))
                                : reinterpret_cast<char*>(s.dev_fifo[local_index_of(config, grank)].get());
         return base + static_cast<std::size_t>(c) * s.fifo_bytes;
@@ -205,7 +207,8 @@ RingEngine::RingEngine(const RingEngineConfig& config, mem::SymmetricAllocator* 
     }
     if (s.net) s.net->start();
     if (bootstrap) bootstrap->barrier();
-    log_info("ring engine: %d channels, %zu-byte FIFOs, edges:%s%s%s", C, s.fifo_bytes, any_p2p ? " peer-to-peer" : "",
+    if (!device_fifos) log_info("ring engine: up to %d clusters, FIFOs in their shared memory", s.clusters);
+    else log_info("ring engine: %d channels, %zu-byte FIFOs, edges:%s%s%s", C, s.fifo_bytes, any_p2p ? " peer-to-peer" : "",
              any_shm ? " host" : "", s.net ? " network" : "");
 }
 

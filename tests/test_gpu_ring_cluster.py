@@ -208,3 +208,25 @@ def test_a_captured_ring():
         comm.check_async_error()
     finally:
         comm.close()
+
+
+def test_a_ring_in_clusters_takes_no_device_memory_for_fifos():
+    def make():
+        return nn.Communicator(devices=[0], loopback_ranks=4, algo="ring", wait_timeout_ms=2000)
+
+    ins = [torch.randn(1 << 16, device="cuda") for _ in range(4)]
+    outs = [torch.empty_like(t) for t in ins]
+    first, second = make(), make()  # the first loads the kernels
+    try:
+        first.all_reduce(outs, ins, op="max")
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        second.all_reduce(outs, ins, op="max")
+        torch.cuda.synchronize()
+        assert free - torch.cuda.mem_get_info()[0] <= 4 << 20  # FIFOs in global memory would be 64 MiB
+        assert all(torch.equal(o, torch.stack(ins).max(0).values) for o in outs)
+        wires = second.ring_channel(1, 0)
+        assert wires["send_fifo"] == wires["recv_fifo"] == 0 and wires["send_head"] != 0 and wires["recv_tail"] != 0
+    finally:
+        first.close()
+        second.close()
