@@ -6,6 +6,8 @@ bounds       — the host is told to pass extents that are too short: the kernel
                first bad index, skip those accesses and still run to its end;
 separate-gpus — emulated ranks synchronise as ranks on GPUs of their own do: the ring's early credit and single
                group of warps at system scope, the peer kernels' barriers with their plan fingerprints;
+separate-gpus-edges — the same at the edges: buffers that are misaligned alike and differently, batches of low-latency words
+               with outputs of their own and in place;
 canary       — the staging arena sits between two pages of canary bytes: they survive staged
                collectives, and a byte overwritten from the host is reported."""
 import os
@@ -49,6 +51,57 @@ def separate_gpus():
                 most = reference(ins, "max").to(dtype)
                 assert all(torch.equal(f, most) for f in full), (algo, transport, ranks, block)
         torch.cuda.synchronize()
+        comm.check_async_error()
+        comm.close()
+
+
+def separate_gpus_edges():
+    """The peer kernels with their meetings over flags: the elements before the first pack and behind the last one of views that
+    are misaligned alike, for every width of pack; the low-latency exchange between threads of different CTAs on both sides of
+    every size of batch. Max and min are exact; sums are added in rank order in fp32 and rounded once."""
+    def combined(ins, op):
+        acc = ins[0].float()
+        for t in ins[1:]:
+            acc = acc + t.float() if op in ("sum", "avg") else (torch.maximum if op == "max" else torch.minimum)(acc, t.float())
+        return (acc * torch.tensor(1.0, device="cuda").div(len(ins)) if op == "avg" else acc).to(ins[0].dtype)
+
+    gen = torch.Generator(device="cuda").manual_seed(77)
+    for algo in ("oneshot", "twoshot"):
+        for ranks in (2, 3, 8):
+            comm = nn.Communicator(devices=[0], loopback_ranks=ranks, algo=algo, wait_timeout_ms=3000)
+            assert "as on GPUs of their own" in comm.describe()
+            for dtype in (torch.float32, torch.bfloat16):
+                esz = torch.empty(0, dtype=dtype).element_size()
+                for k, count in enumerate([1, 32 // esz, 48 // esz - 1, 62 // esz, 64 // esz + 1, 257, 30001, (1 << 18) + 5]):
+                    for shifts in ([1] * ranks, [5] * ranks, [16 // esz + 1] * ranks, [32 // esz - 1] * ranks, [(3 * r) % 5 for r in range(ranks)]):
+                        op = ["sum", "avg", "max", "min"][(k + shifts[0]) % 4]
+                        ins = [torch.randn(count + 64, device="cuda", generator=gen).to(dtype)[s:s + count] for s in shifts]
+                        raw = [torch.full((count + 64,), 7.0, device="cuda", dtype=dtype) for _ in range(ranks)]
+                        outs = [t[s:s + count] for t, s in zip(raw, shifts)]
+                        expect = combined(ins, op)
+                        if algo == "twoshot" and k % 2:  # in place
+                            for t, o in zip(ins, outs):
+                                o.copy_(t)
+                            comm.all_reduce(outs, outs, op=op)
+                        else:
+                            comm.all_reduce(outs, ins, op=op)
+                        assert comm.last_call()["algo"] == algo
+                        for t, o, s in zip(raw, outs, shifts):
+                            assert torch.equal(o, expect), (algo, ranks, dtype, count, shifts, op)
+                            assert (t[:s] == 7.0).all() and (t[s + count:] == 7.0).all(), (algo, ranks, dtype, count, shifts, op)
+            comm.check_async_error()
+            comm.close()
+    for ranks in (2, 3, 8):
+        comm = nn.Communicator(devices=[0], loopback_ranks=ranks, algo="ll", wait_timeout_ms=3000)
+        for k, words in enumerate([4096, 4097, 5, 16384, 16385, 32768, 1, 32767, 20480, 16383] * 2):
+            ins = [torch.randn(words * 2, device="cuda", generator=gen).half() for _ in range(ranks)]
+            outs = [torch.full_like(t, float("nan")) for t in ins]
+            op = ["sum", "avg", "max", "min"][k % 4]
+            expect = combined(ins, op)
+            comm.all_reduce(outs, ins, op=op)
+            assert comm.last_call()["algo"] == "ll" and all(torch.equal(o, expect) for o in outs), (ranks, words, op)
+            comm.all_reduce(ins, ins, op=op)
+            assert all(torch.equal(o, expect) for o in ins), (ranks, words, op, "in place")
         comm.check_async_error()
         comm.close()
 
@@ -103,6 +156,8 @@ def main():
         comm.close()
     elif mode == "separate-gpus":
         separate_gpus()
+    elif mode == "separate-gpus-edges":
+        separate_gpus_edges()
     elif mode == "canary":
         smash = os.environ.pop("B200CCL_DEBUG_SMASH_CANARY", None)
         comm = nn.Communicator(devices=[0], loopback_ranks=4, algo="pipeline", wait_timeout_ms=3000, staging_bytes=8 << 20)

@@ -37,6 +37,12 @@ def test_emulated_ranks_synchronise_as_on_gpus_of_their_own():
     assert rc == 0 and "WORKER OK" in out, out
 
 
+def test_meetings_over_flags_with_misaligned_buffers_and_batches_of_words():
+    # What the product library runs between GPUs only: its emulated ranks have nothing to meet for.
+    rc, out = run("separate-gpus-edges")
+    assert rc == 0 and "WORKER OK" in out, out
+
+
 def test_canary_pages_around_the_staging_arena():
     rc, out = run("canary")
     assert rc == 0 and "WORKER OK" in out, out
