@@ -64,7 +64,7 @@ struct CallInfo {
     bool staged_in = false;   // input went through the staging arena
     bool staged_out = false;  // output went through the staging arena
     bool vectorized = false;  // every buffer and block is a whole number of aligned 16-byte packs (pack_bytes says what was moved)
-    int pack_bytes = 0;       // bytes one thread moves per access: 32, 16 or the element size (0: not applicable)
+    int pack_bytes = 0;       // bytes one thread loads per access: 32, 16 or the element size (0: not applicable)
 };
 
 class Communicator {

@@ -259,7 +259,7 @@ reduce_kernel(const __grid_constant__ ParamT param) {
 
     // 3b. The elements of a ragged or misaligned message that fill no pack, one per thread of CTA 0, in the last rank's shard.
     if constexpr (!kNvls) {
-        const unsigned ends = a.head + a.tail;  // at most 14 + 15
+        const unsigned ends = a.head + a.tail;  // at most 15 + 15 (2-byte elements, 32-byte packs): a CTA has 32 threads at least
         if (ends != 0 && blockIdx.x == 0 && threadIdx.x < ends && (mode == kShardWhole || rank == n - 1)) {
             const u64 e = threadIdx.x < a.head ? threadIdx.x : a.len * kElems + threadIdx.x;
             auto first = [&](const void* base) { return static_cast<const T*>(base) - a.head; };

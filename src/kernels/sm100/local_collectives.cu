@@ -13,11 +13,11 @@
 // and loop (one or two per SM, interleaved or contiguous, 16- to 256-byte windows per thread, and TMA bulk
 // copies through shared memory), float sum: 8 ranks x 64 MiB 157.8 us (6.81 TB/s) against 172.7-181.5 us;
 // 2 ranks x 512 MiB 308.8 us (6.96 TB/s) against 322-375 us; one rank, 64 MiB 21.2 us against 22.9 us for a
-// TMA bulk-copy kernel with one CTA per SM. More packs per thread, or 128 or 512 threads, change less than 1 %.
-// CTAs loop only where the caller caps their number.
+// TMA bulk-copy kernel with one CTA per SM. At these sizes more packs per thread, or 128 or 512 threads, change less than 1 %;
+// small grids and reduce_scatter run 128 threads (start_tiles()). CTAs loop only where the caller caps their number.
 //
-// Lengths and addresses need no alignment beyond the element's. Packs are cut where the INPUTS are aligned; the
-// elements before the first and after the last pack of a segment are handled one by one by the CTA of its first
+// Lengths and addresses need no alignment beyond the element's. Packs are cut where the INPUTS are aligned (copies whose
+// outputs are aligned differently: where the outputs are, see local_shift_copy_kernel); the elements before the first and after the last pack of a segment are handled one by one by the CTA of its first
 // tile. Where the outputs are aligned differently (blocks of a ragged reduce_scatter or all_gather), bytes move
 // between neighbouring lanes by shuffle so that loads and stores are aligned vectors all the same.
 #include "kernels/sm100/local_collectives.h"
@@ -348,7 +348,7 @@ cudaError_t start_copy(Plan& p, LocalLaunch* made) {
     if (p.how == Plan::kAlike) return start_tiles<__half>(local_kernel<__half, OpAdd, 1, false, kBytes, kThreads>, p, made, local_kernel<__half, OpAdd, 1, false, kBytes, kThreads / 2>);
     if (p.how == Plan::kShifted) {
         const cudaError_t st = start_tiles<__half>(local_shift_copy_kernel<__half>, p, made);
-        made->pack_bytes = 16;
+        made->pack_bytes = 16;  // of its loads
         return st;
     }
     return start_op<__half, OpAdd>(p, made);
