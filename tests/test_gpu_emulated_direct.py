@@ -152,3 +152,31 @@ def test_ctas_that_loop_have_the_threads_of_a_whole_cta(algo, ranks):
     finally:
         for comm in caps.values():
             comm.close()
+
+
+@pytest.mark.parametrize("algo, cap", [("oneshot", 0), ("oneshot", 2), ("twoshot", 0), ("twoshot", 2), ("ll", 0)])
+def test_captured_calls_follow_one_another(algo, cap):
+    # Dependent launches as edges of a graph, with CTAs that loop and without; each call reads what the one before wrote.
+    comm = nn.Communicator(devices=[0], loopback_ranks=4, algo=algo, max_ctas=cap, wait_timeout_ms=2000)
+    try:
+        count = 32768 if algo == "ll" else 300007
+        ins = [torch.randn(count, device="cuda") for _ in range(4)]
+        a, b, c = ([torch.empty_like(t) for t in ins] for _ in range(3))
+        comm.all_reduce(a, ins, op="max")
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            comm.all_reduce(a, ins, op="max")
+            comm.all_reduce(b, a, op="min")
+            comm.all_reduce(c, b, op="max")
+        for _ in range(5):
+            for t in ins:
+                t.normal_()
+            graph.replay()
+            torch.cuda.synchronize()
+            expect = torch.stack(ins).max(0).values
+            assert all(torch.equal(o, expect) for o in a + b + c)
+        assert comm.last_call()["algo"] == algo
+        comm.check_async_error()
+    finally:
+        comm.close()
